@@ -179,6 +179,7 @@ struct DevScene {
     int32_t border;
     float background[3];
     int32_t force_background;
+    int32_t narea;                // area lights
 };
 
 }  // namespace hk

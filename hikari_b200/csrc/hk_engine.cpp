@@ -42,10 +42,8 @@ WfEngine::WfEngine(const DevScene &S, int sm_count, const WfEngineConfig &cfg) :
     W_.pix.p = (float4 *)(rec + 48);
     W_.rng.p = (uint4 *)(rec + 64);
     W_.hit.p = (float4 *)(rec + 80);
-    W_.prev_wi.p = (float4 *)(rec + 96);
-    W_.prev_wo.p = (float4 *)(rec + 112);
-    W_.lacc.p = (float4 *)(rec + 128);
-    W_.prev_pdf.p = (float *)(rec + 144);
+    W_.lacc.p = (float4 *)(rec + 96);
+    W_.prev_pdf.p = (float *)(rec + 112);
     int *q = queues_.as<int>();
     W_.eq[0] = q; W_.eq[1] = q + N;
     W_.idle[0] = q + 2 * N; W_.idle[1] = q + 3 * N;

@@ -861,6 +861,7 @@ void build_scene(hk_scene *s) {
     }
     s->b_emitter_area.upload(emitter_area); track(s->b_emitter_area);
     s->b_area.upload(area); track(s->b_area);
+    D.narea = (int32_t)area.size();
     s->b_light_tris.upload(ltris); track(s->b_light_tris);
     s->b_light_normals.upload(lnorms); track(s->b_light_normals);
     s->b_light_cdf.upload(lcdf); track(s->b_light_cdf);

@@ -100,13 +100,12 @@ struct WfCounters {
     unsigned int log_rays[2][kWfLaunchLog];
 };
 
-// Path state: one 160-byte record per slot, five 32-byte sectors, the fields
-// a kernel reads together in one sector: (ray o, ray d) extend and shade;
-// (throughput, pixel) shade and regen; (rng, hit) shade; (previous BSDF record
-// wi, wo) shade at emitter hits; (radiance, previous pdf) regen and the
-// next-event reductions.  Slots are visited in queue order, i.e. scattered, so
+// Path state: one 128-byte record per slot (one cache line), four 32-byte
+// sectors, the fields a kernel reads together in one sector: (ray o, ray d)
+// extend and shade; (throughput, pixel) shade and regen; (rng, hit) shade;
+// (radiance, previous pdf) regen and the next-event reductions.  Slots are visited in queue order, i.e. scattered, so
 // a separate array per field would fetch a whole sector for each 16-byte field.
-constexpr size_t kSlotBytes = 160;
+constexpr size_t kSlotBytes = 128;
 // One field of every slot's record: f[slot] is the field of that slot.
 template <class T>
 struct SlotField {
@@ -127,11 +126,9 @@ struct WfState {
     SlotField<float4> pix;        //  48: film x, film y, bits(job), bits(depth | flags << 16)
     SlotField<uint4> rng;         //  64: pcg32 state, increment
     SlotField<float4> hit;        //  80: t, u, v, bits(tri in leaf order or -1)
-    SlotField<float4> prev_wi;    //  96: previous vertex: BSDF record wi.xyz, bits(bsdf id)
-    SlotField<float4> prev_wo;    // 112: previous vertex: BSDF record wo.xyz, bits(measure)
-    SlotField<float4> lacc;       // 128: radiance.xyz (next-event terms added atomically), -
-    SlotField<float> prev_pdf;    // 144: previous vertex: its BSDF's pdf of the sampled direction (textured
-                                  //      materials only)
+    SlotField<float4> lacc;       //  96: radiance.xyz (next-event terms added atomically), -
+    SlotField<float> prev_pdf;    // 112: previous vertex: its BSDF's pdf of the sampled direction (scenes with
+                                  //      area lights, whose hits weigh by it)
     // queues
     int *eq[2];
     int *idle[2];
