@@ -77,22 +77,24 @@ WfEngine::WfEngine(const DevScene &S, int sm_count, const WfEngineConfig &cfg) :
     L_.lean_extend = cfg_.reg_lean & 1;
     L_.lean_shadow = (cfg_.reg_lean >> 1) & 1;
     L_.lean_shade = (cfg_.reg_lean >> 2) & 1;
-    L_.shadow_tests = cfg_.shadow_tests >= 0 && cfg_.shadow_tests <= 2 ? cfg_.shadow_tests : 0;
-    L_.closest_tests = cfg_.closest_tests == 2 ? 2 : 0;
     auto grid = [&](int which, int threads) {
         const bool lean = which == 0 ? L_.lean_extend : (which == 2 ? L_.lean_shadow : (which == 1 ? L_.lean_shade : false));
-        const bool shared = (which == 2 && L_.shadow_tests == 2) || (which == 0 && L_.closest_tests == 2);
-        return std::max(1, sm_count * std::max(1, wf_occupancy(which, threads, S.accel, lean, shared)));
+        return std::max(1, sm_count * std::max(1, wf_occupancy(which, threads, S.accel, lean)));
     };
     L_.blocks_extend = grid(0, L_.threads_extend);
     L_.blocks_shade = grid(1, L_.threads_shade);
     L_.blocks_shadow = grid(2, L_.threads_shadow);
     L_.blocks_regen = grid(3, L_.threads_regen);
-    L_.fetch_steps = cfg_.fetch_steps > 0 ? cfg_.fetch_steps : (S.accel == kAccelBvh8 ? 3 : 8);
-    L_.fetch_min_idle = std::max(1, std::min(32, cfg_.fetch_min_idle));
+    // idle lanes before a refill, 8-wide tree: a refill costs the warp about 140
+    // instructions and a partly filled test batch, an idle lane a 32nd of the
+    // rest (64-sphere scene, ms of 33.5M paths at 4 / 8 / 12 lanes: closest hit
+    // 24.5 / 21.8 / 21.0, shadow 33.7 / 33.0 / 33.5)
+    const bool w8 = S.accel == kAccelBvh8;
+    L_.fetch_steps = cfg_.fetch_steps > 0 ? cfg_.fetch_steps : 8;
+    L_.fetch_min_idle = cfg_.fetch_min_idle > 0 ? std::min(32, cfg_.fetch_min_idle) : (w8 ? 12 : 1);
     L_.fetch_steps_shadow = cfg_.fetch_steps_shadow > 0 ? cfg_.fetch_steps_shadow : L_.fetch_steps;
-    L_.fetch_min_idle_shadow = cfg_.fetch_min_idle_shadow > 0 ? std::min(32, cfg_.fetch_min_idle_shadow)
-                                                              : L_.fetch_min_idle;
+    const int shadow_idle = cfg_.fetch_min_idle_shadow > 0 ? cfg_.fetch_min_idle_shadow : cfg_.fetch_min_idle;
+    L_.fetch_min_idle_shadow = shadow_idle > 0 ? std::min(32, shadow_idle) : (w8 ? 8 : 1);
     HK_CUDA(cudaGetLastError());
     reset();
 }

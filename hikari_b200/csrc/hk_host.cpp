@@ -1016,7 +1016,7 @@ hk::WfEngine &wf_ensure(hk_scene *s, const hk::WfEngineConfig &c) {
         if (o.capacity == c.capacity && o.threads_extend == c.threads_extend && o.threads_shade == c.threads_shade &&
             o.fetch_steps == c.fetch_steps && o.fetch_min_idle == c.fetch_min_idle &&
             o.fetch_steps_shadow == c.fetch_steps_shadow && o.fetch_min_idle_shadow == c.fetch_min_idle_shadow &&
-            o.reg_lean == c.reg_lean && o.shadow_tests == c.shadow_tests && o.closest_tests == c.closest_tests)
+            o.reg_lean == c.reg_lean)
             return *s->wf;
         s->wf.reset();
     }
@@ -1596,12 +1596,10 @@ int hk_render_batch(hk_scene *s, const hk_render_job *jobs, int njobs, const hk_
         ec.threads_extend = c.threads_extend > 0 ? c.threads_extend : 128;
         ec.threads_shade = c.threads_shade > 0 ? c.threads_shade : 128;
         ec.fetch_steps = std::max(0, std::min(1024, c.fetch_steps));
-        ec.fetch_min_idle = c.fetch_min_idle > 0 ? std::min(32, c.fetch_min_idle) : 1;
+        ec.fetch_min_idle = c.fetch_min_idle > 0 ? std::min(32, c.fetch_min_idle) : 0;
         ec.fetch_steps_shadow = std::max(0, std::min(1024, c.fetch_steps_shadow));
         ec.fetch_min_idle_shadow = c.fetch_min_idle_shadow > 0 ? std::min(32, c.fetch_min_idle_shadow) : 0;
         ec.reg_lean = c.reg_lean & 7;
-        ec.shadow_tests = c.shadow_tests >= 0 && c.shadow_tests <= 2 ? c.shadow_tests : 0;
-        ec.closest_tests = c.closest_tests == 2 ? 2 : 0;
         hk::WfEngine &E = wf_ensure(s, ec);
         cudaStream_t user = (cudaStream_t)stream, st = E.stream();
         // order after the caller's stream (the films may have been cleared there)
@@ -1702,8 +1700,8 @@ int hk_wavefront_autotune(hk_scene *s, const hk_render_desc *probe, hk_wavefront
         const int caps[] = {1 << 20, 1 << 21, 1 << 22};
         const int threads[] = {64, 128, 256};
         const int checks[] = {16, 64};
-        const int steps8[] = {2, 3, 6}, steps2[] = {4, 8, 16};
-        const int min_idle[] = {1, 8, 16};
+        const int steps2[] = {4, 8, 16};   // binary tree
+        const int min_idle[] = {4, 8, 12, 16};
         // a configuration's time: the better of two timed renders after a warm one
         // (one timed render lets run-to-run noise of a few percent pick the configuration)
         auto run = [&](const hk_wavefront_config &c) {
@@ -1744,9 +1742,11 @@ int hk_wavefront_autotune(hk_scene *s, const hk_render_desc *probe, hk_wavefront
             float ms = run(c);
             if (ms < best_t) { best_t = ms; bc = c; }
         }
-        // dynamic ray fetch: node visits between refills, idle lanes before a refill
+        // dynamic ray fetch: node visits between refills (binary tree), idle lanes before a refill
+        const bool w2 = s->dev.accel == hk::kAccelBvh2;
         c = bc;
-        for (int k : (s->dev.accel == hk::kAccelBvh8 ? steps8 : steps2)) {
+        for (int k : steps2) {
+            if (!w2) break;
             c.fetch_steps = k;
             float ms = run(c);
             if (ms < best_t) { best_t = ms; bc = c; }
@@ -1772,7 +1772,8 @@ int hk_wavefront_autotune(hk_scene *s, const hk_render_desc *probe, hk_wavefront
         }
         // the shadow rays' own refill interval and idle-lane threshold
         c = bc;
-        for (int k : (s->dev.accel == hk::kAccelBvh8 ? steps8 : steps2)) {
+        for (int k : steps2) {
+            if (!w2) break;
             c.fetch_steps_shadow = k;
             float ms = run(c);
             if (ms < best_t) { best_t = ms; bc = c; }
@@ -1780,21 +1781,6 @@ int hk_wavefront_autotune(hk_scene *s, const hk_render_desc *probe, hk_wavefront
         c = bc;
         for (int k : min_idle) {
             c.fetch_min_idle_shadow = k;
-            float ms = run(c);
-            if (ms < best_t) { best_t = ms; bc = c; }
-        }
-        // the shadow rays' triangle tests postponed or shared out over the warp (8-wide tree only)
-        if (s->dev.accel == hk::kAccelBvh8) {
-            c = bc;
-            for (int k : {1, 2}) {
-                if (k == 1 && !s->dev.postpone) continue;
-                c.shadow_tests = k;
-                float ms = run(c);
-                if (ms < best_t) { best_t = ms; bc = c; }
-            }
-            // and the closest-hit rays' shared out
-            c = bc;
-            c.closest_tests = 2;
             float ms = run(c);
             if (ms < best_t) { best_t = ms; bc = c; }
         }

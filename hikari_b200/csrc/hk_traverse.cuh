@@ -291,7 +291,8 @@ __device__ __forceinline__ bool trace_bvh2(const DevScene &S, const Ray &ray, Hi
 // hit bits 0..23).  Hit bits of internal children sit at slot ^ (7 ^ octant),
 // so the lowest set bit is the nearest child.  A warp vote postpones the
 // triangle tests of lanes that are few among the active ones while they still
-// have nodes to visit, so that lanes intersect triangles together.
+// have nodes to visit, so that lanes intersect triangles together (closest-hit
+// rays).  The wavefront's traversal kernels walk this tree in hk_wf_trace.cuh.
 
 constexpr int kShStack = 8;   // entries per thread kept in shared memory
 
@@ -401,7 +402,7 @@ struct Bvh8Walker {
             tg = ng;   // a postponed triangle group from the stack (or nothing)
             ng = make_uint2(0u, 0u);
         }
-        if (kAnyHit ? S.postpone_any : S.postpone) {   // any-hit rays only where the launch asks
+        if (!kAnyHit && S.postpone) {
             const unsigned act = __activemask();
             const unsigned want = __ballot_sync(act, tg.y != 0u);
             if (tg.y != 0u && ng.y > 0x00ffffffu && __popc(want) * 5 < __popc(act)) {
@@ -435,192 +436,6 @@ struct Bvh8Walker {
             ng = stk.pop();
         }
         return false;
-    }
-
-    // One step of an any-hit ray with the warp's triangle tests shared out:
-    // every lane of the warp calls it (alive: the lane holds a ray).  Alive
-    // lanes visit a node (or pop a triangle group); the triangles of all
-    // lanes' groups are then numbered in lane order and tested 32 at a time,
-    // lane j taking triangle r + j of the numbering against its owner's ray
-    // (rays: the warp's rays in shared memory, origin + tmin then direction +
-    // tmax per lane), and a lane is occluded when any of its triangles is.
-    // The serial loop of step() runs as many rounds as the warp's largest
-    // group, with the other lanes idle; this runs ceil(sum / 32).
-    __device__ __forceinline__ bool step_any_shared(const DevScene &S, bool alive, const float4 *rays) {
-        const unsigned lane = threadIdx.x & 31u;
-        uint2 grp = make_uint2(0u, 0u);
-        if (alive) {
-            if (ng.y > 0x00ffffffu) {
-                const uint32_t b = __ffs(ng.y >> 24) - 1;
-                ng.y &= ~(1u << (24 + b));
-                const uint32_t slot = b ^ ko;
-                const uint32_t child = ng.x + __popc(ng.y & 0xffu & ((1u << slot) - 1u));
-                if (ng.y > 0x00ffffffu) stk.push(ng);
-                visit(S, child);
-                grp = tg;
-            } else {
-                grp = ng;   // a postponed triangle group from the stack (or nothing)
-                ng = make_uint2(0u, 0u);
-            }
-            tg = make_uint2(0u, 0u);
-        }
-        const uint32_t cnt = __popc(grp.y);
-        uint32_t incl = cnt;   // inclusive prefix of the counts in lane order
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= (unsigned)o) incl += v;
-        }
-        const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-        const uint32_t excl = incl - cnt;
-        ntri += cnt;
-        bool occluded = false;
-        for (uint32_t r = 0; r < total; r += 32) {   // warp-uniform
-            const uint32_t w = r + lane;
-            // owner: the number of lanes whose inclusive prefix is <= w
-            // (binary lifting; every index read stays within 0..31)
-            uint32_t own = 0;
-#pragma unroll
-            for (uint32_t b = 16; b > 0; b >>= 1) {
-                const uint32_t v = __shfl_sync(0xffffffffu, incl, own + b - 1);
-                if (v <= w) own += b;
-            }
-            const uint32_t obase = __shfl_sync(0xffffffffu, grp.x, own);
-            const uint32_t omask = __shfl_sync(0xffffffffu, grp.y, own);
-            const uint32_t oexcl = __shfl_sync(0xffffffffu, excl, own);
-            bool hit = false;
-            if (w < total) {
-                const uint32_t tri = obase + __fns(omask, 0u, (int)(w - oexcl) + 1);
-                const float4 *tp = S.tris + 3 * (size_t)tri;
-                const float4 p0 = ldg4(tp), p1 = ldg4(tp + 1), p2 = ldg4(tp + 2);
-                const float4 ro = rays[2 * own], rd = rays[2 * own + 1];
-                hit = occludes_mt(xyz(ro), xyz(rd), xyz(p0), xyz(p1), xyz(p2), ro.w, rd.w);
-            }
-            const uint32_t hb = __ballot_sync(0xffffffffu, hit);
-            // the lanes that tested this lane's triangles in round r
-            const int lo = max((int)excl - (int)r, 0), hi = min((int)incl - (int)r, 32);
-            if (lo < hi) {
-                const uint32_t upto = hi >= 32 ? 0xffffffffu : ((1u << hi) - 1u);
-                if (hb & upto & ~((1u << lo) - 1u)) occluded = true;
-            }
-        }
-        if (!alive) return false;
-        if (occluded) {
-            found = true;
-            return true;
-        }
-        if (ng.y <= 0x00ffffffu) {
-            if (stk.sp == 0) return true;
-            ng = stk.pop();
-        }
-        return false;
-    }
-
-    // One step of a closest-hit ray with the warp's triangle tests shared out,
-    // numbered and dealt as in step_any_shared: lane j of round r tests
-    // triangle r + j with the watertight test against its owner's ray (rays:
-    // origin + tmin and the packed watertight constants per lane; the owner's
-    // current tmax by shuffle).  Per owner the hit of least t wins and, on
-    // equal t, the one later in the owner's test order: the hit that the
-    // serial loop of step() keeps, since it accepts t <= tmax and then shrinks
-    // tmax to t.  A group that spans two rounds sees the first round's tmax in
-    // the second, as the serial loop would.
-    __device__ __forceinline__ bool step_closest_shared(const DevScene &S, bool alive, const float4 *rays) {
-        const unsigned lane = threadIdx.x & 31u;
-        uint2 grp = make_uint2(0u, 0u);
-        if (alive) {
-            if (ng.y > 0x00ffffffu) {
-                const uint32_t b = __ffs(ng.y >> 24) - 1;
-                ng.y &= ~(1u << (24 + b));
-                const uint32_t slot = b ^ ko;
-                const uint32_t child = ng.x + __popc(ng.y & 0xffu & ((1u << slot) - 1u));
-                if (ng.y > 0x00ffffffu) stk.push(ng);
-                visit(S, child);
-                grp = tg;
-            } else {
-                grp = ng;
-                ng = make_uint2(0u, 0u);
-            }
-            tg = make_uint2(0u, 0u);
-        }
-        const uint32_t cnt = __popc(grp.y);
-        uint32_t incl = cnt;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= (unsigned)o) incl += v;
-        }
-        const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-        const uint32_t excl = incl - cnt;
-        ntri += cnt;
-        for (uint32_t r = 0; r < total; r += 32) {   // warp-uniform
-            const uint32_t w = r + lane;
-            uint32_t own = 0;
-#pragma unroll
-            for (uint32_t b = 16; b > 0; b >>= 1) {
-                const uint32_t v = __shfl_sync(0xffffffffu, incl, own + b - 1);
-                if (v <= w) own += b;
-            }
-            const uint32_t obase = __shfl_sync(0xffffffffu, grp.x, own);
-            const uint32_t omask = __shfl_sync(0xffffffffu, grp.y, own);
-            const uint32_t oexcl = __shfl_sync(0xffffffffu, excl, own);
-            const float otmax = __shfl_sync(0xffffffffu, tmax, own);
-            // (t, 31 - lane): the least key is the least t, then the latest lane
-            unsigned long long key = ~0ull;
-            float tt = 0.0f, uu = 0.0f, vv = 0.0f;
-            uint32_t tri = 0u;
-            if (w < total) {
-                tri = obase + __fns(omask, 0u, (int)(w - oexcl) + 1);
-                const float4 *tp = S.tris + 3 * (size_t)tri;
-                const float4 p0 = ldg4(tp), p1 = ldg4(tp + 1), p2 = ldg4(tp + 2);
-                const float4 ro = rays[2 * own], rw = rays[2 * own + 1];
-                const uint32_t kp = __float_as_uint(rw.w);
-                WatertightRay wr;
-                wr.kx = (int)(kp & 3u);
-                wr.ky = (int)((kp >> 2) & 3u);
-                wr.kz = (int)((kp >> 4) & 3u);
-                wr.sx = rw.x;
-                wr.sy = rw.y;
-                wr.sz = rw.z;
-                if (intersect_watertight(wr, xyz(ro), xyz(p0), xyz(p1), xyz(p2), ro.w, otmax, tt, uu, vv)) {
-                    const uint32_t tb = __float_as_uint(tt);
-                    const uint32_t ord = (tb & 0x80000000u) ? ~tb : (tb | 0x80000000u);   // order of the floats
-                    key = ((unsigned long long)ord << 32) | (31u - lane);
-                }
-            }
-            // least key within each owner's run of lanes (runs are contiguous)
-#pragma unroll
-            for (int s = 1; s < 32; s <<= 1) {
-                const unsigned long long k2 = __shfl_down_sync(0xffffffffu, key, s);
-                const uint32_t o2 = __shfl_down_sync(0xffffffffu, own, s);
-                if (lane + (unsigned)s < 32u && o2 == own && k2 < key) key = k2;
-            }
-            // this lane's run in round r starts at lane lo
-            const int lo = max((int)excl - (int)r, 0), hi = min((int)incl - (int)r, 32);
-            const unsigned long long mk = __shfl_sync(0xffffffffu, key, lo < hi ? lo : 0);
-            const uint32_t wl = 31u - (uint32_t)(mk & 31u);
-            const float wt = __shfl_sync(0xffffffffu, tt, wl), wu = __shfl_sync(0xffffffffu, uu, wl),
-                        wv = __shfl_sync(0xffffffffu, vv, wl);
-            const uint32_t wtri = __shfl_sync(0xffffffffu, tri, wl);
-            if (lo < hi && mk != ~0ull) {
-                found = true;
-                hit.t = wt; hit.u = wu; hit.v = wv; hit.tri = (int)wtri;
-                tmax = wt;
-            }
-        }
-        if (!alive) return false;
-        if (ng.y <= 0x00ffffffu) {
-            if (stk.sp == 0) return true;
-            ng = stk.pop();
-        }
-        return false;
-    }
-
-    // The per-lane record step_closest_shared reads: origin + tmin, and the
-    // watertight constants with kx | ky << 2 | kz << 4 in the last word.
-    __device__ __forceinline__ void closest_record(float4 *dst) const {
-        dst[0] = make_float4(o.x, o.y, o.z, tmin);
-        dst[1] = make_float4(w.sx, w.sy, w.sz, __uint_as_float((uint32_t)w.kx | ((uint32_t)w.ky << 2) | ((uint32_t)w.kz << 4)));
     }
 
     // Intersect the 8 children of node `child`: ng / tg become its groups.
@@ -766,71 +581,6 @@ __device__ __forceinline__ void trace_queue(const DevScene &S, Walker &wk, unsig
                 }
             }
         }
-    }
-}
-
-// trace_queue with the warp's triangle tests shared out
-// (Bvh8Walker::step_any_shared for any-hit rays, step_closest_shared for
-// closest-hit rays): the same refills, but every lane takes every step, lanes
-// without a ray as idle partners.  rays: 2 float4 per thread of the block
-// (shared memory), written here when a lane takes a ray.
-template <bool kAnyHit, class Walker, class Load, class Store>
-__device__ __forceinline__ void trace_queue_shared(const DevScene &S, Walker &wk, unsigned *fetch, unsigned n,
-                                                   int steps, int min_idle, float4 *rays, Load load, Store store,
-                                                   TravStats &st) {
-    const unsigned lane = threadIdx.x & 31u;
-    float4 *mine = rays + 2 * threadIdx.x;
-    const float4 *warp_rays = rays + 2 * (threadIdx.x & ~31u);
-    int item = -1;
-    bool exhausted = false;
-    unsigned chunk_next = 0, chunk_end = 0;
-    for (;;) {
-        const unsigned want = __ballot_sync(0xffffffffu, item < 0 && !exhausted);
-        const unsigned busy = __ballot_sync(0xffffffffu, item >= 0);
-        if (want && (busy == 0u || __popc(want) >= min_idle)) {
-            const unsigned k = __popc(want), rank = __popc(want & ((1u << lane) - 1u));
-            const unsigned avail = chunk_end - chunk_next;
-            unsigned idx = chunk_next + rank;
-            if (k > avail) {
-                unsigned base = 0;
-                if ((int)lane == __ffs(want) - 1) base = atomicAdd(fetch, kFetchChunk);
-                base = __shfl_sync(0xffffffffu, base, __ffs(want) - 1);
-                if (rank >= avail) idx = base + (rank - avail);
-                chunk_next = base + (k - avail);
-                chunk_end = base + kFetchChunk;
-            } else {
-                chunk_next += k;
-            }
-            if (want >> lane & 1u) {
-                if (idx < n) {
-                    item = (int)idx;
-                    const Ray r = load(item);
-                    wk.begin(S, r);
-                    if constexpr (kAnyHit) {
-                        mine[0] = make_float4(r.o.x, r.o.y, r.o.z, r.tmin);
-                        mine[1] = make_float4(r.d.x, r.d.y, r.d.z, r.tmax);
-                    } else {
-                        wk.closest_record(mine);
-                    }
-                } else {
-                    exhausted = true;
-                }
-            }
-        }
-        if (!__any_sync(0xffffffffu, item >= 0)) break;
-        __syncwarp();   // the new rays are visible to the warp's other lanes
-        for (int k = 0; k < steps; ++k) {
-            bool done;
-            if constexpr (kAnyHit) done = wk.step_any_shared(S, item >= 0, warp_rays);
-            else done = wk.step_closest_shared(S, item >= 0, warp_rays);
-            if (item >= 0 && done) {
-                wk.template end<kAnyHit>(S, st);
-                store(item, wk);
-                item = -1;
-            }
-            if (!__any_sync(0xffffffffu, item >= 0)) break;
-        }
-        __syncwarp();   // every read of a lane's ray precedes its replacement
     }
 }
 

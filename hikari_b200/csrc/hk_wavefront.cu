@@ -15,7 +15,8 @@
 //           added to their path's radiance
 //
 // This file holds regen and the launch sequence; the queue helpers and the
-// extend / shade / shadow kernels are in hk_wf_kernels.cuh.
+// shade kernels are in hk_wf_kernels.cuh, the extend and shadow kernels in
+// hk_wf_trace.cuh.
 //
 // The estimator is the reference's: the next-event MIS weight of an
 // unoccluded emitter is its own pl / (pl + pb) (the reference updates its
@@ -30,12 +31,12 @@ namespace hk {
 
 // The traversal and shade kernels are instantiated in hk_wf_trace_*.cu and
 // hk_wf_shade_*.cu; this file only calls their launchers.
-extern template cudaError_t wf_launch_extend_t<kAccelBvh8>(const DevScene &, const WfState &, const WfLaunchConfig &, int, cudaStream_t);
-extern template cudaError_t wf_launch_extend_t<kAccelBvh2>(const DevScene &, const WfState &, const WfLaunchConfig &, int, cudaStream_t);
-extern template cudaError_t wf_launch_shadow_t<kAccelBvh8>(const DevScene &, const WfState &, const WfLaunchConfig &, cudaStream_t);
-extern template cudaError_t wf_launch_shadow_t<kAccelBvh2>(const DevScene &, const WfState &, const WfLaunchConfig &, cudaStream_t);
-extern template int wf_trace_occupancy_t<kAccelBvh8>(int, int, bool, bool);
-extern template int wf_trace_occupancy_t<kAccelBvh2>(int, int, bool, bool);
+template <int kAccel>
+cudaError_t wf_launch_extend_t(const DevScene &, const WfState &, const WfLaunchConfig &, int, cudaStream_t);
+template <int kAccel>
+cudaError_t wf_launch_shadow_t(const DevScene &, const WfState &, const WfLaunchConfig &, cudaStream_t);
+template <int kAccel>
+int wf_trace_occupancy_t(int, int, bool);
 #define HK_WF_SHADE_EXTERN(K)                                                                                           \
     extern template cudaError_t wf_launch_shade_t<K>(const DevScene &, const WfState &, const WfLaunchConfig &, int, \
                                                      cudaStream_t);                                                 \
@@ -289,14 +290,14 @@ cudaError_t wf_launch_phase(const DevScene &S, const WfState &W, const WfLaunchC
     return cudaGetLastError();
 }
 
-int wf_occupancy(int which, int threads, int accel, bool lean, bool shared) {
+int wf_occupancy(int which, int threads, int accel, bool lean) {
     int n = 0;
     const bool w8 = accel == kAccelBvh8;
     switch (which) {
     case 0:
     case 2:
-        return w8 ? wf_trace_occupancy_t<kAccelBvh8>(which, threads, lean, shared)
-                  : wf_trace_occupancy_t<kAccelBvh2>(which, threads, lean, shared);
+        return w8 ? wf_trace_occupancy_t<kAccelBvh8>(which, threads, lean)
+                  : wf_trace_occupancy_t<kAccelBvh2>(which, threads, lean);
     case 1: return wf_shade_occupancy_t<5>(threads, lean);
     default: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, wf_regen_kernel, threads, 0); break;
     }

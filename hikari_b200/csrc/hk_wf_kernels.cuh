@@ -1,8 +1,8 @@
 // Wavefront pathMIS kernels shared by the wavefront translation units: the
-// queue helpers, the extend and shadow (traversal) kernels and the shade
-// kernel template.  hk_wavefront.cu holds regen and the launch sequence;
-// hk_wf_trace_*.cu instantiate the traversal kernels per tree kind and
-// hk_wf_shade_*.cu the shade kernels per queue, so they compile in parallel.
+// queue helpers and the shade kernel template.  hk_wavefront.cu holds regen
+// and the launch sequence; hk_wf_trace_*.cu instantiate the traversal kernels
+// (hk_wf_trace.cuh) per tree kind and hk_wf_shade_*.cu the shade kernels per
+// queue, so they compile in parallel.
 #pragma once
 #include "hk_shading.cuh"
 #include "hk_wavefront.h"
@@ -92,85 +92,6 @@ __device__ __forceinline__ void splat_global(const DevScene &S, const WfJob &J, 
         }
     }
 }
-// ------------------------------------------------------------ extend
-// Shared memory of the traversal short stacks: kShStack entries per thread.
-__device__ __forceinline__ SharedStack make_stack() {
-    extern __shared__ uint2 wf_stack_smem[];
-    SharedStack s;
-    s.sh = wf_stack_smem + threadIdx.x;
-    s.stride = (int)blockDim.x;
-    s.spill = nullptr;
-    return s;
-}
-
-// The traversal kernels come in two register budgets: kMinBlocks = 0 leaves
-// the budget to the compiler; kLeanBlocks asks for five resident blocks of
-// 256 threads (at most 48 registers), more warps to hide the latency of the
-// node and triangle fetches at the price of some spilling.  The autotuner
-// picks per kernel (hk_wavefront_config.reg_lean).
-constexpr int kLeanBlocks = 5;
-
-// kShared: the warp's triangle tests shared out over its lanes (8-wide tree;
-// the block's ray records in dynamic shared memory after the stacks).
-template <int kAccel, int kMinBlocks, bool kShared>
-__global__ void __launch_bounds__(256, kMinBlocks) wf_extend_kernel(DevScene S, WfState W, int cur, int steps, int min_idle) {
-    const unsigned n = W.ctr->eq_count[cur];
-    TravStats ts;
-    WalkerOf<kAccel, SharedStack> wk;
-    std::conditional_t<kAccel == kAccelBvh8, uint2, int> stack_mem[kAccel == kAccelBvh8 ? kStackSize - kShStack : kStackSize];
-    if constexpr (kAccel == kAccelBvh8) {
-        wk.stk = make_stack();
-        wk.stk.spill = stack_mem;
-    } else {
-        wk.stack = stack_mem;
-    }
-    int slot = -1;
-    auto load = [&](int i) {
-        slot = W.eq[cur][i];
-        const float4 o = W.ray_o[slot], d = W.ray_d[slot];
-        Ray r;
-        r.o = v3(o.x, o.y, o.z);
-        r.d = v3(d.x, d.y, d.z);
-        r.tmin = o.w;
-        r.tmax = d.w;
-        return r;
-    };
-    auto store = [&](int, const auto &w) {
-        int type = 0;
-        if (w.found) {
-            const int mesh = __float_as_int(__ldg(S.tris + 3 * w.hit.tri + 1).w);
-            const DevBsdf &B = S.bsdfs[S.meshes[mesh].bsdf];
-            const bool map = B.type == kBumpMap || B.type == kNormalMap;
-            type = B.deep ? kWfGenericQueue : wf_queue_of(B.type, B.textured != 0, map ? S.bsdfs[B.nested].type : -1);
-            if (map && S.bsdfs[B.nested].deep) type = kWfGenericQueue;   // a map over a deep stack of layers
-        }
-        W.hit[slot] = make_float4(w.hit.t, w.hit.u, w.hit.v, __int_as_float(w.found ? w.hit.tri : -1));
-        W.sq[type][warp_append_keyed(W.ctr->sq_count, type)] = slot;
-    };
-    if constexpr (kShared && kAccel == kAccelBvh8) {
-        extern __shared__ uint2 wf_stack_smem[];
-        float4 *rays = reinterpret_cast<float4 *>(wf_stack_smem + (size_t)blockDim.x * kShStack);
-        trace_queue_shared<false>(S, wk, &W.ctr->ext_fetch, n, steps, min_idle, rays, load, store, ts);
-    } else {
-        trace_queue<false>(S, wk, &W.ctr->ext_fetch, n, steps, min_idle, load, store, ts);
-    }
-    unsigned long long nv = ts.nodes, nt = ts.tris;
-    for (int o = 16; o > 0; o >>= 1) {
-        nv += __shfl_down_sync(0xffffffffu, nv, o);
-        nt += __shfl_down_sync(0xffffffffu, nt, o);
-    }
-    if (lane_id() == 0 && (nv || nt)) {
-        atomicAdd(&W.ctr->node_visits, nv);
-        atomicAdd(&W.ctr->tri_tests, nt);
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        atomicAdd(&W.ctr->rays, (unsigned long long)n);
-        const unsigned k = W.ctr->log_n[0];   // one thread per launch; launches are stream-ordered
-        if (k < (unsigned)kWfLaunchLog) W.ctr->log_rays[0][k] = n;
-        W.ctr->log_n[0] = k + 1;
-    }
-}
-
 // ------------------------------------------------------------ shade
 __device__ __forceinline__ void finish(const WfState &W, int slot) { W.fq[warp_append(&W.ctr->fq_count)] = slot; }
 
@@ -376,143 +297,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) wf_shade_kernel(DevScene S, W
     }
 }
 
-// ------------------------------------------------------------ shadow
-// kShared: the warp's triangle tests shared out over its lanes (8-wide tree;
-// the block's rays in dynamic shared memory after the stacks).
-template <int kAccel, int kMinBlocks, bool kShared>
-__global__ void __launch_bounds__(256, kMinBlocks) wf_shadow_kernel(DevScene S, WfState W, int steps, int min_idle) {
-    const unsigned n = min(W.ctr->shadow_count, (unsigned)W.max_shadow);
-    TravStats ts;
-    WalkerOf<kAccel, SharedStack> wk;
-    std::conditional_t<kAccel == kAccelBvh8, uint2, int> stack_mem[kAccel == kAccelBvh8 ? kStackSize - kShStack : kStackSize];
-    if constexpr (kAccel == kAccelBvh8) {
-        wk.stk = make_stack();
-        wk.stk.spill = stack_mem;
-    } else {
-        wk.stack = stack_mem;
-    }
-    int slot = -1;
-    auto load = [&](int i) {
-        const float4 o = W.sh_o[i], d = W.sh_d[i];
-        slot = __float_as_int(o.w);
-        Ray r;
-        r.o = v3(o.x, o.y, o.z);
-        r.d = v3(d.x, d.y, d.z);
-        r.tmin = kRayEps;
-        r.tmax = 1.0f - kRayEps;
-        return r;
-    };
-    auto store = [&](int i, const auto &w) {
-        if (!w.found) {
-            const float4 c = W.sh_c[i];
-            red_add_v4(W.lacc + slot, c.x, c.y, c.z, 0.0f);
-        }
-    };
-    if constexpr (kShared && kAccel == kAccelBvh8) {
-        extern __shared__ uint2 wf_stack_smem[];
-        float4 *rays = reinterpret_cast<float4 *>(wf_stack_smem + (size_t)blockDim.x * kShStack);
-        trace_queue_shared<true>(S, wk, &W.ctr->sh_fetch, n, steps, min_idle, rays, load, store, ts);
-    } else {
-        trace_queue<true>(S, wk, &W.ctr->sh_fetch, n, steps, min_idle, load, store, ts);
-    }
-    unsigned long long nv = ts.nodes, nt = ts.tris;
-    for (int o = 16; o > 0; o >>= 1) {
-        nv += __shfl_down_sync(0xffffffffu, nv, o);
-        nt += __shfl_down_sync(0xffffffffu, nt, o);
-    }
-    if (lane_id() == 0 && (nv || nt)) {
-        atomicAdd(&W.ctr->node_visits_shadow, nv);
-        atomicAdd(&W.ctr->tri_tests_shadow, nt);
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        atomicAdd(&W.ctr->shadow_rays, (unsigned long long)n);
-        const unsigned k = W.ctr->log_n[1];
-        if (k < (unsigned)kWfLaunchLog) W.ctr->log_rays[1][k] = n;
-        W.ctr->log_n[1] = k + 1;
-    }
-}
-
 // ------------------------------------------------------------ launchers
-__host__ inline size_t wf_stack_bytes(int threads) { return (size_t)threads * kShStack * sizeof(uint2); }
-
-// dynamic shared memory of a traversal launch: the short stacks, and the ray
-// records where the triangle tests are shared out
-__host__ inline size_t wf_shadow_smem(int threads, bool shared) {
-    return wf_stack_bytes(threads) + (shared ? (size_t)threads * 2 * sizeof(float4) : 0);
-}
-template <int kAccel>
-cudaError_t wf_launch_extend_t(const DevScene &S, const WfState &W, const WfLaunchConfig &C, int cur, cudaStream_t st) {
-    const bool shared = kAccel == kAccelBvh8 && C.closest_tests == 2;
-    const size_t smem = kAccel == kAccelBvh8 ? wf_shadow_smem(C.threads_extend, shared) : 0;
-    const int a = C.fetch_steps, b = C.fetch_min_idle;
-    if (shared) {
-        if (C.lean_extend)
-            wf_extend_kernel<kAccel, kLeanBlocks, true><<<C.blocks_extend, C.threads_extend, smem, st>>>(S, W, cur, a, b);
-        else
-            wf_extend_kernel<kAccel, 0, true><<<C.blocks_extend, C.threads_extend, smem, st>>>(S, W, cur, a, b);
-    } else {
-        if (C.lean_extend)
-            wf_extend_kernel<kAccel, kLeanBlocks, false><<<C.blocks_extend, C.threads_extend, smem, st>>>(S, W, cur, a, b);
-        else
-            wf_extend_kernel<kAccel, 0, false><<<C.blocks_extend, C.threads_extend, smem, st>>>(S, W, cur, a, b);
-    }
-    return cudaGetLastError();
-}
-template <int kAccel>
-cudaError_t wf_launch_shadow_t(const DevScene &S, const WfState &W, const WfLaunchConfig &C, cudaStream_t st) {
-    const bool shared = kAccel == kAccelBvh8 && C.shadow_tests == 2;
-    const size_t smem = kAccel == kAccelBvh8 ? wf_shadow_smem(C.threads_shadow, shared) : 0;
-    DevScene SS = S;
-    SS.postpone_any = S.postpone && C.shadow_tests == 1 ? 1 : 0;
-    const int a = C.fetch_steps_shadow, b = C.fetch_min_idle_shadow;
-    if (shared) {
-        if (C.lean_shadow)
-            wf_shadow_kernel<kAccel, kLeanBlocks, true><<<C.blocks_shadow, C.threads_shadow, smem, st>>>(SS, W, a, b);
-        else
-            wf_shadow_kernel<kAccel, 0, true><<<C.blocks_shadow, C.threads_shadow, smem, st>>>(SS, W, a, b);
-    } else {
-        if (C.lean_shadow)
-            wf_shadow_kernel<kAccel, kLeanBlocks, false><<<C.blocks_shadow, C.threads_shadow, smem, st>>>(SS, W, a, b);
-        else
-            wf_shadow_kernel<kAccel, 0, false><<<C.blocks_shadow, C.threads_shadow, smem, st>>>(SS, W, a, b);
-    }
-    return cudaGetLastError();
-}
-// which: 0 extend, 2 shadow; lean: the kLeanBlocks register budget; shared:
-// the kernel with shared triangle tests
-template <int kAccel>
-int wf_trace_occupancy_t(int which, int threads, bool lean, bool shared) {
-    int n = 0;
-    shared = shared && kAccel == kAccelBvh8;
-    if (which == 0) {
-        const size_t smem = kAccel == kAccelBvh8 ? wf_shadow_smem(threads, shared) : 0;
-        if (shared) {
-            if (lean)
-                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, wf_extend_kernel<kAccel, kLeanBlocks, true>, threads,
-                                                              smem);
-            else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, wf_extend_kernel<kAccel, 0, true>, threads, smem);
-        } else {
-            if (lean)
-                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, wf_extend_kernel<kAccel, kLeanBlocks, false>, threads,
-                                                              smem);
-            else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, wf_extend_kernel<kAccel, 0, false>, threads, smem);
-        }
-    } else {
-        const size_t smem = kAccel == kAccelBvh8 ? wf_shadow_smem(threads, shared) : 0;
-        if (shared) {
-            if (lean)
-                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, wf_shadow_kernel<kAccel, kLeanBlocks, true>, threads,
-                                                              smem);
-            else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, wf_shadow_kernel<kAccel, 0, true>, threads, smem);
-        } else {
-            if (lean)
-                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, wf_shadow_kernel<kAccel, kLeanBlocks, false>, threads,
-                                                              smem);
-            else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, wf_shadow_kernel<kAccel, 0, false>, threads, smem);
-        }
-    }
-    return n;
-}
 template <int kType>
 cudaError_t wf_launch_shade_t(const DevScene &S, const WfState &W, const WfLaunchConfig &C, int nxt, cudaStream_t st) {
     if constexpr (kType <= 5) {

@@ -292,24 +292,18 @@ typedef struct {
     float *kernel_ms;              /* optional host float[4]: adds the device time of the regen, extend,
                                       shade and shadow phases (timed with events, no graph) */
     int32_t *kernel_launches;      /* optional host int32[4]: adds the kernel launches per phase */
-    int32_t fetch_steps;           /* node visits of a ray between refills of the traversal lanes
-                                      (0 = 8 for the binary tree, 3 for the 8-wide tree) */
+    int32_t fetch_steps;           /* binary tree: node visits of a ray between refills of the traversal
+                                      lanes (0 = 8) */
     int32_t fetch_min_idle;        /* idle lanes of a warp before it refills while others still
-                                      traverse (0 = 1: refill at once) */
+                                      traverse (0 = 12 for the 8-wide tree, 1 for the binary tree) */
     int32_t fetch_steps_shadow;    /* the same two for the shadow (any-hit) rays; 0 = the closest-hit */
-    int32_t fetch_min_idle_shadow; /*   rays' values */
+    int32_t fetch_min_idle_shadow; /*   rays' values where given, else 8 and 8 (binary tree: 8 and 1) */
     int32_t reg_lean;              /* bit 0 / bit 1: the extend / shadow kernel with a register budget of
                                       48 (five resident blocks of 256 threads) instead of the compiler's;
                                       bit 2: the shade kernels of untextured materials with 64 (four
                                       resident blocks of 256 threads) */
-    int32_t shadow_tests;          /* triangle tests of the shadow rays (8-wide tree): 0 each lane tests
-                                      its own; 1 the same, postponed like closest-hit rays' while few
-                                      lanes of the warp have triangles; 2 shared out over the warp, 32
-                                      at a time */
-    int32_t closest_tests;         /* triangle tests of the closest-hit rays (8-wide tree): 0 each lane
-                                      tests its own, postponed while few lanes of the warp have
-                                      triangles; 2 shared out over the warp, 32 at a time, the least t
-                                      of each ray kept (the later test on equal t, as the serial loop) */
+    int32_t shadow_tests;          /* 0, 1 or 2 (8-wide tree): earlier forms of the rays' triangle tests; */
+    int32_t closest_tests;         /*   every value now runs the one form, tests queued per warp */
     int32_t sample_major;          /* 0: each image's work is dealt tile by tile (all samples of a 16 x 16
                                       tile, then the next); 1: sample by sample over the whole image.
                                       Images agree up to the order of the film's float additions */

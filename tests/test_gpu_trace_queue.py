@@ -1,0 +1,62 @@
+"""The wavefront's per-warp queue of triangle tests at the sizes where it can go
+wrong: leaf groups that overfill the ring, warps with fewer rays than lanes,
+refills at the first and at the last idle lane.
+
+The megakernel traces the same sample streams one ray per thread and tests
+each ray's triangles in order, so images agree up to the order of the film's
+float additions (a few hundred terms per pixel at 2^-24 each: 1e-5 relative,
+and 1e-6 of the largest value where terms cancel) and ray counts exactly."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+import hikari_b200 as hk  # noqa: E402
+from hikari_b200 import scenes  # noqa: E402
+from hikari_b200.scenedesc import BSDF_DIFFUSE, BSDFDesc, CameraDesc, FilterDesc, MeshDesc, SceneDesc  # noqa: E402
+
+
+def _sheets(n, width, height):
+    """n large triangles facing the camera, one behind another and jittered, so that a ray meets most of their
+    boxes in one node, lit by a quad beside the camera."""
+    rng = np.random.default_rng(n)
+    sd = SceneDesc()
+    pos, idx = [], []
+    for k in range(n):
+        z = -0.05 * k + 0.01 * rng.random()
+        c = rng.uniform(-0.3, 0.3, 2)
+        for a in (0.5, 2.6, 4.7):   # counter-clockwise as seen from +z
+            pos.append((c[0] + 1.2 * np.cos(a), c[1] + 1.2 * np.sin(a), z))
+        idx.append((3 * k, 3 * k + 1, 3 * k + 2))
+    sd.meshes.append(MeshDesc(np.float32(pos), np.uint32(idx), BSDFDesc(type=BSDF_DIFFUSE, kd=[0.7, 0.6, 0.5])))
+    lp, li = scenes.quad((-1, 2, 1), (1, 2, 1), (1, 2, 3), (-1, 2, 3))
+    n0 = np.cross(lp[1] - lp[0], lp[2] - lp[0])
+    if n0[1] > 0:
+        lp = lp[::-1].copy()
+    sd.meshes.append(MeshDesc(lp, li, BSDFDesc(type=BSDF_DIFFUSE, kd=[0.0, 0.0, 0.0]), radiance=[4.0, 5.0, 6.0]))
+    sd.camera = CameraDesc(width, height, scenes.look_at((0, 0.2, 3.0), (0, 0, 0), (0, 1, 0)), 50.0, 1e-4, 1e4)
+    sd.filter = FilterDesc(2, 2.0, 0.5)
+    sd.depth = 8
+    return sd
+
+
+def _agree(a, ca, b, cb):
+    scale = float(np.abs(a).max())
+    assert scale > 0
+    assert tuple(ca[:3]) == tuple(cb[:3]), f"rays, shadow rays, dropped: {ca[:3]} vs {cb[:3]}"
+    assert np.allclose(a, b, rtol=1e-5, atol=1e-6 * scale), f"max abs difference {np.abs(a - b).max():.3e} of {scale}"
+
+
+# 1 and 3: one leaf; 24: a node full of three-triangle leaves (32 lanes x 24 tests overfill the 64-entry ring); 25, 70: beyond
+@pytest.mark.parametrize("n", [1, 3, 24, 25, 70])
+@pytest.mark.parametrize("size", [(1, 1), (37, 29)])
+def test_queued_triangle_tests_agree_with_the_serial_order(n, size):
+    gs = hk.Scene.from_desc(_sheets(n, *size))
+    gs.set_image_form(hk.FORM_MEGAKERNEL)
+    a, ca = gs.render_image(16, 8, seed=5)
+    gs.set_image_form(hk.FORM_WAVEFRONT)
+    for idle in (0, 1, 32):
+        gs.set_wavefront_config(dict(fetch_min_idle=idle, fetch_min_idle_shadow=idle))
+        b, cb = gs.render_image(16, 8, seed=5)
+        _agree(a, ca, b, cb)
