@@ -81,11 +81,7 @@ def _host_gb() -> float:
 def _unit_gb(cmd) -> float:
     """Peak host memory (GB) the unit's compile is expected to take."""
     name = next((os.path.basename(a) for a in cmd if a.endswith((".cu", ".cpp"))), "")
-    if name in ("hk_render_b8t.cu", "hk_render_b2t.cu", "hk_wf_shade_3.cu"):
-        return 22.0
-    if name.startswith("hk_render_"):
-        return 10.0
-    return 3.0
+    return 7.0 if name.startswith("hk_render_") or name in ("hk_wf_shade_3.cu", "hk_batch_4.cu") else 3.0
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -106,9 +102,9 @@ def build(force: bool = False, verbose: bool = False) -> str:
             print(" ".join(cmd))
         cmds.append(cmd)
     # translation units compile in parallel (SOURCES lists the slowest first)
-    # within a host-memory budget: ptxas takes about 20 GB for the textured
-    # megakernels and the run-time-dispatched shade kernel, 9 GB for the other
-    # megakernels and a few GB for the rest
+    # within a host-memory budget: ptxas takes up to 7 GB for the units that
+    # dispatch over every BSDF type at run time (the megakernels, the generic
+    # shade kernel, the layered BSDF batch), under 3 GB for the rest
     total = max(16.0, _host_gb() * 0.8)
     budget = [total]
     cv = threading.Condition()

@@ -1436,6 +1436,17 @@ __device__ __forceinline__ V3 bsdf_sample(const DevBsdf *bs, int id, BRec &r, fl
     return layer_sample(bs, b, r, ux, uy, u1);
 }
 
+// The same as calls: one copy of the dispatch over every type per kernel that
+// shades more than one of them.  Inlined at each use (two or three pdfs, an
+// eval and a sample, each again under the bumpMap / normalMap wrappers) the
+// dispatch outgrew the instruction cache, and ptxas took 13 minutes and 20 GB
+// for such a kernel.
+static __device__ __noinline__ V3 bsdf_eval_n(const DevBsdf *bs, int id, const BRec &r) { return bsdf_eval(bs, id, r); }
+static __device__ __noinline__ float bsdf_pdf_n(const DevBsdf *bs, int id, const BRec &r) { return bsdf_pdf(bs, id, r); }
+static __device__ __noinline__ V3 bsdf_sample_n(const DevBsdf *bs, int id, BRec &r, float ux, float uy, float u1) {
+    return bsdf_sample(bs, id, r, ux, uy, u1);
+}
+
 // ---- bumpMap / normalMap (src/bsdf/BumpMapBSDF.cpp, src/bsdf/NormalMapBSDF.cpp).
 // The perturbed frame depends on the intersection only, so the shading code
 // computes it once per vertex (perturbed_frames, hk_shading.cuh) and these
@@ -1455,12 +1466,12 @@ __device__ __forceinline__ bool bump_record(const BumpFrames &f, const BRec &r, 
 static __device__ __noinline__ V3 bump_eval(const DevBsdf *bs, int id, const BRec &r, const BumpFrames &f) {
     BRec q;
     if (!bump_record(f, r, q)) return v3(0, 0, 0);
-    return bsdf_eval(bs, bs[id].nested, q);
+    return bsdf_eval_n(bs, bs[id].nested, q);
 }
 static __device__ __noinline__ float bump_pdf(const DevBsdf *bs, int id, const BRec &r, const BumpFrames &f) {
     BRec q;
     if (!bump_record(f, r, q)) return 0.0f;
-    return bsdf_pdf(bs, bs[id].nested, q);
+    return bsdf_pdf_n(bs, bs[id].nested, q);
 }
 // BumpMapBSDF::Sample (:22)
 static __device__ __noinline__ V3 bump_sample(const DevBsdf *bs, int id, BRec &r, float ux, float uy, float u1,
@@ -1470,7 +1481,7 @@ static __device__ __noinline__ V3 bump_sample(const DevBsdf *bs, int id, BRec &r
     q.wo = v3(0, 0, 0);
     q.measure = kMeasureUnknown;
     if (r.wi.z * q.wi.z <= 0.0f) return v3(0, 0, 0);
-    const V3 res = bsdf_sample(bs, bs[id].nested, q, ux, uy, u1);
+    const V3 res = bsdf_sample_n(bs, bs[id].nested, q, ux, uy, u1);
     if (!is_zero(res)) {
         r.wo = to_local(f.sh, to_world(f.pf, q.wo));
         r.eta = q.eta;
@@ -1481,14 +1492,14 @@ static __device__ __noinline__ V3 bump_sample(const DevBsdf *bs, int id, BRec &r
 }
 // run-time dispatch including the wrappers (f is read only for them)
 __device__ __forceinline__ V3 bsdf_eval_b(const DevBsdf *bs, int id, const BRec &r, const BumpFrames &f) {
-    return is_bump(bs[id]) ? bump_eval(bs, id, r, f) : bsdf_eval(bs, id, r);
+    return is_bump(bs[id]) ? bump_eval(bs, id, r, f) : bsdf_eval_n(bs, id, r);
 }
 __device__ __forceinline__ float bsdf_pdf_b(const DevBsdf *bs, int id, const BRec &r, const BumpFrames &f) {
-    return is_bump(bs[id]) ? bump_pdf(bs, id, r, f) : bsdf_pdf(bs, id, r);
+    return is_bump(bs[id]) ? bump_pdf(bs, id, r, f) : bsdf_pdf_n(bs, id, r);
 }
 __device__ __forceinline__ V3 bsdf_sample_b(const DevBsdf *bs, int id, BRec &r, float ux, float uy, float u1,
                                             const BumpFrames &f) {
-    return is_bump(bs[id]) ? bump_sample(bs, id, r, ux, uy, u1, f) : bsdf_sample(bs, id, r, ux, uy, u1);
+    return is_bump(bs[id]) ? bump_sample(bs, id, r, ux, uy, u1, f) : bsdf_sample_n(bs, id, r, ux, uy, u1);
 }
 
 }  // namespace hk
@@ -1500,7 +1511,7 @@ namespace hk {
 template <int BT>
 __device__ __forceinline__ V3 bsdf_eval_t(const DevBsdf *bs, int id, const BRec &r) {
     const DevBsdf &b = bs[id];
-    if constexpr (BT < 0) return bsdf_eval(bs, id, r);
+    if constexpr (BT < 0) return bsdf_eval_n(bs, id, r);
     else if constexpr (BT == kDiffuse) return diffuse_eval(b, r);
     else if constexpr (BT == kRoughConductor) return conductor_eval(b, r);
     else if constexpr (BT == kRoughDielectric) return dielectric_eval(b, r);
@@ -1517,7 +1528,7 @@ __device__ __forceinline__ V3 bsdf_eval_t(const DevBsdf *bs, int id, const BRec 
 template <int BT>
 __device__ __forceinline__ float bsdf_pdf_t(const DevBsdf *bs, int id, const BRec &r) {
     const DevBsdf &b = bs[id];
-    if constexpr (BT < 0) return bsdf_pdf(bs, id, r);
+    if constexpr (BT < 0) return bsdf_pdf_n(bs, id, r);
     else if constexpr (BT == kDiffuse) return diffuse_pdf(r);
     else if constexpr (BT == kRoughConductor) return conductor_pdf(b, r);
     else if constexpr (BT == kRoughDielectric) return dielectric_pdf(b, r);
@@ -1533,7 +1544,7 @@ __device__ __forceinline__ float bsdf_pdf_t(const DevBsdf *bs, int id, const BRe
 template <int BT>
 __device__ __forceinline__ V3 bsdf_sample_t(const DevBsdf *bs, int id, BRec &r, float ux, float uy, float u1) {
     const DevBsdf &b = bs[id];
-    if constexpr (BT < 0) return bsdf_sample(bs, id, r, ux, uy, u1);
+    if constexpr (BT < 0) return bsdf_sample_n(bs, id, r, ux, uy, u1);
     else if constexpr (BT == kDiffuse) return diffuse_sample(b, r, ux, uy);
     else if constexpr (BT == kRoughConductor) return conductor_sample(b, r, ux, uy);
     else if constexpr (BT == kRoughDielectric) return dielectric_sample(b, r, ux, uy, u1);

@@ -101,7 +101,7 @@ struct alignas(16) DevMesh {
     int32_t has_normals;   // vertex normals present -> interpolated shading frame
     int32_t has_uv;        // texture coordinates present (with normals: the frame follows dP/du)
     float radiance[3];     // area emitter radiance
-    float pad1;
+    int32_t shade_queue;   // wavefront shade queue of the mesh's BSDF (wf_queue_of_bsdf)
 };
 
 // Area emitter: triangles of its mesh in mesh order with the area CDF
@@ -179,6 +179,7 @@ struct DevScene {
     float background[3];
     int32_t force_background;
     int32_t narea;                // area lights
+    uint32_t shade_queues;        // wavefront shade queues that a path in this scene can reach (bit per queue)
 };
 
 }  // namespace hk

@@ -78,13 +78,28 @@ WfEngine::WfEngine(const DevScene &S, int sm_count, const WfEngineConfig &cfg) :
     L_.lean_shadow = (cfg_.reg_lean >> 1) & 1;
     L_.lean_shade = (cfg_.reg_lean >> 2) & 1;
     auto grid = [&](int which, int threads) {
-        const bool lean = which == 0 ? L_.lean_extend : (which == 2 ? L_.lean_shadow : (which == 1 ? L_.lean_shade : false));
+        const bool lean = which == 0 ? L_.lean_extend : (which == 2 ? L_.lean_shadow : false);
         return std::max(1, sm_count * std::max(1, wf_occupancy(which, threads, S.accel, lean)));
     };
     L_.blocks_extend = grid(0, L_.threads_extend);
-    L_.blocks_shade = grid(1, L_.threads_shade);
+    L_.shade_queues = S.shade_queues;
+    int nshade = 0;
+    for (int q = 0; q < kWfTypes; ++q) {
+        if (!(S.shade_queues >> q & 1u)) continue;
+        L_.blocks_shade[q] = std::max(1, sm_count * std::max(1, wf_shade_occupancy(q, L_.threads_shade, L_.lean_shade)));
+        ++nshade;
+    }
     L_.blocks_shadow = grid(2, L_.threads_shadow);
     L_.blocks_regen = grid(3, L_.threads_regen);
+    if (!cfg_.serve) {
+        L_.nfork = std::min(kWfForks, nshade - 1);
+        if (L_.nfork > 0) HK_CUDA(cudaEventCreateWithFlags(&L_.ev_fork, cudaEventDisableTiming));
+        for (int f = 0; f < L_.nfork; ++f) {
+            HK_CUDA(cudaStreamCreateWithFlags(&L_.fork[f], cudaStreamNonBlocking));
+            HK_CUDA(cudaEventCreateWithFlags(&L_.ev_join[f], cudaEventDisableTiming));
+        }
+    }
+    W_.recycle = cfg_.serve ? 1 : 0;
     // idle lanes before a refill, 8-wide tree: a refill costs the warp about 140
     // instructions and a partly filled test batch, an idle lane a 32nd of the
     // rest (64-sphere scene, ms of 33.5M paths at 4 / 8 / 12 lanes: closest hit
@@ -104,6 +119,12 @@ WfEngine::~WfEngine() {
         if (s) cudaStreamSynchronize(s);
     if (exec_) cudaGraphExecDestroy(exec_);
     if (graph_) cudaGraphDestroy(graph_);
+    if (loop_exec_) cudaGraphExecDestroy(loop_exec_);
+    if (loop_graph_) cudaGraphDestroy(loop_graph_);
+    for (cudaEvent_t e : {L_.ev_fork, L_.ev_join[0], L_.ev_join[1], L_.ev_join[2]})
+        if (e) cudaEventDestroy(e);
+    for (cudaStream_t s : L_.fork)
+        if (s) cudaStreamDestroy(s);
     for (cudaEvent_t e : {ev_done_, ev_plan_, ev_switch_, pe_[0], pe_[1]})
         if (e) cudaEventDestroy(e);
     for (cudaStream_t s : streams_)
@@ -118,9 +139,9 @@ void WfEngine::set_priority(bool high) {
     stream_ = target;
 }
 
-void WfEngine::reset() {
+void WfEngine::reset(int slots) {
     set_plan({}, 0);
-    HK_CUDA(wf_launch_init(W_, stream_));
+    HK_CUDA(wf_launch_init(W_, slots > 0 ? std::min(slots, W_.capacity) : W_.capacity, stream_));
 }
 
 void WfEngine::set_job(int slot, WfJob J) {
@@ -163,6 +184,38 @@ void WfEngine::capture() {
     HK_CUDA(cudaGraphInstantiate(&exec_, graph_, 0));
 }
 
+void WfEngine::capture_loop() {
+    HK_CUDA(cudaGraphCreate(&loop_graph_, 0));
+    cudaGraphConditionalHandle handle;
+    HK_CUDA(cudaGraphConditionalHandleCreate(&handle, loop_graph_, 1, cudaGraphCondAssignDefault));
+    cudaGraphNodeParams np = {};
+    np.type = cudaGraphNodeTypeConditional;
+    np.conditional.handle = handle;
+    np.conditional.type = cudaGraphCondTypeWhile;
+    np.conditional.size = 1;
+    cudaGraphNode_t node;
+    HK_CUDA(cudaGraphAddNode(&node, loop_graph_, nullptr, 0, &np));
+    cudaGraph_t body = np.conditional.phGraph_out[0];
+    WfState W = W_;
+    W.cond = handle;
+    HK_CUDA(cudaStreamBeginCaptureToGraph(stream_, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
+    const cudaError_t e0 = wf_launch_iteration(S_, W, L_, 0, stream_);
+    const cudaError_t e1 = wf_launch_iteration(S_, W, L_, 1, stream_);
+    const cudaError_t ec = cudaStreamEndCapture(stream_, &body);
+    if (e0 != cudaSuccess || e1 != cudaSuccess || ec != cudaSuccess)
+        throw HkError{HK_ERR_CUDA, "wavefront graph capture failed"};
+    HK_CUDA(cudaGraphInstantiate(&loop_exec_, loop_graph_, 0));
+}
+
+void WfEngine::run_to_end() {
+    if (!loop_exec_) {
+        if (loop_graph_) cudaGraphDestroy(loop_graph_);   // an earlier attempt failed half way
+        loop_graph_ = nullptr;
+        capture_loop();
+    }
+    HK_CUDA(cudaGraphLaunch(loop_exec_, stream_));
+}
+
 void WfEngine::run(int iterations, bool use_graph, float *kernel_ms, int32_t *kernel_launches) {
     iterations += iterations & 1;   // the queues ping-pong: whole pairs only
     if (kernel_ms) {
@@ -170,7 +223,7 @@ void WfEngine::run(int iterations, bool use_graph, float *kernel_ms, int32_t *ke
             HK_CUDA(cudaEventCreate(&pe_[0]));
             HK_CUDA(cudaEventCreate(&pe_[1]));
         }
-        const int phase_launches[4] = {2, 1, kWfTypes, 1};
+        const int phase_launches[4] = {1, 1, __builtin_popcount(L_.shade_queues), 1};
         for (int k = 0; k < iterations; ++k)
             for (int ph = 0; ph < 4; ++ph) {
                 HK_CUDA(cudaEventRecord(pe_[0], stream_));

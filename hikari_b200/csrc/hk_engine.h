@@ -23,6 +23,8 @@ struct WfEngineConfig {
     int fetch_min_idle = 0;   // idle lanes before a warp refills while others traverse (0: per-kernel default)
     int fetch_steps_shadow = 0;      // the same for the shadow rays (0: the closest-hit value where one is given)
     int fetch_min_idle_shadow = 0;
+    bool fit_capacity = false;   // capacity was chosen from the work, not by the caller
+    bool serve = false;   // plans follow one another; one stream (run), no device-side loop
     int reg_lean = 0;   // bit 0: extend, bit 1: shadow, bit 2: untextured shade kernels with the smaller register budget
 };
 
@@ -45,8 +47,8 @@ public:
     // before those of low-priority engines sharing the GPU.
     void set_priority(bool high);
 
-    // Empty pool (every slot idle), zero statistics, empty plan.  Async on stream().
-    void reset();
+    // Empty pool (the first `slots` slots idle, 0: all), zero statistics, empty plan.  Async on stream().
+    void reset(int slots = 0);
     // Job-table entry `slot`: its finished counter is zeroed and J.finished set.  Async;
     // the slot must not be in use by paths in flight.
     void set_job(int slot, WfJob J);
@@ -55,6 +57,10 @@ public:
     // `iterations` (even) wavefront iterations, from the graph or as plain launches.
     // With kernel_ms (host float[4]) each phase is timed with events and added.
     void run(int iterations, bool use_graph, float *kernel_ms = nullptr, int32_t *kernel_launches = nullptr);
+    // Iterations until the plan is dealt and no path is in flight, or at least
+    // kWfMaxLoops pairs of them: one graph launch whose while node regen
+    // steers, so the host neither polls nor overshoots.  Async.
+    void run_to_end();
     // Copy the counters and the job table's finished counters to the host mirrors
     // and record done_event(); read them after the event completed.
     void fetch_status();
@@ -71,6 +77,7 @@ public:
 
 private:
     void capture();
+    void capture_loop();
     DevScene S_;
     WfEngineConfig cfg_;
     WfLaunchConfig L_{};
@@ -88,6 +95,8 @@ private:
     cudaEvent_t ev_done_ = nullptr, ev_plan_ = nullptr, pe_[2] = {nullptr, nullptr};
     cudaGraph_t graph_ = nullptr;
     cudaGraphExec_t exec_ = nullptr;
+    cudaGraph_t loop_graph_ = nullptr;   // one while node over a pair of iterations
+    cudaGraphExec_t loop_exec_ = nullptr;
 };
 
 }  // namespace hk

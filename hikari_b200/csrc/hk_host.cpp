@@ -690,6 +690,8 @@ void build_scene(hk_scene *s) {
     D.bsdfs = s->b_bsdfs.as<hk::DevBsdf>();
     D.nbsdfs = (int)bs.size();
 
+    D.shade_queues = 1u;   // the miss queue; the meshes add theirs
+
     // meshes, global triangles
     std::vector<hk::DevMesh> dm;
     uint64_t ntris = 0;
@@ -724,6 +726,8 @@ void build_scene(hk_scene *s) {
         d.has_normals = !m.nrm.empty();
         d.has_uv = !m.uv.empty();
         for (int c = 0; c < 3; c++) d.radiance[c] = m.radiance[c];
+        d.shade_queue = hk::wf_queue_of_bsdf(bs.data(), m.bsdf);
+        D.shade_queues |= 1u << d.shade_queue;
         dm.push_back(d);
         size_t nv = m.pos.size() / 3;
         for (size_t v = 0; v < nv; ++v)
@@ -1013,7 +1017,9 @@ void require_scene_size(const hk_scene *s, const hk_render_desc &d) {
 hk::WfEngine &wf_ensure(hk_scene *s, const hk::WfEngineConfig &c) {
     if (s->wf) {
         const hk::WfEngineConfig &o = s->wf->config();
-        if (o.capacity == c.capacity && o.threads_extend == c.threads_extend && o.threads_shade == c.threads_shade &&
+        // a pool fitted to an earlier call's work serves every call that needs no more slots
+        const bool fits = o.capacity == c.capacity || (o.fit_capacity && c.fit_capacity && o.capacity >= c.capacity);
+        if (fits && o.fit_capacity == c.fit_capacity && o.threads_extend == c.threads_extend && o.threads_shade == c.threads_shade &&
             o.fetch_steps == c.fetch_steps && o.fetch_min_idle == c.fetch_min_idle &&
             o.fetch_steps_shadow == c.fetch_steps_shadow && o.fetch_min_idle_shadow == c.fetch_min_idle_shadow &&
             o.reg_lean == c.reg_lean)
@@ -1592,7 +1598,7 @@ int hk_render_batch(hk_scene *s, const hk_render_job *jobs, int njobs, const hk_
         hk_wavefront_config c{};
         if (cfg) c = *cfg;
         hk::WfEngineConfig ec;
-        ec.capacity = std::max(1024, std::min(c.capacity > 0 ? c.capacity : (1 << 21), 1 << 26));
+        ec.capacity = std::max(1024, std::min(c.capacity, 1 << 26));
         ec.threads_extend = c.threads_extend > 0 ? c.threads_extend : 128;
         ec.threads_shade = c.threads_shade > 0 ? c.threads_shade : 128;
         ec.fetch_steps = std::max(0, std::min(1024, c.fetch_steps));
@@ -1600,6 +1606,22 @@ int hk_render_batch(hk_scene *s, const hk_render_job *jobs, int njobs, const hk_
         ec.fetch_steps_shadow = std::max(0, std::min(1024, c.fetch_steps_shadow));
         ec.fetch_min_idle_shadow = c.fetch_min_idle_shadow > 0 ? std::min(32, c.fetch_min_idle_shadow) : 0;
         ec.reg_lean = c.reg_lean & 7;
+        std::vector<hk::WfJob> table(njobs);
+        std::vector<hk::WfSeg> plan(njobs);
+        uint64_t total = 0;
+        for (int j = 0; j < njobs; ++j) {
+            if (!jobs[j].film_dev) throw HkError{HK_ERR_INVALID, "bad job: null film"};
+            table[j] = hk::make_wf_job(s, jobs[j].desc);
+            table[j].sample_major = c.sample_major ? 1 : 0;
+            table[j].film = jobs[j].film_dev;
+            plan[j] = hk::WfSeg{total, 0, j, 0};
+            total += table[j].work_count;
+        }
+        if (c.capacity <= 0) {   // as many slots as the work can use, from 2^14 to 2^21
+            ec.fit_capacity = true;
+            ec.capacity = 1 << 14;
+            while (ec.capacity < (1 << 21) && (uint64_t)ec.capacity < total) ec.capacity *= 2;
+        }
         hk::WfEngine &E = wf_ensure(s, ec);
         cudaStream_t user = (cudaStream_t)stream, st = E.stream();
         // order after the caller's stream (the films may have been cleared there)
@@ -1611,18 +1633,8 @@ int hk_render_batch(hk_scene *s, const hk_render_job *jobs, int njobs, const hk_
         } guard{ev};
         HK_CUDA(cudaEventRecord(ev, user));
         HK_CUDA(cudaStreamWaitEvent(st, ev, 0));
-        std::vector<hk::WfSeg> plan(njobs);
-        uint64_t total = 0;
-        E.reset();
-        for (int j = 0; j < njobs; ++j) {
-            if (!jobs[j].film_dev) throw HkError{HK_ERR_INVALID, "bad job: null film"};
-            hk::WfJob J = hk::make_wf_job(s, jobs[j].desc);
-            J.sample_major = c.sample_major ? 1 : 0;
-            J.film = jobs[j].film_dev;
-            E.set_job(j, J);
-            plan[j] = hk::WfSeg{total, 0, j, 0};
-            total += J.work_count;
-        }
+        E.reset((int)std::min<uint64_t>(total, (uint64_t)ec.capacity));
+        for (int j = 0; j < njobs; ++j) E.set_job(j, table[j]);
         E.set_plan(plan, total);
         const bool profile = c.kernel_ms != nullptr;
         const bool use_graph = c.no_graph == 0 && !profile;
@@ -1630,7 +1642,8 @@ int hk_render_batch(hk_scene *s, const hk_render_job *jobs, int njobs, const hk_
         uint64_t iters = 0;
         const uint64_t max_iters = 1ull << 40;
         for (;;) {
-            E.run(per_check, use_graph, c.kernel_ms, c.kernel_launches);
+            if (use_graph) E.run_to_end();
+            else E.run(per_check, false, c.kernel_ms, c.kernel_launches);
             iters += per_check;
             E.fetch_status();
             HK_CUDA(cudaEventSynchronize(E.done_event()));

@@ -104,8 +104,8 @@ __device__ V3 li_pathmis(const DevScene &S, Pcg32 &rng, Ray ray, float px, float
                     pb = bsdf_pdf_b(S.bsdfs, bsdf, br, bf);
                     f = bsdf_eval_b(S.bsdfs, bsdf, br, bf);
                 } else {
-                    pb = bsdf_pdf(S.bsdfs, bsdf, br);
-                    f = bsdf_eval(S.bsdfs, bsdf, br);
+                    pb = bsdf_pdf_n(S.bsdfs, bsdf, br);
+                    f = bsdf_eval_n(S.bsdfs, bsdf, br);
                 }
                 const float w = (pl + pb != 0.0f) ? pl / (pl + pb) : w_ems;
                 const float c = fabsf(br.wo.z);
@@ -133,7 +133,7 @@ __device__ V3 li_pathmis(const DevScene &S, Pcg32 &rng, Ray ray, float px, float
         float u1 = needs_u1(S.bsdfs, bsdf) ? rng.nextf() : 0.0f;
         V3 F;
         if constexpr (kTex) F = bsdf_sample_b(S.bsdfs, bsdf, br, sx, sy, u1, bf);
-        else F = bsdf_sample(S.bsdfs, bsdf, br, sx, sy, u1);
+        else F = bsdf_sample_n(S.bsdfs, bsdf, br, sx, sy, u1);
         ray.o = it.p;
         ray.d = to_world(it.sh, br.wo);
         ray.tmin = kRayEps;
@@ -163,7 +163,7 @@ __device__ V3 li_pathmis(const DevScene &S, Pcg32 &rng, Ray ray, float px, float
                 float plm = area_pdf(AL, er);
                 float pbm;
                 if constexpr (kTex) pbm = bsdf_pdf_b(S.bsdfs, bsdf, br, bf);
-                else pbm = bsdf_pdf(S.bsdfs, bsdf, br);
+                else pbm = bsdf_pdf_n(S.bsdfs, bsdf, br);
                 if (pbm + plm != 0.0f) w_mats = pbm / (pbm + plm);
             }
         }

@@ -233,6 +233,7 @@ void hk_server::admit(const std::vector<SceneEntry *> &sc) {
             // the server's pool size and block sizes; the traversal knobs of
             // the scene's own configuration where it has one (autotuned)
             hk::WfEngineConfig sec = ec;
+            sec.serve = true;
             if (*e.view.has_cfg) {
                 const hk_wavefront_config &t = *e.view.cfg;
                 sec.fetch_steps = std::max(0, std::min(1024, t.fetch_steps));

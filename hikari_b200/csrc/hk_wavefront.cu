@@ -27,6 +27,8 @@
 // discards the hit of a terminated path, which changes nothing).
 #include "hk_wf_kernels.cuh"
 
+#include <algorithm>
+
 namespace hk {
 
 // The traversal and shade kernels are instantiated in hk_wf_trace_*.cu and
@@ -59,18 +61,20 @@ HK_WF_SHADE_EXTERN(14);
 HK_WF_SHADE_EXTERN(15);
 HK_WF_SHADE_EXTERN(16);
 #undef HK_WF_SHADE_EXTERN
-static_assert(kWfTypes == 17, "launch_shade_all launches one kernel per shade queue");
+static_assert(kWfTypes == 17, "one shade kernel per queue");
 
 // ------------------------------------------------------------ regen
-// Splat and retire the finished paths, then give every finished or idle slot
-// new work from the dispatch plan; slots that find none wait in the next idle
+// Splat and retire the finished paths, then give finished and idle slots new
+// work from the dispatch plan; slots that find none wait in the next idle
 // list.  Queues read here: fq, idle[cur]; written: eq[cur], idle[cur ^ 1].
 // Slot i of the n slots that want work (finished paths first, then idle
 // slots) takes plan item next_work + i: the items are dealt without an
-// atomic, and wf_reset_kernel advances next_work by n afterwards.  An item
+// atomic, and the last block to finish advances next_work by n.  An item
 // whose pixel lies outside its image (the partial tiles at the right and
 // bottom edges) counts as work done and leaves its slot idle until the next
-// iteration.  Appends to the extend and idle lists, the per-job finished
+// iteration.  Where no plan follows this one (W.recycle == 0), idle slots
+// beyond the plan's end are dropped, so that a draining pool touches only the
+// paths still in flight (a quarter of a 2^22-path image's iterations drain).  Appends to the extend and idle lists, the per-job finished
 // counts and the change of the in-flight count are gathered per block in
 // shared memory and added once per block and round: a global atomic per warp
 // on a handful of addresses serialises at the L2.
@@ -83,9 +87,11 @@ __global__ void __launch_bounds__(256) wf_regen_kernel(DevScene S, WfState W, in
     if (threadIdx.x == 0) s_active = 0;
     __syncthreads();
     const int nf = (int)W.ctr->fq_count;
-    const int n = nf + (int)W.ctr->idle_count[cur];
     const uint64_t total = W.ctr->total_work;
     const uint64_t first = W.ctr->next_work;
+    int n = nf + (int)W.ctr->idle_count[cur];
+    const bool drained = !W.recycle && first + (uint64_t)n >= total;   // this pass deals the plan's last item
+    if (drained) n = max(nf, (int)min((uint64_t)n, total - min(first, total)));
     const int nseg = (int)W.ctr->seg_count;
     const unsigned lane = lane_id(), warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     unsigned long long dropped = 0;
@@ -149,7 +155,7 @@ __global__ void __launch_bounds__(256) wf_regen_kernel(DevScene S, WfState W, in
             }
         }
         // block-aggregated appends: one atomic per list per block and round
-        const bool to_idle = i < n && !started;
+        const bool to_idle = i < n && !started && !drained;
         const unsigned be = __ballot_sync(0xffffffffu, started), bi = __ballot_sync(0xffffffffu, to_idle);
         if (lane == 0) {
             s_warp[0][warp] = __popc(be);
@@ -179,37 +185,46 @@ __global__ void __launch_bounds__(256) wf_regen_kernel(DevScene S, WfState W, in
     __syncthreads();
     for (int k = threadIdx.x; k < kWfMaxJobs; k += blockDim.x)
         if (s_finished[k]) atomicAdd(W.jobs[k].finished, (unsigned long long)s_finished[k]);
-    if (threadIdx.x == 0 && s_active) atomicAdd(&W.ctr->active, (unsigned)s_active);
-}
-
-// Reset the counters of the queues consumed by regen and of those the next
-// phases fill.
-__global__ void wf_reset_kernel(WfState W, int cur) {
+    // the last block through resets the counters of the queues consumed here
+    // and of those that the next phases fill, and decides whether the
+    // device-side loop goes on
     if (threadIdx.x == 0) {
-        // regen dealt plan items next_work .. next_work + n - 1 to its n slots
-        const unsigned long long dealt = W.ctr->next_work + W.ctr->fq_count + W.ctr->idle_count[cur];
-        W.ctr->next_work = dealt < W.ctr->total_work ? dealt : W.ctr->total_work;
-        W.ctr->fq_count = 0;
-        W.ctr->idle_count[cur] = 0;
-        W.ctr->eq_count[cur ^ 1] = 0;
-        W.ctr->shadow_count = 0;
-        W.ctr->ext_fetch = 0;
-        W.ctr->sh_fetch = 0;
+        WfCounters *c = W.ctr;
+        if (s_active) atomicAdd(&c->active, (unsigned)s_active);
+        __threadfence();
+        if (atomicAdd(&c->regen_done, 1u) == gridDim.x - 1u) {
+            __threadfence();
+            const unsigned long long dealt = first + (uint64_t)n;
+            const unsigned long long next = dealt < total ? dealt : total;
+            c->regen_done = 0u;
+            c->next_work = next;
+            c->fq_count = 0u;
+            c->idle_count[cur] = 0u;
+            c->eq_count[cur ^ 1] = 0u;
+            c->shadow_count = 0u;
+            c->ext_fetch = 0u;
+            c->sh_fetch = 0u;
+            for (int t = 0; t < kWfTypes; ++t) c->sq_count[t] = 0u;
+            if (W.cond && cur == 1) {
+                const bool more = (atomicAdd(&c->active, 0u) != 0u || next < total) && ++c->loops < kWfMaxLoops;
+                if (!more) c->loops = 0u;
+                cudaGraphSetConditional(W.cond, more ? 1u : 0u);
+            }
+        }
     }
-    if (threadIdx.x < kWfTypes) W.ctr->sq_count[threadIdx.x] = 0;
 }
 
-// Empty pool: every slot in idle list 0, all queues and statistics zero.
-__global__ void wf_init_kernel(WfState W) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < W.capacity; i += gridDim.x * blockDim.x) W.idle[0][i] = i;
+// Empty pool: the first `slots` slots in idle list 0, all queues and statistics zero.
+__global__ void wf_init_kernel(WfState W, int slots) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < slots; i += gridDim.x * blockDim.x) W.idle[0][i] = i;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         WfCounters *c = W.ctr;
         c->eq_count[0] = c->eq_count[1] = 0;
-        c->idle_count[0] = (unsigned)W.capacity;
+        c->idle_count[0] = (unsigned)slots;
         c->idle_count[1] = 0;
         for (int t = 0; t < kWfTypes; ++t) c->sq_count[t] = 0;
         c->fq_count = c->shadow_count = c->active = 0;
-        c->ext_fetch = c->sh_fetch = 0;
+        c->ext_fetch = c->sh_fetch = c->regen_done = c->loops = 0;
         c->rays = c->shadow_rays = c->dropped = 0;
         c->node_visits = c->tri_tests = c->node_visits_shadow = c->tri_tests_shadow = 0;
         c->log_n[0] = c->log_n[1] = 0;
@@ -235,24 +250,31 @@ static cudaError_t launch_extend(const DevScene &S, const WfState &W, const WfLa
 static cudaError_t launch_shadow(const DevScene &S, const WfState &W, const WfLaunchConfig &C, cudaStream_t st) {
     return S.accel == kAccelBvh8 ? wf_launch_shadow_t<kAccelBvh8>(S, W, C, st) : wf_launch_shadow_t<kAccelBvh2>(S, W, C, st);
 }
+// The shade kernels of the queues that the scene can reach.  They are dealt to
+// the launch stream and its forks: each runs one wave or less in the later
+// iterations, so side by side they fill the SMs that one alone leaves idle.
+template <int kType>
+struct ShadeLaunch {
+    static void run(const DevScene &S, const WfState &W, const WfLaunchConfig &C, int nxt, cudaStream_t st, int &k) {
+        if (C.shade_queues >> kType & 1u) {
+            const int lane = k++ % (C.nfork + 1);
+            wf_launch_shade_t<kType>(S, W, C, nxt, lane == 0 ? st : C.fork[lane - 1]);
+        }
+        if constexpr (kType + 1 < kWfTypes) ShadeLaunch<kType + 1>::run(S, W, C, nxt, st, k);
+    }
+};
 static cudaError_t launch_shade_all(const DevScene &S, const WfState &W, const WfLaunchConfig &C, int nxt, cudaStream_t st) {
-    wf_launch_shade_t<0>(S, W, C, nxt, st);
-    wf_launch_shade_t<1>(S, W, C, nxt, st);
-    wf_launch_shade_t<2>(S, W, C, nxt, st);
-    wf_launch_shade_t<3>(S, W, C, nxt, st);
-    wf_launch_shade_t<4>(S, W, C, nxt, st);
-    wf_launch_shade_t<5>(S, W, C, nxt, st);
-    wf_launch_shade_t<6>(S, W, C, nxt, st);
-    wf_launch_shade_t<7>(S, W, C, nxt, st);
-    wf_launch_shade_t<8>(S, W, C, nxt, st);
-    wf_launch_shade_t<9>(S, W, C, nxt, st);
-    wf_launch_shade_t<10>(S, W, C, nxt, st);
-    wf_launch_shade_t<11>(S, W, C, nxt, st);
-    wf_launch_shade_t<12>(S, W, C, nxt, st);
-    wf_launch_shade_t<13>(S, W, C, nxt, st);
-    wf_launch_shade_t<14>(S, W, C, nxt, st);
-    wf_launch_shade_t<15>(S, W, C, nxt, st);
-    return wf_launch_shade_t<16>(S, W, C, nxt, st);
+    if (C.nfork > 0) {
+        cudaEventRecord(C.ev_fork, st);
+        for (int f = 0; f < C.nfork; ++f) cudaStreamWaitEvent(C.fork[f], C.ev_fork, 0);
+    }
+    int k = 0;
+    ShadeLaunch<0>::run(S, W, C, nxt, st, k);
+    for (int f = 0; f < C.nfork; ++f) {
+        cudaEventRecord(C.ev_join[f], C.fork[f]);
+        cudaStreamWaitEvent(st, C.ev_join[f], 0);
+    }
+    return cudaGetLastError();
 }
 
 cudaError_t wf_launch_counters_add(const WfState &W, unsigned long long *out, cudaStream_t st) {
@@ -260,15 +282,14 @@ cudaError_t wf_launch_counters_add(const WfState &W, unsigned long long *out, cu
     return cudaGetLastError();
 }
 
-cudaError_t wf_launch_init(const WfState &W, cudaStream_t st) {
-    wf_init_kernel<<<(W.capacity + 255) / 256, 256, 0, st>>>(W);
+cudaError_t wf_launch_init(const WfState &W, int slots, cudaStream_t st) {
+    wf_init_kernel<<<std::max(1, std::min((slots + 255) / 256, 4096)), 256, 0, st>>>(W, slots);
     return cudaGetLastError();
 }
 
 cudaError_t wf_launch_iteration(const DevScene &S, const WfState &W, const WfLaunchConfig &C, int cur, cudaStream_t st) {
     const int nxt = cur ^ 1;
     wf_regen_kernel<<<C.blocks_regen, C.threads_regen, 0, st>>>(S, W, cur);
-    wf_reset_kernel<<<1, 32, 0, st>>>(W, cur);
     launch_extend(S, W, C, cur, st);
     launch_shade_all(S, W, C, nxt, st);
     launch_shadow(S, W, C, st);
@@ -281,8 +302,7 @@ cudaError_t wf_launch_phase(const DevScene &S, const WfState &W, const WfLaunchC
     switch (phase) {
     case 0:
         wf_regen_kernel<<<C.blocks_regen, C.threads_regen, 0, st>>>(S, W, cur);
-        wf_reset_kernel<<<1, 32, 0, st>>>(W, cur);
-        break;
+            break;
     case 1: launch_extend(S, W, C, cur, st); break;
     case 2: launch_shade_all(S, W, C, nxt, st); break;
     default: launch_shadow(S, W, C, st); break;
@@ -291,17 +311,20 @@ cudaError_t wf_launch_phase(const DevScene &S, const WfState &W, const WfLaunchC
 }
 
 int wf_occupancy(int which, int threads, int accel, bool lean) {
-    int n = 0;
-    const bool w8 = accel == kAccelBvh8;
-    switch (which) {
-    case 0:
-    case 2:
-        return w8 ? wf_trace_occupancy_t<kAccelBvh8>(which, threads, lean)
-                  : wf_trace_occupancy_t<kAccelBvh2>(which, threads, lean);
-    case 1: return wf_shade_occupancy_t<5>(threads, lean);
-    default: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, wf_regen_kernel, threads, 0); break;
+    if (which == 3) {
+        int n = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, wf_regen_kernel, threads, 0);
+        return n;
     }
-    return n;
+    return accel == kAccelBvh8 ? wf_trace_occupancy_t<kAccelBvh8>(which, threads, lean)
+                               : wf_trace_occupancy_t<kAccelBvh2>(which, threads, lean);
 }
+template <int kType>
+static int shade_occupancy(int queue, int threads, bool lean) {
+    if (queue == kType) return wf_shade_occupancy_t<kType>(threads, lean);
+    if constexpr (kType + 1 < kWfTypes) return shade_occupancy<kType + 1>(queue, threads, lean);
+    return 0;
+}
+int wf_shade_occupancy(int queue, int threads, bool lean) { return shade_occupancy<0>(queue, threads, lean); }
 
 }  // namespace hk

@@ -39,6 +39,14 @@ __host__ __device__ constexpr int wf_queue_of(int bsdf_type, bool textured = fal
                       ? kWfBumpQueue0 + nested_type
                       : kWfGenericQueue);
 }
+// Shade queue of BSDF id: deep stacks of layers (and maps over them) are
+// dispatched at run time whatever their top-level type.
+__host__ __device__ inline int wf_queue_of_bsdf(const DevBsdf *bs, int id) {
+    const DevBsdf &b = bs[id];
+    const bool map = b.type == kBumpMap || b.type == kNormalMap;
+    if (b.deep || (map && bs[b.nested].deep)) return kWfGenericQueue;
+    return wf_queue_of(b.type, b.textured != 0, map ? bs[b.nested].type : -1);
+}
 constexpr int kWfMaxJobs = 1024;   // job table entries of one engine
 constexpr int kWfMaxSegs = 4096;   // pieces of one dispatch plan
 constexpr int kWfTileSide = 16;
@@ -90,6 +98,8 @@ struct WfCounters {
     unsigned int shadow_count;         // next-event shadow rays
     unsigned int active;               // paths in flight
     unsigned int ext_fetch, sh_fetch;  // rays claimed by the extend / shadow kernels (dynamic fetch)
+    unsigned int regen_done;           // blocks of the running regen launch that are through
+    unsigned int loops;                // passes of the device-side loop since its launch
     unsigned int pad1;
     unsigned long long rays, shadow_rays, dropped;
     unsigned long long node_visits, tri_tests;                 // closest-hit traversal (extend)
@@ -140,14 +150,22 @@ struct WfState {
     WfCounters *ctr;
     const WfJob *jobs;
     const WfSeg *segs;
+    int recycle;                       // plans follow one another (serving): slots without work stay in the idle list
+    unsigned long long cond;           // handle of the while node that repeats the iterations (0: none)
 };
 
 // flags in the high half of pix.w
 constexpr uint32_t kWfFlagForceMats = 1u;   // previous BSDF sample was EDiscrete
 
+constexpr int kWfForks = 3;             // streams beside the launch stream that shade kernels are dealt to
+constexpr unsigned kWfMaxLoops = 1u << 14;   // passes of the device-side loop before it returns to the host
 struct WfLaunchConfig {
     int blocks_extend, threads_extend;
-    int blocks_shade, threads_shade;
+    int blocks_shade[kWfTypes], threads_shade;
+    uint32_t shade_queues;             // queues the scene can reach; the kernels of the others are not launched
+    int nfork;                         // forks in use
+    cudaStream_t fork[kWfForks];
+    cudaEvent_t ev_fork, ev_join[kWfForks];
     int blocks_shadow, threads_shadow;
     int blocks_regen, threads_regen;
     // dynamic ray fetch of the extend kernel: node visits between refills (binary tree), idle lanes before a refill
@@ -157,8 +175,9 @@ struct WfLaunchConfig {
     int lean_shade;                                  // untextured shade kernels with the smaller register budget
 };
 
-// empty pool: every slot idle, queues and statistics zero (the dispatch head is the host's)
-cudaError_t wf_launch_init(const WfState &W, cudaStream_t st);
+// empty pool: the first `slots` slots idle (the others unused), queues and
+// statistics zero (the dispatch head is the host's)
+cudaError_t wf_launch_init(const WfState &W, int slots, cudaStream_t st);
 // one iteration with extend queue `cur` (0/1)
 cudaError_t wf_launch_iteration(const DevScene &S, const WfState &W, const WfLaunchConfig &C, int cur, cudaStream_t st);
 // one phase of an iteration: 0 regen + reset, 1 extend, 2 shade (all materials), 3 shadow
@@ -166,8 +185,9 @@ cudaError_t wf_launch_phase(const DevScene &S, const WfState &W, const WfLaunchC
                             cudaStream_t st);
 // out[0..6] += rays, shadow rays, dropped, node visits, triangle tests, shadow node visits, shadow tests
 cudaError_t wf_launch_counters_add(const WfState &W, unsigned long long *out, cudaStream_t st);
-// resident blocks per SM of a kernel (which: 0 extend, 1 shade, 2 shadow, 3
-// regen); lean: the traversal kernels' smaller register budget
+// resident blocks per SM of a kernel (which: 0 extend, 2 shadow, 3 regen) and
+// of a queue's shade kernel; lean: the smaller register budget
 int wf_occupancy(int which, int threads, int accel, bool lean = false);
+int wf_shade_occupancy(int queue, int threads, bool lean);
 
 }  // namespace hk

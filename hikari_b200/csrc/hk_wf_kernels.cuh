@@ -302,11 +302,11 @@ template <int kType>
 cudaError_t wf_launch_shade_t(const DevScene &S, const WfState &W, const WfLaunchConfig &C, int nxt, cudaStream_t st) {
     if constexpr (kType <= 5) {
         if (C.lean_shade) {
-            wf_shade_kernel<kType, kLeanShade><<<C.blocks_shade, C.threads_shade, 0, st>>>(S, W, nxt);
+            wf_shade_kernel<kType, kLeanShade><<<C.blocks_shade[kType], C.threads_shade, 0, st>>>(S, W, nxt);
             return cudaGetLastError();
         }
     }
-    wf_shade_kernel<kType><<<C.blocks_shade, C.threads_shade, 0, st>>>(S, W, nxt);
+    wf_shade_kernel<kType><<<C.blocks_shade[kType], C.threads_shade, 0, st>>>(S, W, nxt);
     return cudaGetLastError();
 }
 template <int kType>

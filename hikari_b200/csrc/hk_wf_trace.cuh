@@ -405,10 +405,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) wf_extend_kernel(DevScene S, 
                 const float4 o = W.ray_o[slot], d = W.ray_d[slot];
                 refine_mt(xyz(o), xyz(d), xyz(ldg4(tp)), xyz(p1), xyz(ldg4(tp + 2)), o.w, d.w, h.t, h.u, h.v);
             }
-            const DevBsdf &B = S.bsdfs[S.meshes[__float_as_int(p1.w)].bsdf];
-            const bool map = B.type == kBumpMap || B.type == kNormalMap;
-            type = B.deep ? kWfGenericQueue : wf_queue_of(B.type, B.textured != 0, map ? S.bsdfs[B.nested].type : -1);
-            if (map && S.bsdfs[B.nested].deep) type = kWfGenericQueue;   // a map over a deep stack of layers
+            type = S.meshes[__float_as_int(p1.w)].shade_queue;
         }
         W.hit[slot] = make_float4(h.t, h.u, h.v, __int_as_float(found ? h.tri : -1));
         W.sq[type][warp_append_keyed(W.ctr->sq_count, type)] = slot;

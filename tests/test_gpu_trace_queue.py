@@ -1,6 +1,6 @@
-"""The wavefront's per-warp queue of triangle tests at the sizes where it can go
-wrong: leaf groups that overfill the ring, warps with fewer rays than lanes,
-refills at the first and at the last idle lane.
+"""The wavefront's per-warp queue of triangle tests and its pool at the sizes
+where they can go wrong: leaf groups that overfill the ring, warps with fewer
+rays than lanes, pools smaller than the work, images with partial tiles.
 
 The megakernel traces the same sample streams one ray per thread and tests
 each ray's triangles in order, so images agree up to the order of the film's
@@ -60,3 +60,24 @@ def test_queued_triangle_tests_agree_with_the_serial_order(n, size):
         gs.set_wavefront_config(dict(fetch_min_idle=idle, fetch_min_idle_shadow=idle))
         b, cb = gs.render_image(16, 8, seed=5)
         _agree(a, ca, b, cb)
+
+
+# pools of 1024 slots (the least) against 33 x 17 and 80 x 56 x 8 paths; 0: fitted to the work, then reused for less and for more
+@pytest.mark.parametrize("no_graph", [False, True])
+def test_pool_sizes_render_the_same_images(no_graph):
+    sd = scenes.cornell_box(width=80, height=56)
+    gs = hk.Scene.from_desc(sd)
+    sizes = [(33, 17), (80, 56), (16, 16)]
+    ref = None
+    for capacity, spp in ((1024, 8), (0, 1), (0, 8), (0, 2), (1 << 16, 8)):
+        films = [torch.zeros(gs.film_shape(w, h), device="cuda") for w, h in sizes]
+        ctr = torch.zeros(7, dtype=torch.int64, device="cuda")
+        gs.render_batch(films, spp, sd.depth, seeds=[1, 2, 3], sizes=sizes, counters=ctr, capacity=capacity,
+                        no_graph=no_graph)
+        if spp != 8:
+            continue
+        got = np.concatenate([f.cpu().numpy().astype(np.float64).reshape(-1) for f in films])
+        c = ctr.cpu().numpy()
+        if ref is None:
+            ref = (got, c)
+        _agree(ref[0], ref[1], got, c)
