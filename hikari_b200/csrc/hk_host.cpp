@@ -250,7 +250,6 @@ struct hk_scene {
     DevBuf b_film, b_rgb, b_scratch;   // scratch: work counter + counters
     std::vector<std::unique_ptr<DevBuf>> batch_films;   // films of hk_render_batch_host
     hk_scene_info info{};
-    int margin_lo = 0, margin_hi = 0;
     int sm_count = 148;
     int device = 0;   // CUDA device the scene was built on
     int image_form = HK_FORM_AUTO;             // form hk_render_image renders with
@@ -969,8 +968,6 @@ void build_scene(hk_scene *s) {
     if (D.border > 8) throw HkError{HK_ERR_INVALID, "reconstruction filter radius too large (max 8.5)"};
     for (int c = 0; c < 3; c++) D.background[c] = s->background[c];
     D.force_background = s->force_background;
-    s->margin_lo = (int)std::ceil(D.border - 0.5f - s->filt_r);
-    s->margin_hi = (int)std::floor(D.border + 0.5f + s->filt_r);
 
     // scratch: [0] work counter (u32 in a u64 slot), [1..3] counters
     s->b_scratch.alloc(16 * sizeof(unsigned long long));
@@ -981,7 +978,7 @@ void build_scene(hk_scene *s) {
     HK_CUDA(cudaGetDevice(&dev));
     s->device = dev;
     HK_CUDA(cudaDeviceGetAttribute(&s->sm_count, cudaDevAttrMultiProcessorCount, dev));
-    for (int a = 0; a < 2; ++a) s->occupancy_of[a] = std::max(1, hk::render_occupancy(s->margin_lo, s->margin_hi, a, D.textured != 0));
+    for (int a = 0; a < 2; ++a) s->occupancy_of[a] = std::max(1, hk::render_occupancy(a, D.textured != 0));
     s->occupancy = s->occupancy_of[D.accel];
     HK_CUDA(cudaGetLastError());
 
@@ -1381,6 +1378,12 @@ int hk_scene_get_info(const hk_scene *s, hk_scene_info *info) {
     });
 }
 
+// Blocks of a megakernel launch: one wave of resident ones, fewer where the paths need fewer lanes.
+static int render_grid(const hk_scene *s, int spp) {
+    const uint64_t paths = (uint64_t)s->width * s->height * (uint64_t)spp;
+    const uint64_t blocks = (paths + hk::kRenderThreads - 1) / hk::kRenderThreads;
+    return (int)std::max<uint64_t>(1, std::min<uint64_t>(blocks, (uint64_t)s->sm_count * s->occupancy));
+}
 int hk_render(hk_scene *s, const hk_render_desc *d, float *film, unsigned long long *counters, void *stream) {
     return guarded([&] {
         require_built(s);
@@ -1391,7 +1394,7 @@ int hk_render(hk_scene *s, const hk_render_desc *d, float *film, unsigned long l
         hk::RenderLaunch P;
         std::memset(&P, 0, sizeof P);
         P.film = film;
-        P.work_counter = (unsigned int *)s->b_scratch.p;
+        P.work_counter = (unsigned long long *)s->b_scratch.p;
         P.counters = counters;
         P.seed = d->seed;
         P.spp = d->spp;
@@ -1399,22 +1402,8 @@ int hk_render(hk_scene *s, const hk_render_desc *d, float *film, unsigned long l
         P.depth = d->depth;
         P.rr_start = d->rr_start;
         P.image_index = d->image_index;
-        P.tiles_x = ((int)s->width + hk::kTile - 1) / hk::kTile;
-        P.tiles_y = ((int)s->height + hk::kTile - 1) / hk::kTile;
-        const int tiles = P.tiles_x * P.tiles_y;
-        const int resident = s->sm_count * s->occupancy;
-        int per_item = d->spp_per_item;
-        if (per_item <= 0) {
-            int chunks = std::max(1, std::min(d->spp, (4 * resident + tiles - 1) / tiles));
-            per_item = (d->spp + chunks - 1) / chunks;
-        }
-        P.spp_per_item = per_item;
-        P.n_chunks = (d->spp + per_item - 1) / per_item;
-        P.n_items = tiles * P.n_chunks;
-        P.margin_lo = s->margin_lo;
-        P.margin_hi = s->margin_hi;
         HK_CUDA(cudaMemsetAsync(s->b_scratch.p, 0, sizeof(unsigned long long), st));
-        int grid = std::min(P.n_items, resident);
+        const int grid = render_grid(s, P.spp);
         if (d->use_camera) {
             hk::DevScene D = s->dev;   // per-call camera pose (passed by value with the launch)
             const float *M = d->camera_to_world;
@@ -1551,7 +1540,7 @@ int hk_render_image_static(hk_scene *s, const hk_render_desc *d, float *rgb_dev,
         hk::RenderLaunch P;
         std::memset(&P, 0, sizeof P);
         P.film = film;
-        P.work_counter = (unsigned int *)hdr;
+        P.work_counter = hdr;
         P.counters = hdr + 1;
         P.seed = d->seed;
         P.spp = d->spp;
@@ -1559,21 +1548,7 @@ int hk_render_image_static(hk_scene *s, const hk_render_desc *d, float *rgb_dev,
         P.depth = d->depth;
         P.rr_start = d->rr_start;
         P.image_index = d->image_index;
-        P.tiles_x = ((int)s->width + hk::kTile - 1) / hk::kTile;
-        P.tiles_y = ((int)s->height + hk::kTile - 1) / hk::kTile;
-        const int tiles = P.tiles_x * P.tiles_y;
-        const int resident = s->sm_count * s->occupancy;
-        int per_item = d->spp_per_item;
-        if (per_item <= 0) {
-            int chunks = std::max(1, std::min(d->spp, (4 * resident + tiles - 1) / tiles));
-            per_item = (d->spp + chunks - 1) / chunks;
-        }
-        P.spp_per_item = per_item;
-        P.n_chunks = (d->spp + per_item - 1) / per_item;
-        P.n_items = tiles * P.n_chunks;
-        P.margin_lo = s->margin_lo;
-        P.margin_hi = s->margin_hi;
-        const int grid = std::min(P.n_items, resident);
+        const int grid = render_grid(s, P.spp);
         hk::DevScene D = s->dev;
         if (d->use_camera) {
             const float *M = d->camera_to_world;

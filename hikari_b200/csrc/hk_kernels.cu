@@ -199,10 +199,9 @@ cudaError_t launch_env_eval(const DevScene &S, uint64_t n, const float *wi, floa
     env_eval_kernel<<<grid_for(n, 128), 128, 0, st>>>(S, n, wi, out, pdf);
     return cudaGetLastError();
 }
-int render_occupancy(int margin_lo, int margin_hi, int accel, bool textured) {
-    if (accel == kAccelBvh8)
-        return textured ? render_occupancy_t<kAccelBvh8, true>(margin_lo, margin_hi) : render_occupancy_t<kAccelBvh8, false>(margin_lo, margin_hi);
-    return textured ? render_occupancy_t<kAccelBvh2, true>(margin_lo, margin_hi) : render_occupancy_t<kAccelBvh2, false>(margin_lo, margin_hi);
+int render_occupancy(int accel, bool textured) {
+    if (accel == kAccelBvh8) return textured ? render_occupancy_t<kAccelBvh8, true>() : render_occupancy_t<kAccelBvh8, false>();
+    return textured ? render_occupancy_t<kAccelBvh2, true>() : render_occupancy_t<kAccelBvh2, false>();
 }
 
 }  // namespace hk

@@ -3,5 +3,5 @@
 
 namespace hk {
 template cudaError_t launch_render_t<kAccelBvh2, false>(const DevScene &, const RenderLaunch &, int, cudaStream_t);
-template int render_occupancy_t<kAccelBvh2, false>(int, int);
+template int render_occupancy_t<kAccelBvh2, false>();
 }  // namespace hk

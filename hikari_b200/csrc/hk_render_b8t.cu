@@ -3,5 +3,5 @@
 
 namespace hk {
 template cudaError_t launch_render_t<kAccelBvh8, true>(const DevScene &, const RenderLaunch &, int, cudaStream_t);
-template int render_occupancy_t<kAccelBvh8, true>(int, int);
+template int render_occupancy_t<kAccelBvh8, true>();
 }  // namespace hk

@@ -451,4 +451,47 @@ __device__ __forceinline__ void camera_diff(const DevScene &S, const float *M, u
             M[8] * b.x + M[9] * b.y + M[10] * b.z);
 }
 
+// ------------------------------------------------------------ sample streams and film
+// Seed of sample s of a render seeded `seed` (splitmix64); the pcg32 sequence
+// is the pixel's, so an image depends on neither the work split nor the form.
+__device__ __forceinline__ uint64_t mix_seed(uint64_t seed, uint64_t s) {
+    uint64_t z = seed + 0x9E3779B97F4A7C15ULL * (s + 1);
+    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ULL;
+    z = (z ^ (z >> 27)) * 0x94D049BB133111EBULL;
+    return z ^ (z >> 31);
+}
+__device__ __forceinline__ void red_add_v4(float4 *addr, float a, float b, float c, float d) {
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(a), "f"(b), "f"(c), "f"(d)
+                 : "memory");
+}
+// ImageBlock::Put (src/core/Block.cpp:95) into a film of a width x height image
+// with one 128-bit reduction per filter tap (scalar ones where the caller's
+// film is not 16-byte aligned).
+__device__ __forceinline__ void splat_film(const DevScene &S, float *film, int width, int height, float px, float py,
+                                           V3 val) {
+    const int B = S.border, FW = width + 2 * B, FH = height + 2 * B;
+    const float cx = px - 0.5f - (0 - B), cy = py - 0.5f - (0 - B);
+    const int x0 = max((int)ceilf(cx - S.filt_radius), 0), y0 = max((int)ceilf(cy - S.filt_radius), 0);
+    const int x1 = min((int)floorf(cx + S.filt_radius), FW - 1), y1 = min((int)floorf(cy + S.filt_radius), FH - 1);
+    const bool aligned = (reinterpret_cast<size_t>(film) & 15) == 0;
+    for (int y = y0; y <= y1; ++y) {
+        const float wy = __ldg(S.ftab + (int)(fabsf((float)y - cy) * S.filt_lookup));
+        for (int x = x0; x <= x1; ++x) {
+            const float wx = __ldg(S.ftab + (int)(fabsf((float)x - cx) * S.filt_lookup));
+            const float w = wx * wy;
+            if (w == 0.0f) continue;
+            float *c = film + 4 * ((size_t)y * FW + x);
+            const float r = (val.x * wx) * wy, g = (val.y * wx) * wy, b = (val.z * wx) * wy;
+            if (aligned) {
+                red_add_v4(reinterpret_cast<float4 *>(c), r, g, b, w);
+            } else {
+                atomicAdd(c, r);
+                atomicAdd(c + 1, g);
+                atomicAdd(c + 2, b);
+                atomicAdd(c + 3, w);
+            }
+        }
+    }
+}
+
 }  // namespace hk

@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(256) wf_regen_kernel(DevScene S, WfState W, in
                 const int pj = __float_as_int(p.z);
                 const WfJob &J = W.jobs[pj];
                 V3 val = v3(L.x, L.y, L.z);
-                if (is_valid(val)) splat_global(S, J, p.x, p.y, val);
+                if (is_valid(val)) splat_film(S, J.film, (int)J.width, (int)J.height, p.x, p.y, val);
                 else ++dropped;
                 atomicAdd(&s_finished[pj], 1u);
                 --active_delta;
@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(256) wf_regen_kernel(DevScene S, WfState W, in
                     atomicAdd(&s_finished[j], 1u);   // counted as work done: no path
                 } else {
                     Pcg32 rng;
-                    rng.seed(wf_mix_seed(J.seed, (uint64_t)J.sample_offset + s),
+                    rng.seed(mix_seed(J.seed, (uint64_t)J.sample_offset + s),
                              (uint64_t)y * J.width + x + (uint64_t)J.image_index * J.width * J.height);
                     float px = (float)x + rng.nextf(), py = (float)y + rng.nextf();
                     Ray r = camera_ray_job(S, J, px, py);

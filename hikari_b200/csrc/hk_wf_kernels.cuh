@@ -33,10 +33,6 @@ __device__ __forceinline__ unsigned warp_append_keyed(unsigned *counters, int ke
     base = __shfl_sync(peers, base, leader);
     return base + rank;
 }
-__device__ __forceinline__ void red_add_v4(float4 *addr, float a, float b, float c, float d) {
-    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(a), "f"(b), "f"(c), "f"(d)
-                 : "memory");
-}
 __device__ __forceinline__ float4 f4(V3 v, float w) { return make_float4(v.x, v.y, v.z, w); }
 
 // PerspectiveCamera::SampleRay (src/camera/PerspectiveCamera.cpp:71) at the
@@ -57,13 +53,6 @@ __device__ __forceinline__ Ray camera_ray_job(const DevScene &S, const WfJob &J,
     return r;
 }
 
-__device__ __forceinline__ uint64_t wf_mix_seed(uint64_t seed, uint64_t s) {
-    uint64_t z = seed + 0x9E3779B97F4A7C15ULL * (s + 1);
-    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ULL;
-    z = (z ^ (z >> 27)) * 0x94D049BB133111EBULL;
-    return z ^ (z >> 31);
-}
-
 // Piece of the current plan that holds plan item w (pieces are sorted by plan_begin).
 __device__ __forceinline__ int find_seg(const WfState &W, uint64_t w, int nseg) {
     int lo = 0, hi = nseg - 1;
@@ -74,24 +63,6 @@ __device__ __forceinline__ int find_seg(const WfState &W, uint64_t w, int nseg) 
     return lo;
 }
 
-// ImageBlock::Put into the job's global film with vector reductions.
-__device__ __forceinline__ void splat_global(const DevScene &S, const WfJob &J, float px, float py, V3 val) {
-    const int B = S.border, FW = (int)J.width + 2 * B, FH = (int)J.height + 2 * B;
-    float *film = J.film;
-    float cx = px - 0.5f - (0 - B), cy = py - 0.5f - (0 - B);
-    int x0 = max((int)ceilf(cx - S.filt_radius), 0), y0 = max((int)ceilf(cy - S.filt_radius), 0);
-    int x1 = min((int)floorf(cx + S.filt_radius), FW - 1), y1 = min((int)floorf(cy + S.filt_radius), FH - 1);
-    float4 *F = reinterpret_cast<float4 *>(film);
-    for (int y = y0; y <= y1; ++y) {
-        float wy = __ldg(S.ftab + (int)(fabsf((float)y - cy) * S.filt_lookup));
-        for (int x = x0; x <= x1; ++x) {
-            float wx = __ldg(S.ftab + (int)(fabsf((float)x - cx) * S.filt_lookup));
-            float w = wx * wy;
-            if (w == 0.0f) continue;
-            red_add_v4(F + (size_t)y * FW + x, (val.x * wx) * wy, (val.y * wx) * wy, (val.z * wx) * wy, w);
-        }
-    }
-}
 // ------------------------------------------------------------ shade
 __device__ __forceinline__ void finish(const WfState &W, int slot) { W.fq[warp_append(&W.ctr->fq_count)] = slot; }
 
