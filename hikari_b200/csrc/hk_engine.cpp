@@ -8,13 +8,14 @@
 namespace hk {
 
 namespace {
-constexpr int kQueueArrays = 2 /*eq*/ + 2 /*idle*/ + kWfTypes /*sq*/ + 1 /*fq*/;
+// queue arrays of one slot id per slot: 2 extend, 2 idle, the scene's shade queues, 1 finished
+int queue_arrays(uint32_t shade_queues) { return 5 + __builtin_popcount(shade_queues); }
 }  // namespace
 
-size_t WfEngine::bytes_for(int capacity, int nemitters) {
+size_t WfEngine::bytes_for(int capacity, int nemitters, uint32_t shade_queues) {
     const size_t N = (size_t)capacity;
     const size_t shadow = N * (size_t)std::max(1, nemitters);
-    return N * kSlotBytes + N * sizeof(int) * kQueueArrays + shadow * 16 * 3 + sizeof(WfCounters) +
+    return N * kSlotBytes + N * sizeof(int) * queue_arrays(shade_queues) + shadow * 16 * 3 + sizeof(WfCounters) +
            (sizeof(WfJob) + sizeof(unsigned long long)) * kWfMaxJobs + sizeof(WfSeg) * kWfMaxSegs;
 }
 
@@ -28,13 +29,13 @@ WfEngine::WfEngine(const DevScene &S, int sm_count, const WfEngineConfig &cfg) :
     W_.capacity = cfg_.capacity;
     W_.max_shadow = cfg_.capacity * std::max(1, S.nemitters);
     state_.alloc(N * kSlotBytes);
-    queues_.alloc(N * sizeof(int) * kQueueArrays);
+    queues_.alloc(N * sizeof(int) * queue_arrays(S.shade_queues));
     shadow_.alloc((size_t)W_.max_shadow * 16 * 3);
     counters_.alloc(sizeof(WfCounters));
     jobs_.alloc(sizeof(WfJob) * kWfMaxJobs);
     finished_.alloc(sizeof(unsigned long long) * kWfMaxJobs);
     segs_.alloc(sizeof(WfSeg) * kWfMaxSegs);
-    bytes_ = bytes_for(cfg_.capacity, S.nemitters);
+    bytes_ = bytes_for(cfg_.capacity, S.nemitters, S.shade_queues);
     char *rec = state_.as<char>();   // slot records (kSlotBytes each, 256-byte aligned base)
     W_.ray_o.p = (float4 *)(rec + 0);
     W_.ray_d.p = (float4 *)(rec + 16);
@@ -47,8 +48,10 @@ WfEngine::WfEngine(const DevScene &S, int sm_count, const WfEngineConfig &cfg) :
     int *q = queues_.as<int>();
     W_.eq[0] = q; W_.eq[1] = q + N;
     W_.idle[0] = q + 2 * N; W_.idle[1] = q + 3 * N;
-    for (int t = 0; t < kWfTypes; ++t) W_.sq[t] = q + (4 + t) * N;
-    W_.fq = q + (4 + kWfTypes) * N;
+    W_.fq = q + 4 * N;
+    q += 5 * N;
+    for (int t = 0; t < kWfTypes; ++t)
+        if (S.shade_queues >> t & 1u) { W_.sq[t] = q; q += N; }
     float4 *sh = shadow_.as<float4>();
     W_.sh_o = sh; W_.sh_d = sh + W_.max_shadow; W_.sh_c = sh + 2 * (size_t)W_.max_shadow;
     W_.ctr = counters_.as<WfCounters>();

@@ -222,7 +222,7 @@ void hk_server::admit(const std::vector<SceneEntry *> &sc) {
         Job *j = queued.front();
         SceneEntry &e = *sc[j->scene];
         const uint64_t need = j->size.film_bytes + j->size.rgb_bytes;
-        const uint64_t pool = e.eng ? 0 : hk::WfEngine::bytes_for(ec.capacity, e.view.dev->nemitters);
+        const uint64_t pool = e.eng ? 0 : hk::WfEngine::bytes_for(ec.capacity, e.view.dev->nemitters, e.view.dev->shade_queues);
         uint64_t used;
         {
             std::lock_guard<std::mutex> lk(mu);

@@ -53,15 +53,29 @@ HK_WF_SHADE_EXTERN(6);
 HK_WF_SHADE_EXTERN(7);
 HK_WF_SHADE_EXTERN(8);
 HK_WF_SHADE_EXTERN(9);
-HK_WF_SHADE_EXTERN(10);
 HK_WF_SHADE_EXTERN(11);
 HK_WF_SHADE_EXTERN(12);
 HK_WF_SHADE_EXTERN(13);
 HK_WF_SHADE_EXTERN(14);
 HK_WF_SHADE_EXTERN(15);
 HK_WF_SHADE_EXTERN(16);
+HK_WF_SHADE_EXTERN(17);
+HK_WF_SHADE_EXTERN(18);
+HK_WF_SHADE_EXTERN(19);
+HK_WF_SHADE_EXTERN(20);
+HK_WF_SHADE_EXTERN(21);
+HK_WF_SHADE_EXTERN(23);
+HK_WF_SHADE_EXTERN(24);
+HK_WF_SHADE_EXTERN(25);
+HK_WF_SHADE_EXTERN(26);
+HK_WF_SHADE_EXTERN(27);
+HK_WF_SHADE_EXTERN(28);
+HK_WF_SHADE_EXTERN(29);
+HK_WF_SHADE_EXTERN(30);
 #undef HK_WF_SHADE_EXTERN
-static_assert(kWfTypes == 17, "one shade kernel per queue");
+static_assert(kWfTypes == 31, "one shade kernel per queue");
+// 10 and 22 (twoSided) have no kernel of their own: wf_queue_of sends them to the generic queue.
+constexpr bool has_shade_kernel(int q) { return q != 1 + kTwoSided && q != kWfTexturedQueue0 + kTwoSided; }
 
 // ------------------------------------------------------------ regen
 // Splat and retire the finished paths, then give finished and idle slots new
@@ -256,9 +270,11 @@ static cudaError_t launch_shadow(const DevScene &S, const WfState &W, const WfLa
 template <int kType>
 struct ShadeLaunch {
     static void run(const DevScene &S, const WfState &W, const WfLaunchConfig &C, int nxt, cudaStream_t st, int &k) {
-        if (C.shade_queues >> kType & 1u) {
-            const int lane = k++ % (C.nfork + 1);
-            wf_launch_shade_t<kType>(S, W, C, nxt, lane == 0 ? st : C.fork[lane - 1]);
+        if constexpr (has_shade_kernel(kType)) {
+            if (C.shade_queues >> kType & 1u) {
+                const int lane = k++ % (C.nfork + 1);
+                wf_launch_shade_t<kType>(S, W, C, nxt, lane == 0 ? st : C.fork[lane - 1]);
+            }
         }
         if constexpr (kType + 1 < kWfTypes) ShadeLaunch<kType + 1>::run(S, W, C, nxt, st, k);
     }
@@ -321,7 +337,9 @@ int wf_occupancy(int which, int threads, int accel, bool lean) {
 }
 template <int kType>
 static int shade_occupancy(int queue, int threads, bool lean) {
-    if (queue == kType) return wf_shade_occupancy_t<kType>(threads, lean);
+    if constexpr (has_shade_kernel(kType)) {
+        if (queue == kType) return wf_shade_occupancy_t<kType>(threads, lean);
+    }
     if constexpr (kType + 1 < kWfTypes) return shade_occupancy<kType + 1>(queue, threads, lean);
     return 0;
 }

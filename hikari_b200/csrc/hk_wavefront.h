@@ -18,26 +18,26 @@
 
 namespace hk {
 
-// Shade queues: 0 miss; 1..5 the rough BSDF types without textures (type +
-// 1), each shaded by a kernel compiled for that type with texture lookups
-// compiled out; 6 the smooth, twoSided, bump- and normal-mapped BSDFs, shaded
-// by one kernel that dispatches at run time; 7..11 the rough BSDF types with
-// textured parameters (type + 7), each shaded by a kernel compiled for that
-// type with texture lookups.
-constexpr int kWfGenericQueue = 6;
-constexpr int kWfTexturedQueue0 = 7;
-constexpr int kWfBumpQueue0 = kWfTexturedQueue0 + kRoughCoating + 1;   // bumpMap / normalMap over a rough type
-constexpr int kWfTypes = kWfBumpQueue0 + kRoughCoating + 1;
-// Shade queue of a hit's top-level BSDF: 0 the miss queue; 1-5 the rough types
-// without textures; 7-11 the same with textures; 12-16 bumpMap / normalMap
-// wrapping a rough type (nested_type); 6 everything else (smooth BSDFs,
-// twoSided, maps over them), dispatched at run time.
+// Shade queues, one kernel each: 0 the misses; 1 + type the BSDF types without
+// textures, each compiled for that type with texture lookups compiled out;
+// 13 + type the same with textured parameters and lookups; 25 + type a bumpMap
+// or normalMap over a rough type; 30 the rest, dispatched at run time: deep
+// stacks of layers, twoSided BSDFs and maps over the smooth types.  A mirror
+// that shared the run-time-dispatched kernel paid for the calls, the 1.4 KB of
+// stack and the divergence of every type: 2.2 ns a vertex in the Cornell box of
+// smooth materials, where a diffuse vertex takes 0.2.
+constexpr int kWfLeafTypes = kRoughDiffuse + 1;
+constexpr int kWfTexturedQueue0 = 1 + kWfLeafTypes;
+constexpr int kWfBumpQueue0 = kWfTexturedQueue0 + kWfLeafTypes;   // bumpMap / normalMap over a rough type
+constexpr int kWfGenericQueue = kWfBumpQueue0 + kRoughCoating + 1;
+constexpr int kWfTypes = kWfGenericQueue + 1;
+// Shade queue of a top-level BSDF type (nested_type: what a map wraps).
 __host__ __device__ constexpr int wf_queue_of(int bsdf_type, bool textured = false, int nested_type = -1) {
-    return bsdf_type <= kRoughCoating
-               ? (textured ? kWfTexturedQueue0 + bsdf_type : bsdf_type + 1)
-               : ((bsdf_type == kBumpMap || bsdf_type == kNormalMap) && nested_type >= 0 && nested_type <= kRoughCoating
-                      ? kWfBumpQueue0 + nested_type
-                      : kWfGenericQueue);
+    return bsdf_type == kTwoSided
+               ? kWfGenericQueue
+               : (bsdf_type <= kRoughDiffuse
+                      ? (textured ? kWfTexturedQueue0 : 1) + bsdf_type
+                      : (nested_type >= 0 && nested_type <= kRoughCoating ? kWfBumpQueue0 + nested_type : kWfGenericQueue));
 }
 // Shade queue of BSDF id: deep stacks of layers (and maps over them) are
 // dispatched at run time whatever their top-level type.

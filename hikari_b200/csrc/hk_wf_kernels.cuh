@@ -103,12 +103,12 @@ __global__ void __launch_bounds__(256, kMinBlocks) wf_shade_kernel(DevScene S, W
             // kBumpQ: a bumpMap / normalMap over the rough type BT (the
             // records move through the perturbed frame, the nested BSDF is
             // evaluated with its type compiled in)
-            constexpr bool kBumpQ = kType >= kWfBumpQueue0;
+            constexpr bool kBumpQ = kType >= kWfBumpQueue0 && kType != kWfGenericQueue;
             constexpr int BT = kType == kWfGenericQueue
                                    ? -1
                                    : (kBumpQ ? kType - kWfBumpQueue0
                                              : (kType >= kWfTexturedQueue0 ? kType - kWfTexturedQueue0 : kType - 1));
-            constexpr bool kTexQ = kType >= kWfGenericQueue;
+            constexpr bool kTexQ = kType >= kWfTexturedQueue0;
             uint4 rs = W.rng[slot];
             Pcg32 rng;
             rng.state = (uint64_t)rs.x | ((uint64_t)rs.y << 32);

@@ -1,4 +1,4 @@
-// Wavefront shade kernels: queue 5 (roughCoating).
+// Wavefront shade kernels: queues 5 (roughCoating).
 #include "hk_wf_kernels.cuh"
 
 namespace hk {
