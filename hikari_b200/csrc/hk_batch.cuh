@@ -25,11 +25,13 @@ __global__ void bsdf_batch_kernel(DevScene S, int bsdf, uint64_t n, const float 
         r.tv = kTex ? uv[2 * i + 1] : 0.0f;
         r.duv = (kTex && duv) ? make_float4(duv[4 * i], duv[4 * i + 1], duv[4 * i + 2], duv[4 * i + 3])
                               : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        V3 w = bsdf_sample_t<BT>(S.bsdfs, bsdf, r, u2[2 * i], u2[2 * i + 1], u1 ? u1[i] : 0.0f);
+        const BsdfVertex bv = bsdf_vertex_t<BT>(S.bsdfs, bsdf, r);
+        float spdf;
+        V3 w = bsdf_sample_pdf_t<BT>(S.bsdfs, bsdf, r, u2[2 * i], u2[2 * i + 1], u1 ? u1[i] : 0.0f, bv, s_pdf != nullptr, spdf);
         if (s_wo) { s_wo[3 * i] = r.wo.x; s_wo[3 * i + 1] = r.wo.y; s_wo[3 * i + 2] = r.wo.z; }
         if (s_w) { s_w[3 * i] = w.x; s_w[3 * i + 1] = w.y; s_w[3 * i + 2] = w.z; }
         if (s_m) s_m[i] = r.measure;
-        if (s_pdf) s_pdf[i] = all_zero(w) ? 0.0f : bsdf_pdf_t<BT>(S.bsdfs, bsdf, r);
+        if (s_pdf) s_pdf[i] = all_zero(w) ? 0.0f : spdf;
         BRec q;
         q.wi = r.wi;
         q.wo = v3(wo[3 * i], wo[3 * i + 1], wo[3 * i + 2]);
@@ -39,11 +41,12 @@ __global__ void bsdf_batch_kernel(DevScene S, int bsdf, uint64_t n, const float 
         q.tu = r.tu;
         q.tv = r.tv;
         q.duv = r.duv;
-        if (e_rgb) {
-            V3 e = bsdf_eval_t<BT>(S.bsdfs, bsdf, q);
-            e_rgb[3 * i] = e.x; e_rgb[3 * i + 1] = e.y; e_rgb[3 * i + 2] = e.z;
+        if (e_rgb || p_pdf) {
+            float pdf;
+            const V3 e = bsdf_eval_pdf_t<BT>(S.bsdfs, bsdf, q, bv, pdf);
+            if (e_rgb) { e_rgb[3 * i] = e.x; e_rgb[3 * i + 1] = e.y; e_rgb[3 * i + 2] = e.z; }
+            if (p_pdf) p_pdf[i] = pdf;
         }
-        if (p_pdf) p_pdf[i] = bsdf_pdf_t<BT>(S.bsdfs, bsdf, q);
     }
 }
 

@@ -58,8 +58,8 @@ __device__ __forceinline__ float mfd_project_roughness(const Mfd &d, V3 v) {   /
     float c2 = v.x * v.x * inv, s2 = v.y * v.y * inv;
     return sqrtf(c2 * d.au * d.au + s2 * d.av * d.av);
 }
-__device__ __forceinline__ float mfd_g1(const Mfd &d, V3 v, V3 m) {   // SmithG1 :82
-    if (dot(v, m) * v.z <= 0.0f) return 0.0f;
+// SmithG1 (:82) past its test of m's side, which is all that m enters
+__device__ __forceinline__ float mfd_g1_of(const Mfd &d, V3 v) {
     float tt = fabsf(tan_theta(v));
     if (tt == 0.0f) return 1.0f;
     float a = mfd_project_roughness(d, v);
@@ -72,6 +72,11 @@ __device__ __forceinline__ float mfd_g1(const Mfd &d, V3 v, V3 m) {   // SmithG1
     float root = a * tt;
     return 2.0f / (1.0f + hypot2(1.0f, root));
 }
+__device__ __forceinline__ float mfd_g1(const Mfd &d, V3 v, V3 m) {
+    return dot(v, m) * v.z <= 0.0f ? 0.0f : mfd_g1_of(d, v);
+}
+// mfd_g1 with mfd_g1_of(d, v) at hand
+__device__ __forceinline__ float mfd_g1_with(float g1, V3 v, V3 m) { return dot(v, m) * v.z <= 0.0f ? 0.0f : g1; }
 __device__ __forceinline__ float mfd_g(const Mfd &d, V3 wi, V3 wo, V3 m) { return mfd_g1(d, wi, m) * mfd_g1(d, wo, m); }
 __device__ __forceinline__ V3 mfd_sample(const Mfd &d, float ux, float uy, float &pdf) {   // SampleAll :148
     float sp, cp, a2;
@@ -517,6 +522,24 @@ __device__ __forceinline__ float conductor_pdf(const DevBsdf &b, const BRec &r) 
     return mfd_pdf(d, h) / (4.0f * fabsf(dot(h, r.wo)));
 }
 
+// Eval and Pdf of one record under ESolidAngle in one pass: the half vector and
+// D are formed once, G1 of wi comes from the caller.  Products and sums are
+// those of conductor_eval and conductor_pdf, so are the results' bits.
+__device__ __forceinline__ V3 conductor_eval_pdf(const DevBsdf &b, const BRec &r, float g1_wi, float &pdf) {
+    const float ci = r.wi.z, co = r.wo.z;
+    pdf = 0.0f;
+    if (ci <= 0.0f || co <= 0.0f) return v3(0, 0, 0);
+    const V3 h = normalize(r.wi + r.wo);
+    const Mfd d = bsdf_mfd(b, r);
+    const float D = mfd_eval(d, h);
+    pdf = (D * h.z) / (4.0f * fabsf(dot(h, r.wo)));
+    if (D == 0.0f) return v3(0, 0, 0);
+    const V3 F = conductor_fresnel(b, dot(h, r.wi)) * par_rgb(b, 1, b.ks, r);
+    const float G = mfd_g1_with(g1_wi, r.wi, h) * mfd_g1(d, r.wo, h);
+    const float dg = D * G, den = 4.0f * ci;
+    return v3(dg * F.x / den, dg * F.y / den, dg * F.z / den);
+}
+
 // ------------------------------------------------------------ roughDielectric
 // src/bsdf/RoughDielectricBSDF.cpp:57-281.  u1 is the Next1D draw the
 // reference takes from the record's sampler inside Sample (:92).
@@ -598,27 +621,62 @@ __device__ __forceinline__ float dielectric_pdf(const DevBsdf &b, const BRec &r)
     return fabsf(pdf * J);
 }
 
+// Eval and Pdf of one record under ESolidAngle in one pass (see conductor_eval_pdf)
+__device__ __forceinline__ V3 dielectric_eval_pdf(const DevBsdf &b, const BRec &r, float g1_wi, float &pdf) {
+    const float ci = r.wi.z, co = r.wo.z;
+    pdf = 0.0f;
+    if (ci == 0.0f) return v3(0, 0, 0);
+    const bool refl = ci * co > 0.0f;
+    const float e = ci > 0.0f ? b.eta : b.inv_eta;
+    const V3 h0 = refl ? normalize(r.wi + r.wo) : normalize(r.wi + r.wo * e);
+    const V3 h = h0 * signum(h0.z);
+    const Mfd d = bsdf_mfd(b, r);
+    float ct;
+    const float F = fresnel_dielectric(dot(r.wi, h), b.eta, b.inv_eta, ct);
+    if (co != 0.0f) {
+        float J;
+        if (refl) {
+            J = 1.0f / (4.0f * dot(r.wo, h0));
+        } else {
+            const float sd = dot(r.wi, h0) + e * dot(r.wo, h0);
+            J = (e * e * dot(r.wo, h0)) / (sd * sd);
+        }
+        Mfd ds = d;
+        const float s = 1.2f - 0.2f * sqrtf(fabsf(ci));
+        ds.au *= s;
+        ds.av *= s;
+        const float pm = mfd_pdf(ds, h) * (refl ? F : (1.0f - F));
+        pdf = fabsf(pm * J);
+    }
+    const float D = mfd_eval(d, h);
+    if (D == 0.0f) return v3(0, 0, 0);
+    const float G = mfd_g1_with(g1_wi, r.wi, h) * mfd_g1(d, r.wo, h);
+    if (refl) return par_rgb(b, 1, b.ks, r) * (F * D * G / (4.0f * fabsf(ci)));
+    const float sd = dot(r.wi, h) + e * dot(r.wo, h);
+    const float val = ((1.0f - F) * D * G * e * e * dot(r.wi, h) * dot(r.wo, h)) / (ci * sd * sd);
+    const float fac = (ci < 0.0f ? b.inv_eta : b.eta);
+    return par_rgb(b, 2, b.ks_refract, r) * fabsf(val * fac * fac);
+}
+
 // ------------------------------------------------------------ roughPlastic
 // The roughness of roughPlastic / roughCoating: the activated constant, or the
 // texture's first channel clamped to [5e-4, 1] (RoughPlasticBSDF.cpp:77)
 __device__ __forceinline__ float coat_alpha(const DevBsdf &b, const BRec &r) {
     return b.alpha_tex ? clampf(par_alpha(b, 4, b.alpha_u, r), 5e-4f, 1.0f) : b.alpha_u;
 }
-// src/bsdf/RoughPlasticBSDF.cpp:66-192
-__device__ __forceinline__ V3 plastic_eval(const DevBsdf &b, const BRec &r) {
-    float ci = r.wi.z, co = r.wo.z;
-    if (r.measure == kMeasureUnknown || ci <= 0.0f || co <= 0.0f) return v3(0, 0, 0);
-    const float a = coat_alpha(b, r);
-    Mfd d = mfd_make(b.distribution, a, a);
+// src/bsdf/RoughPlasticBSDF.cpp:66-192.  h, D: the half vector and D at it;
+// t_ci: rft_eval at wi; g1_wi: mfd_g1_of wi; past the tests of Eval.
+__device__ __forceinline__ V3 plastic_value(const DevBsdf &b, const BRec &r, const Mfd &d, V3 h, float D, float t_ci,
+                                            float g1_wi) {
+    const float ci = r.wi.z, co = r.wo.z;
     float ct;
-    V3 h = normalize(r.wi + r.wo);
-    float D = mfd_eval(d, h);
-    float F = fresnel_dielectric(dot(r.wi, h), b.eta, b.inv_eta, ct);
-    float G = mfd_g(d, r.wi, r.wi, h);   // G(Wi, Wi, H) as the reference does (:146)
+    const float F = fresnel_dielectric(dot(r.wi, h), b.eta, b.inv_eta, ct);
+    const float g1 = mfd_g1_with(g1_wi, r.wi, h);
+    const float G = g1 * g1;   // G(Wi, Wi, H) as the reference does (:146)
     float val = F * D * G / (4.0f * ci);
     V3 res = par_rgb(b, 1, b.ks, r) * val;
     V3 dif = par_rgb(b, 0, b.kd, r);
-    float t12 = rft_eval(b, ci, d.au), t21 = rft_eval(b, co, d.au);
+    float t12 = t_ci, t21 = rft_eval(b, co, d.au);
     float fdr = plastic_fdr(b, d.au);
     if (b.nonlinear) dif = v3(dif.x / (1.0f - dif.x * fdr), dif.y / (1.0f - dif.y * fdr), dif.z / (1.0f - dif.z * fdr));
     else dif = dif / (1.0f - fdr);
@@ -626,34 +684,56 @@ __device__ __forceinline__ V3 plastic_eval(const DevBsdf &b, const BRec &r) {
     float k = (float)(kInvPiD * co * t12 * t21 * b.inv_eta2);
     return res + dif * k;
 }
-__device__ __forceinline__ float plastic_spec_pdf(const DevBsdf &b, float ci, float alpha) {
-    float sp = 1.0f - rft_eval(b, ci, alpha);
+__device__ __forceinline__ Mfd coat_mfd(const DevBsdf &b, const BRec &r) {
+    const float a = coat_alpha(b, r);
+    return mfd_make(b.distribution, a, a);
+}
+__device__ __forceinline__ V3 plastic_eval(const DevBsdf &b, const BRec &r) {
+    if (r.measure == kMeasureUnknown || r.wi.z <= 0.0f || r.wo.z <= 0.0f) return v3(0, 0, 0);
+    const Mfd d = coat_mfd(b, r);
+    const V3 h = normalize(r.wi + r.wo);
+    return plastic_value(b, r, d, h, mfd_eval(d, h), rft_eval(b, r.wi.z, d.au), mfd_g1_of(d, r.wi));
+}
+// Specular sampling weight, t_ci: rft_eval at wi
+__device__ __forceinline__ float coat_spec_pdf(const DevBsdf &b, float t_ci) {
+    float sp = 1.0f - t_ci;
     return (sp * b.spec_w) / (sp * b.spec_w + (1.0f - sp) * (1.0f - b.spec_w));
 }
-__device__ __forceinline__ float plastic_pdf(const DevBsdf &b, const BRec &r) {
-    float ci = r.wi.z, co = r.wo.z;
-    if (r.measure == kMeasureUnknown || ci <= 0.0f || co <= 0.0f) return 0.0f;
-    const float a = coat_alpha(b, r);
-    Mfd d = mfd_make(b.distribution, a, a);
-    V3 h = normalize(r.wi + r.wo);
-    float sp = plastic_spec_pdf(b, ci, d.au), dp = 1.0f - sp;
-    float J = 1.0f / (4.0f * dot(r.wo, h));
-    float res = mfd_pdf(d, h) * J * sp;
-    res += dp * cos_hemi_pdf(r.wo);
-    return res;
+// Pdf past its tests
+__device__ __forceinline__ float plastic_density(const BRec &r, V3 h, float D, float sp) {
+    const float dp = 1.0f - sp;
+    const float J = 1.0f / (4.0f * dot(r.wo, h));
+    return (D * h.z) * J * sp + dp * cos_hemi_pdf(r.wo);
 }
-__device__ __forceinline__ V3 plastic_sample(const DevBsdf &b, BRec &r, float ux, float uy) {
+__device__ __forceinline__ float plastic_pdf(const DevBsdf &b, const BRec &r) {
+    if (r.measure == kMeasureUnknown || r.wi.z <= 0.0f || r.wo.z <= 0.0f) return 0.0f;
+    const Mfd d = coat_mfd(b, r);
+    const V3 h = normalize(r.wi + r.wo);
+    return plastic_density(r, h, mfd_eval(d, h), coat_spec_pdf(b, rft_eval(b, r.wi.z, d.au)));
+}
+__device__ __forceinline__ V3 plastic_eval_pdf(const DevBsdf &b, const BRec &r, float g1_wi, float t_ci, float &pdf) {
+    pdf = 0.0f;
+    if (r.wi.z <= 0.0f || r.wo.z <= 0.0f) return v3(0, 0, 0);
+    const Mfd d = coat_mfd(b, r);
+    const V3 h = normalize(r.wi + r.wo);
+    const float D = mfd_eval(d, h);
+    pdf = plastic_density(r, h, D, coat_spec_pdf(b, t_ci));
+    return plastic_value(b, r, d, h, D, t_ci, g1_wi);
+}
+// pdf: that of the sampled direction, as plastic_pdf gives it
+__device__ __forceinline__ V3 plastic_sample(const DevBsdf &b, BRec &r, float ux, float uy, float g1_wi, float t_ci,
+                                             float &pdf) {
+    pdf = 0.0f;
     float ci = r.wi.z;
     if (ci <= 0.0f) return v3(0, 0, 0);
-    const float a = coat_alpha(b, r);
-    Mfd d = mfd_make(b.distribution, a, a);
-    float sp = plastic_spec_pdf(b, ci, d.au), dp = 1.0f - sp;
+    const Mfd d = coat_mfd(b, r);
+    const float sp = coat_spec_pdf(b, t_ci);
     bool spec;
     if (uy < sp) { uy /= sp; spec = true; }
     else { uy = (uy - sp) / (1.0f - sp); spec = false; }
     if (spec) {
-        float pdf;
-        V3 m = mfd_sample(d, ux, uy, pdf);
+        float mp;
+        V3 m = mfd_sample(d, ux, uy, mp);
         r.wo = reflect_m(r.wi, m);
         r.measure = kMeasureDiscrete;
     } else {
@@ -662,10 +742,18 @@ __device__ __forceinline__ V3 plastic_sample(const DevBsdf &b, BRec &r, float ux
     }
     r.eta = 1.0f;
     V3 h = normalize(r.wi + r.wo);
-    float J = 1.0f / (4.0f * dot(r.wo, h));
-    float P = mfd_pdf(d, h) * J * sp + dp * cos_hemi_pdf(r.wo);
+    const float D = mfd_eval(d, h);
+    const float P = plastic_density(r, h, D, sp);
     if (P == 0.0f) return v3(0, 0, 0);
-    return plastic_eval(b, r) / P;
+    if (r.wo.z <= 0.0f) return v3(0, 0, 0) / P;
+    pdf = P;
+    return plastic_value(b, r, d, h, D, t_ci, g1_wi) / P;
+}
+__device__ __forceinline__ V3 plastic_sample(const DevBsdf &b, BRec &r, float ux, float uy) {
+    if (r.wi.z <= 0.0f) return v3(0, 0, 0);
+    const Mfd d = coat_mfd(b, r);
+    float pdf;
+    return plastic_sample(b, r, ux, uy, mfd_g1_of(d, r.wi), rft_eval(b, r.wi.z, d.au), pdf);
 }
 
 // ------------------------------------------------------------ smooth BSDFs
@@ -923,24 +1011,40 @@ __device__ __forceinline__ V3 coat_refract(V3 wi, float inv_eta) {   // RefractI
     float ct = sqrtf(1.0f - st2);
     return v3(inv_eta * wi.x, inv_eta * wi.y, entering ? ct : -ct);
 }
-__device__ __forceinline__ V3 coating_eval(const DevBsdf &b, const DevBsdf &nb, const BRec &r) {
-    float ci = r.wi.z, co = r.wo.z;
-    if (ci * co <= 0.0f) return v3(0, 0, 0);
-    const float a = coat_alpha(b, r);
-    Mfd d = mfd_make(b.distribution, a, a);
-    V3 h = normalize(r.wi + r.wo) * signum(r.wo.z);
-    float ct;
-    float D = mfd_eval(d, h);
-    float F = fresnel_dielectric(fabsf(dot(r.wi, h)), b.eta, b.inv_eta, ct);
-    float G = mfd_g(d, r.wi, r.wo, h);
-    float den = 4.0f * fabsf(ci);
-    const V3 ks = par_rgb(b, 1, b.ks, r);
-    V3 res = v3((((ks.x * F) * D) * G) / den, (((ks.y * F) * D) * G) / den, (((ks.z * F) * D) * G) / den);
+// Eval and Pdf of a leaf BSDF under ESolidAngle
+__device__ __forceinline__ V3 leaf_eval_pdf(const DevBsdf &b, const BRec &r, float &pdf) {
+    switch (b.type) {
+    case kRoughConductor: return conductor_eval_pdf(b, r, mfd_g1_of(bsdf_mfd(b, r), r.wi), pdf);
+    case kRoughDielectric: return dielectric_eval_pdf(b, r, mfd_g1_of(bsdf_mfd(b, r), r.wi), pdf);
+    case kRoughPlastic: {
+        const Mfd d = coat_mfd(b, r);
+        return plastic_eval_pdf(b, r, mfd_g1_of(d, r.wi), rft_eval(b, r.wi.z, d.au), pdf);
+    }
+    default:
+        pdf = leaf_pdf(b, r);
+        return leaf_eval(b, r);
+    }
+}
+// The record below the layer: both directions refracted into it
+__device__ __forceinline__ BRec coat_inner(const DevBsdf &b, const BRec &r) {
     BRec ri = r;
     ri.wi = coat_refract(r.wi, b.inv_eta);
     ri.wo = coat_refract(r.wo, b.inv_eta);
-    V3 nv = leaf_eval(nb, ri);
-    float ti = rft_eval(b, fabsf(ci), d.au), to = rft_eval(b, fabsf(co), d.au);
+    return ri;
+}
+// Eval past its test of sides.  h, D: the half vector on wo's side and D at it;
+// ri, nv: the inner record and the nested BSDF's value at it; t_ci: rft_eval at
+// |cos wi|; g1_wi: mfd_g1_of wi.
+__device__ __forceinline__ V3 coating_value(const DevBsdf &b, const BRec &r, const Mfd &d, V3 h, float D, const BRec &ri,
+                                            V3 nv, float g1_wi, float t_ci) {
+    const float ci = r.wi.z, co = r.wo.z;
+    float ct;
+    float F = fresnel_dielectric(fabsf(dot(r.wi, h)), b.eta, b.inv_eta, ct);
+    float G = mfd_g1_with(g1_wi, r.wi, h) * mfd_g1(d, r.wo, h);
+    float den = 4.0f * fabsf(ci);
+    const V3 ks = par_rgb(b, 1, b.ks, r);
+    V3 res = v3((((ks.x * F) * D) * G) / den, (((ks.y * F) * D) * G) / den, (((ks.z * F) * D) * G) / den);
+    float ti = t_ci, to = rft_eval(b, fabsf(co), d.au);
     nv = v3(nv.x * ti * to, nv.y * ti * to, nv.z * ti * to);
     V3 sa = par_rgb(b, 3, b.sigma_a, r) * b.thickness;
     if (!is_zero(sa)) {
@@ -950,38 +1054,58 @@ __device__ __forceinline__ V3 coating_eval(const DevBsdf &b, const DevBsdf &nb, 
     if (r.measure == kMeasureSolidAngle) nv = nv * (b.inv_eta * b.inv_eta * r.wo.z / ri.wo.z);
     return res + nv;
 }
-__device__ __forceinline__ float coating_pdf(const DevBsdf &b, const DevBsdf &nb, const BRec &r) {
-    V3 h = normalize(r.wi + r.wo) * signum(r.wo.z);
-    const float a = coat_alpha(b, r);
-    Mfd d = mfd_make(b.distribution, a, a);
-    float ci = r.wi.z, co = r.wo.z;
-    float r12 = 1.0f - rft_eval(b, fabsf(ci), d.au);
-    float sp = (r12 * b.spec_w) / (r12 * b.spec_w + (1.0f - r12) * (1.0f - b.spec_w));
-    float np = 1.0f - sp;
+// Pdf; p: the nested BSDF's pdf of the inner record, sp: the specular sampling weight
+__device__ __forceinline__ float coating_density(const DevBsdf &b, const BRec &r, V3 h, float D, const BRec &ri, float p,
+                                                 float sp) {
+    const float ci = r.wi.z, co = r.wo.z;
+    const float np = 1.0f - sp;
     float res = 0.0f;
     if (ci * co > 0.0f) {
         float J = 1.0f / (4.0f * fabsf(dot(r.wo, h)));
-        res = mfd_pdf(d, h) * J * sp;
+        res = (D * h.z) * J * sp;
     }
-    BRec ri = r;
-    ri.wi = coat_refract(r.wi, b.inv_eta);
-    ri.wo = coat_refract(r.wo, b.inv_eta);
-    float p = leaf_pdf(nb, ri);
     if (ri.measure == kMeasureSolidAngle) p *= b.inv_eta * b.inv_eta * co / ri.wo.z;
     return res + p * np;
 }
-__device__ __forceinline__ V3 coating_sample(const DevBsdf &b, const DevBsdf &nb, BRec &r, float ux, float uy, float u1) {
-    const float a = coat_alpha(b, r);
-    Mfd d = mfd_make(b.distribution, a, a);
-    float aci = fabsf(r.wi.z);
-    float r12 = 1.0f - rft_eval(b, aci, d.au);
-    float sp = (r12 * b.spec_w) / (r12 * b.spec_w + (1.0f - r12) * (1.0f - b.spec_w));
+__device__ __forceinline__ V3 coating_eval(const DevBsdf &b, const DevBsdf &nb, const BRec &r) {
+    if (r.wi.z * r.wo.z <= 0.0f) return v3(0, 0, 0);
+    const Mfd d = coat_mfd(b, r);
+    V3 h = normalize(r.wi + r.wo) * signum(r.wo.z);
+    const BRec ri = coat_inner(b, r);
+    return coating_value(b, r, d, h, mfd_eval(d, h), ri, leaf_eval(nb, ri), mfd_g1_of(d, r.wi),
+                         rft_eval(b, fabsf(r.wi.z), d.au));
+}
+__device__ __forceinline__ float coating_pdf(const DevBsdf &b, const DevBsdf &nb, const BRec &r) {
+    V3 h = normalize(r.wi + r.wo) * signum(r.wo.z);
+    const Mfd d = coat_mfd(b, r);
+    const BRec ri = coat_inner(b, r);
+    return coating_density(b, r, h, mfd_eval(d, h), ri, leaf_pdf(nb, ri), coat_spec_pdf(b, rft_eval(b, fabsf(r.wi.z), d.au)));
+}
+// Both, for a record under ESolidAngle
+__device__ __forceinline__ V3 coating_eval_pdf(const DevBsdf &b, const DevBsdf &nb, const BRec &r, float g1_wi, float t_ci,
+                                               float &pdf) {
+    const V3 h = normalize(r.wi + r.wo) * signum(r.wo.z);
+    const Mfd d = coat_mfd(b, r);
+    const float D = mfd_eval(d, h);
+    const BRec ri = coat_inner(b, r);
+    float p;
+    const V3 nv = leaf_eval_pdf(nb, ri, p);
+    pdf = coating_density(b, r, h, D, ri, p, coat_spec_pdf(b, t_ci));
+    if (r.wi.z * r.wo.z <= 0.0f) return v3(0, 0, 0);
+    return coating_value(b, r, d, h, D, ri, nv, g1_wi, t_ci);
+}
+// pdf: that of the sampled direction, as coating_pdf gives it
+__device__ __forceinline__ V3 coating_sample(const DevBsdf &b, const DevBsdf &nb, BRec &r, float ux, float uy, float u1,
+                                             float g1_wi, float t_ci, float &pdf) {
+    const Mfd d = coat_mfd(b, r);
+    const float sp = coat_spec_pdf(b, t_ci);
     bool spec;
+    pdf = 0.0f;
     if (ux < sp) { spec = true; ux /= sp; }
     else { spec = false; ux = (ux - sp) / (1.0f - sp); }
     if (spec) {
-        float pdf;
-        V3 m = mfd_sample(d, ux, uy, pdf);
+        float mp;
+        V3 m = mfd_sample(d, ux, uy, mp);
         r.wo = reflect_m(r.wi, m);
         r.measure = kMeasureDiscrete;
         r.eta = 1.0f;
@@ -995,9 +1119,18 @@ __device__ __forceinline__ V3 coating_sample(const DevBsdf &b, const DevBsdf &nb
         r.wo = coat_refract(r.wo, b.eta);
         if (is_zero(r.wo)) return v3(0, 0, 0);
     }
-    float P = coating_pdf(b, nb, r);
-    if (P == 0.0f) return v3(0, 0, 0);
-    return coating_eval(b, nb, r) / P;
+    const V3 h = normalize(r.wi + r.wo) * signum(r.wo.z);
+    const float D = mfd_eval(d, h);
+    const BRec ri = coat_inner(b, r);
+    pdf = coating_density(b, r, h, D, ri, leaf_pdf(nb, ri), sp);
+    if (pdf == 0.0f) return v3(0, 0, 0);
+    if (r.wi.z * r.wo.z <= 0.0f) return v3(0, 0, 0) / pdf;
+    return coating_value(b, r, d, h, D, ri, leaf_eval(nb, ri), g1_wi, t_ci) / pdf;
+}
+__device__ __forceinline__ V3 coating_sample(const DevBsdf &b, const DevBsdf &nb, BRec &r, float ux, float uy, float u1) {
+    const Mfd d = coat_mfd(b, r);
+    float pdf;
+    return coating_sample(b, nb, r, ux, uy, u1, mfd_g1_of(d, r.wi), rft_eval(b, fabsf(r.wi.z), d.au), pdf);
 }
 
 // ------------------------------------------------------------ coating
@@ -1557,6 +1690,51 @@ __device__ __forceinline__ V3 bsdf_sample_t(const DevBsdf *bs, int id, BRec &r, 
     else if constexpr (BT == kCoating) return scoating_sample(b, bs[b.nested], r, ux, uy, u1);
     else if constexpr (BT == kRoughDiffuse) return roughdiffuse_sample(b, r, ux, uy);
     else return twosided_sample(bs, b, r, ux, uy, u1);
+}
+
+// What the records of one vertex share, from wi alone: G1 of wi and the rough
+// transmittance at it (a powf and a cubic table lookup).
+struct BsdfVertex {
+    float g1_wi, t_ci;
+};
+template <int BT>
+__device__ __forceinline__ BsdfVertex bsdf_vertex_t(const DevBsdf *bs, int id, const BRec &r) {
+    BsdfVertex v{0.0f, 0.0f};
+    const DevBsdf &b = bs[id];
+    if constexpr (BT == kRoughConductor || BT == kRoughDielectric) {
+        v.g1_wi = mfd_g1_of(bsdf_mfd(b, r), r.wi);
+    } else if constexpr (BT == kRoughPlastic || BT == kRoughCoating) {
+        const Mfd d = coat_mfd(b, r);
+        v.g1_wi = mfd_g1_of(d, r.wi);
+        v.t_ci = rft_eval(b, BT == kRoughCoating ? fabsf(r.wi.z) : r.wi.z, d.au);
+    }
+    return v;
+}
+// Eval and Pdf of a next-event record (ESolidAngle) at vertex v
+template <int BT>
+__device__ __forceinline__ V3 bsdf_eval_pdf_t(const DevBsdf *bs, int id, const BRec &r, const BsdfVertex &v, float &pdf) {
+    const DevBsdf &b = bs[id];
+    if constexpr (BT == kRoughConductor) return conductor_eval_pdf(b, r, v.g1_wi, pdf);
+    else if constexpr (BT == kRoughDielectric) return dielectric_eval_pdf(b, r, v.g1_wi, pdf);
+    else if constexpr (BT == kRoughPlastic) return plastic_eval_pdf(b, r, v.g1_wi, v.t_ci, pdf);
+    else if constexpr (BT == kRoughCoating) return coating_eval_pdf(b, bs[b.nested], r, v.g1_wi, v.t_ci, pdf);
+    else {
+        pdf = bsdf_pdf_t<BT>(bs, id, r);
+        return bsdf_eval_t<BT>(bs, id, r);
+    }
+}
+// Sample at vertex v; want_pdf: also the pdf of the sampled direction
+template <int BT>
+__device__ __forceinline__ V3 bsdf_sample_pdf_t(const DevBsdf *bs, int id, BRec &r, float ux, float uy, float u1,
+                                                const BsdfVertex &v, bool want_pdf, float &pdf) {
+    const DevBsdf &b = bs[id];
+    if constexpr (BT == kRoughPlastic) return plastic_sample(b, r, ux, uy, v.g1_wi, v.t_ci, pdf);
+    else if constexpr (BT == kRoughCoating) return coating_sample(b, bs[b.nested], r, ux, uy, u1, v.g1_wi, v.t_ci, pdf);
+    else {
+        const V3 w = bsdf_sample_t<BT>(bs, id, r, ux, uy, u1);
+        pdf = want_pdf && !all_zero(w) ? bsdf_pdf_t<BT>(bs, id, r) : 0.0f;
+        return w;
+    }
 }
 
 // bumpMap / normalMap id wrapping a BSDF of type BT known at compile time:

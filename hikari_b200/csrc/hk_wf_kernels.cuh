@@ -159,6 +159,19 @@ __global__ void __launch_bounds__(256, kMinBlocks) wf_shade_kernel(DevScene S, W
             }
             // next-event estimation over every emitter (PathMISIntegrator.cpp:83-109)
             const V3 wi_local = to_local(it.sh, rd * -1.0f);
+            BsdfVertex bv;   // the typed kernels'
+            if constexpr (BT >= 0 && !kBumpQ) {
+                BRec br;
+                br.wi = wi_local;
+                br.tex = kTexQ;
+                br.tu = it.u;
+                br.tv = it.v;
+                if constexpr (kTexQ) {
+                    br.duv = duv;
+                    br.geo = geo;
+                }
+                bv = bsdf_vertex_t<BT>(S.bsdfs, bsdf, br);
+            }
             for (int e = 0; e < S.nemitters; ++e) {
                 ERec er;
                 er.ref = it.p;
@@ -190,8 +203,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) wf_shade_kernel(DevScene S, W
                     pb = bump_pdf_t<BT>(S.bsdfs, bsdf, br, bf);
                     f = bump_eval_t<BT>(S.bsdfs, bsdf, br, bf);
                 } else {
-                    pb = bsdf_pdf_t<BT>(S.bsdfs, bsdf, br);
-                    f = bsdf_eval_t<BT>(S.bsdfs, bsdf, br);
+                    f = bsdf_eval_pdf_t<BT>(S.bsdfs, bsdf, br, bv, pb);
                 }
                 float w = (pl + pb != 0.0f) ? pl / (pl + pb) : 1.0f;
                 float c = fabsf(br.wo.z);
@@ -221,9 +233,10 @@ __global__ void __launch_bounds__(256, kMinBlocks) wf_shade_kernel(DevScene S, W
             float sx = rng.nextf(), sy = rng.nextf();
             float u1 = needs_u1(S.bsdfs, bsdf) ? rng.nextf() : 0.0f;
             V3 F;
+            float spdf = 0.0f;   // the typed kernels' pdf of the sampled direction
             if constexpr (BT < 0) F = bsdf_sample_b(S.bsdfs, bsdf, br, sx, sy, u1, bf);
             else if constexpr (kBumpQ) F = bump_sample_t<BT>(S.bsdfs, bsdf, br, sx, sy, u1, bf);
-            else F = bsdf_sample_t<BT>(S.bsdfs, bsdf, br, sx, sy, u1);
+            else F = bsdf_sample_pdf_t<BT>(S.bsdfs, bsdf, br, sx, sy, u1, bv, S.narea != 0, spdf);
             beta = beta * F;
             bool alive = !is_zero(beta);
             if (alive) {
@@ -259,7 +272,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) wf_shade_kernel(DevScene S, W
                 pr.eta = 0.0f;
                 if constexpr (BT < 0) W.prev_pdf[slot] = bsdf_pdf_b(S.bsdfs, bsdf, pr, bf);
                 else if constexpr (kBumpQ) W.prev_pdf[slot] = bump_pdf_t<BT>(S.bsdfs, bsdf, pr, bf);
-                else W.prev_pdf[slot] = bsdf_pdf_t<BT>(S.bsdfs, bsdf, pr);
+                else W.prev_pdf[slot] = spdf;
             }
             W.rng[slot] = make_uint4((uint32_t)rng.state, (uint32_t)(rng.state >> 32), (uint32_t)rng.inc,
                                      (uint32_t)(rng.inc >> 32));
