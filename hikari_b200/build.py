@@ -23,7 +23,7 @@ SOURCES = ["hk_batch_4.cu", "hk_render_b8.cu", "hk_render_b8t.cu", "hk_render_b2
            "hk_batch_0.cu", "hk_batch_1.cu", "hk_batch_2.cu", "hk_batch_3.cu", "hk_batch_5.cu",
            "hk_kernels.cu", "hk_wavefront.cu", "hk_lbvh.cu", "hk_host.cpp", "hk_engine.cpp", "hk_server.cpp", "hk_bvh.cpp", "hk_xml.cpp",
            "hk_obj.cpp", "hk_mipmap.cpp", "hk_image.cpp"]
-HEADERS = ["hk_megakernel.cuh", "hk_batch.cuh", "hk_wf_kernels.cuh", "hk_wf_trace.cuh", "hk_device.h", "hk_math.cuh", "hk_bsdf.cuh", "hk_traverse.cuh", "hk_shading.cuh", "hk_kernels.h",
+HEADERS = ["hk_megakernel.cuh", "hk_batch.cuh", "hk_wf_kernels.cuh", "hk_wf_trace.cuh", "hk_device.h", "hk_math.cuh", "hk_bsdf.cuh", "hk_traverse.cuh", "hk_traverse8.cuh", "hk_shading.cuh", "hk_kernels.h",
            "hk_bvh.h", "hk_xml.h", "hk_wavefront.h", "hk_engine.h", "hk_hostutil.h", "hk_internal.h", "hk_obj.h", "hk_mipmap.h"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ARCH + ["-O3", "-lineinfo", "-fmad=false", "-std=c++17", "-Xcompiler", "-fPIC,-O2,-pthread",

@@ -152,6 +152,7 @@ void WfEngine::set_job(int slot, WfJob J) {
     // Each slot has its own staging entry; a slot is rewritten only after its
     // previous job ended, long after that job's copy ran.
     J.finished = finished_.as<unsigned long long>() + slot;
+    job_count_ = std::max(job_count_, slot + 1);
     h_jobs_.p[slot] = J;
     HK_CUDA(cudaMemcpyAsync(jobs_.as<WfJob>() + slot, h_jobs_.p + slot, sizeof(WfJob), cudaMemcpyHostToDevice, stream_));
     HK_CUDA(cudaMemsetAsync(finished_.as<unsigned long long>() + slot, 0, sizeof(unsigned long long), stream_));
@@ -168,9 +169,9 @@ void WfEngine::set_plan(const std::vector<WfSeg> &segs, uint64_t total) {
     h.next_work = 0;
     h.total_work = total;
     h.seg_count = (unsigned)segs.size();
-    h.pad0 = 0;
-    // the dispatch head: next_work, total_work, seg_count (first 20 bytes)
-    HK_CUDA(cudaMemcpyAsync(W_.ctr, &h, offsetof(WfCounters, pad0), cudaMemcpyHostToDevice, stream_));
+    h.job_count = (unsigned)job_count_;
+    // the dispatch head: next_work, total_work, seg_count, job_count (first 24 bytes)
+    HK_CUDA(cudaMemcpyAsync(W_.ctr, &h, offsetof(WfCounters, eq_count), cudaMemcpyHostToDevice, stream_));
     HK_CUDA(cudaEventRecord(ev_plan_, stream_));
 }
 

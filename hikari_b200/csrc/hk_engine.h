@@ -83,6 +83,7 @@ private:
     WfLaunchConfig L_{};
     WfState W_{};
     size_t bytes_ = 0;
+    int job_count_ = 0;   // highest job slot ever set + 1
     DevBuf state_, queues_, shadow_, counters_, jobs_, finished_, segs_;
     PinnedBuf<WfCounters> h_ctr_;
     PinnedBuf<unsigned long long> h_fin_;

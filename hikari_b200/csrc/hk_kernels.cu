@@ -4,13 +4,17 @@
 //   * the dispatch from the launch interface to the megakernel
 //     (hk_megakernel.cuh, instantiated in hk_render_*.cu) and the BSDF batch
 //     (hk_batch.cuh, instantiated in hk_batch_*.cu).
+#include <algorithm>
 #include <cstdio>
 #include <mutex>
 
 #include "hk_kernels.h"
 #include "hk_shading.cuh"
+#include "hk_traverse8.cuh"
 
 namespace hk {
+constexpr int kTraceThreads = 128;
+
 // Block.cpp:61 ToBitmap: interior pixels divided by their filter weight.
 __global__ void film_resolve_kernel(const float *film, float *rgb, int W, int H, int B) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -25,33 +29,64 @@ __global__ void film_resolve_kernel(const float *film, float *rgb, int W, int H,
 }
 
 // Ray queries: rays are n x 8 floats (o, d, tmin, tmax).  Reported triangle
-// ids are the ORIGINAL global triangle indices (mesh order).
-template <int kAccel>
-__global__ void trace_rays_kernel(DevScene S, uint64_t n, const float *rays, int32_t *tri, float *t, float *u, float *v,
-                                  int any_hit, unsigned long long *visit_counter) {
+// ids are the ORIGINAL global triangle indices (mesh order).  In the 8-wide
+// tree a warp takes per_warp consecutive rays and shares their tests
+// (trace_queue8); in the binary tree each thread walks its own.
+template <int kAccel, bool kAnyHit>
+__global__ void __launch_bounds__(kTraceThreads) trace_rays_kernel(DevScene S, uint64_t n, uint32_t per_warp, const float *rays,
+                                                                   int32_t *tri, float *t, float *u, float *v,
+                                                                   unsigned long long *visit_counter) {
     TravStats ts;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+    auto load = [&](uint64_t i) {   // ray i
         const float4 *rp = reinterpret_cast<const float4 *>(rays + 8 * i);
-        float4 a = __ldg(rp), b = __ldg(rp + 1);
+        const float4 a = __ldg(rp), b = __ldg(rp + 1);
         Ray r;
         r.o = v3(a.x, a.y, a.z);
         r.d = v3(a.w, b.x, b.y);
         r.tmin = b.z;
         r.tmax = b.w;
-        Hit h;
-        bool f = any_hit ? trace<kAccel, true>(S, r, h, ts) : trace<kAccel, false>(S, r, h, ts);
-        if (any_hit) { tri[i] = f ? 1 : 0; continue; }
-        tri[i] = f ? __float_as_int(__ldg(S.tris + 3 * h.tri).w) : -1;
-        if (t) t[i] = f ? h.t : 0.0f;
-        if (u) u[i] = f ? h.u : 0.0f;
-        if (v) v[i] = f ? h.v : 0.0f;
+        return r;
+    };
+    auto put = [&](uint64_t i, bool f, const Hit &h) {
+        if constexpr (kAnyHit) {
+            tri[i] = f ? 1 : 0;
+        } else {
+            tri[i] = f ? __float_as_int(__ldg(S.tris + 3 * (size_t)h.tri).w) : -1;
+            if (t) t[i] = f ? h.t : 0.0f;
+            if (u) u[i] = f ? h.u : 0.0f;
+            if (v) v[i] = f ? h.v : 0.0f;
+        }
+    };
+    if constexpr (kAccel == kAccelBvh8) {
+        const uint64_t warp = blockIdx.x * (uint64_t)(blockDim.x / 32) + threadIdx.x / 32;
+        const uint64_t begin = min(n, warp * per_warp);
+        const unsigned cnt = (unsigned)min((uint64_t)per_warp, n - begin);
+        trace_queue8<kAnyHit, false>(S, 0u, cnt, cnt, kAnyHit ? 8 : 12, [&] { return cnt; },
+                              [&](int i) { return load(begin + (uint64_t)i); }, [&](int i, bool f, Hit h) {
+            const uint64_t k = begin + (uint64_t)i;
+            if constexpr (!kAnyHit) {
+                if (f) {   // t and the barycentrics with the reference's arithmetic
+                    const Ray r = load(k);
+                    const float4 *tp = S.tris + 3 * (size_t)h.tri;
+                    refine_mt(r.o, r.d, xyz(ldg4(tp)), xyz(ldg4(tp + 1)), xyz(ldg4(tp + 2)), r.tmin, r.tmax, h.t, h.u, h.v);
+                }
+            }
+            put(k, f, h);
+        }, ts);
+    } else {
+        for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+            Hit h;
+            const bool f = trace<kAccel, kAnyHit>(S, load(i), h, ts);
+            put(i, f, h);
+        }
     }
     if (visit_counter) {
         unsigned long long nodes = ts.nodes, tris = ts.tris;
-        for (int o = 16; o > 0; o >>= 1) {
-            nodes += __shfl_down_sync(0xffffffffu, nodes, o);
-            tris += __shfl_down_sync(0xffffffffu, tris, o);
-        }
+        if constexpr (kAccel != kAccelBvh8)   // there every lane has its warp's sums
+            for (int o = 16; o > 0; o >>= 1) {
+                nodes += __shfl_down_sync(0xffffffffu, nodes, o);
+                tris += __shfl_down_sync(0xffffffffu, tris, o);
+            }
         if ((threadIdx.x & 31) == 0) {
             atomicAdd(visit_counter, nodes);
             atomicAdd(visit_counter + 1, tris);
@@ -155,13 +190,31 @@ cudaError_t launch_resolve(const float *film, float *rgb, int W, int H, int B, c
     film_resolve_kernel<<<(n + 255) / 256, 256, 0, st>>>(film, rgb, W, H, B);
     return cudaGetLastError();
 }
+template <int kAccel, bool kAnyHit>
+static cudaError_t launch_trace_t(const DevScene &S, uint64_t n, const float *rays, int32_t *tri, float *t, float *u, float *v,
+                                  unsigned long long *visits, cudaStream_t st) {
+    if constexpr (kAccel == kAccelBvh8) {
+        // 32 rays a warp fill the GPU's 4736 resident warps up to 150 thousand
+        // rays; above, up to 128, so that lanes refill while blocks still
+        // follow one another and even out the warps' times
+        const uint64_t per_warp = std::max<uint64_t>(32, std::min<uint64_t>(128, n / (148 * 32)));
+        const uint64_t warps = (n + per_warp - 1) / per_warp, per_block = kTraceThreads / 32;
+        const size_t smem = trace8_smem(kAnyHit, kTraceThreads);
+        trace_rays_kernel<kAccel, kAnyHit><<<(unsigned)((warps + per_block - 1) / per_block), kTraceThreads, smem, st>>>(
+            S, n, (uint32_t)per_warp, rays, tri, t, u, v, visits);
+    } else {
+        trace_rays_kernel<kAccel, kAnyHit><<<grid_for(n, kTraceThreads), kTraceThreads, 0, st>>>(S, n, 0u, rays, tri, t, u, v,
+                                                                                                 visits);
+    }
+    return cudaGetLastError();
+}
 cudaError_t launch_trace(const DevScene &S, uint64_t n, const float *rays, int32_t *tri, float *t, float *u, float *v,
                          int any_hit, unsigned long long *visits, cudaStream_t st) {
     if (S.accel == kAccelBvh8)
-        trace_rays_kernel<kAccelBvh8><<<grid_for(n, 128), 128, 0, st>>>(S, n, rays, tri, t, u, v, any_hit, visits);
-    else
-        trace_rays_kernel<kAccelBvh2><<<grid_for(n, 128), 128, 0, st>>>(S, n, rays, tri, t, u, v, any_hit, visits);
-    return cudaGetLastError();
+        return any_hit ? launch_trace_t<kAccelBvh8, true>(S, n, rays, tri, t, u, v, visits, st)
+                       : launch_trace_t<kAccelBvh8, false>(S, n, rays, tri, t, u, v, visits, st);
+    return any_hit ? launch_trace_t<kAccelBvh2, true>(S, n, rays, tri, t, u, v, visits, st)
+                   : launch_trace_t<kAccelBvh2, false>(S, n, rays, tri, t, u, v, visits, st);
 }
 cudaError_t launch_bsdf_batch(const DevScene &S, int bsdf, int type, uint64_t n, const float *wi, const float *u2, const float *u1,
                               const float *wo, const float *uv, const float *duv, float *s_wo, float *s_w, float *s_pdf,

@@ -1,0 +1,361 @@
+// Traversal of the 8-wide tree by warps that share their triangle tests, for
+// kernels that trace a queue of rays: the wavefront's extend and shadow kernels
+// and the ray queries.
+//
+// The 8-wide tree is walked by warps whose lanes hold one ray each and share
+// one queue of triangle tests (trace_queue8): a step visits one node per lane,
+// the triangles that the visits hit are appended to a 64-entry ring in shared
+// memory as (triangle, owner lane), and a batch of 32 is tested, one triangle
+// per lane, whenever 32 are pending.  The kernels are bound by instruction
+// issue (77% of the slots) and by the ALU pipe (68%: the node test's byte
+// permutes, min / max and compares run there at half rate), not by DRAM (7%),
+// so what counts is warp instructions per ray.  A lane that tests its own
+// triangles keeps the warp for as many rounds as the largest leaf group with
+// the other lanes idle (13 active lanes per instruction); testing each step's
+// triangles at once, shared out over the lanes, fills half of a round (14
+// triangles on average) and pays for numbering triangles and finding owners in
+// every round.  1024^2 x 32 spp, ns per ray, own / shared out at once / ring:
+// 64-sphere scene (1.3M triangles) shadow 0.319 / 0.280 / 0.245, closest hit
+// 0.466 / 0.413 / 0.266; glass sphere (0.33M) shadow 0.485 / 0.391 / 0.324,
+// closest hit 0.549 / 0.473 / 0.307; Cornell box (36 triangles, two visits a
+// ray) shadow 0.124 / 0.129 / 0.120, closest hit 0.161 / 0.174 / 0.134.
+#pragma once
+#include "hk_traverse.cuh"
+
+namespace hk {
+
+constexpr unsigned kTriRing = 64;      // pending triangle tests per warp (a power of two, at least 2 x 32)
+constexpr unsigned kTriOwnerShift = kLeafCountShift;   // scenes hold fewer than 2^27 triangles: the owner lane sits above
+constexpr uint32_t kTriMask = (1u << kTriOwnerShift) - 1u;
+
+// A ray's constants of the node test.
+struct NodeRay {
+    V3 o;
+    V3 i;                // 1 / d
+    float tmin, tmax;    // tmax with the same slack
+    uint32_t oct;
+};
+
+__device__ __forceinline__ void node_ray_begin(NodeRay &q, const Ray &ray) {
+    q.o = ray.o;
+    // |1/d| <= 1e20 keeps 2^23 steps of up to 2^38 (the largest step the build emits) finite
+    const float tiny = 1e-20f, slack = 1.00000024f;
+    const V3 d = ray.d;
+    const V3 dd = v3(fabsf(d.x) < tiny ? copysignf(tiny, d.x) : d.x, fabsf(d.y) < tiny ? copysignf(tiny, d.y) : d.y,
+                     fabsf(d.z) < tiny ? copysignf(tiny, d.z) : d.z);
+    const V3 i = v3(1.0f / dd.x, 1.0f / dd.y, 1.0f / dd.z);
+    q.i = i;
+    q.oct = (i.x < 0.0f ? 1u : 0u) | (i.y < 0.0f ? 2u : 0u) | (i.z < 0.0f ? 4u : 0u);
+    q.tmin = ray.tmin;
+    q.tmax = ray.tmax * slack + 1e-30f;
+}
+
+// Intersect the 8 children of a node (hk_bvh.h): its node group and triangle group.
+template <bool kUnit>
+__device__ __forceinline__ void visit8(const DevScene &S, uint32_t child, const NodeRay &q, uint2 &ng, uint2 &tg) {
+    const uint4 *np = S.wnodes + 5 * (size_t)child;
+    const uint4 n0 = ldg4u(np), n1 = ldg4u(np + 1), n2 = ldg4u(np + 2), n3 = ldg4u(np + 3), n4 = ldg4u(np + 4);
+    const uint32_t oct = q.oct, ko = 7u ^ oct;
+    // plane step and offset per axis of the near (x) and far (y) planes; offsets
+    // are shifted by -2^23 steps (qbyte_biased).  The far planes' constants are
+    // scaled by 1 + 2^-22 (two ulps): the slack that keeps boxes of zero
+    // thickness costs nothing per child.
+    const float sx = __uint_as_float((n0.w << 23) & 0x7f800000u), sy = __uint_as_float((n0.w << 15) & 0x7f800000u),
+                sz = __uint_as_float((n0.w << 7) & 0x7f800000u);
+    const float px = __uint_as_float(n0.x) - q.o.x, py = __uint_as_float(n0.y) - q.o.y, pz = __uint_as_float(n0.z) - q.o.z;
+    const float slack = 1.00000024f;
+    const V3 f = q.i * slack;
+    const float2 ax = make_float2(sx * q.i.x, sx * f.x), ay = make_float2(sy * q.i.y, sy * f.y),
+                 az = make_float2(sz * q.i.z, sz * f.z);
+    const float2 bx = make_float2(__fmaf_rn(-8388608.0f, ax.x, px * q.i.x), __fmaf_rn(-8388608.0f, ax.y, px * f.x));
+    const float2 by = make_float2(__fmaf_rn(-8388608.0f, ay.x, py * q.i.y), __fmaf_rn(-8388608.0f, ay.y, py * f.y));
+    const float2 bz = make_float2(__fmaf_rn(-8388608.0f, az.x, pz * q.i.z), __fmaf_rn(-8388608.0f, az.y, pz * f.z));
+    const uint32_t imask = n0.w >> 24;
+    // meta of internal children: slot ^ (7 ^ octant) in the position bits
+    const uint32_t in0 = ((imask & 0xfu) * 0x00204081u) & 0x01010101u;
+    const uint32_t in1 = ((imask >> 4) * 0x00204081u) & 0x01010101u;
+    const uint32_t meta0 = n1.z ^ (in0 * ko), meta1 = n1.w ^ (in1 * ko);
+    // near / far planes per axis (lo planes first for a positive direction)
+    const uint32_t nx0 = oct & 1u ? n3.z : n2.x, nx1 = oct & 1u ? n3.w : n2.y;
+    const uint32_t fx0 = oct & 1u ? n2.x : n3.z, fx1 = oct & 1u ? n2.y : n3.w;
+    const uint32_t ny0 = oct & 2u ? n4.x : n2.z, ny1 = oct & 2u ? n4.y : n2.w;
+    const uint32_t fy0 = oct & 2u ? n2.z : n4.x, fy1 = oct & 2u ? n2.w : n4.y;
+    const uint32_t nz0 = oct & 4u ? n4.z : n3.x, nz1 = oct & 4u ? n4.w : n3.y;
+    const uint32_t fz0 = oct & 4u ? n3.x : n4.z, fz1 = oct & 4u ? n3.y : n4.w;
+    uint32_t hits = 0;
+    const float t0 = kUnit ? kRayEps : q.tmin, t1 = kUnit ? (1.0f - kRayEps) * 1.00000024f : q.tmax;
+    auto test_child = [&](auto kk, uint32_t xn, uint32_t xf, uint32_t yn, uint32_t yf, uint32_t zn, uint32_t zf,
+                          uint32_t meta) {
+        constexpr int k = decltype(kk)::value;
+        const float2 tx = make_float2(__fmaf_rn(qbyte_biased<k>(xn), ax.x, bx.x), __fmaf_rn(qbyte_biased<k>(xf), ax.y, bx.y));
+        const float2 ty = make_float2(__fmaf_rn(qbyte_biased<k>(yn), ay.x, by.x), __fmaf_rn(qbyte_biased<k>(yf), ay.y, by.y));
+        const float2 tz = make_float2(__fmaf_rn(qbyte_biased<k>(zn), az.x, bz.x), __fmaf_rn(qbyte_biased<k>(zf), az.y, bz.y));
+        const float tn = fmax3f(tx.x, ty.x, fmaxf(tz.x, t0));
+        const float tf = fmin3f(tx.y, ty.y, fminf(tz.y, t1));
+        const uint32_t m = __byte_perm(meta, 0u, 0x4440u | k);
+        if (tn <= tf) hits |= __funnelshift_l(0u, m >> 5, m);   // shifted by the low five bits of m
+    };
+    test_child(std::integral_constant<int, 0>{}, nx0, fx0, ny0, fy0, nz0, fz0, meta0);
+    test_child(std::integral_constant<int, 1>{}, nx0, fx0, ny0, fy0, nz0, fz0, meta0);
+    test_child(std::integral_constant<int, 2>{}, nx0, fx0, ny0, fy0, nz0, fz0, meta0);
+    test_child(std::integral_constant<int, 3>{}, nx0, fx0, ny0, fy0, nz0, fz0, meta0);
+    test_child(std::integral_constant<int, 0>{}, nx1, fx1, ny1, fy1, nz1, fz1, meta1);
+    test_child(std::integral_constant<int, 1>{}, nx1, fx1, ny1, fy1, nz1, fz1, meta1);
+    test_child(std::integral_constant<int, 2>{}, nx1, fx1, ny1, fy1, nz1, fz1, meta1);
+    test_child(std::integral_constant<int, 3>{}, nx1, fx1, ny1, fy1, nz1, fz1, meta1);
+    ng = make_uint2(n1.x, (hits & 0xff000000u) | imask);
+    tg = make_uint2(n1.y, hits & 0x00ffffffu);
+}
+
+// Shared memory of one warp of the 8-wide traversal kernels: the lanes' rays as
+// the triangle test reads them (two float4 each), the short stacks (kShStack
+// entries of 32 lanes), the ring; for closest-hit rays also the lanes' hits so
+// far (t, u, v, triangle) and their tmax.  One base address per warp and
+// constant offsets from it keep the addresses out of the registers.
+template <bool kAnyHit>
+struct WarpSmem {
+    float4 rays[64];
+    float4 hits[kAnyHit ? 1 : 32];
+    uint2 stack[kShStack * 32];
+    uint32_t ring[kTriRing];
+    uint32_t tmaxs[kAnyHit ? 4 : 32];
+};
+constexpr size_t trace8_smem(bool any_hit, int threads) {
+    return (size_t)(threads / 32) * (any_hit ? sizeof(WarpSmem<true>) : sizeof(WarpSmem<false>));
+}
+
+// Floats as unsigned integers in the floats' order, and back.
+__device__ __forceinline__ uint32_t ordered_bits(float t) {
+    const uint32_t b = __float_as_uint(t + 0.0f);   // -0 becomes +0
+    return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+}
+__device__ __forceinline__ float from_ordered(uint32_t b) {
+    return __uint_as_float((b & 0x80000000u) ? (b & 0x7fffffffu) : ~b);
+}
+
+// Traverses n rays of a queue: lanes are refilled as in trace_queue
+// (hk_traverse.cuh), node visits and triangle tests as described at the top.
+// The warp starts with entries first to last - 1; claim(), called by one lane,
+// takes the next kFetchChunk ones and returns the first of them (n or more: none
+// are left).
+// load(i) returns ray i; store(i, found, hit) consumes the result.  st counts
+// the warp's visits and tests (the same in every lane).  kUnit: every ray's
+// range is [kRayEps, 1 - kRayEps], a segment between two points.  A lane
+// whose walk has ended, or whose any-hit ray is found occluded, waits until
+// min_idle lanes are without a walk; the ring is then tested to its end, so no
+// entry outlives its ray, the rays are stored and the lanes refilled.
+//
+// Closest-hit rays keep the hit that the serial loop keeps: tests run in the
+// order a ray met its triangles (ring order, and lane order within a batch),
+// a hit needs t <= tmax as of the batch's start, the least t of the batch
+// wins, and of equal ones the latest.  That tmax shrinks a batch late only
+// adds visits and tests, never a hit.
+template <bool kAnyHit, bool kUnit, class Claim, class Load, class Store>
+__device__ __forceinline__ void trace_queue8(const DevScene &S, unsigned first, unsigned last, unsigned n,
+                                             int min_idle, Claim claim, Load load, Store store, TravStats &st) {
+    extern __shared__ float4 trace_smem[];
+    const unsigned lane = threadIdx.x & 31u;
+    WarpSmem<kAnyHit> &sm = reinterpret_cast<WarpSmem<kAnyHit> *>(trace_smem)[threadIdx.x >> 5];
+    uint2 spill[kStackSize - kShStack];   // entries of the stack past the short one
+    int sp = 0;
+
+    NodeRay nr;
+    uint2 ng = make_uint2(0u, 0u);
+    int item = -1;
+    bool live = false, found = false, exhausted = false;
+    unsigned head = 0, pend = 0;              // warp-uniform: the ring's first entry and number of entries
+    unsigned chunk_next = first, chunk_end = last;   // warp-uniform: unhanded entries of the warp's chunk
+
+    // Test the ring's first cnt (at most 32) entries, one per lane.
+    auto test_batch = [&](unsigned cnt) {
+        __syncwarp();   // the entries and the rays are visible
+        const bool act = lane < cnt;
+        const uint32_t e = act ? sm.ring[(head + lane) & (kTriRing - 1u)] : 0u;
+        const uint32_t own = e >> kTriOwnerShift, tri = e & kTriMask;
+        head += cnt;
+        pend -= cnt;
+        if constexpr (kAnyHit) {
+            bool hit = false;
+            if (act) {
+                const float4 *tp = S.tris + 3 * (size_t)tri;
+                const float4 p0 = ldg4(tp), p1 = ldg4(tp + 1), p2 = ldg4(tp + 2);
+                const float4 ro = sm.rays[2 * own], rd = sm.rays[2 * own + 1];
+                hit = occludes_mt(xyz(ro), xyz(rd), xyz(p0), xyz(p1), xyz(p2), kUnit ? kRayEps : ro.w,
+                                  kUnit ? 1.0f - kRayEps : rd.w);
+            }
+            const uint32_t occluded = __reduce_or_sync(0xffffffffu, hit ? 1u << own : 0u);
+            if (occluded >> lane & 1u) {
+                found = true;
+                live = false;
+            }
+        } else {
+            bool hit = false;
+            float tt = 0.0f, uu = 0.0f, vv = 0.0f;
+            if (act) {
+                const float4 *tp = S.tris + 3 * (size_t)tri;
+                const float4 p0 = ldg4(tp), p1 = ldg4(tp + 1), p2 = ldg4(tp + 2);
+                const float4 ro = sm.rays[2 * own], rw = sm.rays[2 * own + 1];
+                const uint32_t kp = __float_as_uint(rw.w);
+                WatertightRay w;
+                w.kx = (int)(kp & 3u);
+                w.ky = (int)((kp >> 2) & 3u);
+                w.kz = (int)((kp >> 4) & 3u);
+                w.sx = rw.x;
+                w.sy = rw.y;
+                w.sz = rw.z;
+                hit = intersect_watertight(w, xyz(ro), xyz(p0), xyz(p1), xyz(p2), ro.w, from_ordered(sm.tmaxs[own]), tt, uu,
+                                           vv);
+            }
+            if (__any_sync(0xffffffffu, hit)) {   // also: every lane has read tmaxs
+                const uint32_t key = ordered_bits(tt);
+                if (hit) atomicMin(&sm.tmaxs[own], key);
+                __syncwarp();
+                const bool least = hit && sm.tmaxs[own] == key;
+                if (least) sm.hits[own] = make_float4(tt, uu, vv, __uint_as_float(tri));
+                __syncwarp();
+                // equal least t of one ray in this batch: the latest stays
+                const bool lost = least && __float_as_uint(sm.hits[own].w) != tri;
+                if (__any_sync(0xffffffffu, lost)) {
+                    for (unsigned l = 0; l < 32; ++l) {
+                        if (lane == l && least) sm.hits[own] = make_float4(tt, uu, vv, __uint_as_float(tri));
+                        __syncwarp();
+                    }
+                }
+                nr.tmax = from_ordered(sm.tmaxs[lane]) * 1.00000024f + 1e-30f;
+            }
+        }
+        __syncwarp();   // reads of the ring precede its next entries
+    };
+
+    for (;;) {
+        // rays for idle lanes
+        const unsigned want = __ballot_sync(0xffffffffu, item < 0 && !exhausted);
+        const unsigned busy = __ballot_sync(0xffffffffu, item >= 0);
+        if (want && (busy == 0u || __popc(want) >= min_idle)) {
+            const unsigned k = __popc(want), rank = __popc(want & ((1u << lane) - 1u));
+            const unsigned avail = chunk_end - chunk_next;
+            unsigned idx = chunk_next + rank;
+            if (k > avail) {   // warp-uniform: claim the next chunk for the lanes past the old one
+                unsigned base = 0;
+                if ((int)lane == __ffs(want) - 1) base = claim();
+                base = __shfl_sync(0xffffffffu, base, __ffs(want) - 1);
+                if (rank >= avail) idx = base + (rank - avail);
+                chunk_next = base + (k - avail);
+                chunk_end = base + kFetchChunk;
+            } else {
+                chunk_next += k;
+            }
+            if (want >> lane & 1u) {
+                if (idx < n) {
+                    item = (int)idx;
+                    const Ray r = load(item);
+                    node_ray_begin(nr, r);
+                    // the root as slot 0 of a virtual parent (nothing for an empty tree)
+                    ng = make_uint2(0u, S.nwnodes == 0 ? 0u : ((1u << (24 + (7u ^ nr.oct))) | 1u));
+                    sp = 0;
+                    found = false;
+                    live = S.nwnodes != 0;
+                    sm.rays[2 * lane] = make_float4(r.o.x, r.o.y, r.o.z, r.tmin);
+                    if constexpr (kAnyHit) {
+                        sm.rays[2 * lane + 1] = make_float4(r.d.x, r.d.y, r.d.z, r.tmax);
+                    } else {
+                        const WatertightRay w = watertight_setup(r.d);
+                        sm.rays[2 * lane + 1] = make_float4(
+                            w.sx, w.sy, w.sz, __uint_as_float((uint32_t)w.kx | ((uint32_t)w.ky << 2) | ((uint32_t)w.kz << 4)));
+                        sm.hits[lane].w = __int_as_float(-1);
+                        sm.tmaxs[lane] = ordered_bits(r.tmax);
+                    }
+                } else {
+                    exhausted = true;
+                }
+            }
+        }
+        if (!__any_sync(0xffffffffu, item >= 0)) break;
+        const unsigned may = __ballot_sync(0xffffffffu, item >= 0 || !exhausted);
+        unsigned walking = __ballot_sync(0xffffffffu, live);
+        __syncwarp();
+        for (;;) {
+            uint2 tg = make_uint2(0u, 0u);
+            if (live) {   // one node per ray
+                const uint32_t ko = 7u ^ nr.oct;
+                const uint32_t b = __ffs(ng.y >> 24) - 1;
+                ng.y &= ~(1u << (24 + b));
+                const uint32_t child = ng.x + __popc(ng.y & 0xffu & ((1u << (b ^ ko)) - 1u));
+                if (ng.y > 0x00ffffffu) {   // the tree's depth bound keeps sp below kStackSize
+                    if (sp < kShStack) sm.stack[32 * sp + lane] = ng;
+                    else if (sp < kStackSize) spill[sp - kShStack] = ng;
+                    ++sp;
+                }
+                visit8<kUnit>(S, child, nr, ng, tg);
+                if (ng.y <= 0x00ffffffu) {
+                    if (sp == 0) {
+                        live = false;
+                    } else {
+                        --sp;
+                        ng = sp < kShStack ? sm.stack[32 * sp + lane] : spill[sp - kShStack];
+                    }
+                }
+            }
+            const uint32_t cnt = __popc(tg.y);
+            if (__any_sync(0xffffffffu, cnt != 0u)) {
+                uint32_t incl = cnt;   // inclusive prefix of the counts in lane order
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= (unsigned)o) incl += v;
+                }
+                const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+                st.tris += total;
+                if (total <= kTriRing - pend) {
+                    uint32_t at = head + pend + (incl - cnt);
+                    while (tg.y != 0u) {
+                        const uint32_t b = __ffs(tg.y) - 1;
+                        tg.y &= tg.y - 1u;
+                        sm.ring[at & (kTriRing - 1u)] = (tg.x + b) | (lane << kTriOwnerShift);
+                        ++at;
+                    }
+                    pend += total;
+                    while (pend >= 32u) test_batch(32u);
+                } else {   // more triangles than the ring has room for: in passes
+                    uint32_t pos = incl - cnt, dealt = 0;
+                    while (dealt < total) {
+                        const uint32_t room = kTriRing - pend;
+                        while (tg.y != 0u && pos < dealt + room) {
+                            const uint32_t b = __ffs(tg.y) - 1;
+                            tg.y &= tg.y - 1u;
+                            sm.ring[(head + pend + (pos - dealt)) & (kTriRing - 1u)] = (tg.x + b) | (lane << kTriOwnerShift);
+                            ++pos;
+                        }
+                        const uint32_t moved = min(total - dealt, room);
+                        pend += moved;
+                        dealt += moved;
+                        while (pend >= 32u) test_batch(32u);
+                    }
+                }
+            }
+            // once min_idle of the lanes that could hold a ray walk none, end their rays and refill
+            st.nodes += __popc(walking);
+            walking = __ballot_sync(0xffffffffu, live);
+            if (walking == 0u || __popc(may & ~walking) >= min_idle) break;
+        }
+        if (__any_sync(0xffffffffu, item >= 0 && !live)) {
+            if (pend) test_batch(pend);   // fewer than 32 are left here
+            if (item >= 0 && !live) {
+                Hit h;
+                h.t = h.u = h.v = 0.0f;
+                h.tri = -1;
+                if constexpr (!kAnyHit) {
+                    const float4 r = sm.hits[lane];
+                    h.t = r.x; h.u = r.y; h.v = r.z;
+                    h.tri = __float_as_int(r.w);
+                    found = h.tri >= 0;
+                }
+                store(item, found, h);
+                item = -1;
+            }
+        }
+        __syncwarp();   // every read of a lane's records precedes their replacement
+    }
+}
+
+}  // namespace hk

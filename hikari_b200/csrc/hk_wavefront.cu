@@ -97,9 +97,7 @@ __global__ void __launch_bounds__(256) wf_regen_kernel(DevScene S, WfState W, in
     __shared__ int s_active;
     __shared__ unsigned s_warp[2][8];   // per-warp counts, then offsets, of the extend / idle appends
     __shared__ unsigned s_base[2];
-    for (int k = threadIdx.x; k < kWfMaxJobs; k += blockDim.x) s_finished[k] = 0u;
-    if (threadIdx.x == 0) s_active = 0;
-    __syncthreads();
+    const int njobs = (int)W.ctr->job_count;
     const int nf = (int)W.ctr->fq_count;
     const uint64_t total = W.ctr->total_work;
     const uint64_t first = W.ctr->next_work;
@@ -107,6 +105,11 @@ __global__ void __launch_bounds__(256) wf_regen_kernel(DevScene S, WfState W, in
     const bool drained = !W.recycle && first + (uint64_t)n >= total;   // this pass deals the plan's last item
     if (drained) n = max(nf, (int)min((uint64_t)n, total - min(first, total)));
     const int nseg = (int)W.ctr->seg_count;
+    const bool some = (int)(blockIdx.x * blockDim.x) < n;   // block-uniform: slots for this block
+    if (some)
+        for (int k = threadIdx.x; k < njobs; k += blockDim.x) s_finished[k] = 0u;
+    if (threadIdx.x == 0) s_active = 0;
+    __syncthreads();
     const unsigned lane = lane_id(), warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     unsigned long long dropped = 0;
     int active_delta = 0;
@@ -197,7 +200,7 @@ __global__ void __launch_bounds__(256) wf_regen_kernel(DevScene S, WfState W, in
     for (int o = 16; o > 0; o >>= 1) active_delta += __shfl_down_sync(0xffffffffu, active_delta, o);
     if (lane == 0 && active_delta) atomicAdd(&s_active, active_delta);
     __syncthreads();
-    for (int k = threadIdx.x; k < kWfMaxJobs; k += blockDim.x)
+    for (int k = threadIdx.x; some && k < njobs; k += blockDim.x)
         if (s_finished[k]) atomicAdd(W.jobs[k].finished, (unsigned long long)s_finished[k]);
     // the last block through resets the counters of the queues consumed here
     // and of those that the next phases fill, and decides whether the

@@ -82,7 +82,7 @@ struct WfSeg {
     int32_t pad;
 };
 
-// Device-wide counters of the engine (one struct in HBM).  The first three
+// Device-wide counters of the engine (one struct in HBM).  The first four
 // fields are the dispatch head, rewritten by the host with each plan.
 constexpr int kWfLaunchLog = 1024;   // launches whose ray counts the counters keep
 
@@ -90,7 +90,7 @@ struct WfCounters {
     unsigned long long next_work;      // next plan item to hand out
     unsigned long long total_work;     // plan items in the current plan
     unsigned int seg_count;            // pieces in the current plan
-    unsigned int pad0;
+    unsigned int job_count;            // job-table entries in use: the highest one set + 1
     unsigned int eq_count[2];          // extend queues (ping-pong)
     unsigned int idle_count[2];        // slots without a path (ping-pong)
     unsigned int sq_count[kWfTypes];   // shade queues per material type

@@ -66,12 +66,14 @@ __device__ __forceinline__ int find_seg(const WfState &W, uint64_t w, int nseg) 
 // ------------------------------------------------------------ shade
 __device__ __forceinline__ void finish(const WfState &W, int slot) { W.fq[warp_append(&W.ctr->fq_count)] = slot; }
 
-// kMinBlocks = 0 leaves the register budget to the compiler; kLeanShade asks
-// for four resident blocks of 256 threads (at most 64 registers): more warps
-// to hide the latency of the path-state and scene gathers, at the price of
-// some spilling.  Only the untextured queues (0-5) come in both budgets.
+// Register budgets: the kernels of untextured materials are held to three
+// resident blocks of 256 threads (80 registers; left to itself the compiler
+// takes up to 122 for the coating, and the shade phase of the 64-sphere scene
+// 16.1 instead of 15.4 ms), the others, whose calls need 128 anyway, are left
+// alone.  kLeanShade asks for four blocks (64 registers, more spilling: 15.0 ms
+// there, but 13.2 instead of 12.5 on the Cornell box); only queues 0-5 have it.
 constexpr int kLeanShade = 4;
-template <int kType, int kMinBlocks = 0>
+template <int kType, int kMinBlocks = kType < kWfTexturedQueue0 ? 3 : 0>
 __global__ void __launch_bounds__(256, kMinBlocks) wf_shade_kernel(DevScene S, WfState W, int nxt) {
     const int n = (int)W.ctr->sq_count[kType];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
