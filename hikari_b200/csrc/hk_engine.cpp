@@ -8,6 +8,8 @@
 namespace hk {
 
 namespace {
+// bytes of an allocation's part
+constexpr size_t part(size_t n) { return (n + 255) & ~(size_t)255; }
 // queue arrays of one slot id per slot: 2 extend, 2 idle, the scene's shade queues, 1 finished
 int queue_arrays(uint32_t shade_queues) { return 5 + __builtin_popcount(shade_queues); }
 }  // namespace
@@ -15,8 +17,9 @@ int queue_arrays(uint32_t shade_queues) { return 5 + __builtin_popcount(shade_qu
 size_t WfEngine::bytes_for(int capacity, int nemitters, uint32_t shade_queues) {
     const size_t N = (size_t)capacity;
     const size_t shadow = N * (size_t)std::max(1, nemitters);
-    return N * kSlotBytes + N * sizeof(int) * queue_arrays(shade_queues) + shadow * 16 * 3 + sizeof(WfCounters) +
-           (sizeof(WfJob) + sizeof(unsigned long long)) * kWfMaxJobs + sizeof(WfSeg) * kWfMaxSegs;
+    return part(N * kSlotBytes) + part(N * sizeof(int) * queue_arrays(shade_queues)) + part(shadow * 16 * 3) +
+           part(sizeof(WfCounters)) + part(sizeof(WfJob) * kWfMaxJobs) + part(sizeof(unsigned long long) * kWfMaxJobs) +
+           part(sizeof(WfSeg) * kWfMaxSegs);
 }
 
 WfEngine::WfEngine(const DevScene &S, int sm_count, const WfEngineConfig &cfg) : S_(S), cfg_(cfg) {
@@ -28,15 +31,34 @@ WfEngine::WfEngine(const DevScene &S, int sm_count, const WfEngineConfig &cfg) :
     const size_t N = (size_t)cfg_.capacity;
     W_.capacity = cfg_.capacity;
     W_.max_shadow = cfg_.capacity * std::max(1, S.nemitters);
-    state_.alloc(N * kSlotBytes);
-    queues_.alloc(N * sizeof(int) * queue_arrays(S.shade_queues));
-    shadow_.alloc((size_t)W_.max_shadow * 16 * 3);
-    counters_.alloc(sizeof(WfCounters));
-    jobs_.alloc(sizeof(WfJob) * kWfMaxJobs);
-    finished_.alloc(sizeof(unsigned long long) * kWfMaxJobs);
-    segs_.alloc(sizeof(WfSeg) * kWfMaxSegs);
     bytes_ = bytes_for(cfg_.capacity, S.nemitters, S.shade_queues);
-    char *rec = state_.as<char>();   // slot records (kSlotBytes each, 256-byte aligned base)
+    // one device and one pinned host allocation, carved up (256-byte aligned parts)
+    mem_.alloc(bytes_);
+    char *at = mem_.as<char>();
+    auto take = [](char *&p, size_t n) {
+        char *r = p;
+        p += part(n);
+        return r;
+    };
+    char *rec = take(at, N * kSlotBytes);   // slot records
+    int *q = (int *)take(at, N * sizeof(int) * queue_arrays(S.shade_queues));
+    float4 *sh = (float4 *)take(at, (size_t)W_.max_shadow * 16 * 3);
+    W_.ctr = (WfCounters *)take(at, sizeof(WfCounters));
+    jobs_ = (WfJob *)take(at, sizeof(WfJob) * kWfMaxJobs);
+    finished_ = (unsigned long long *)take(at, sizeof(unsigned long long) * kWfMaxJobs);
+    segs_ = (WfSeg *)take(at, sizeof(WfSeg) * kWfMaxSegs);
+    W_.jobs = jobs_;
+    W_.segs = segs_;
+    const size_t host_bytes = 2 * part(sizeof(WfCounters)) + part(sizeof(unsigned long long) * kWfMaxJobs) +
+                              part(sizeof(WfJob) * kWfMaxJobs) + part(sizeof(WfSeg) * kWfMaxSegs);
+    host_.alloc(host_bytes);
+    std::memset(host_.p, 0, host_bytes);
+    at = host_.p;
+    h_ctr_ = (WfCounters *)take(at, sizeof(WfCounters));
+    h_head_ = (WfCounters *)take(at, sizeof(WfCounters));
+    h_fin_ = (unsigned long long *)take(at, sizeof(unsigned long long) * kWfMaxJobs);
+    h_jobs_ = (WfJob *)take(at, sizeof(WfJob) * kWfMaxJobs);
+    h_segs_ = (WfSeg *)take(at, sizeof(WfSeg) * kWfMaxSegs);
     W_.ray_o.p = (float4 *)(rec + 0);
     W_.ray_d.p = (float4 *)(rec + 16);
     W_.beta.p = (float4 *)(rec + 32);
@@ -45,25 +67,13 @@ WfEngine::WfEngine(const DevScene &S, int sm_count, const WfEngineConfig &cfg) :
     W_.hit.p = (float4 *)(rec + 80);
     W_.lacc.p = (float4 *)(rec + 96);
     W_.prev_pdf.p = (float *)(rec + 112);
-    int *q = queues_.as<int>();
     W_.eq[0] = q; W_.eq[1] = q + N;
     W_.idle[0] = q + 2 * N; W_.idle[1] = q + 3 * N;
     W_.fq = q + 4 * N;
     q += 5 * N;
     for (int t = 0; t < kWfTypes; ++t)
         if (S.shade_queues >> t & 1u) { W_.sq[t] = q; q += N; }
-    float4 *sh = shadow_.as<float4>();
     W_.sh_o = sh; W_.sh_d = sh + W_.max_shadow; W_.sh_c = sh + 2 * (size_t)W_.max_shadow;
-    W_.ctr = counters_.as<WfCounters>();
-    W_.jobs = jobs_.as<WfJob>();
-    W_.segs = segs_.as<WfSeg>();
-    h_ctr_.alloc(1);
-    h_fin_.alloc(kWfMaxJobs);
-    h_jobs_.alloc(kWfMaxJobs);
-    h_segs_.alloc(kWfMaxSegs);
-    h_head_.alloc(1);
-    std::memset(h_ctr_.p, 0, sizeof(WfCounters));
-    std::memset(h_fin_.p, 0, sizeof(unsigned long long) * kWfMaxJobs);
     int least = 0, greatest = 0;
     HK_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
     HK_CUDA(cudaStreamCreateWithPriority(&streams_[0], cudaStreamNonBlocking, least));
@@ -144,28 +154,34 @@ void WfEngine::set_priority(bool high) {
 
 void WfEngine::reset(int slots) {
     set_plan({}, 0);
-    HK_CUDA(wf_launch_init(W_, slots > 0 ? std::min(slots, W_.capacity) : W_.capacity, stream_));
+    HK_CUDA(wf_launch_init(W_, slots > 0 ? std::min(slots, W_.capacity) : W_.capacity, WfJob{}, stream_));
+}
+
+void WfEngine::begin(WfJob J, int slots) {
+    J.finished = finished_;
+    job_count_ = std::max(job_count_, 1);
+    HK_CUDA(wf_launch_init(W_, std::min(slots, W_.capacity), J, stream_));
 }
 
 void WfEngine::set_job(int slot, WfJob J) {
     if (slot < 0 || slot >= kWfMaxJobs) throw HkError{HK_ERR_INVALID, "job slot out of range"};
     // Each slot has its own staging entry; a slot is rewritten only after its
     // previous job ended, long after that job's copy ran.
-    J.finished = finished_.as<unsigned long long>() + slot;
+    J.finished = finished_ + slot;
     job_count_ = std::max(job_count_, slot + 1);
-    h_jobs_.p[slot] = J;
-    HK_CUDA(cudaMemcpyAsync(jobs_.as<WfJob>() + slot, h_jobs_.p + slot, sizeof(WfJob), cudaMemcpyHostToDevice, stream_));
-    HK_CUDA(cudaMemsetAsync(finished_.as<unsigned long long>() + slot, 0, sizeof(unsigned long long), stream_));
+    h_jobs_[slot] = J;
+    HK_CUDA(cudaMemcpyAsync(jobs_ + slot, h_jobs_ + slot, sizeof(WfJob), cudaMemcpyHostToDevice, stream_));
+    HK_CUDA(cudaMemsetAsync(finished_ + slot, 0, sizeof(unsigned long long), stream_));
 }
 
 void WfEngine::set_plan(const std::vector<WfSeg> &segs, uint64_t total) {
     if (segs.size() > (size_t)kWfMaxSegs) throw HkError{HK_ERR_INVALID, "dispatch plan has too many pieces"};
     HK_CUDA(cudaEventSynchronize(ev_plan_));   // the staging copies of the previous plan have run
     if (!segs.empty()) {
-        std::memcpy(h_segs_.p, segs.data(), sizeof(WfSeg) * segs.size());
-        HK_CUDA(cudaMemcpyAsync(segs_.p, h_segs_.p, sizeof(WfSeg) * segs.size(), cudaMemcpyHostToDevice, stream_));
+        std::memcpy(h_segs_, segs.data(), sizeof(WfSeg) * segs.size());
+        HK_CUDA(cudaMemcpyAsync(segs_, h_segs_, sizeof(WfSeg) * segs.size(), cudaMemcpyHostToDevice, stream_));
     }
-    WfCounters &h = *h_head_.p;
+    WfCounters &h = *h_head_;
     h.next_work = 0;
     h.total_work = total;
     h.seg_count = (unsigned)segs.size();
@@ -250,13 +266,15 @@ void WfEngine::run(int iterations, bool use_graph, float *kernel_ms, int32_t *ke
 }
 
 void WfEngine::fetch_status() {
-    HK_CUDA(cudaMemcpyAsync(h_ctr_.p, W_.ctr, offsetof(WfCounters, log_n), cudaMemcpyDeviceToHost, stream_));
-    HK_CUDA(cudaMemcpyAsync(h_fin_.p, finished_.p, sizeof(unsigned long long) * kWfMaxJobs, cudaMemcpyDeviceToHost,
+    HK_CUDA(cudaMemcpyAsync(h_ctr_, W_.ctr, offsetof(WfCounters, log_n), cudaMemcpyDeviceToHost, stream_));
+    HK_CUDA(cudaMemcpyAsync(h_fin_, finished_, sizeof(unsigned long long) * kWfMaxJobs, cudaMemcpyDeviceToHost,
                             stream_));
     HK_CUDA(cudaEventRecord(ev_done_, stream_));
 }
 
-void WfEngine::add_counters(unsigned long long *out_dev) { HK_CUDA(wf_launch_counters_add(W_, out_dev, stream_)); }
+void WfEngine::add_counters(unsigned long long *out_dev, bool sum) {
+    HK_CUDA(wf_launch_counters_add(W_, out_dev, sum, stream_));
+}
 
 int WfEngine::launch_log(int which, uint32_t *rays, int max) {
     unsigned n = 0;

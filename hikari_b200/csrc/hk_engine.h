@@ -49,6 +49,9 @@ public:
 
     // Empty pool (the first `slots` slots idle, 0: all), zero statistics, empty plan.  Async on stream().
     void reset(int slots = 0);
+    // The start of a render of one job: reset(slots), the job in entry 0 and its
+    // plan, in one launch without staging copies.  Async, and never waits.
+    void begin(WfJob J, int slots);
     // Job-table entry `slot`: its finished counter is zeroed and J.finished set.  Async;
     // the slot must not be in use by paths in flight.
     void set_job(int slot, WfJob J);
@@ -65,10 +68,11 @@ public:
     // and record done_event(); read them after the event completed.
     void fetch_status();
     cudaEvent_t done_event() const { return ev_done_; }
-    const WfCounters &status() const { return *h_ctr_.p; }
-    const unsigned long long *finished() const { return h_fin_.p; }
-    // Add the statistics to a caller's 7-slot device array.  Async.
-    void add_counters(unsigned long long *out_dev);
+    const WfCounters &status() const { return *h_ctr_; }
+    const unsigned long long *finished() const { return h_fin_; }
+    // Add the statistics to a caller's 7-slot device array (sum: 5 slots, the
+    // traversal totals over both ray kinds).  Async.
+    void add_counters(unsigned long long *out_dev, bool sum = false);
     // Rays of each extend (which 0) / shadow (which 1) launch since the last
     // reset, in launch order: up to max of them into rays (host); returns the
     // number of launches.  Synchronises the engine's stream.
@@ -84,12 +88,15 @@ private:
     WfState W_{};
     size_t bytes_ = 0;
     int job_count_ = 0;   // highest job slot ever set + 1
-    DevBuf state_, queues_, shadow_, counters_, jobs_, finished_, segs_;
-    PinnedBuf<WfCounters> h_ctr_;
-    PinnedBuf<unsigned long long> h_fin_;
-    PinnedBuf<WfJob> h_jobs_;
-    PinnedBuf<WfSeg> h_segs_;
-    PinnedBuf<WfCounters> h_head_;
+    DevBuf mem_;             // slot records, queues, shadow queue, counters, job table, plan
+    PinnedBuf<char> host_;   // the host mirrors below
+    WfCounters *h_ctr_ = nullptr, *h_head_ = nullptr;
+    unsigned long long *h_fin_ = nullptr;
+    WfJob *h_jobs_ = nullptr;
+    WfSeg *h_segs_ = nullptr;
+    WfJob *jobs_ = nullptr;   // device
+    WfSeg *segs_ = nullptr;
+    unsigned long long *finished_ = nullptr;
     cudaStream_t stream_ = nullptr;             // current: streams_[0] or streams_[1]
     cudaStream_t streams_[2] = {nullptr, nullptr};   // low, high priority
     cudaEvent_t ev_switch_ = nullptr;

@@ -259,7 +259,10 @@ struct hk_scene {
     hk_wavefront_config wf_cfg{};              // wavefront configuration of hk_render_image
     int occupancy = 1;        // resident megakernel CTAs per SM for the traversed tree
     int occupancy_of[2] = {1, 1};
-    std::unique_ptr<hk::WfEngine> wf;   // wavefront engine (allocated on first use)
+    // wavefront engines, allocated on first use: of the pool size that a caller
+    // named, and fitted to the work; the one that rendered last
+    std::unique_ptr<hk::WfEngine> wf, wf_fit;
+    hk::WfEngine *wf_last = nullptr;
 };
 
 namespace {
@@ -574,6 +577,12 @@ hk::DevBsdf activate_bsdf(const hk_scene *s, const hk_bsdf_desc &d, int n_bsdfs,
     return b;
 }
 
+void drop_engines(hk_scene *s) {
+    s->wf_last = nullptr;
+    s->wf.reset();
+    s->wf_fit.reset();
+}
+
 void build_scene(hk_scene *s) {
     if (s->meshes.empty()) throw HkError{HK_ERR_INVALID, "scene has no meshes"};
     if (s->width == 0 || s->height == 0) throw HkError{HK_ERR_INVALID, "camera has an empty film"};
@@ -586,7 +595,7 @@ void build_scene(hk_scene *s) {
         if ((t == hk::kBumpMap || t == hk::kNormalMap) && (m.nrm.empty() || m.uv.empty()))
             throw HkError{HK_ERR_INVALID, "a mesh with a bumpMap / normalMap BSDF needs vertex normals and texture coordinates"};
     }
-    s->wf.reset();   // the engine holds a copy of the device description that is rebuilt here
+    drop_engines(s);   // they hold a copy of the device description that is rebuilt here
     hk::DevScene &D = s->dev;
     std::memset(&D, 0, sizeof D);
     size_t dev_bytes = 0;
@@ -1011,20 +1020,34 @@ void require_scene_size(const hk_scene *s, const hk_render_desc &d) {
 }
 
 // ------------------------------------------------------------ wavefront engine
+// The scene's engine of configuration c.  Pools fitted to the work and pools
+// that a caller sized are kept apart, so that alternating calls of the two kinds
+// do not rebuild them; a fitted one serves every call that needs no more slots.
 hk::WfEngine &wf_ensure(hk_scene *s, const hk::WfEngineConfig &c) {
-    if (s->wf) {
-        const hk::WfEngineConfig &o = s->wf->config();
-        // a pool fitted to an earlier call's work serves every call that needs no more slots
-        const bool fits = o.capacity == c.capacity || (o.fit_capacity && c.fit_capacity && o.capacity >= c.capacity);
-        if (fits && o.fit_capacity == c.fit_capacity && o.threads_extend == c.threads_extend && o.threads_shade == c.threads_shade &&
-            o.fetch_steps == c.fetch_steps && o.fetch_min_idle == c.fetch_min_idle &&
+    std::unique_ptr<hk::WfEngine> &e = c.fit_capacity ? s->wf_fit : s->wf;
+    if (e) {
+        const hk::WfEngineConfig &o = e->config();
+        if ((c.fit_capacity ? o.capacity >= c.capacity : o.capacity == c.capacity) && o.threads_extend == c.threads_extend &&
+            o.threads_shade == c.threads_shade && o.fetch_steps == c.fetch_steps && o.fetch_min_idle == c.fetch_min_idle &&
             o.fetch_steps_shadow == c.fetch_steps_shadow && o.fetch_min_idle_shadow == c.fetch_min_idle_shadow &&
-            o.reg_lean == c.reg_lean)
-            return *s->wf;
-        s->wf.reset();
+            o.reg_lean == c.reg_lean) {
+            s->wf_last = e.get();
+            return *e;
+        }
+        if (s->wf_last == e.get()) s->wf_last = nullptr;
+        e.reset();
     }
-    s->wf.reset(new hk::WfEngine(s->dev, s->sm_count, c));
-    return *s->wf;
+    try {
+        e.reset(new hk::WfEngine(s->dev, s->sm_count, c));
+    } catch (const HkError &) {
+        if (c.fit_capacity || !s->wf_fit) throw;
+        cudaGetLastError();   // short of memory: the fitted pool makes room
+        if (s->wf_last == s->wf_fit.get()) s->wf_last = nullptr;
+        s->wf_fit.reset();
+        e.reset(new hk::WfEngine(s->dev, s->sm_count, c));
+    }
+    s->wf_last = e.get();
+    return *e;
 }
 
 }  // namespace
@@ -1311,8 +1334,8 @@ int hk_wavefront_launch_log(hk_scene *s, int32_t which, uint32_t *rays_host, int
         require_built(s);
         if ((which != 0 && which != 1) || max < 0 || (max > 0 && !rays_host) || !launches)
             throw HkError{HK_ERR_INVALID, "bad arguments"};
-        if (!s->wf) throw HkError{HK_ERR_INVALID, "the scene has not rendered with the wavefront integrator"};
-        *launches = s->wf->launch_log(which, rays_host, max);
+        if (!s->wf_last) throw HkError{HK_ERR_INVALID, "the scene has not rendered with the wavefront integrator"};
+        *launches = s->wf_last->launch_log(which, rays_host, max);
         return HK_OK;
     });
 }
@@ -1343,7 +1366,7 @@ int hk_scene_set_accel(hk_scene *s, int32_t accel) {
         s->dev.accel = accel;
         s->info.accel = accel;
         s->occupancy = s->occupancy_of[accel];
-        s->wf.reset();   // the engine holds a copy of the device description
+        drop_engines(s);   // they hold a copy of the device description
         return HK_OK;
     });
 }
@@ -1378,6 +1401,79 @@ int hk_scene_get_info(const hk_scene *s, hk_scene_info *info) {
     });
 }
 
+static hk::WfEngineConfig engine_config(const hk_wavefront_config &c, uint64_t work) {
+    hk::WfEngineConfig ec;
+    ec.capacity = std::max(1024, std::min(c.capacity, 1 << 26));
+    ec.threads_extend = c.threads_extend > 0 ? c.threads_extend : 128;
+    ec.threads_shade = c.threads_shade > 0 ? c.threads_shade : 128;
+    ec.fetch_steps = std::max(0, std::min(1024, c.fetch_steps));
+    ec.fetch_min_idle = c.fetch_min_idle > 0 ? std::min(32, c.fetch_min_idle) : 0;
+    ec.fetch_steps_shadow = std::max(0, std::min(1024, c.fetch_steps_shadow));
+    ec.fetch_min_idle_shadow = c.fetch_min_idle_shadow > 0 ? std::min(32, c.fetch_min_idle_shadow) : 0;
+    ec.reg_lean = c.reg_lean & 7;
+    if (c.capacity <= 0) {   // as many slots as the work can use, from 2^14 to 2^21
+        ec.fit_capacity = true;
+        ec.capacity = 1 << 14;
+        while (ec.capacity < (1 << 21) && (uint64_t)ec.capacity < work) ec.capacity *= 2;
+    }
+    return ec;
+}
+// Whether a render of the scene's own image goes to the wavefront: from 2^18
+// paths on.  Measured on five scenes (Cornell boxes of diffuse and of smooth
+// materials, a glass sphere, 64 spheres, textures; depth 16), megakernel /
+// wavefront: 2^16 paths 0.8-4.8 / 0.8-2.5 ms, 2^18 paths 1.5-13.8 / 1.2-3.1 ms,
+// 2^20 paths 4-46 / 2.5-4.9 ms; below 2^16 the wavefront's five launches a
+// bounce cost more than the megakernel's divergence, and a scene's first
+// wavefront render spends 2 ms on its pool and graph.
+static bool work_for_wavefront(const hk_scene *s, const hk_render_desc &d) {
+    if (s->image_form == HK_FORM_MEGAKERNEL || d.depth < 1 || d.depth > 65535) return false;
+    return (uint64_t)s->width * s->height * (uint64_t)d.spp >= (1ull << 18);
+}
+// hk_render through the wavefront, asynchronous on `stream` like the
+// megakernel: one launch that sets the pool, job and plan up, one graph whose
+// loop ends by itself, one for the counters.  False (nothing launched) where
+// the stream is being captured into a graph, which cannot hold a loop, where
+// the loop's bound might be reached, or where there is no memory for the pool.
+static bool render_wavefront_async(hk_scene *s, const hk_render_desc &d, float *film, unsigned long long *counters,
+                                   cudaStream_t stream) {
+    const hk_wavefront_config c = s->has_wf_cfg ? s->wf_cfg : hk_wavefront_config{};
+    if (c.no_graph) return false;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return false;
+    }
+    hk_render_desc own = d;
+    own.width = own.height = 0;
+    hk::WfJob J = hk::make_wf_job(s, own);
+    J.film = film;
+    J.sample_major = c.sample_major ? 1 : 0;
+    const hk::WfEngineConfig ec = engine_config(c, J.work_count);
+    // every pass of the loop (a pair of iterations) advances each slot in use by two vertices
+    if ((J.work_count / (uint64_t)ec.capacity + 1) * (uint64_t)d.depth + 64 > hk::kWfMaxLoops) return false;
+    hk::WfEngine *E;
+    try {
+        E = &wf_ensure(s, ec);
+    } catch (const HkError &e) {
+        if (e.code == HK_ERR_INVALID) throw;
+        cudaGetLastError();
+        return false;
+    }
+    cudaEvent_t ev;
+    HK_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    struct EvGuard {
+        cudaEvent_t e;
+        ~EvGuard() { cudaEventDestroy(e); }
+    } guard{ev};
+    HK_CUDA(cudaEventRecord(ev, stream));
+    HK_CUDA(cudaStreamWaitEvent(E->stream(), ev, 0));
+    E->begin(J, (int)std::min<uint64_t>(J.work_count, (uint64_t)ec.capacity));
+    E->run_to_end();
+    if (counters) E->add_counters(counters, true);
+    HK_CUDA(cudaEventRecord(ev, E->stream()));
+    HK_CUDA(cudaStreamWaitEvent(stream, ev, 0));
+    return true;
+}
 // Blocks of a megakernel launch: one wave of resident ones, fewer where the paths need fewer lanes.
 static int render_grid(const hk_scene *s, int spp) {
     const uint64_t paths = (uint64_t)s->width * s->height * (uint64_t)spp;
@@ -1390,7 +1486,9 @@ int hk_render(hk_scene *s, const hk_render_desc *d, float *film, unsigned long l
         if (!d || !film) throw HkError{HK_ERR_INVALID, "bad arguments"};
         if (d->spp <= 0 || d->depth < 0) throw HkError{HK_ERR_INVALID, "spp must be > 0 and depth >= 0"};
         require_scene_size(s, *d);
+        if (d->use_camera && d->camera_to_world[15] == 0.0f) throw HkError{HK_ERR_INVALID, "camera_to_world has w = 0"};
         cudaStream_t st = (cudaStream_t)stream;
+        if (work_for_wavefront(s, *d) && render_wavefront_async(s, *d, film, counters, st)) return HK_OK;
         hk::RenderLaunch P;
         std::memset(&P, 0, sizeof P);
         P.film = film;
@@ -1428,16 +1526,6 @@ int hk_film_resolve(hk_scene *s, const float *film, float *rgb, void *stream) {
         return HK_OK;
     });
 }
-// Whether hk_render_image renders this call with the wavefront: always for
-// HK_FORM_WAVEFRONT; for HK_FORM_AUTO once the image has at least 256 x 256
-// pixels and 2^22 paths (below that a pool of path slots cannot fill the GPU
-// better than the megakernel's persistent tiles).
-static bool image_uses_wavefront(const hk_scene *s, const hk_render_desc &d) {
-    if (s->image_form == HK_FORM_WAVEFRONT) return true;
-    if (s->image_form == HK_FORM_MEGAKERNEL) return false;
-    const uint64_t px = (uint64_t)s->width * s->height;
-    return px >= 65536 && px * (uint64_t)std::max(d.spp, 0) >= (1ull << 22);
-}
 int hk_render_image(hk_scene *s, const hk_render_desc *d, float *rgb_host, unsigned long long *counters, void *stream) {
     return guarded([&] {
         require_built(s);
@@ -1449,11 +1537,12 @@ int hk_render_image(hk_scene *s, const hk_render_desc *d, float *rgb_host, unsig
         size_t film_bytes = FW * FH * 4 * sizeof(float), rgb_bytes = (size_t)s->width * s->height * 3 * sizeof(float);
         if (s->b_film.bytes < film_bytes) s->b_film.alloc(film_bytes);
         if (s->b_rgb.bytes < rgb_bytes) s->b_rgb.alloc(rgb_bytes);
-        // counters: [1..5] the megakernel's, [8..14] the wavefront's 7
+        // counters: [1..5] those of hk_render, [8..14] hk_render_batch's 7
         unsigned long long *ctr = (unsigned long long *)s->b_scratch.p + 1;
         unsigned long long *ctr7 = (unsigned long long *)s->b_scratch.p + 8;
         HK_CUDA(cudaMemsetAsync(s->b_film.p, 0, film_bytes, st));
-        const bool wave = image_uses_wavefront(s, *d);
+        // HK_FORM_WAVEFRONT: small images too, through the batch
+        const bool wave = s->image_form == HK_FORM_WAVEFRONT;
         int rc;
         if (wave) {
             HK_CUDA(cudaMemsetAsync(ctr7, 0, 7 * sizeof(unsigned long long), st));
@@ -1572,15 +1661,6 @@ int hk_render_batch(hk_scene *s, const hk_render_job *jobs, int njobs, const hk_
         if (!jobs || njobs <= 0 || njobs > hk::kWfMaxJobs) throw HkError{HK_ERR_INVALID, "need 1..1024 jobs"};
         hk_wavefront_config c{};
         if (cfg) c = *cfg;
-        hk::WfEngineConfig ec;
-        ec.capacity = std::max(1024, std::min(c.capacity, 1 << 26));
-        ec.threads_extend = c.threads_extend > 0 ? c.threads_extend : 128;
-        ec.threads_shade = c.threads_shade > 0 ? c.threads_shade : 128;
-        ec.fetch_steps = std::max(0, std::min(1024, c.fetch_steps));
-        ec.fetch_min_idle = c.fetch_min_idle > 0 ? std::min(32, c.fetch_min_idle) : 0;
-        ec.fetch_steps_shadow = std::max(0, std::min(1024, c.fetch_steps_shadow));
-        ec.fetch_min_idle_shadow = c.fetch_min_idle_shadow > 0 ? std::min(32, c.fetch_min_idle_shadow) : 0;
-        ec.reg_lean = c.reg_lean & 7;
         std::vector<hk::WfJob> table(njobs);
         std::vector<hk::WfSeg> plan(njobs);
         uint64_t total = 0;
@@ -1592,11 +1672,7 @@ int hk_render_batch(hk_scene *s, const hk_render_job *jobs, int njobs, const hk_
             plan[j] = hk::WfSeg{total, 0, j, 0};
             total += table[j].work_count;
         }
-        if (c.capacity <= 0) {   // as many slots as the work can use, from 2^14 to 2^21
-            ec.fit_capacity = true;
-            ec.capacity = 1 << 14;
-            while (ec.capacity < (1 << 21) && (uint64_t)ec.capacity < total) ec.capacity *= 2;
-        }
+        const hk::WfEngineConfig ec = engine_config(c, total);
         hk::WfEngine &E = wf_ensure(s, ec);
         cudaStream_t user = (cudaStream_t)stream, st = E.stream();
         // order after the caller's stream (the films may have been cleared there)
@@ -1687,7 +1763,6 @@ int hk_wavefront_autotune(hk_scene *s, const hk_render_desc *probe, hk_wavefront
         hk_wavefront_config bc{};
         const int caps[] = {1 << 20, 1 << 21, 1 << 22};
         const int threads[] = {64, 128, 256};
-        const int checks[] = {16, 64};
         const int steps2[] = {4, 8, 16};   // binary tree
         const int min_idle[] = {4, 8, 12, 16};
         // a configuration's time: the better of two timed renders after a warm one
@@ -1709,7 +1784,7 @@ int hk_wavefront_autotune(hk_scene *s, const hk_render_desc *probe, hk_wavefront
             }
             return best_ms;
         };
-        // coordinate descent: capacity, then block sizes, then the check interval
+        // coordinate descent: capacity, then block sizes
         hk_wavefront_config c{};
         c.threads_extend = 128; c.threads_shade = 128; c.iterations_per_check = 16;
         for (int cap : caps) {
@@ -1724,12 +1799,6 @@ int hk_wavefront_autotune(hk_scene *s, const hk_render_desc *probe, hk_wavefront
                 float ms = run(c);
                 if (ms < best_t) { best_t = ms; bc = c; }
             }
-        c = bc;
-        for (int k : checks) {
-            c.iterations_per_check = k;
-            float ms = run(c);
-            if (ms < best_t) { best_t = ms; bc = c; }
-        }
         // dynamic ray fetch: node visits between refills (binary tree), idle lanes before a refill
         const bool w2 = s->dev.accel == hk::kAccelBvh2;
         c = bc;

@@ -231,8 +231,11 @@ __global__ void __launch_bounds__(256) wf_regen_kernel(DevScene S, WfState W, in
     }
 }
 
-// Empty pool: the first `slots` slots in idle list 0, all queues and statistics zero.
-__global__ void wf_init_kernel(WfState W, int slots) {
+// Empty pool: the first `slots` slots in idle list 0, all queues and statistics
+// zero.  With a job (work_count > 0) also the table of that one job and its plan:
+// the whole start of a render in one launch, its input passed by value, so a
+// caller can queue renders without the host waiting for a staging buffer.
+__global__ void wf_init_kernel(WfState W, int slots, WfJob J) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < slots; i += gridDim.x * blockDim.x) W.idle[0][i] = i;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         WfCounters *c = W.ctr;
@@ -245,17 +248,28 @@ __global__ void wf_init_kernel(WfState W, int slots) {
         c->rays = c->shadow_rays = c->dropped = 0;
         c->node_visits = c->tri_tests = c->node_visits_shadow = c->tri_tests_shadow = 0;
         c->log_n[0] = c->log_n[1] = 0;
+        if (J.work_count > 0) {
+            c->next_work = 0;
+            c->total_work = J.work_count;
+            c->seg_count = 1;
+            c->job_count = 1;
+            const_cast<WfJob *>(W.jobs)[0] = J;
+            const_cast<WfSeg *>(W.segs)[0] = WfSeg{0, 0, 0, 0};
+            *J.finished = 0;
+        }
     }
 }
 
-// Add the engine's statistics to a caller's 7-slot u64 array.
-__global__ void wf_counters_add_kernel(const WfCounters *c, unsigned long long *out) {
+// Add the engine's statistics to a caller's 7-slot u64 array, or to a 5-slot one
+// with the traversal totals of both ray kinds (sum).
+__global__ void wf_counters_add_kernel(const WfCounters *c, unsigned long long *out, bool sum) {
     if (threadIdx.x != 0) return;
     out[0] += c->rays;
     out[1] += c->shadow_rays;
     out[2] += c->dropped;
-    out[3] += c->node_visits;
-    out[4] += c->tri_tests;
+    out[3] += c->node_visits + (sum ? c->node_visits_shadow : 0);
+    out[4] += c->tri_tests + (sum ? c->tri_tests_shadow : 0);
+    if (sum) return;
     out[5] += c->node_visits_shadow;
     out[6] += c->tri_tests_shadow;
 }
@@ -296,13 +310,13 @@ static cudaError_t launch_shade_all(const DevScene &S, const WfState &W, const W
     return cudaGetLastError();
 }
 
-cudaError_t wf_launch_counters_add(const WfState &W, unsigned long long *out, cudaStream_t st) {
-    wf_counters_add_kernel<<<1, 32, 0, st>>>(W.ctr, out);
+cudaError_t wf_launch_counters_add(const WfState &W, unsigned long long *out, bool sum, cudaStream_t st) {
+    wf_counters_add_kernel<<<1, 32, 0, st>>>(W.ctr, out, sum);
     return cudaGetLastError();
 }
 
-cudaError_t wf_launch_init(const WfState &W, int slots, cudaStream_t st) {
-    wf_init_kernel<<<std::max(1, std::min((slots + 255) / 256, 4096)), 256, 0, st>>>(W, slots);
+cudaError_t wf_launch_init(const WfState &W, int slots, const WfJob &J, cudaStream_t st) {
+    wf_init_kernel<<<std::max(1, std::min((slots + 255) / 256, 4096)), 256, 0, st>>>(W, slots, J);
     return cudaGetLastError();
 }
 

@@ -176,15 +176,17 @@ struct WfLaunchConfig {
 };
 
 // empty pool: the first `slots` slots idle (the others unused), queues and
-// statistics zero (the dispatch head is the host's)
-cudaError_t wf_launch_init(const WfState &W, int slots, cudaStream_t st);
+// statistics zero; J with work: job 0 and the whole plan, otherwise the job
+// table and the dispatch head are the host's
+cudaError_t wf_launch_init(const WfState &W, int slots, const WfJob &J, cudaStream_t st);
 // one iteration with extend queue `cur` (0/1)
 cudaError_t wf_launch_iteration(const DevScene &S, const WfState &W, const WfLaunchConfig &C, int cur, cudaStream_t st);
 // one phase of an iteration: 0 regen + reset, 1 extend, 2 shade (all materials), 3 shadow
 cudaError_t wf_launch_phase(const DevScene &S, const WfState &W, const WfLaunchConfig &C, int cur, int phase,
                             cudaStream_t st);
-// out[0..6] += rays, shadow rays, dropped, node visits, triangle tests, shadow node visits, shadow tests
-cudaError_t wf_launch_counters_add(const WfState &W, unsigned long long *out, cudaStream_t st);
+// out[0..6] += rays, shadow rays, dropped, node visits, triangle tests, shadow
+// node visits, shadow tests; sum: out[0..4] with the visits and tests of both kinds
+cudaError_t wf_launch_counters_add(const WfState &W, unsigned long long *out, bool sum, cudaStream_t st);
 // resident blocks per SM of a kernel (which: 0 extend, 2 shadow, 3 regen) and
 // of a queue's shade kernel; lean: the smaller register budget
 int wf_occupancy(int which, int threads, int accel, bool lean = false);

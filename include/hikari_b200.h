@@ -244,7 +244,7 @@ typedef struct {
     int32_t sample_offset;  /* index of the first sample (progressive accumulation) */
     uint64_t seed;
     int32_t image_index;    /* decorrelates streams of several images of one scene */
-    int32_t spp_per_item;   /* 0 = automatic work split */
+    int32_t spp_per_item;   /* unused: lanes take paths as they become free */
     int32_t use_camera;     /* 1: render from camera_to_world instead of the scene camera */
     float camera_to_world[16];
     int32_t width, height;  /* image size; 0 = the scene camera's (wavefront and serving only:
@@ -254,7 +254,12 @@ typedef struct {
 /* Accumulate spp samples per pixel into film_dev ((H+2B)*(W+2B)*4 floats of
  * RGB*w and w, B = ceil(radius - 0.5)); counters_dev (optional, 5 x u64) gets
  * closest-hit rays, shadow rays, dropped (invalid) samples, BVH node visits
- * and triangle tests added. */
+ * and triangle tests added.  Asynchronous on `stream`.  Renders of 2^18 paths
+ * and more go to the wavefront integrator (its pool, sized to the work, is
+ * allocated on first use and kept by the scene), smaller ones, captures of the
+ * stream into a graph and calls without memory for the pool to the megakernel;
+ * HK_FORM_MEGAKERNEL keeps all of them there.  Both forms draw the same
+ * per-sample streams. */
 int hk_render(hk_scene *s, const hk_render_desc *desc, float *film_dev, unsigned long long *counters_dev,
               void *stream);
 /* film -> H*W*3 RGB (ImageBlock::ToBitmap, src/core/Block.cpp:61) */
@@ -263,16 +268,16 @@ int hk_film_resolve(hk_scene *s, const float *film_dev, float *rgb_dev, void *st
  * makes in place of Render's block loop (src/Main.cpp:46-147): render into
  * the scene's own film, resolve and copy the H*W*3 float image to host memory
  * rgb_host.  counters (host, 5) optional: as hk_render's (node visits and
- * triangle tests summed over closest-hit and shadow rays).  The image is
- * rendered with the wavefront integrator (hk_render_batch, one job) when the
- * scene's image form says so -- by default once it has at least 256 x 256
- * pixels and 2^22 paths -- else with the megakernel (hk_render).  Both run the
- * same estimator on the same per-sample streams: the images agree up to the
- * order of the film's float additions. */
+ * triangle tests summed over closest-hit and shadow rays).  HK_FORM_WAVEFRONT
+ * renders with the wavefront integrator whatever the size (hk_render_batch, one
+ * job), otherwise hk_render picks the form.  Both run the same estimator on the
+ * same per-sample streams: the images agree up to the order of the film's float
+ * additions. */
 int hk_render_image(hk_scene *s, const hk_render_desc *desc, float *rgb_host, unsigned long long *counters,
                     void *stream);
 enum { HK_FORM_AUTO = 0, HK_FORM_MEGAKERNEL = 1, HK_FORM_WAVEFRONT = 2 };
-/* The form hk_render_image renders with (HK_FORM_AUTO by default). */
+/* The form hk_render_image renders with (HK_FORM_AUTO by default);
+ * HK_FORM_MEGAKERNEL holds for hk_render too. */
 int hk_scene_set_image_form(hk_scene *s, int32_t form);
 
 /* ---- wavefront rendering (the batched form) ---- */
@@ -284,11 +289,11 @@ typedef struct {
 } hk_render_job;
 
 typedef struct {
-    int32_t capacity;              /* path slots in flight (0 = 2^21) */
+    int32_t capacity;              /* path slots in flight (0 = as many as the work can use, 2^14 to 2^21) */
     int32_t threads_extend;        /* block size of the extend/shadow kernels (0 = 128) */
     int32_t threads_shade;         /* block size of the shade kernels (0 = 128) */
-    int32_t iterations_per_check;  /* iterations between host termination checks (0 = 16) */
-    int32_t no_graph;              /* 1: launch kernels directly instead of replaying a CUDA graph */
+    int32_t iterations_per_check;  /* no_graph: iterations between host termination checks (0 = 16) */
+    int32_t no_graph;              /* 1: launch kernels directly instead of a CUDA graph that loops on the device */
     float *kernel_ms;              /* optional host float[4]: adds the device time of the regen, extend,
                                       shade and shadow phases (timed with events, no graph) */
     int32_t *kernel_launches;      /* optional host int32[4]: adds the kernel launches per phase */
@@ -327,9 +332,9 @@ int hk_render_batch_host(hk_scene *s, const hk_render_desc *descs, int n, const 
                          float *const *rgb_host, unsigned long long *counters_host, void *stream);
 
 /* Autotuner: render `probe` (one image) under candidate configurations --
- * slot capacity 2^20..2^22, block sizes 64/128/256, termination-check
- * interval 16/64, traversal refill interval and idle-lane threshold -- by
- * coordinate descent and return the fastest. */
+ * slot capacity 2^20..2^22, block sizes 64/128/256, traversal refill interval
+ * and idle-lane threshold, register budgets, dispatch order -- by coordinate
+ * descent and return the fastest. */
 int hk_wavefront_autotune(hk_scene *s, const hk_render_desc *probe, hk_wavefront_config *best, float *best_ms);
 /* The wavefront configuration hk_render_image uses (NULL: the defaults of
  * hk_render_batch).  hk_wavefront_autotune sets it to the configuration it

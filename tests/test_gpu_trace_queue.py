@@ -81,3 +81,36 @@ def test_pool_sizes_render_the_same_images(no_graph):
         if ref is None:
             ref = (got, c)
         _agree(ref[0], ref[1], got, c)
+
+
+# 512 x 512 x 1 and 256 x 256 x 4: 2^18 paths, the least that hk_render gives to the wavefront; 511 x 512: below; 1024 x 257: ragged
+@pytest.mark.parametrize("size,spp", [((512, 512), 1), ((256, 256), 4), ((511, 512), 1), ((1024, 257), 1)])
+def test_queued_film_renders_agree_with_the_megakernel(size, spp):
+    sd = scenes.cornell_box(width=size[0], height=size[1])
+    gs = hk.Scene.from_desc(sd)
+    out = []
+    for form in (hk.FORM_MEGAKERNEL, hk.FORM_AUTO):
+        gs.set_image_form(form)
+        film = torch.zeros(gs.film_shape(), device="cuda")
+        ctr = torch.zeros(5, dtype=torch.int64, device="cuda")
+        for k in range(3):   # three calls on the stream, none waited for
+            gs.render(film, spp, sd.depth, seed=7, sample_offset=k * spp, counters=ctr)
+        out.append((film.cpu().numpy().astype(np.float64), ctr.cpu().numpy()))
+    _agree(*out[0], *out[1])
+
+
+def test_film_render_is_still_captured():
+    """A capture of hk_render holds the megakernel whatever the size: a graph with a loop cannot be captured."""
+    sd = scenes.cornell_box(width=512, height=512)
+    gs = hk.Scene.from_desc(sd)
+    film, ref = (torch.zeros(gs.film_shape(), device="cuda") for _ in range(2))
+    gs.render(ref, 2, sd.depth, seed=3)   # the wavefront
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        gs.render(film, 2, sd.depth, seed=3)
+    film.zero_()
+    g.replay()
+    torch.cuda.synchronize()
+    a, b = ref.cpu().numpy(), film.cpu().numpy()
+    assert np.allclose(a, b, rtol=1e-5, atol=1e-6 * float(np.abs(a).max()))
