@@ -30,7 +30,7 @@ __device__ __forceinline__ void trace_rays(const DevScene &S, unsigned *fetch, u
         const unsigned warps = gridDim.x * (blockDim.x / 32u), warp = blockIdx.x * (blockDim.x / 32u) + threadIdx.x / 32u;
         const unsigned own = min(kFetchChunk, (n + warps - 1u) / warps);
         const unsigned first = min(n, warp * own), last = min(n, first + own);
-        trace_queue8<kAnyHit, kAnyHit>(S, first, last, n, min_idle,
+        trace_queue8<kAnyHit, kAnyHit ? kRangeUnit : kRangeWave>(S, first, last, n, min_idle,
                               [&] { return own < kFetchChunk ? n : warps * kFetchChunk + atomicAdd(fetch, kFetchChunk); },
                               load, store, ts);
     } else {

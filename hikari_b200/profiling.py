@@ -186,7 +186,8 @@ def render(argv):
                     fetch_min_idle=a.fetch_min_idle, iterations_per_check=a.iterations_per_check,
                     fetch_steps_shadow=a.fetch_steps_shadow, fetch_min_idle_shadow=a.fetch_min_idle_shadow,
                     reg_lean=a.reg_lean, shadow_tests=a.shadow_tests, closest_tests=a.closest_tests,
-                    sample_major=a.sample_major)
+                    sample_major=a.sample_major,
+                    no_graph=True)   # plain launches: ncu does not list the kernels of a graph's loop
     torch.cuda.synchronize()
     c = [int(x) for x in ctr.cpu().tolist()]
     names = ["rays", "shadow_rays", "dropped", "node_visits", "tri_tests", "node_visits_shadow", "tri_tests_shadow"]
