@@ -387,9 +387,9 @@ class Scene:
         return self.desc.camera.width if self.desc else None
 
     def set_image_form(self, form: int) -> None:
-        """The form render_image renders with: FORM_AUTO (the wavefront for
-        images of at least 256 x 256 pixels and 2^22 paths), FORM_MEGAKERNEL
-        or FORM_WAVEFRONT."""
+        """The form render and render_image render with: FORM_AUTO (the wavefront
+        from 2^18 paths on), FORM_MEGAKERNEL, or FORM_WAVEFRONT (render_image
+        whatever the size)."""
         check(lib().hk_scene_set_image_form(self.h, form))
 
     def set_wavefront_config(self, cfg: Optional[dict]) -> None:

@@ -15,6 +15,7 @@
 
 namespace hk {
 
+struct TexVals;
 struct BRec {
     V3 wi, wo;
     float eta;
@@ -22,6 +23,7 @@ struct BRec {
     float tu, tv;   // texture coordinates of the intersection (Record.Isect.UV)
     float4 duv;     // their screen-space partials (dUdX, dVdX, dUdY, dVdY): a camera ray's first hit, else 0
     bool tex;       // textures are looked up (false in kernels that shade untextured materials only)
+    const TexVals *looked = nullptr;   // values looked up already at this vertex, or none
     // what the wireframe and curvature textures read at the intersection: the
     // distance from P to the nearest edge line of the hit triangle, the mean
     // and the Gaussian curvature (tex_geometry); without an intersection the
@@ -439,17 +441,30 @@ __device__ __forceinline__ V3 pattern_eval(const DevTexture &t, float u, float v
 }
 // A BSDF parameter at the query's intersection: its texture or its constant.
 // slot: 0 kd, 1 ks, 2 ks_refract, 3 sigma_a, 4 alpha(U), 5 alphaV
+// The textured parameters of one BSDF at a vertex, looked up once for its next-
+// event records and its sample: a lookup depends on the hit alone, and a
+// filtered one reads eight to dozens of texels.
+struct TexVals {
+    const DevBsdf *b;
+    V3 v[6];   // by slot, where the slot is textured
+};
 __device__ __forceinline__ V3 par_rgb(const DevBsdf &b, int slot, const float *c, const BRec &r) {
     if (r.tex) {
         const int t = b.tex[slot];
-        if (t) return tex_eval(b.textures, t - 1, r.tu, r.tv, r.duv, true, r.geo);
+        if (t) {
+            if (r.looked && r.looked->b == &b) return r.looked->v[slot];
+            return tex_eval(b.textures, t - 1, r.tu, r.tv, r.duv, true, r.geo);
+        }
     }
     return ld_rgb(c);
 }
 __device__ __forceinline__ float par_alpha(const DevBsdf &b, int slot, float c, const BRec &r) {
     if (r.tex) {
         const int t = b.tex[slot];
-        if (t) return tex_eval(b.textures, t - 1, r.tu, r.tv, r.duv, true, r.geo).x;
+        if (t) {
+            if (r.looked && r.looked->b == &b) return r.looked->v[slot].x;
+            return tex_eval(b.textures, t - 1, r.tu, r.tv, r.duv, true, r.geo).x;
+        }
     }
     return c;
 }
@@ -1692,6 +1707,29 @@ __device__ __forceinline__ V3 bsdf_sample_t(const DevBsdf *bs, int id, BRec &r, 
     else return twosided_sample(bs, b, r, ux, uy, u1);
 }
 
+// Texture slots (kd, ks, ks_refract, sigma_a, alpha_u, alpha_v) that a type reads.
+constexpr unsigned tex_slots(int type) {
+    return type == kDiffuse ? 0x01u
+         : type == kRoughConductor ? 0x32u
+         : type == kRoughDielectric ? 0x36u
+         : type == kRoughPlastic ? 0x13u
+         : type == kRoughCoating ? 0x1au
+         : type == kConductor ? 0x02u
+         : type == kDielectric ? 0x06u
+         : type == kPlastic ? 0x03u
+         : type == kCoating ? 0x0au
+         : type == kRoughDiffuse ? 0x11u
+                                 : 0u;
+}
+// Look up the textured ones of BSDF id, of type BT, for record r.
+template <int BT>
+__device__ __forceinline__ void tex_look_up(const DevBsdf *bs, int id, const BRec &r, TexVals &t) {
+    const DevBsdf &b = bs[id];
+    t.b = &b;
+#pragma unroll
+    for (int k = 0; k < 6; ++k)
+        if ((tex_slots(BT) >> k & 1u) && b.tex[k]) t.v[k] = tex_eval(b.textures, b.tex[k] - 1, r.tu, r.tv, r.duv, true, r.geo);
+}
 // What the records of one vertex share, from wi alone: G1 of wi and the rough
 // transmittance at it (a powf and a cubic table lookup).
 struct BsdfVertex {
@@ -1739,11 +1777,20 @@ __device__ __forceinline__ V3 bsdf_sample_pdf_t(const DevBsdf *bs, int id, BRec 
 
 // bumpMap / normalMap id wrapping a BSDF of type BT known at compile time:
 // the wrappers above with the nested call dispatched statically
+// The vertex terms of the nested BSDF: wi moved into the perturbed frame
 template <int BT>
-__device__ __forceinline__ V3 bump_eval_t(const DevBsdf *bs, int id, const BRec &r, const BumpFrames &f) {
+__device__ __forceinline__ BsdfVertex bump_vertex_t(const DevBsdf *bs, int id, const BRec &r, const BumpFrames &f) {
+    BRec q = r;
+    q.wi = to_local(f.pf, to_world(f.sh, r.wi));
+    return bsdf_vertex_t<BT>(bs, bs[id].nested, q);
+}
+template <int BT>
+__device__ __forceinline__ V3 bump_eval_pdf_t(const DevBsdf *bs, int id, const BRec &r, const BumpFrames &f,
+                                              const BsdfVertex &v, float &pdf) {
     BRec q;
+    pdf = 0.0f;
     if (!bump_record(f, r, q)) return v3(0, 0, 0);
-    return bsdf_eval_t<BT>(bs, bs[id].nested, q);
+    return bsdf_eval_pdf_t<BT>(bs, bs[id].nested, q, v, pdf);
 }
 template <int BT>
 __device__ __forceinline__ float bump_pdf_t(const DevBsdf *bs, int id, const BRec &r, const BumpFrames &f) {

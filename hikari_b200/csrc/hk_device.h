@@ -179,7 +179,7 @@ struct DevScene {
     float background[3];
     int32_t force_background;
     int32_t narea;                // area lights
-    uint32_t shade_queues;        // wavefront shade queues that a path in this scene can reach (bit per queue)
+    uint64_t shade_queues;        // wavefront shade queues that a path in this scene can reach (bit per queue)
 };
 
 }  // namespace hk

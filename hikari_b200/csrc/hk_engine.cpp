@@ -11,10 +11,10 @@ namespace {
 // bytes of an allocation's part
 constexpr size_t part(size_t n) { return (n + 255) & ~(size_t)255; }
 // queue arrays of one slot id per slot: 2 extend, 2 idle, the scene's shade queues, 1 finished
-int queue_arrays(uint32_t shade_queues) { return 5 + __builtin_popcount(shade_queues); }
+int queue_arrays(uint64_t shade_queues) { return 5 + __builtin_popcountll(shade_queues); }
 }  // namespace
 
-size_t WfEngine::bytes_for(int capacity, int nemitters, uint32_t shade_queues) {
+size_t WfEngine::bytes_for(int capacity, int nemitters, uint64_t shade_queues) {
     const size_t N = (size_t)capacity;
     const size_t shadow = N * (size_t)std::max(1, nemitters);
     return part(N * kSlotBytes) + part(N * sizeof(int) * queue_arrays(shade_queues)) + part(shadow * 16 * 3) +
@@ -243,7 +243,7 @@ void WfEngine::run(int iterations, bool use_graph, float *kernel_ms, int32_t *ke
             HK_CUDA(cudaEventCreate(&pe_[0]));
             HK_CUDA(cudaEventCreate(&pe_[1]));
         }
-        const int phase_launches[4] = {1, 1, __builtin_popcount(L_.shade_queues), 1};
+        const int phase_launches[4] = {1, 1, __builtin_popcountll(L_.shade_queues), 1};
         for (int k = 0; k < iterations; ++k)
             for (int ph = 0; ph < 4; ++ph) {
                 HK_CUDA(cudaEventRecord(pe_[0], stream_));

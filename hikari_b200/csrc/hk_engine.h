@@ -37,7 +37,7 @@ public:
     WfEngine &operator=(const WfEngine &) = delete;
 
     // Device bytes an engine of this capacity holds for a scene with nemitters emitters and these shade queues.
-    static size_t bytes_for(int capacity, int nemitters, uint32_t shade_queues);
+    static size_t bytes_for(int capacity, int nemitters, uint64_t shade_queues);
     size_t device_bytes() const { return bytes_; }
     const WfEngineConfig &config() const { return cfg_; }
     // The stream the engine's work goes to next (one of two of different priority).

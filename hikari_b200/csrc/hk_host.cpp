@@ -735,7 +735,7 @@ void build_scene(hk_scene *s) {
         d.has_uv = !m.uv.empty();
         for (int c = 0; c < 3; c++) d.radiance[c] = m.radiance[c];
         d.shade_queue = hk::wf_queue_of_bsdf(bs.data(), m.bsdf);
-        D.shade_queues |= 1u << d.shade_queue;
+        D.shade_queues |= 1ull << d.shade_queue;
         dm.push_back(d);
         size_t nv = m.pos.size() / 3;
         for (size_t v = 0; v < nv; ++v)

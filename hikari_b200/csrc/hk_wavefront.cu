@@ -72,10 +72,16 @@ HK_WF_SHADE_EXTERN(27);
 HK_WF_SHADE_EXTERN(28);
 HK_WF_SHADE_EXTERN(29);
 HK_WF_SHADE_EXTERN(30);
+HK_WF_SHADE_EXTERN(31);
+HK_WF_SHADE_EXTERN(32);
+HK_WF_SHADE_EXTERN(33);
+HK_WF_SHADE_EXTERN(35);
+HK_WF_SHADE_EXTERN(36);
+HK_WF_SHADE_EXTERN(37);
 #undef HK_WF_SHADE_EXTERN
-static_assert(kWfTypes == 31, "one shade kernel per queue");
-// 10 and 22 (twoSided) have no kernel of their own: wf_queue_of sends them to the generic queue.
-constexpr bool has_shade_kernel(int q) { return q != 1 + kTwoSided && q != kWfTexturedQueue0 + kTwoSided; }
+static_assert(kWfTypes == 38, "one shade kernel per queue");
+// TwoSided BSDFs (10, 22, 34) have no kernel of their own: wf_queue_of sends them to the generic queue.
+constexpr bool has_shade_kernel(int q) { return q == 0 || q == kWfGenericQueue || (q - 1) % kWfLeafTypes != kTwoSided; }
 
 // ------------------------------------------------------------ regen
 // Splat and retire the finished paths, then give finished and idle slots new

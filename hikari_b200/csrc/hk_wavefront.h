@@ -21,15 +21,15 @@ namespace hk {
 // Shade queues, one kernel each: 0 the misses; 1 + type the BSDF types without
 // textures, each compiled for that type with texture lookups compiled out;
 // 13 + type the same with textured parameters and lookups; 25 + type a bumpMap
-// or normalMap over a rough type; 30 the rest, dispatched at run time: deep
-// stacks of layers, twoSided BSDFs and maps over the smooth types.  A mirror
+// or normalMap over that type; 37 the rest, dispatched at run time: deep stacks
+// of layers, twoSided BSDFs and maps over them.  A mirror
 // that shared the run-time-dispatched kernel paid for the calls, the 1.4 KB of
 // stack and the divergence of every type: 2.2 ns a vertex in the Cornell box of
 // smooth materials, where a diffuse vertex takes 0.2.
 constexpr int kWfLeafTypes = kRoughDiffuse + 1;
 constexpr int kWfTexturedQueue0 = 1 + kWfLeafTypes;
-constexpr int kWfBumpQueue0 = kWfTexturedQueue0 + kWfLeafTypes;   // bumpMap / normalMap over a rough type
-constexpr int kWfGenericQueue = kWfBumpQueue0 + kRoughCoating + 1;
+constexpr int kWfBumpQueue0 = kWfTexturedQueue0 + kWfLeafTypes;   // bumpMap / normalMap over the type
+constexpr int kWfGenericQueue = kWfBumpQueue0 + kWfLeafTypes;
 constexpr int kWfTypes = kWfGenericQueue + 1;
 // Shade queue of a top-level BSDF type (nested_type: what a map wraps).
 __host__ __device__ constexpr int wf_queue_of(int bsdf_type, bool textured = false, int nested_type = -1) {
@@ -37,7 +37,9 @@ __host__ __device__ constexpr int wf_queue_of(int bsdf_type, bool textured = fal
                ? kWfGenericQueue
                : (bsdf_type <= kRoughDiffuse
                       ? (textured ? kWfTexturedQueue0 : 1) + bsdf_type
-                      : (nested_type >= 0 && nested_type <= kRoughCoating ? kWfBumpQueue0 + nested_type : kWfGenericQueue));
+                      : (nested_type >= 0 && nested_type <= kRoughDiffuse && nested_type != kTwoSided
+                             ? kWfBumpQueue0 + nested_type
+                             : kWfGenericQueue));
 }
 // Shade queue of BSDF id: deep stacks of layers (and maps over them) are
 // dispatched at run time whatever their top-level type.
@@ -162,7 +164,7 @@ constexpr unsigned kWfMaxLoops = 1u << 14;   // passes of the device-side loop b
 struct WfLaunchConfig {
     int blocks_extend, threads_extend;
     int blocks_shade[kWfTypes], threads_shade;
-    uint32_t shade_queues;             // queues the scene can reach; the kernels of the others are not launched
+    uint64_t shade_queues;             // queues the scene can reach; the kernels of the others are not launched
     int nfork;                         // forks in use
     cudaStream_t fork[kWfForks];
     cudaEvent_t ev_fork, ev_join[kWfForks];

@@ -162,7 +162,8 @@ __global__ void __launch_bounds__(256, kMinBlocks) wf_shade_kernel(DevScene S, W
             // next-event estimation over every emitter (PathMISIntegrator.cpp:83-109)
             const V3 wi_local = to_local(it.sh, rd * -1.0f);
             BsdfVertex bv;   // the typed kernels'
-            if constexpr (BT >= 0 && !kBumpQ) {
+            TexVals looked;  // the typed kernels' of textured materials
+            if constexpr (BT >= 0) {
                 BRec br;
                 br.wi = wi_local;
                 br.tex = kTexQ;
@@ -171,8 +172,11 @@ __global__ void __launch_bounds__(256, kMinBlocks) wf_shade_kernel(DevScene S, W
                 if constexpr (kTexQ) {
                     br.duv = duv;
                     br.geo = geo;
+                    tex_look_up<BT>(S.bsdfs, kBumpQ ? S.bsdfs[bsdf].nested : bsdf, br, looked);
+                    br.looked = &looked;
                 }
-                bv = bsdf_vertex_t<BT>(S.bsdfs, bsdf, br);
+                if constexpr (kBumpQ) bv = bump_vertex_t<BT>(S.bsdfs, bsdf, br, bf);
+                else bv = bsdf_vertex_t<BT>(S.bsdfs, bsdf, br);
             }
             for (int e = 0; e < S.nemitters; ++e) {
                 ERec er;
@@ -194,6 +198,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) wf_shade_kernel(DevScene S, W
                 if constexpr (kTexQ) {   // unread where lookups are compiled out
                     br.duv = duv;
                     br.geo = geo;
+                    if constexpr (BT >= 0) br.looked = &looked;
                 }
                 float pl = er.pdf;
                 float pb;
@@ -202,8 +207,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) wf_shade_kernel(DevScene S, W
                     pb = bsdf_pdf_b(S.bsdfs, bsdf, br, bf);
                     f = bsdf_eval_b(S.bsdfs, bsdf, br, bf);
                 } else if constexpr (kBumpQ) {
-                    pb = bump_pdf_t<BT>(S.bsdfs, bsdf, br, bf);
-                    f = bump_eval_t<BT>(S.bsdfs, bsdf, br, bf);
+                    f = bump_eval_pdf_t<BT>(S.bsdfs, bsdf, br, bf, bv, pb);
                 } else {
                     f = bsdf_eval_pdf_t<BT>(S.bsdfs, bsdf, br, bv, pb);
                 }
@@ -231,6 +235,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) wf_shade_kernel(DevScene S, W
             if constexpr (kTexQ) {
                 br.duv = duv;
                 br.geo = geo;
+                if constexpr (BT >= 0) br.looked = &looked;
             }
             float sx = rng.nextf(), sy = rng.nextf();
             float u1 = needs_u1(S.bsdfs, bsdf) ? rng.nextf() : 0.0f;
