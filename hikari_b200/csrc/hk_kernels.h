@@ -19,6 +19,7 @@ struct RenderLaunch {
     int sample_offset;                    // first sample index (progressive rendering)
     int depth, rr_start;
     int image_index;
+    unsigned lanes;                       // lanes of each warp that take paths (1 to 32)
 };
 
 // Static scratch of hk_render_image_static: a 256-byte header ([0] work

@@ -149,8 +149,8 @@ __device__ __forceinline__ bool path_vertex(const DevScene &S, Path &P, int dept
 
 // ------------------------------------------------------------ megakernel
 // Paths are numbered sample by sample over the image, 16 x 16 tile by tile
-// within a sample, and dealt to warps 32 at a time; a lane whose path has ended
-// takes the next one at its warp's next vertex.  With a lane per pixel that
+// within a sample, and dealt to warps P.lanes at a time; a lane whose path has
+// ended takes the next one at its warp's next vertex.  With a lane per pixel that
 // ran its samples one after another, a warp waited at each sample for its
 // longest path (roulette at p = 0.95: the longest of 32 has four times the
 // mean's vertices), and a block for its slowest tile item.
@@ -161,7 +161,8 @@ __global__ void __launch_bounds__(kRenderThreads, kRenderBlocks) render_pathmis_
     PathCounters pc{0, 0, TravStats()};
     uint32_t dropped = 0;
     Path p;
-    bool have = false, exhausted = false;
+    // few paths: fewer lanes of each warp take part, so that more warps do
+    bool have = false, exhausted = lane >= P.lanes;
     uint64_t next = 0, end = 0;   // warp-uniform: undealt paths of the warp's chunk
     for (;;) {
         const unsigned want = __ballot_sync(0xffffffffu, !have && !exhausted);
@@ -171,11 +172,11 @@ __global__ void __launch_bounds__(kRenderThreads, kRenderBlocks) render_pathmis_
             uint64_t i = next + rank;
             if (k > avail) {   // claim the next chunk for the lanes past the old one
                 unsigned long long base = 0;
-                if ((int)lane == __ffs(want) - 1) base = atomicAdd(P.work_counter, 32ull);
+                if ((int)lane == __ffs(want) - 1) base = atomicAdd(P.work_counter, (unsigned long long)P.lanes);
                 base = __shfl_sync(0xffffffffu, base, __ffs(want) - 1);
                 if (rank >= avail) i = base + (rank - avail);
                 next = base + (k - avail);
-                end = base + 32;
+                end = base + P.lanes;
             } else {
                 next += k;
             }

@@ -1,4 +1,5 @@
-"""The wavefront's shade kernels for one BSDF type, textured and perturbed.
+"""The wavefront's shade kernels for one BSDF type, textured and perturbed,
+and the megakernel's spread of few paths over its warps.
 
 Both forms walk the same sample streams.  The megakernel evaluates every
 material with the BSDF that looks its textures up at each use; a shade queue's
@@ -53,3 +54,9 @@ def test_textures_looked_up_once_per_vertex(name, over):
     for m in sd.meshes[1:6]:
         m.bsdf = b
     _both(sd, 4)
+
+
+# one path; under and over one path per scheduler's warp (592 of 148 SMs); the last sizes of partly and of fully filled warps
+@pytest.mark.parametrize("size", [(1, 1), (24, 24), (25, 24), (135, 136), (138, 138)])
+def test_few_paths_are_spread_over_the_warps(size):
+    _both(scenes.lights_scene(width=size[0], height=size[1], shading_normals=True, textured=True), 1)
