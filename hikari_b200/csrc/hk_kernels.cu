@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(kTraceThreads) trace_rays_kernel(DevScene S, u
         const uint64_t warp = blockIdx.x * (uint64_t)(blockDim.x / 32) + threadIdx.x / 32;
         const uint64_t begin = min(n, warp * per_warp);
         const unsigned cnt = (unsigned)min((uint64_t)per_warp, n - begin);
-        trace_queue8<kAnyHit, kRangeAny>(S, 0u, cnt, cnt, kAnyHit ? 8 : 12, [&] { return cnt; },
+        trace_queue8<kAnyHit, kRangeAny>(S, 0u, cnt, cnt, 0u, kAnyHit ? 8 : 12, [&](unsigned &) { return cnt; },
                               [&](int i) { return load(begin + (uint64_t)i); }, [&](int i, bool f, Hit h) {
             const uint64_t k = begin + (uint64_t)i;
             if constexpr (!kAnyHit) {

@@ -24,6 +24,7 @@
 
 namespace hk {
 
+constexpr unsigned kClaim8 = 32;       // rays that a warp claims at once
 constexpr unsigned kTriRing = 64;      // pending triangle tests per warp (a power of two, at least 2 x 32)
 constexpr unsigned kTriOwnerShift = kLeafCountShift;   // scenes hold fewer than 2^27 triangles: the owner lane sits above
 constexpr uint32_t kTriMask = (1u << kTriOwnerShift) - 1u;
@@ -176,9 +177,9 @@ __device__ __forceinline__ float from_ordered(uint32_t b) {
 
 // Traverses n rays of a queue: lanes are refilled as in trace_queue
 // (hk_traverse.cuh), node visits and triangle tests as described at the top.
-// The warp starts with entries first to last - 1; claim(), called by one lane,
-// takes the next kFetchChunk ones and returns the first of them (n or more: none
-// are left).
+// The warp starts with entries first to last - 1; claim(part), called by one
+// lane, takes the next kClaim8 ones and returns the first of them (n or more:
+// none are left); part is the warp's, kept from claim to claim.
 // load(i) returns ray i; store(i, found, hit) consumes the result.  st counts
 // the warp's visits and tests (the same in every lane).  kUnit: every ray's
 // range is [kRayEps, 1 - kRayEps], a segment between two points.  A lane
@@ -193,7 +194,7 @@ __device__ __forceinline__ float from_ordered(uint32_t b) {
 // adds visits and tests, never a hit.
 template <bool kAnyHit, int kForm, class Claim, class Load, class Store>
 __device__ __forceinline__ void trace_queue8(const DevScene &S, unsigned first, unsigned last, unsigned n,
-                                             int min_idle, Claim claim, Load load, Store store, TravStats &st) {
+                                             unsigned part, int min_idle, Claim claim, Load load, Store store, TravStats &st) {
     constexpr bool kUnit = kForm == kRangeUnit;
     extern __shared__ float4 trace_smem[];
     const unsigned lane = threadIdx.x & 31u;
@@ -280,11 +281,12 @@ __device__ __forceinline__ void trace_queue8(const DevScene &S, unsigned first, 
             unsigned idx = chunk_next + rank;
             if (k > avail) {   // warp-uniform: claim the next chunk for the lanes past the old one
                 unsigned base = 0;
-                if ((int)lane == __ffs(want) - 1) base = claim();
+                if ((int)lane == __ffs(want) - 1) base = claim(part);
                 base = __shfl_sync(0xffffffffu, base, __ffs(want) - 1);
+                part = __shfl_sync(0xffffffffu, part, __ffs(want) - 1);
                 if (rank >= avail) idx = base + (rank - avail);
                 chunk_next = base + (k - avail);
-                chunk_end = base + kFetchChunk;
+                chunk_end = base + kClaim8;
             } else {
                 chunk_next += k;
             }

@@ -225,8 +225,7 @@ __global__ void __launch_bounds__(256) wf_regen_kernel(DevScene S, WfState W, in
             c->idle_count[cur] = 0u;
             c->eq_count[cur ^ 1] = 0u;
             c->shadow_count = 0u;
-            c->ext_fetch = 0u;
-            c->sh_fetch = 0u;
+            for (unsigned k = 0; k < kWfFetchParts; ++k) c->ext_fetch[k * kWfFetchStride] = c->sh_fetch[k * kWfFetchStride] = 0u;
             for (int t = 0; t < kWfTypes; ++t) c->sq_count[t] = 0u;
             if (W.cond && cur == 1) {
                 const bool more = (atomicAdd(&c->active, 0u) != 0u || next < total) && ++c->loops < kWfMaxLoops;
@@ -250,7 +249,8 @@ __global__ void wf_init_kernel(WfState W, int slots, WfJob J) {
         c->idle_count[1] = 0;
         for (int t = 0; t < kWfTypes; ++t) c->sq_count[t] = 0;
         c->fq_count = c->shadow_count = c->active = 0;
-        c->ext_fetch = c->sh_fetch = c->regen_done = c->loops = 0;
+        for (unsigned k = 0; k < kWfFetchParts; ++k) c->ext_fetch[k * kWfFetchStride] = c->sh_fetch[k * kWfFetchStride] = 0;
+        c->regen_done = c->loops = 0;
         c->rays = c->shadow_rays = c->dropped = 0;
         c->node_visits = c->tri_tests = c->node_visits_shadow = c->tri_tests_shadow = 0;
         c->log_n[0] = c->log_n[1] = 0;

@@ -88,6 +88,9 @@ struct WfSeg {
 // fields are the dispatch head, rewritten by the host with each plan.
 constexpr int kWfLaunchLog = 1024;   // launches whose ray counts the counters keep
 
+// Parts of a ray queue, each with a counter of its own, and the counters' spacing (a cache line of 128 bytes).
+constexpr unsigned kWfFetchParts = 8, kWfFetchStride = 32;
+
 struct WfCounters {
     unsigned long long next_work;      // next plan item to hand out
     unsigned long long total_work;     // plan items in the current plan
@@ -99,13 +102,14 @@ struct WfCounters {
     unsigned int fq_count;             // finished paths awaiting splat + regeneration
     unsigned int shadow_count;         // next-event shadow rays
     unsigned int active;               // paths in flight
-    unsigned int ext_fetch, sh_fetch;  // rays claimed by the extend / shadow kernels (dynamic fetch)
     unsigned int regen_done;           // blocks of the running regen launch that are through
     unsigned int loops;                // passes of the device-side loop since its launch
     unsigned int pad1;
     unsigned long long rays, shadow_rays, dropped;
     unsigned long long node_visits, tri_tests;                 // closest-hit traversal (extend)
     unsigned long long node_visits_shadow, tri_tests_shadow;   // any-hit traversal (shadow)
+    // rays claimed by the extend / shadow kernels (dynamic fetch): one counter per part of the queue, a cache line each
+    unsigned int ext_fetch[kWfFetchParts * kWfFetchStride], sh_fetch[kWfFetchParts * kWfFetchStride];
     // rays of each extend (0) / shadow (1) launch since the last reset, in
     // launch order (profiling; the host's status copies stop before it)
     unsigned int log_n[2];

@@ -21,18 +21,34 @@ template <int kAccel, bool kAnyHit, class Load, class Store>
 __device__ __forceinline__ void trace_rays(const DevScene &S, unsigned *fetch, unsigned n, int steps, int min_idle,
                                            Load load, Store store, TravStats &ts) {
     if constexpr (kAccel == kAccelBvh8) {
-        // Every warp starts with an equal share of the queue, at most
-        // kFetchChunk rays, so that a short queue (a small image, the last
-        // bounces of a large one) is spread over all warps and costs no atomic:
-        // with chunks claimed from the start, 4096 rays of a Cornell box went to
-        // 32 warps and took 58 us; so they take 12.  The rest of a long queue is
-        // claimed.
+        // Every warp starts with an equal share of the queue, at most kClaim8
+        // rays, so that a short queue (a small image, the last bounces of a large
+        // one) is spread over all warps and costs no atomic: with chunks of 128
+        // claimed from the start, 4096 rays of a Cornell box went to 32 warps and
+        // took 58 us; so they take 12.  The rest is claimed 32 rays at a time: a
+        // claim of 128 near the end kept a warp for a quarter of a launch of 2^21
+        // rays while others idled (64-sphere scene, 0.304 ns per closest-hit ray,
+        // 0.265 with 32).  One counter would bound cheap rays (Cornell box,
+        // shadow 0.132 -> 0.190 ns), so the rest is cut into kWfFetchParts parts
+        // with a counter and a cache line each; a warp moves on to the next part
+        // when one is used up.
         const unsigned warps = gridDim.x * (blockDim.x / 32u), warp = blockIdx.x * (blockDim.x / 32u) + threadIdx.x / 32u;
-        const unsigned own = min(kFetchChunk, (n + warps - 1u) / warps);
+        const unsigned own = min(kClaim8, (n + warps - 1u) / warps);
         const unsigned first = min(n, warp * own), last = min(n, first + own);
-        trace_queue8<kAnyHit, kAnyHit ? kRangeUnit : kRangeWave>(S, first, last, n, min_idle,
-                              [&] { return own < kFetchChunk ? n : warps * kFetchChunk + atomicAdd(fetch, kFetchChunk); },
-                              load, store, ts);
+        auto claim = [&](unsigned &part) {
+            const unsigned dealt = gridDim.x * (blockDim.x / 32u) * kClaim8;
+            if (n <= dealt) return n;
+            // entries of a part: a multiple of kClaim8
+            const unsigned len = ((n - dealt + kWfFetchParts * kClaim8 - 1u) / (kWfFetchParts * kClaim8)) * kClaim8;
+            for (unsigned k = 0; k < kWfFetchParts; ++k) {
+                const unsigned at = atomicAdd(fetch + part * kWfFetchStride, kClaim8);
+                if (at < len && dealt + part * len + at < n) return dealt + part * len + at;
+                part = part + 1u == kWfFetchParts ? 0u : part + 1u;
+            }
+            return n;
+        };
+        trace_queue8<kAnyHit, kAnyHit ? kRangeUnit : kRangeWave>(S, first, last, n, warp % kWfFetchParts, min_idle, claim, load,
+                                                                 store, ts);
     } else {
         Bvh2Walker wk;
         int stack_mem[kStackSize];
@@ -95,7 +111,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) wf_extend_kernel(DevScene S, 
         W.hit[slot] = make_float4(h.t, h.u, h.v, __int_as_float(found ? h.tri : -1));
         W.sq[type][warp_append_keyed(W.ctr->sq_count, type)] = slot;
     };
-    trace_rays<kAccel, false>(S, &W.ctr->ext_fetch, n, steps, min_idle, load, store, ts);
+    trace_rays<kAccel, false>(S, W.ctr->ext_fetch, n, steps, min_idle, load, store, ts);
     add_stats<kAccel>(ts, &W.ctr->node_visits, &W.ctr->tri_tests);
     log_launch(W.ctr, 0, n);
 }
@@ -120,7 +136,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) wf_shadow_kernel(DevScene S, 
             red_add_v4(W.lacc + slot, c.x, c.y, c.z, 0.0f);
         }
     };
-    trace_rays<kAccel, true>(S, &W.ctr->sh_fetch, n, steps, min_idle, load, store, ts);
+    trace_rays<kAccel, true>(S, W.ctr->sh_fetch, n, steps, min_idle, load, store, ts);
     add_stats<kAccel>(ts, &W.ctr->node_visits_shadow, &W.ctr->tri_tests_shadow);
     log_launch(W.ctr, 1, n);
 }

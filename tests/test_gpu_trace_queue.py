@@ -114,3 +114,19 @@ def test_film_render_is_still_captured():
     torch.cuda.synchronize()
     a, b = ref.cpu().numpy(), film.cpu().numpy()
     assert np.allclose(a, b, rtol=1e-5, atol=1e-6 * float(np.abs(a).max()))
+
+
+# first bounces of 151552 rays: 32 for each warp of 148 x 4 blocks, none left to claim; 151560: one claim of 8; 152144, 302253: the
+# parts of the rest ragged, the last ones empty or cut; capacity 1 << 17: all dealt
+@pytest.mark.parametrize("size", [(592, 256), (421, 360), (592, 257), (777, 389)])
+@pytest.mark.parametrize("threads", [128, 256])
+def test_each_ray_of_a_queue_is_claimed_once(size, threads):
+    sd = scenes.cornell_box(width=size[0], height=size[1])
+    gs = hk.Scene.from_desc(sd)
+    gs.set_image_form(hk.FORM_MEGAKERNEL)
+    a, ca = gs.render_image(1, 6, seed=2)
+    gs.set_image_form(hk.FORM_WAVEFRONT)
+    for capacity in (1 << 17, 1 << 19):
+        gs.set_wavefront_config(dict(capacity=capacity, threads_extend=threads))
+        b, cb = gs.render_image(1, 6, seed=2)
+        _agree(a, ca, b, cb)
