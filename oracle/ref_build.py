@@ -67,7 +67,7 @@ def _newer(obj, *deps):
 
 
 def build(ref: str = "/root/reference", jobs: int = 0) -> str:
-    if not os.path.isdir(ref):
+    if not os.path.isdir(os.path.join(ref, "src")):   # an empty folder is no checkout
         raise FileNotFoundError(f"reference checkout not found at {ref}")
     shim = os.path.join(OUT, "shim")
     objd = os.path.join(OUT, "obj")
