@@ -559,7 +559,7 @@ BvhPair build_bvh_pair(const float *tris, uint32_t n) {
         const uint32_t child_base = (uint32_t)(W.size() / 20);
         W.resize(W.size() + 20 * (size_t)ninternal, 0u);
         const uint32_t tri_base = (uint32_t)order.size();
-        uint32_t imask = 0, meta[8] = {0};
+        uint32_t imask = 0, slots = 0;
         Todo kids[8];
         int nkids = 0;
         uint32_t j = 0;
@@ -570,12 +570,12 @@ BvhPair build_bvh_pair(const float *tris, uint32_t n) {
             if (c < 0) continue;
             if (!is_leaf8(c)) {
                 imask |= 1u << s;
-                meta[s] = 1u << 5 | (24u + (uint32_t)s);   // one hit bit at 24 + slot
+                slots |= 1u << (4 * s);
                 kids[nkids++] = {child_base + j++, c, t.depth + 1};
             } else {
                 const uint32_t off = (uint32_t)order.size() - tri_base, cnt = sub_count[c];
                 if (cnt < 1 || cnt > 3 || off > 21) throw std::runtime_error("BVH8 leaf layout");
-                meta[s] = ((1u << cnt) - 1u) << 5 | off;   // cnt hit bits from off
+                slots |= ((1u << cnt) - 1u) << (4 * s + 1);
                 place_subtree(c, (uint32_t)order.size());
                 for (uint32_t k = 0; k < cnt; k++) order.push_back(T.order[sub_start[c] + k]);
             }
@@ -584,8 +584,7 @@ BvhPair build_bvh_pair(const float *tris, uint32_t n) {
         w[3] = imask << 24;
         w[4] = child_base;
         w[5] = tri_base;
-        w[6] = meta[0] | meta[1] << 8 | meta[2] << 16 | meta[3] << 24;
-        w[7] = meta[4] | meta[5] << 8 | meta[6] << 16 | meta[7] << 24;
+        w[6] = slots;
         quantize(w, nodes[t.b].box, cb);
         for (int q = nkids - 1; q >= 0; --q) todo.push_back(kids[q]);
     }
@@ -636,22 +635,23 @@ std::string check_bvh8(const std::vector<uint32_t> &W, const std::vector<uint32_
         auto q = [&](int plane, int k, int s) { return (double)((w[8 + 2 * (plane * 3 + k) + s / 4] >> (8 * (s % 4))) & 0xffu); };
         uint32_t j = 0;
         for (int s = 0; s < 8; s++) {
-            const uint32_t m = (s < 4 ? w[6] : w[7]) >> (8 * (s & 3)) & 0xffu;
+            const uint32_t m = w[6] >> (4 * s) & 0xfu;
             double lo[3], hi[3];
             for (int k = 0; k < 3; k++) {
                 lo[k] = (double)p[k] + q(0, k, s) * scale[k];
                 hi[k] = (double)p[k] + q(1, k, s) * scale[k];
             }
             if (imask >> s & 1u) {
-                if (m != (0x38u | (uint32_t)s)) return "8-wide internal child meta";
+                if (m != 1u) return "8-wide internal child bits";
                 const uint32_t c = w[4] + j++;
                 if (c >= nw || node_ref[c]) return "8-wide child index out of range or shared";
                 node_ref[c] = 1;
                 Item ci{c, {lo[0], lo[1], lo[2]}, {hi[0], hi[1], hi[2]}};
                 todo.push_back(ci);
             } else if (m) {
-                const uint32_t cnt = (uint32_t)__builtin_popcount(m >> 5), off = m & 31u;
-                if ((m >> 5) != (1u << cnt) - 1u) return "8-wide leaf meta is not a unary count";
+                const uint32_t cnt = (uint32_t)__builtin_popcount(m >> 1),
+                               off = (uint32_t)__builtin_popcount(w[6] & 0xeeeeeeeeu & ((1u << (4 * s)) - 1u));
+                if (m != ((1u << cnt) - 1u) << 1) return "8-wide leaf bits are not a unary count";
                 for (uint32_t k = 0; k < cnt; k++) {
                     const uint32_t pos = w[5] + off + k;
                     if (pos >= n || tri_ref[pos]) return "8-wide leaf triangle out of range or shared";

@@ -25,13 +25,18 @@ Bvh2 build_bvh2(const float *tris, uint32_t ntris, int max_leaf = 4);
 //          by one step on every side)
 //   w4     index of the first internal child node (children are consecutive)
 //   w5     index of the node's first triangle (leaf children's triangles are consecutive)
-//   w6, w7 meta byte per child slot, bits << 5 | position: a hit sets `bits`
-//          at `position` of the node's hit word -- leaf: count ones at its
-//          first triangle's offset 0..21 from w5; internal: one bit at 24 +
-//          slot (the traversal XORs the slot with the ray octant); 0 = empty
+//   w6     four bits per child slot (slot s: 4 s): bit 0 an internal child, bits
+//          1..3 a leaf's triangles, count ones from bit 1; 0 = empty.  A leaf's
+//          triangles follow those of the leaves in lower slots, so the triangle
+//          of a bit is w5 plus the number of triangle bits below it
+//   w7     0
 //   w8..19 q_lo.x[8], q_lo.y[8], q_lo.z[8], q_hi.x[8], q_hi.y[8], q_hi.z[8]
 // A child in slot s lies on the negative side of axis k when bit k of s is
 // set, so a ray visits children in the order s ^ (7 ^ octant) near first.
+// With a meta byte per slot (Ylitie et al.: bits << 5 | position in the hit
+// word) a hit took four instructions of the pipe that bounds the traversal
+// (extract, shift, shift, or); with four bits per slot at a fixed place it is
+// one predicated or, and slots are put in visiting order once per node.
 struct Bvh8 {
     std::vector<uint32_t> nodes;
     uint32_t depth = 0;

@@ -323,7 +323,7 @@ __global__ void collapse_kernel(const unsigned long long *keys, int n, const int
         const uint32_t tri_base = nleaf_tris ? atomicAdd(&ctr[1], nleaf_tris) : atomicAdd(&ctr[1], 0u);
         if (fr.wide >= max_wide) { atomicExch(&ctr[3], 2u); continue; }
         uint32_t *w = wnodes + 20 * (size_t)fr.wide;
-        uint32_t imask = 0, meta[8] = {0, 0, 0, 0, 0, 0, 0, 0}, j = 0, off = 0;
+        uint32_t imask = 0, slots = 0, j = 0, off = 0;
         Box3 cb[8];
         bool used[8];
         for (int s = 0; s < 8; s++) {
@@ -334,13 +334,13 @@ __global__ void collapse_kernel(const unsigned long long *keys, int n, const int
             const uint32_t cnt = node_count(range, n, c);
             if (cnt > 3u) {
                 imask |= 1u << s;
-                meta[s] = 1u << 5 | (24u + (uint32_t)s);
+                slots |= 1u << (4 * s);
                 const uint32_t o = atomicAdd(&ctr[2], 1u);
                 if (o < max_wide) out[o] = Frontier{child_base + j, c};
                 else atomicExch(&ctr[3], 2u);
                 ++j;
             } else {
-                meta[s] = ((1u << cnt) - 1u) << 5 | off;
+                slots |= ((1u << cnt) - 1u) << (4 * s + 1);
                 const uint32_t first = node_first(range, n, c);
                 for (uint32_t k = 0; k < cnt; k++) {
                     if (tri_base + off + k < (uint32_t)n && first + k < (uint32_t)n)
@@ -354,8 +354,8 @@ __global__ void collapse_kernel(const unsigned long long *keys, int n, const int
         w[3] = imask << 24;
         w[4] = child_base;
         w[5] = tri_base;
-        w[6] = meta[0] | meta[1] << 8 | meta[2] << 16 | meta[3] << 24;
-        w[7] = meta[4] | meta[5] << 8 | meta[6] << 16 | meta[7] << 24;
+        w[6] = slots;
+        w[7] = 0u;
         if (!quantize_dev(w, nb, cb, used)) atomicExch(&ctr[3], 1u);
     }
 }

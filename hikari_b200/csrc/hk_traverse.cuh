@@ -285,14 +285,47 @@ __device__ __forceinline__ bool trace_bvh2(const DevScene &S, const Ray &ray, Hi
 }
 
 // ------------------------------------------------------------ 8-wide tree
-// Traversal of the compressed 8-wide BVH (hk_bvh.h), following Ylitie, Karras
-// and Laine (HPG 2017): a node group is (first child index, hit bits of the
-// internal children << 24 | imask), a triangle group is (first triangle,
-// hit bits 0..23).  Hit bits of internal children sit at slot ^ (7 ^ octant),
-// so the lowest set bit is the nearest child.  A warp vote postpones the
-// triangle tests of lanes that are few among the active ones while they still
-// have nodes to visit, so that lanes intersect triangles together (closest-hit
-// rays).  The wavefront's traversal kernels walk this tree in hk_wf_trace.cuh.
+// Traversal of the compressed 8-wide BVH (hk_bvh.h), after Ylitie, Karras and
+// Laine (HPG 2017).  A child slot has four bits of a word: a node group is
+// (first child index, word), bit 0 of nibble slot ^ octant a hit internal child
+// and bit 1 of nibble slot an internal child, so the highest hit bit is the
+// nearest child; a triangle group is (node, hit triangle bits 1..3 of each
+// nibble).  A warp vote postpones the triangle tests of lanes that are few
+// among the active ones while they still have nodes to visit, so that lanes
+// intersect triangles together (closest-hit rays).  The kernels that trace a
+// queue of rays walk this tree in hk_traverse8.cuh.
+
+constexpr uint32_t kSlotNode = 0x11111111u, kSlotTris = 0xeeeeeeeeu;   // bits of a node's slot word, and of the hits in it
+
+// A ray's visiting order ko as visit8 and next_child use it: ko << 2, and the
+// byte permute that applies its upper bits.
+__device__ __forceinline__ uint32_t slot_order(uint32_t ko) {
+    return ko << 2 | (0x3210u ^ (ko >> 1) * 0x1111u) << 16;
+}
+// Hits of internal children (bit 0 of nibble slot) moved to nibble slot ^ ko.
+__device__ __forceinline__ uint32_t order_hits(uint32_t h, uint32_t order) {
+    const uint32_t r = __byte_perm(h, 0u, order >> 16), s = order & 4u;
+    return ((r >> s) & 0x0f0f0f0fu) | ((r << s) & 0xf0f0f0f0u);
+}
+// The group of a visited node: slots is its word, hv the word's bits that were hit.
+__device__ __forceinline__ uint2 node_group(uint32_t first, uint32_t slots, uint32_t hv, uint32_t order) {
+    return make_uint2(first, order_hits(hv & kSlotNode, order) | (slots & kSlotNode) << 1);
+}
+// The root as slot 0 of a virtual parent.
+__device__ __forceinline__ uint2 root_group(bool any, uint32_t order) {
+    return make_uint2(0u, any ? (1u << (order & 0x1cu) | 2u) : 0u);
+}
+// Takes the group's next child in order.
+__device__ __forceinline__ uint32_t next_child(uint2 &ng, uint32_t order) {
+    const uint32_t b = 31u - __clz(ng.y & kSlotNode);
+    ng.y ^= 1u << b;
+    const uint32_t at = b ^ (order & 0x1cu);
+    return ng.x + __popc(ng.y & (kSlotNode << 1) & ((1u << at) - 1u));
+}
+// Offset from the node's first triangle of the triangle at bit b.
+__device__ __forceinline__ uint32_t tri_offset(uint32_t slots, uint32_t b) {
+    return __popc(slots & kSlotTris & ((1u << b) - 1u));
+}
 
 constexpr int kShStack = 8;   // entries per thread kept in shared memory
 
@@ -307,33 +340,8 @@ struct LocalStack {
     __device__ __forceinline__ uint2 pop() { return e[--sp]; }
 };
 
-// Short stack: the top kShStack entries of each thread in shared memory
-// (sh[k * stride], one column per thread), deeper entries in local memory.
-struct SharedStack {
-    uint2 *sh;
-    int stride;
-    int sp = 0;
-    uint2 *spill;   // kStackSize - kShStack entries in local memory, owned by the caller
-    __device__ __forceinline__ void push(uint2 v) {
-        if (sp < kShStack) sh[sp++ * stride] = v;
-        else if (sp < kStackSize) { spill[sp - kShStack] = v; ++sp; }
-    }
-    __device__ __forceinline__ uint2 pop() {
-        --sp;
-        return sp < kShStack ? sh[sp * stride] : spill[sp - kShStack];
-    }
-};
-
 __device__ __forceinline__ uint4 ldg4u(const uint4 *p) { return __ldg(p); }
 
-// Byte k of x as a float in [0, 255]: a byte permute builds the float
-// 2^23 + q (exponent byte 0x4B, q in the low mantissa byte), and subtracting
-// 2^23 is exact -- two full-rate instructions instead of an integer-to-float
-// conversion.
-template <int k>
-__device__ __forceinline__ float qbyte(uint32_t x) {
-    return __uint_as_float(__byte_perm(x, 0x4B000000u, 0x7440u | k)) - 8388608.0f;
-}
 // Two FMAs in one instruction (PTX fma.rn.f32x2, sm_100a): each lane is an
 // IEEE round-to-nearest FMA, the same result as two __fmaf_rn.
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
@@ -346,9 +354,10 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
     return r;
 }
 
-// The float 2^23 + q without the subtraction: the slab offsets of a node are
-// shifted by -2^23 steps instead (one rounding of at most half a step, which
-// the one-step padding of the quantised boxes absorbs).
+// Byte k of x as the float 2^23 + q: a byte permute puts q into the low
+// mantissa byte.  The slab offsets of a node are shifted by -2^23 steps (one
+// rounding of at most half a step, which the one-step padding of the quantised
+// boxes absorbs).
 template <int k>
 __device__ __forceinline__ float qbyte_biased(uint32_t x) {
     return __uint_as_float(__byte_perm(x, 0x4B000000u, 0x7440u | k));
@@ -359,8 +368,9 @@ struct Bvh8Walker {
     V3 o, d, idir;
     float tmin, tmax, tmax0;
     WatertightRay w;
-    uint32_t oct, ko;
+    uint32_t oct, order;
     uint2 ng, tg;
+    uint32_t tri0, slots;   // of the triangle group's node
     bool found;
     Hit hit;
     uint32_t nvis, ntri;
@@ -375,12 +385,11 @@ struct Bvh8Walker {
                          fabsf(d.z) < tiny ? copysignf(tiny, d.z) : d.z);
         idir = v3(1.0f / dd.x, 1.0f / dd.y, 1.0f / dd.z);
         oct = (idir.x < 0.0f ? 1u : 0u) | (idir.y < 0.0f ? 2u : 0u) | (idir.z < 0.0f ? 4u : 0u);
-        ko = 7u ^ oct;
+        order = slot_order(oct);
         w = watertight_setup(d);
         tmin = ray.tmin;
         tmax = tmax0 = ray.tmax;
-        // the root as slot 0 of a virtual parent (nothing for an empty tree)
-        ng = make_uint2(0u, S.nwnodes == 0 ? 0u : ((1u << (24 + ko)) | 1u));
+        ng = root_group(S.nwnodes != 0, order);
         tg = make_uint2(0u, 0u);
         stk.sp = 0;
         found = false;
@@ -391,27 +400,29 @@ struct Bvh8Walker {
     // One node visit (or one popped triangle group) and its triangle tests.
     template <bool kAnyHit>
     __device__ __forceinline__ bool step(const DevScene &S) {
-        if (ng.y > 0x00ffffffu) {
-            const uint32_t b = __ffs(ng.y >> 24) - 1;
-            ng.y &= ~(1u << (24 + b));
-            const uint32_t slot = b ^ ko;
-            const uint32_t child = ng.x + __popc(ng.y & 0xffu & ((1u << slot) - 1u));
-            if (ng.y > 0x00ffffffu) stk.push(ng);
+        if (ng.y & kSlotNode) {
+            const uint32_t child = next_child(ng, order);
+            if (ng.y & kSlotNode) stk.push(ng);
             visit(S, child);
         } else {
             tg = ng;   // a postponed triangle group from the stack (or nothing)
             ng = make_uint2(0u, 0u);
+            if (tg.y != 0u) {
+                const uint4 n1 = ldg4u(S.wnodes + 5 * (size_t)tg.x + 1);
+                tri0 = n1.y;
+                slots = n1.z;
+            }
         }
         if (!kAnyHit && S.postpone) {
             const unsigned act = __activemask();
             const unsigned want = __ballot_sync(act, tg.y != 0u);
-            if (tg.y != 0u && ng.y > 0x00ffffffu && __popc(want) * 5 < __popc(act)) {
+            if (tg.y != 0u && (ng.y & kSlotNode) && __popc(want) * 5 < __popc(act)) {
                 stk.push(tg);
                 tg.y = 0u;
             }
         }
         while (tg.y != 0u) {
-            const uint32_t tri = tg.x + (__ffs(tg.y) - 1);
+            const uint32_t tri = tri0 + tri_offset(slots, __ffs(tg.y) - 1);
             tg.y &= tg.y - 1u;
             ++ntri;
             const float4 *tp = S.tris + 3 * (size_t)tri;
@@ -431,7 +442,7 @@ struct Bvh8Walker {
                 }
             }
         }
-        if (ng.y <= 0x00ffffffu) {
+        if (!(ng.y & kSlotNode)) {
             if (stk.sp == 0) return true;
             ng = stk.pop();
         }
@@ -449,11 +460,6 @@ struct Bvh8Walker {
         const float ox = __fmaf_rn(-8388608.0f, adx, (__uint_as_float(n0.x) - o.x) * idir.x);
         const float oy = __fmaf_rn(-8388608.0f, ady, (__uint_as_float(n0.y) - o.y) * idir.y);
         const float oz = __fmaf_rn(-8388608.0f, adz, (__uint_as_float(n0.z) - o.z) * idir.z);
-        const uint32_t imask = n0.w >> 24;
-        // meta of internal children: slot ^ (7 ^ octant) in the position bits
-        const uint32_t in0 = ((imask & 0xfu) * 0x00204081u) & 0x01010101u;
-        const uint32_t in1 = ((imask >> 4) * 0x00204081u) & 0x01010101u;
-        const uint32_t meta0 = n1.z ^ (in0 * ko), meta1 = n1.w ^ (in1 * ko);
         // near / far planes per axis (lo planes first for a positive direction)
         const uint32_t nx0 = oct & 1u ? n3.z : n2.x, nx1 = oct & 1u ? n3.w : n2.y;
         const uint32_t fx0 = oct & 1u ? n2.x : n3.z, fx1 = oct & 1u ? n2.y : n3.w;
@@ -465,28 +471,28 @@ struct Bvh8Walker {
         const float t0 = tmin, t1 = tmax;
         const float2 adx2 = make_float2(adx, adx), ady2 = make_float2(ady, ady), adz2 = make_float2(adz, adz);
         const float2 ox2 = make_float2(ox, ox), oy2 = make_float2(oy, oy), oz2 = make_float2(oz, oz);
-        auto test_child = [&](auto kk, uint32_t xn, uint32_t xf, uint32_t yn, uint32_t yf, uint32_t zn, uint32_t zf,
-                              uint32_t meta) {
-            constexpr int k = decltype(kk)::value;
+        auto test_child = [&](auto kk, uint32_t xn, uint32_t xf, uint32_t yn, uint32_t yf, uint32_t zn, uint32_t zf) {
+            constexpr int c = decltype(kk)::value, k = c & 3;
             // near and far plane of an axis in one packed FMA
             const float2 tx = fma2(make_float2(qbyte_biased<k>(xn), qbyte_biased<k>(xf)), adx2, ox2);
             const float2 ty = fma2(make_float2(qbyte_biased<k>(yn), qbyte_biased<k>(yf)), ady2, oy2);
             const float2 tz = fma2(make_float2(qbyte_biased<k>(zn), qbyte_biased<k>(zf)), adz2, oz2);
             const float tn = fmax3f(tx.x, ty.x, fmaxf(tz.x, t0));
             const float tf = fmin3f(tx.y, ty.y, fminf(tz.y, t1));
-            const uint32_t m = __byte_perm(meta, 0u, 0x4440u | k);
-            if (tn <= tf * 1.00000024f + 1e-30f) hits |= (m >> 5) << (m & 31u);
+            if (tn <= tf * 1.00000024f + 1e-30f) hits |= 0xfu << (4 * c);
         };
-        test_child(std::integral_constant<int, 0>{}, nx0, fx0, ny0, fy0, nz0, fz0, meta0);
-        test_child(std::integral_constant<int, 1>{}, nx0, fx0, ny0, fy0, nz0, fz0, meta0);
-        test_child(std::integral_constant<int, 2>{}, nx0, fx0, ny0, fy0, nz0, fz0, meta0);
-        test_child(std::integral_constant<int, 3>{}, nx0, fx0, ny0, fy0, nz0, fz0, meta0);
-        test_child(std::integral_constant<int, 0>{}, nx1, fx1, ny1, fy1, nz1, fz1, meta1);
-        test_child(std::integral_constant<int, 1>{}, nx1, fx1, ny1, fy1, nz1, fz1, meta1);
-        test_child(std::integral_constant<int, 2>{}, nx1, fx1, ny1, fy1, nz1, fz1, meta1);
-        test_child(std::integral_constant<int, 3>{}, nx1, fx1, ny1, fy1, nz1, fz1, meta1);
-        ng = make_uint2(n1.x, (hits & 0xff000000u) | imask);
-        tg = make_uint2(n1.y, hits & 0x00ffffffu);
+        test_child(std::integral_constant<int, 0>{}, nx0, fx0, ny0, fy0, nz0, fz0);
+        test_child(std::integral_constant<int, 1>{}, nx0, fx0, ny0, fy0, nz0, fz0);
+        test_child(std::integral_constant<int, 2>{}, nx0, fx0, ny0, fy0, nz0, fz0);
+        test_child(std::integral_constant<int, 3>{}, nx0, fx0, ny0, fy0, nz0, fz0);
+        test_child(std::integral_constant<int, 4>{}, nx1, fx1, ny1, fy1, nz1, fz1);
+        test_child(std::integral_constant<int, 5>{}, nx1, fx1, ny1, fy1, nz1, fz1);
+        test_child(std::integral_constant<int, 6>{}, nx1, fx1, ny1, fy1, nz1, fz1);
+        test_child(std::integral_constant<int, 7>{}, nx1, fx1, ny1, fy1, nz1, fz1);
+        tri0 = n1.y;
+        slots = n1.z;
+        ng = node_group(n1.x, slots, hits & slots, order);
+        tg = make_uint2(child, hits & slots & kSlotTris);
     }
 
     template <bool kAnyHit>

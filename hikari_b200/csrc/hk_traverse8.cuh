@@ -4,7 +4,7 @@
 //
 // The 8-wide tree is walked by warps whose lanes hold one ray each and share
 // one queue of triangle tests (trace_queue8): a step visits one node per lane,
-// the triangles that the visits hit are appended to a 64-entry ring in shared
+// the triangles that the visits hit are appended to a 128-entry ring in shared
 // memory as (triangle, owner lane), and a batch of 32 is tested, one triangle
 // per lane, whenever 32 are pending.  The kernels are bound by instruction
 // issue (77% of the slots) and by the ALU pipe (68%: the node test's byte
@@ -25,7 +25,12 @@
 namespace hk {
 
 constexpr unsigned kClaim8 = 32;       // rays that a warp claims at once
-constexpr unsigned kTriRing = 64;      // pending triangle tests per warp (a power of two, at least 2 x 32)
+// Pending triangle tests per warp (a power of two, at least 2 x 32).  A step of
+// a small scene queues a hundred (Cornell box: 3 per ray and visit), which a
+// ring of 64 takes in passes; 256 take L1 from the nodes of large ones (whole
+// render with 64 / 128 / 256, ms: Cornell box 29.3 / 28.2 / 28.0, 64-sphere scene
+// 66.3 / 66.1 / 66.2, glass sphere 52.3 / 52.1 / 52.2).
+constexpr unsigned kTriRing = 128;
 constexpr unsigned kTriOwnerShift = kLeafCountShift;   // scenes hold fewer than 2^27 triangles: the owner lane sits above
 constexpr uint32_t kTriMask = (1u << kTriOwnerShift) - 1u;
 
@@ -51,10 +56,10 @@ struct NodeRay {
     V3 o;
     V3 i;                // 1 / d
     float tmin, tmax;    // tmax with the same slack
-    uint32_t oct;
+    uint32_t oct;        // slot_order of the ray | its octant << 5
 };
 
-template <int kForm>
+template <bool kAnyHit, int kForm>
 __device__ __forceinline__ void node_ray_begin(NodeRay &q, const Ray &ray) {
     q.o = ray.o;
     // |1/d| <= 1e20 keeps 2^23 steps of up to 2^38 (the largest step the build emits) finite
@@ -64,7 +69,8 @@ __device__ __forceinline__ void node_ray_begin(NodeRay &q, const Ray &ray) {
                      fabsf(d.z) < tiny ? copysignf(tiny, d.z) : d.z);
     const V3 i = v3(1.0f / dd.x, 1.0f / dd.y, 1.0f / dd.z);
     q.i = i;
-    q.oct = (i.x < 0.0f ? 1u : 0u) | (i.y < 0.0f ? 2u : 0u) | (i.z < 0.0f ? 4u : 0u);
+    const uint32_t oct = (i.x < 0.0f ? 1u : 0u) | (i.y < 0.0f ? 2u : 0u) | (i.z < 0.0f ? 4u : 0u);
+    q.oct = slot_order(kAnyHit ? 7u ^ oct : oct) | oct << 5;
     q.tmin = ray.tmin;
     q.tmax = ray.tmax * slack + 1e-30f;
     if (kForm == kRangeWave) {
@@ -73,17 +79,24 @@ __device__ __forceinline__ void node_ray_begin(NodeRay &q, const Ray &ray) {
     }
 }
 
-// Children are visited in slot ^ ko order: near first for closest hits.  Any-hit
+// Children are visited from the highest nibble slot ^ ko down: near first for closest hits.  Any-hit
 // rays go far first: they start on a surface whose own neighbourhood fills the
 // near boxes without occluding, and what occludes them does so as well met last
 // (visits and ns per shadow ray, near / far first: 64-sphere scene 9.95 / 9.54,
 // 0.232 / 0.227; glass sphere 9.65 / 7.28, 0.309 / 0.261).
-// Intersect the 8 children of a node (hk_bvh.h): its node group and triangle group.
-template <bool kAnyHit, int kForm>
-__device__ __forceinline__ void visit8(const DevScene &S, uint32_t child, const NodeRay &q, uint2 &ng, uint2 &tg) {
+// Intersect the 8 children of a node (hk_bvh.h): its node group and triangle
+// group (first triangle, hit triangle bits), and its slot word.  A hit child is
+// one predicated or; with a meta byte per slot, shifted to its place for each
+// child, and one queue entry per turn of the loop instead of one leaf, closest-
+// hit rays took 0.272 ns instead of 0.258 and shadow rays 0.232 instead of 0.221
+// (64-sphere scene; glass sphere 0.311 / 0.297 and 0.288 / 0.275, Cornell box
+// 0.136 / 0.128 and 0.128 / 0.123).
+template <int kForm>
+__device__ __forceinline__ void visit8(const DevScene &S, uint32_t child, const NodeRay &q, uint2 &ng, uint2 &tg,
+                                       uint32_t &slots) {
     const uint4 *np = S.wnodes + 5 * (size_t)child;
     const uint4 n0 = ldg4u(np), n1 = ldg4u(np + 1), n2 = ldg4u(np + 2), n3 = ldg4u(np + 3), n4 = ldg4u(np + 4);
-    const uint32_t oct = q.oct, ko = kAnyHit ? oct : 7u ^ oct;
+    const uint32_t oct = q.oct >> 5;
     // plane step and offset per axis of the near (x) and far (y) planes; offsets
     // are shifted by -2^23 steps (qbyte_biased).  The far planes' constants are
     // scaled by 1 + 2^-22 (two ulps): the slack that keeps boxes of zero
@@ -100,11 +113,6 @@ __device__ __forceinline__ void visit8(const DevScene &S, uint32_t child, const 
     const float2 bx = make_float2(__fmaf_rn(-8388608.0f, ax.x, off(px, q.i.x)), __fmaf_rn(-8388608.0f, ax.y, off(px, f.x)));
     const float2 by = make_float2(__fmaf_rn(-8388608.0f, ay.x, off(py, q.i.y)), __fmaf_rn(-8388608.0f, ay.y, off(py, f.y)));
     const float2 bz = make_float2(__fmaf_rn(-8388608.0f, az.x, off(pz, q.i.z)), __fmaf_rn(-8388608.0f, az.y, off(pz, f.z)));
-    const uint32_t imask = n0.w >> 24;
-    // meta of internal children: slot ^ (7 ^ octant) in the position bits
-    const uint32_t in0 = ((imask & 0xfu) * 0x00204081u) & 0x01010101u;
-    const uint32_t in1 = ((imask >> 4) * 0x00204081u) & 0x01010101u;
-    const uint32_t meta0 = n1.z ^ (in0 * ko), meta1 = n1.w ^ (in1 * ko);
     // near / far planes per axis (lo planes first for a positive direction)
     const uint32_t nx0 = oct & 1u ? n3.z : n2.x, nx1 = oct & 1u ? n3.w : n2.y;
     const uint32_t fx0 = oct & 1u ? n2.x : n3.z, fx1 = oct & 1u ? n2.y : n3.w;
@@ -115,9 +123,8 @@ __device__ __forceinline__ void visit8(const DevScene &S, uint32_t child, const 
     uint32_t hits = 0;
     constexpr bool kUnit = kForm == kRangeUnit;
     const float t0 = kUnit ? kRayEps : q.tmin, t1 = kUnit ? (1.0f - kRayEps) * 1.00000024f : q.tmax;
-    auto test_child = [&](auto kk, uint32_t xn, uint32_t xf, uint32_t yn, uint32_t yf, uint32_t zn, uint32_t zf,
-                          uint32_t meta) {
-        constexpr int k = decltype(kk)::value;
+    auto test_child = [&](auto kk, uint32_t xn, uint32_t xf, uint32_t yn, uint32_t yf, uint32_t zn, uint32_t zf) {
+        constexpr int c = decltype(kk)::value, k = c & 3;
         if constexpr (kForm != kRangeAny) {
             const float2 tx = make_float2(fma_sat(qbyte_biased<k>(xn), ax.x, bx.x), fma_sat(qbyte_biased<k>(xf), ax.y, bx.y));
             const float2 ty = make_float2(fma_sat(qbyte_biased<k>(yn), ay.x, by.x), fma_sat(qbyte_biased<k>(yf), ay.y, by.y));
@@ -125,8 +132,7 @@ __device__ __forceinline__ void visit8(const DevScene &S, uint32_t child, const 
             const float tn = fmax3f(tx.x, ty.x, tz.x);
             const float tf3 = fmin3f(tx.y, ty.y, tz.y);
             const float tf = kUnit ? tf3 : fminf(tf3, t1);
-            const uint32_t m = __byte_perm(meta, 0u, 0x4440u | k);
-            if (tn < tf) hits |= __funnelshift_l(0u, m >> 5, m);
+            if (tn < tf) hits |= 0xfu << (4 * c);
             return;
         }
         const float2 tx = make_float2(__fmaf_rn(qbyte_biased<k>(xn), ax.x, bx.x), __fmaf_rn(qbyte_biased<k>(xf), ax.y, bx.y));
@@ -134,19 +140,19 @@ __device__ __forceinline__ void visit8(const DevScene &S, uint32_t child, const 
         const float2 tz = make_float2(__fmaf_rn(qbyte_biased<k>(zn), az.x, bz.x), __fmaf_rn(qbyte_biased<k>(zf), az.y, bz.y));
         const float tn = fmax3f(tx.x, ty.x, fmaxf(tz.x, t0));
         const float tf = fmin3f(tx.y, ty.y, fminf(tz.y, t1));
-        const uint32_t m = __byte_perm(meta, 0u, 0x4440u | k);
-        if (tn <= tf) hits |= __funnelshift_l(0u, m >> 5, m);   // shifted by the low five bits of m
+        if (tn <= tf) hits |= 0xfu << (4 * c);
     };
-    test_child(std::integral_constant<int, 0>{}, nx0, fx0, ny0, fy0, nz0, fz0, meta0);
-    test_child(std::integral_constant<int, 1>{}, nx0, fx0, ny0, fy0, nz0, fz0, meta0);
-    test_child(std::integral_constant<int, 2>{}, nx0, fx0, ny0, fy0, nz0, fz0, meta0);
-    test_child(std::integral_constant<int, 3>{}, nx0, fx0, ny0, fy0, nz0, fz0, meta0);
-    test_child(std::integral_constant<int, 0>{}, nx1, fx1, ny1, fy1, nz1, fz1, meta1);
-    test_child(std::integral_constant<int, 1>{}, nx1, fx1, ny1, fy1, nz1, fz1, meta1);
-    test_child(std::integral_constant<int, 2>{}, nx1, fx1, ny1, fy1, nz1, fz1, meta1);
-    test_child(std::integral_constant<int, 3>{}, nx1, fx1, ny1, fy1, nz1, fz1, meta1);
-    ng = make_uint2(n1.x, (hits & 0xff000000u) | imask);
-    tg = make_uint2(n1.y, hits & 0x00ffffffu);
+    test_child(std::integral_constant<int, 0>{}, nx0, fx0, ny0, fy0, nz0, fz0);
+    test_child(std::integral_constant<int, 1>{}, nx0, fx0, ny0, fy0, nz0, fz0);
+    test_child(std::integral_constant<int, 2>{}, nx0, fx0, ny0, fy0, nz0, fz0);
+    test_child(std::integral_constant<int, 3>{}, nx0, fx0, ny0, fy0, nz0, fz0);
+    test_child(std::integral_constant<int, 4>{}, nx1, fx1, ny1, fy1, nz1, fz1);
+    test_child(std::integral_constant<int, 5>{}, nx1, fx1, ny1, fy1, nz1, fz1);
+    test_child(std::integral_constant<int, 6>{}, nx1, fx1, ny1, fy1, nz1, fz1);
+    test_child(std::integral_constant<int, 7>{}, nx1, fx1, ny1, fy1, nz1, fz1);
+    slots = n1.z;
+    ng = node_group(n1.x, slots, hits & slots, q.oct);
+    tg = make_uint2(n1.y, hits & slots & kSlotTris);
 }
 
 // Shared memory of one warp of the 8-wide traversal kernels: the lanes' rays as
@@ -294,11 +300,8 @@ __device__ __forceinline__ void trace_queue8(const DevScene &S, unsigned first, 
                 if (idx < n) {
                     item = (int)idx;
                     const Ray r = load(item);
-                    node_ray_begin<kForm>(nr, r);
-                    // the root as slot 0 of a virtual parent (nothing for an empty tree)
-                    
-                    ng = make_uint2(0u, S.nwnodes == 0 ? 0u : ((1u << (24 + (kAnyHit ? nr.oct : 7u ^ nr.oct))) | 1u));
-
+                    node_ray_begin<kAnyHit, kForm>(nr, r);
+                    ng = root_group(S.nwnodes != 0, nr.oct);
                     sp = 0;
                     found = false;
                     live = S.nwnodes != 0;
@@ -323,18 +326,16 @@ __device__ __forceinline__ void trace_queue8(const DevScene &S, unsigned first, 
         __syncwarp();
         for (;;) {
             uint2 tg = make_uint2(0u, 0u);
+            uint32_t slots = 0;
             if (live) {   // one node per ray
-                const uint32_t ko = kAnyHit ? nr.oct : 7u ^ nr.oct;
-                const uint32_t b = __ffs(ng.y >> 24) - 1;
-                ng.y &= ~(1u << (24 + b));
-                const uint32_t child = ng.x + __popc(ng.y & 0xffu & ((1u << (b ^ ko)) - 1u));
-                if (ng.y > 0x00ffffffu) {   // the tree's depth bound keeps sp below kStackSize
+                const uint32_t child = next_child(ng, nr.oct);
+                if (ng.y & kSlotNode) {   // the tree's depth bound keeps sp below kStackSize
                     if (sp < kShStack) sm.stack[32 * sp + lane] = ng;
                     else if (sp < kStackSize) spill[sp - kShStack] = ng;
                     ++sp;
                 }
-                visit8<kAnyHit, kForm>(S, child, nr, ng, tg);
-                if (ng.y <= 0x00ffffffu) {
+                visit8<kForm>(S, child, nr, ng, tg, slots);
+                if (!(ng.y & kSlotNode)) {
                     if (sp == 0) {
                         live = false;
                     } else {
@@ -355,14 +356,18 @@ __device__ __forceinline__ void trace_queue8(const DevScene &S, unsigned first, 
                 const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
                 st.tris += total;
                 if (total <= kTriRing - pend) {
-                    // from the highest bit down, from the last position back: ring order is bit order
+                    // leaf by leaf, from the highest slot down and the last position back: ring order is
+                    // bit order (a hit leaf has all its triangles' bits set, so bit b & 3 counts them)
                     uint32_t at = head + pend + incl;
                     const uint32_t base = tg.x | (lane << kTriOwnerShift);
                     while (tg.y != 0u) {
-                        const uint32_t b = 31u - __clz(tg.y);
-                        tg.y ^= 1u << b;
-                        --at;
-                        sm.ring[at & (kTriRing - 1u)] = base + b;
+                        const uint32_t b = 31u - __clz(tg.y), below = (1u << (b & 28u)) - 1u, leaf = b & 3u;
+                        tg.y &= below;
+                        at -= leaf;
+                        const uint32_t e = base + __popc(slots & kSlotTris & below);
+                        sm.ring[at & (kTriRing - 1u)] = e;
+                        if (leaf > 1u) sm.ring[(at + 1u) & (kTriRing - 1u)] = e + 1u;
+                        if (leaf > 2u) sm.ring[(at + 2u) & (kTriRing - 1u)] = e + 2u;
                     }
                     pend += total;
                     while (pend >= 32u) test_batch(32u);
@@ -373,7 +378,7 @@ __device__ __forceinline__ void trace_queue8(const DevScene &S, unsigned first, 
                         while (tg.y != 0u && pos < dealt + room) {
                             const uint32_t b = __ffs(tg.y) - 1;
                             tg.y &= tg.y - 1u;
-                            sm.ring[(head + pend + (pos - dealt)) & (kTriRing - 1u)] = (tg.x + b) | (lane << kTriOwnerShift);
+                            sm.ring[(head + pend + (pos - dealt)) & (kTriRing - 1u)] = (tg.x + tri_offset(slots, b)) | (lane << kTriOwnerShift);
                             ++pos;
                         }
                         const uint32_t moved = min(total - dealt, room);

@@ -48,7 +48,7 @@ def _agree(a, ca, b, cb):
     assert np.allclose(a, b, rtol=1e-5, atol=1e-6 * scale), f"max abs difference {np.abs(a - b).max():.3e} of {scale}"
 
 
-# 1 and 3: one leaf; 24: a node full of three-triangle leaves (32 lanes x 24 tests overfill the 64-entry ring); 25, 70: beyond
+# 1 and 3: one leaf; 24: a node full of three-triangle leaves (32 lanes x 24 tests overfill the ring); 25, 70: beyond
 @pytest.mark.parametrize("n", [1, 3, 24, 25, 70])
 @pytest.mark.parametrize("size", [(1, 1), (37, 29)])
 def test_queued_triangle_tests_agree_with_the_serial_order(n, size):
