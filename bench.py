@@ -44,8 +44,8 @@ FALLBACK_HBM_GBS = 6650.0
 # (dram__bytes_read.sum + dram__bytes_write.sum), L2 bytes (lts__t_bytes.sum)
 # and warp instructions issued (smsp__inst_executed.sum).  The bench scales them
 # by the rays of its own launches.
-TRAVERSAL_PER_RAY = {"bvh8": {"extend": {"dram": 231.40, "l2": 964.0, "inst": 343.9},
-                              "shadow": {"dram": 114.43, "l2": 798.4, "inst": 241.9}}}
+TRAVERSAL_PER_RAY = {"bvh8": {"extend": {"dram": 294.10, "l2": 1065.2, "inst": 259.6},
+                              "shadow": {"dram": 194.11, "l2": 860.8, "inst": 200.2}}}
 SMS, SCHEDULERS_PER_SM = 148, 4
 MEASURED_SM_MAX_MHZ = 1965.0
 
@@ -626,6 +626,8 @@ def main():
     counters = torch.zeros(n_ctr, dtype=torch.int64, device="cuda")
     cam_list = [c for c in cams] if cams[0] is not None else None
     tuned, tune_ms = {}, None
+    if not wave:
+        gs.set_image_form(hk.FORM_MEGAKERNEL)
     if wave:
         tuned, tune_ms = gs.autotune(min(32, spp), depth, camera=cams[0])   # untimed set-up
         for kv in args.set:
@@ -773,12 +775,14 @@ def main():
         f = films[0]
         f.zero_()
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        gs.set_image_form(hk.FORM_MEGAKERNEL)   # hk_render gives a sample of this size to the wavefront
         gs.render(f, spp=ps, depth=depth, seed=3, camera=cams[0])
         torch.cuda.synchronize()
         e0.record(stream)
         gs.render(f, spp=ps, depth=depth, seed=4, camera=cams[0])
         e1.record(stream)
         torch.cuda.synchronize()
+        gs.set_image_form(hk.FORM_AUTO)
         plain = {"mpaths_per_s": W * H * ps / (e0.elapsed_time(e1) / 1e3) / 1e6,
                  "sample": f"view 0, {W}x{H} x {ps} spp, render_pathmis_kernel"}
     # the drop-in call a pathMISCuda plugin's RenderImage makes (hk_render_image:
