@@ -14,7 +14,7 @@
 //   shadow  any-hit of every queued shadow ray; unoccluded contributions are
 //           added to their path's radiance
 //
-// This file holds regen and the launch sequence; the queue helpers and the
+// This file holds regen and the launches of an iteration; the queue helpers and the
 // shade kernels are in hk_wf_kernels.cuh, the extend and shadow kernels in
 // hk_wf_trace.cuh.
 //
@@ -94,10 +94,11 @@ constexpr bool has_shade_kernel(int q) { return q == 0 || q == kWfGenericQueue |
 // bottom edges) counts as work done and leaves its slot idle until the next
 // iteration.  Where no plan follows this one (W.recycle == 0), idle slots
 // beyond the plan's end are dropped, so that a draining pool touches only the
-// paths still in flight (a quarter of a 2^22-path image's iterations drain).  Appends to the extend and idle lists, the per-job finished
-// counts and the change of the in-flight count are gathered per block in
-// shared memory and added once per block and round: a global atomic per warp
-// on a handful of addresses serialises at the L2.
+// paths still in flight (a quarter of a 2^22-path image's iterations drain).
+// Appends to the extend and idle lists, the per-job finished counts and the
+// change of the in-flight count are gathered per block in shared memory and
+// added once per block and round: a global atomic per warp on a handful of
+// addresses serialises at the L2.
 __global__ void __launch_bounds__(256) wf_regen_kernel(DevScene S, WfState W, int cur) {
     __shared__ unsigned s_finished[kWfMaxJobs];
     __shared__ int s_active;

@@ -8,7 +8,8 @@
 // rays, BSDF sampling, Russian roulette) -> shadow (any-hit, add unoccluded
 // next-event terms).  Kernels use fixed persistent grids and read queue sizes
 // and the dispatch plan from HBM, so iterations are captured once in a CUDA
-// graph and replayed; jobs and plans change between replays.
+// graph, looped on the device or replayed by the host; jobs and plans change
+// between launches.
 #pragma once
 #include <cuda_runtime.h>
 

@@ -1,6 +1,6 @@
 // Wavefront pathMIS kernels shared by the wavefront translation units: the
 // queue helpers and the shade kernel template.  hk_wavefront.cu holds regen
-// and the launch sequence; hk_wf_trace_*.cu instantiate the traversal kernels
+// and the launches of an iteration; hk_wf_trace_*.cu instantiate the traversal kernels
 // (hk_wf_trace.cuh) per tree kind and hk_wf_shade_*.cu the shade kernels per
 // queue, so they compile in parallel.
 #pragma once

@@ -316,7 +316,7 @@ typedef struct {
 
 /* Render every job of the batch with the wavefront integrator: a pool of path
  * slots shared by all images, compacted ray queues, one shading kernel per
- * material type, and iterations replayed from a CUDA graph.  Same estimator
+ * material type, and a loop over the iterations steered on the device.  Same estimator
  * as hk_render (PathMISIntegrator::Li, src/integrator/PathMISIntegrator.cpp:16).
  * Returns when every job is done; counters_dev (optional, 7 x u64) gets rays,
  * shadow rays, dropped samples, node visits and triangle tests of the
