@@ -28,6 +28,8 @@ WfEngine::WfEngine(const DevScene &S, int sm_count, const WfEngineConfig &cfg) :
     for (int t : {cfg_.threads_extend, cfg_.threads_shade})
         if (t % 32 != 0 || t <= 0 || t > 256)
             throw HkError{HK_ERR_INVALID, "wavefront block sizes must be multiples of 32 up to 256"};
+    if (!fits(cfg_.capacity, S.nemitters))
+        throw HkError{HK_ERR_INVALID, "wavefront capacity x emitters must be below 2^31"};
     const size_t N = (size_t)cfg_.capacity;
     W_.capacity = cfg_.capacity;
     W_.max_shadow = cfg_.capacity * std::max(1, S.nemitters);

@@ -4,6 +4,7 @@
 // the serving loop keeps one engine per resident scene and adds jobs to it
 // while it runs.
 #pragma once
+#include <algorithm>
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -37,6 +38,8 @@ public:
     WfEngine &operator=(const WfEngine &) = delete;
 
     // Device bytes an engine of this capacity holds for a scene with nemitters emitters and these shade queues.
+    // Shadow records are numbered in 32 bits: one for every slot and emitter.
+    static bool fits(int capacity, int nemitters) { return (int64_t)capacity * std::max(1, nemitters) < (1ll << 31); }
     static size_t bytes_for(int capacity, int nemitters, uint64_t shade_queues);
     size_t device_bytes() const { return bytes_; }
     const WfEngineConfig &config() const { return cfg_; }

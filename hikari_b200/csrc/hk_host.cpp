@@ -1401,7 +1401,7 @@ int hk_scene_get_info(const hk_scene *s, hk_scene_info *info) {
     });
 }
 
-static hk::WfEngineConfig engine_config(const hk_wavefront_config &c, uint64_t work) {
+static hk::WfEngineConfig engine_config(const hk_wavefront_config &c, uint64_t work, int nemitters) {
     hk::WfEngineConfig ec;
     ec.capacity = std::max(1024, std::min(c.capacity, 1 << 26));
     ec.threads_extend = c.threads_extend > 0 ? c.threads_extend : 128;
@@ -1414,7 +1414,9 @@ static hk::WfEngineConfig engine_config(const hk_wavefront_config &c, uint64_t w
     if (c.capacity <= 0) {   // as many slots as the work can use, from 2^14 to 2^21
         ec.fit_capacity = true;
         ec.capacity = 1 << 14;
-        while (ec.capacity < (1 << 21) && (uint64_t)ec.capacity < work) ec.capacity *= 2;
+        // a slot has a shadow record for every emitter: fewer than 2^28 of them (13 GB) past the least pool
+        while (ec.capacity < (1 << 21) && (uint64_t)ec.capacity < work && (int64_t)ec.capacity * nemitters < (1 << 27))
+            ec.capacity *= 2;
     }
     return ec;
 }
@@ -1448,9 +1450,10 @@ static bool render_wavefront_async(hk_scene *s, const hk_render_desc &d, float *
     hk::WfJob J = hk::make_wf_job(s, own);
     J.film = film;
     J.sample_major = c.sample_major ? 1 : 0;
-    const hk::WfEngineConfig ec = engine_config(c, J.work_count);
+    const hk::WfEngineConfig ec = engine_config(c, J.work_count, s->dev.nemitters);
     // every pass of the loop (a pair of iterations) advances each slot in use by two vertices
     if ((J.work_count / (uint64_t)ec.capacity + 1) * (uint64_t)d.depth + 64 > hk::kWfMaxLoops) return false;
+    if (!hk::WfEngine::fits(ec.capacity, s->dev.nemitters)) return false;
     hk::WfEngine *E;
     try {
         E = &wf_ensure(s, ec);
@@ -1680,7 +1683,7 @@ int hk_render_batch(hk_scene *s, const hk_render_job *jobs, int njobs, const hk_
             plan[j] = hk::WfSeg{total, 0, j, 0};
             total += table[j].work_count;
         }
-        const hk::WfEngineConfig ec = engine_config(c, total);
+        const hk::WfEngineConfig ec = engine_config(c, total, s->dev.nemitters);
         hk::WfEngine &E = wf_ensure(s, ec);
         cudaStream_t user = (cudaStream_t)stream, st = E.stream();
         // order after the caller's stream (the films may have been cleared there)

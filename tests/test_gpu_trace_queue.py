@@ -130,3 +130,26 @@ def test_each_ray_of_a_queue_is_claimed_once(size, threads):
         gs.set_wavefront_config(dict(capacity=capacity, threads_extend=threads))
         b, cb = gs.render_image(1, 6, seed=2)
         _agree(a, ca, b, cb)
+
+
+def test_pool_with_many_emitters():
+    """1100 area lights: a pool of 2^18 slots would hold more than 2^28 shadow records, the fitted one holds fewer.
+    A path's radiance is a sum of 1100 terms a vertex in any order: 2^-24 each. A capacity that needs 2^31 is refused."""
+    sd = scenes.cornell_box(width=512, height=512)
+    lp, li = scenes.quad((0, 0, 0), (0.01, 0, 0), (0.01, 0, 0.01), (0, 0, 0.01))
+    for k in range(1099):
+        off = np.float32([-0.9 + 0.05 * (k % 36), 1.97, -0.9 + 0.05 * (k // 36)])
+        sd.meshes.append(MeshDesc(lp + off, li, BSDFDesc(type=BSDF_DIFFUSE, kd=[0.0, 0.0, 0.0]), radiance=[9.0, 8.0, 7.0]))
+    gs = hk.Scene.from_desc(sd)
+    out = []
+    for form in (hk.FORM_MEGAKERNEL, hk.FORM_AUTO):
+        gs.set_image_form(form)
+        film = torch.zeros(gs.film_shape(), device="cuda")
+        ctr = torch.zeros(5, dtype=torch.int64, device="cuda")
+        gs.render(film, 1, 2, seed=7, counters=ctr)
+        out.append((film.cpu().numpy().astype(np.float64), ctr.cpu().numpy()))
+    (a, ca), (b, cb) = out
+    assert tuple(ca[:3]) == tuple(cb[:3])
+    assert np.allclose(a, b, rtol=1100 * 2.0 ** -24, atol=1e-6 * float(np.abs(a).max()))
+    with pytest.raises(hk.HikariError):
+        gs.render_batch([film], 1, 2, seeds=[1], capacity=1 << 21)
