@@ -153,3 +153,20 @@ def test_pool_with_many_emitters():
     assert np.allclose(a, b, rtol=1100 * 2.0 ** -24, atol=1e-6 * float(np.abs(a).max()))
     with pytest.raises(hk.HikariError):
         gs.render_batch([film], 1, 2, seeds=[1], capacity=1 << 21)
+
+
+# powers of two: every coordinate, and so every distance and box, scales exactly; the last camera stands 2^40.9 away
+@pytest.mark.parametrize("exponent,away,fov", [(-6, 3.8, 40.0), (0, 3.8, 40.0), (30, 3.8, 40.0), (30, 1945.6, 0.08)])
+def test_scaled_scenes(exponent, away, fov):
+    f = np.float32(2.0 ** exponent)
+    sd = scenes.cornell_box(width=32, height=32)
+    for m in sd.meshes:
+        m.positions = m.positions * f
+    sd.camera = CameraDesc(32, 32, scenes.look_at((0, 1 * f, away * f), (0, 1 * f, 0), (0, 1, 0)), fov, float(1e-4 * f),
+                           float(1e4 * f))
+    gs = hk.Scene.from_desc(sd)
+    gs.set_image_form(hk.FORM_MEGAKERNEL)
+    a, ca = gs.render_image(16, 8, seed=5)
+    gs.set_image_form(hk.FORM_WAVEFRONT)
+    b, cb = gs.render_image(16, 8, seed=5)
+    _agree(a, ca, b, cb)
