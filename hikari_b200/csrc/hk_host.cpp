@@ -1420,16 +1420,17 @@ static hk::WfEngineConfig engine_config(const hk_wavefront_config &c, uint64_t w
     }
     return ec;
 }
-// Whether a render of the scene's own image goes to the wavefront: from 2^18
+// Whether a render of the scene's own image goes to the wavefront: from 2^17
 // paths on.  Measured on five scenes (Cornell boxes of diffuse and of smooth
 // materials, a glass sphere, 64 spheres, textures; depth 16), megakernel /
 // wavefront: 2^16 paths 0.8-4.8 / 0.8-2.5 ms, 2^18 paths 1.5-13.8 / 1.2-3.1 ms,
 // 2^20 paths 4-46 / 2.5-4.9 ms; below 2^16 the wavefront's five launches a
-// bounce cost more than the megakernel's divergence, and a scene's first
+// bounce cost more than the megakernel's divergence, between 2^16 and 2^17 a
+// mesh of one conductor still does better in the megakernel (1.1 / 1.7 ms), and a scene's first
 // wavefront render spends 2 ms on its pool and graph.
 static bool work_for_wavefront(const hk_scene *s, const hk_render_desc &d) {
     if (s->image_form == HK_FORM_MEGAKERNEL || d.depth < 1 || d.depth > 65535) return false;
-    return (uint64_t)s->width * s->height * (uint64_t)d.spp >= (1ull << 18);
+    return (uint64_t)s->width * s->height * (uint64_t)d.spp >= (1ull << 17);
 }
 // hk_render through the wavefront, asynchronous on `stream` like the
 // megakernel: one launch that sets the pool, job and plan up, one graph whose

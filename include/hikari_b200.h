@@ -254,7 +254,7 @@ typedef struct {
 /* Accumulate spp samples per pixel into film_dev ((H+2B)*(W+2B)*4 floats of
  * RGB*w and w, B = ceil(radius - 0.5)); counters_dev (optional, 5 x u64) gets
  * closest-hit rays, shadow rays, dropped (invalid) samples, BVH node visits
- * and triangle tests added.  Asynchronous on `stream`.  Renders of 2^18 paths
+ * and triangle tests added.  Asynchronous on `stream`.  Renders of 2^17 paths
  * and more go to the wavefront integrator (its pool, sized to the work, is
  * allocated on first use and kept by the scene), smaller ones, captures of the
  * stream into a graph and calls without memory for the pool to the megakernel;
