@@ -1435,8 +1435,14 @@ static bool work_for_wavefront(const hk_scene *s, const hk_render_desc &d) {
 // hk_render through the wavefront, asynchronous on `stream` like the
 // megakernel: one launch that sets the pool, job and plan up, one graph whose
 // loop ends by itself, one for the counters.  False (nothing launched) where
-// the stream is being captured into a graph, which cannot hold a loop, where
-// the loop's bound might be reached, or where there is no memory for the pool.
+// the stream is being captured into a graph, which cannot hold a loop, or where
+// there is no memory for the pool.
+//
+// The loop of one graph launch ends after kWfMaxLoops passes, done or not, so the
+// graph is queued as often as the work could ask for: a path keeps its slot for
+// at most `depth` iterations, slots wait only once the plan is dealt, and a pass is two
+// iterations.  Roulette ends most paths long before their depth; a launch that
+// finds the pool empty ends after one pass.
 static bool render_wavefront_async(hk_scene *s, const hk_render_desc &d, float *film, unsigned long long *counters,
                                    cudaStream_t stream) {
     const hk_wavefront_config c = s->has_wf_cfg ? s->wf_cfg : hk_wavefront_config{};
@@ -1452,8 +1458,10 @@ static bool render_wavefront_async(hk_scene *s, const hk_render_desc &d, float *
     J.film = film;
     J.sample_major = c.sample_major ? 1 : 0;
     const hk::WfEngineConfig ec = engine_config(c, J.work_count, s->dev.nemitters);
-    // every pass of the loop (a pair of iterations) advances each slot in use by two vertices
-    if ((J.work_count / (uint64_t)ec.capacity + 1) * (uint64_t)d.depth + 64 > hk::kWfMaxLoops) return false;
+    const uint64_t slots = std::min<uint64_t>(J.work_count, (uint64_t)ec.capacity);
+    const uint64_t turns = (J.work_count + slots - 1) / slots + 1;   // paths of a slot one after another, and the last of all
+    if (turns > (1ull << 40)) return false;                          // 2^54 paths and more
+    const uint64_t passes = (turns * (uint64_t)d.depth) / 2 + 2;
     if (!hk::WfEngine::fits(ec.capacity, s->dev.nemitters)) return false;
     hk::WfEngine *E;
     try {
@@ -1471,8 +1479,8 @@ static bool render_wavefront_async(hk_scene *s, const hk_render_desc &d, float *
     } guard{ev};
     HK_CUDA(cudaEventRecord(ev, stream));
     HK_CUDA(cudaStreamWaitEvent(E->stream(), ev, 0));
-    E->begin(J, (int)std::min<uint64_t>(J.work_count, (uint64_t)ec.capacity));
-    E->run_to_end();
+    E->begin(J, (int)slots);
+    for (uint64_t p = 0; p < passes; p += hk::kWfMaxLoops) E->run_to_end();
     if (counters) E->add_counters(counters, true);
     HK_CUDA(cudaEventRecord(ev, E->stream()));
     HK_CUDA(cudaStreamWaitEvent(stream, ev, 0));

@@ -1,0 +1,57 @@
+"""Renders whose form, pool or launches the library chooses, at the lines of
+those rules (the rules themselves: test_host_routes.py)."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+import hikari_b200 as hk  # noqa: E402
+from hikari_b200 import scenes  # noqa: E402
+from hikari_b200.scenedesc import BSDF_DIFFUSE, BSDFDesc, CameraDesc, FilterDesc, MeshDesc, SceneDesc  # noqa: E402
+
+
+def _closed_room(side):
+    """A cube without openings, seen from inside: a path ends at its depth or in roulette alone."""
+    sd = SceneDesc()
+    c = [np.float32([x, y, z]) for x in (-1, 1) for y in (-1, 1) for z in (-1, 1)]
+    for q in ((0, 1, 3, 2), (4, 6, 7, 5), (0, 4, 5, 1), (2, 3, 7, 6), (0, 2, 6, 4), (1, 5, 7, 3)):
+        p, i = scenes.quad(*(c[k] for k in q))
+        n = np.cross(p[i[0][1]] - p[i[0][0]], p[i[0][2]] - p[i[0][0]])
+        if np.dot(n, p.mean(0)) > 0:   # facing inwards
+            i = i[:, ::-1].copy()
+        sd.meshes.append(MeshDesc(p, i, BSDFDesc(type=BSDF_DIFFUSE, kd=[0.9, 0.9, 0.9])))
+    lp, li = scenes.quad((-0.2, 0.99, -0.2), (0.2, 0.99, -0.2), (0.2, 0.99, 0.2), (-0.2, 0.99, 0.2))
+    if np.cross(lp[li[0][1]] - lp[li[0][0]], lp[li[0][2]] - lp[li[0][0]])[1] > 0:
+        li = li[:, ::-1].copy()
+    sd.meshes.append(MeshDesc(lp, li, BSDFDesc(type=BSDF_DIFFUSE, kd=[0.5, 0.5, 0.5]), radiance=[4.0, 5.0, 6.0]))
+    sd.camera = CameraDesc(side, side, scenes.look_at((0, 0, 0.9), (0, 0, 0), (0, 1, 0)), 60.0, 1e-4, 1e4)
+    sd.filter = FilterDesc(2, 2.0, 0.5)
+    return sd
+
+
+def _launches(gs, which=0):
+    n = C.c_int32()
+    buf = np.zeros(1, np.uint32)
+    hk.check(hk.lib().hk_wavefront_launch_log(gs.h, which, buf.ctypes.data, 1, C.byref(n)))
+    return n.value
+
+
+def test_render_of_more_passes_than_a_launch_of_the_loop_holds():
+    """2^20 paths of 64 vertices in a pool of 2^10 slots: 2^16 iterations, a launch of the loop ends after 2^15.
+    The film's weights say that every path was splatted once: up to 1024 terms a pixel (64 samples, 16 filter taps) in
+    any order, 2^-24 each; the mean radiance may differ by what a few of the 2^26 rays that graze an edge change."""
+    gs = hk.Scene.from_desc(_closed_room(128))
+    gs.set_wavefront_config(dict(capacity=1024))
+    films = []
+    for form in (hk.FORM_MEGAKERNEL, hk.FORM_AUTO):
+        gs.set_image_form(form)
+        film = torch.zeros(gs.film_shape(), device="cuda")
+        gs.render(film, 64, 64, seed=3, rr_start=64)
+        films.append(film.cpu().numpy().astype(np.float64))
+    assert _launches(gs) > 1 << 15
+    a, b = films
+    assert np.allclose(a[..., 3], b[..., 3], rtol=1024 * 2.0 ** -24)
+    assert abs(b[..., :3].mean() / a[..., :3].mean() - 1) < 1e-4

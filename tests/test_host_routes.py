@@ -1,0 +1,107 @@
+"""The library's host decisions -- form, pool, launches, streams, devices,
+memory -- against a CUDA runtime of host memory (fake_cuda.cpp): its own host
+sources, compiled with g++, over a fake that logs what would be launched."""
+import concurrent.futures
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+import hikari_b200 as hk
+from hikari_b200 import build, scenes
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+SOURCES = [os.path.join(build.CSRC, f) for f in build.SOURCES if f.endswith(".cpp")] + [os.path.join(HERE, "fake_cuda.cpp")]
+
+
+@pytest.fixture(scope="module")
+def fake_lib(tmp_path_factory):
+    out = tmp_path_factory.mktemp("fake_cuda")
+    so = str(out / "libhikari_fake.so")
+
+    def compile_one(src):
+        obj = str(out / (os.path.basename(src) + ".o"))
+        subprocess.run(["g++", "-std=c++17", "-O1", "-fPIC", "-pthread", "-I/usr/local/cuda/include", "-I" + build.CSRC, "-c",
+                        src, "-o", obj], check=True)
+        return obj
+
+    with concurrent.futures.ThreadPoolExecutor() as pool:
+        objs = list(pool.map(compile_one, SOURCES))
+    # -Bsymbolic: the fake's entry points, also where a real runtime is loaded already
+    subprocess.run(["g++", "-shared", "-Wl,-Bsymbolic,--no-undefined", "-o", so] + objs + ["-lz", "-lpthread"], check=True)
+    return so
+
+
+class Fake:
+    """The fake's controls."""
+
+    def __init__(self, so):
+        L = C.CDLL(so)
+        L.fake_log.restype = C.c_char_p
+        L.fake_live.restype = C.c_size_t
+        L.fake_limit.argtypes = [C.c_size_t]
+        L.fake_passes_left.restype = C.c_uint64
+        L.fake_stream.restype = C.c_void_p
+        self.L = L
+
+    def log(self):
+        """What was launched since the last call."""
+        text = self.L.fake_log().decode().split("\n")[:-1]
+        self.L.fake_clear()
+        return text
+
+    def forms(self):
+        """The forms of the renders since the last call, one word per render."""
+        return [x.split()[0] for x in self.log() if x.startswith(("mega", "begin"))]
+
+    def live(self):
+        return self.L.fake_live()
+
+
+@pytest.fixture
+def fake(fake_lib, monkeypatch):
+    monkeypatch.setattr(hk, "LIB_PATH", fake_lib)
+    monkeypatch.setattr(hk, "_lib", None)
+    f = Fake(fake_lib)
+    f.made = []
+    f.log()
+    yield f
+    for s in f.made:   # while the fake is the library
+        s.close()
+    f.L.fake_limit(C.c_size_t(-1).value)
+    f.L.fake_device(0)
+    f.L.fake_other_capture(0)
+    f.L.fake_user_capturing(0)
+    f.L.fake_fail_instantiate(0)
+
+
+def _scene(fake, width=64, height=64, lights=1):
+    """A Cornell box; lights > 1: as many area lights."""
+    sd = scenes.cornell_box(width=width, height=height)
+    light = next(m for m in sd.meshes if m.radiance is not None)
+    for k in range(lights - 1):
+        sd.meshes.append(light)
+    s = hk.Scene.from_desc(sd)
+    fake.made.append(s)
+    fake.log()
+    return s
+
+
+def _render(s, spp, depth=16, **kw):
+    film = np.zeros(4, np.float32)   # the fake writes no film
+    s.render(film, spp, depth, stream=0, **kw)
+
+
+# 2^29 paths of depth 64; 2^25 of depth 1000; 2^19 of depth 64 in the least pool; the deepest that the path state holds
+@pytest.mark.parametrize("width,spp,depth,capacity", [(256, 8192, 64, 0), (256, 16384, 64, 0), (1024, 32, 1000, 0),
+                                                      (64, 128, 64, 1024), (256, 2, 65535, 0)])
+def test_long_and_deep_renders_stay_on_the_wavefront(fake, width, spp, depth, capacity):
+    s = _scene(fake, width, width)
+    if capacity:
+        s.set_wavefront_config(dict(capacity=capacity))
+    _render(s, spp, depth)
+    assert fake.forms() == ["begin"]
+    # as many launches of the loop as the work can need if every path reaches its depth
+    assert fake.L.fake_passes_left() == 0
