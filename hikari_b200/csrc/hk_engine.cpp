@@ -30,6 +30,7 @@ WfEngine::WfEngine(const DevScene &S, int sm_count, const WfEngineConfig &cfg) :
             throw HkError{HK_ERR_INVALID, "wavefront block sizes must be multiples of 32 up to 256"};
     if (!fits(cfg_.capacity, S.nemitters))
         throw HkError{HK_ERR_INVALID, "wavefront capacity x emitters must be below 2^31"};
+    HK_CUDA(cudaGetDevice(&device_));
     const size_t N = (size_t)cfg_.capacity;
     W_.capacity = cfg_.capacity;
     W_.max_shadow = cfg_.capacity * std::max(1, S.nemitters);

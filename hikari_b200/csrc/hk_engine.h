@@ -43,6 +43,7 @@ public:
     static size_t bytes_for(int capacity, int nemitters, uint64_t shade_queues);
     size_t device_bytes() const { return bytes_; }
     const WfEngineConfig &config() const { return cfg_; }
+    int device() const { return device_; }   // the device that was current when the engine was made: its memory, streams and events
     // The stream the engine's work goes to next (one of two of different priority).
     cudaStream_t stream() const { return stream_; }
     // Move later work to the high- or low-priority stream, ordered after all
@@ -90,6 +91,7 @@ private:
     WfLaunchConfig L_{};
     WfState W_{};
     size_t bytes_ = 0;
+    int device_ = 0;
     int job_count_ = 0;   // highest job slot ever set + 1
     DevBuf mem_;             // slot records, queues, shadow queue, counters, job table, plan
     PinnedBuf<char> host_;   // the host mirrors below

@@ -1020,14 +1020,16 @@ void require_scene_size(const hk_scene *s, const hk_render_desc &d) {
 }
 
 // ------------------------------------------------------------ wavefront engine
-// The scene's engine of configuration c.  Pools fitted to the work and pools
+// The scene's engine of configuration c on the current device.  Pools fitted to the work and pools
 // that a caller sized are kept apart, so that alternating calls of the two kinds
 // do not rebuild them; a fitted one serves every call that needs no more slots.
 hk::WfEngine &wf_ensure(hk_scene *s, const hk::WfEngineConfig &c) {
     std::unique_ptr<hk::WfEngine> &e = c.fit_capacity ? s->wf_fit : s->wf;
+    int dev = 0;
+    HK_CUDA(cudaGetDevice(&dev));
     if (e) {
         const hk::WfEngineConfig &o = e->config();
-        if ((c.fit_capacity ? o.capacity >= c.capacity : o.capacity == c.capacity) && o.threads_extend == c.threads_extend &&
+        if (e->device() == dev && (c.fit_capacity ? o.capacity >= c.capacity : o.capacity == c.capacity) && o.threads_extend == c.threads_extend &&
             o.threads_shade == c.threads_shade && o.fetch_steps == c.fetch_steps && o.fetch_min_idle == c.fetch_min_idle &&
             o.fetch_steps_shadow == c.fetch_steps_shadow && o.fetch_min_idle_shadow == c.fetch_min_idle_shadow &&
             o.reg_lean == c.reg_lean) {
@@ -1435,8 +1437,9 @@ static bool work_for_wavefront(const hk_scene *s, const hk_render_desc &d) {
 // hk_render through the wavefront, asynchronous on `stream` like the
 // megakernel: one launch that sets the pool, job and plan up, one graph whose
 // loop ends by itself, one for the counters.  False (nothing launched) where
-// the stream is being captured into a graph, which cannot hold a loop, or where
-// there is no memory for the pool.
+// the stream is being captured into a graph, which cannot hold a loop, where
+// another device than the scene's is current (the megakernel runs there and
+// reads the scene as a peer), or where there is no memory for the pool.
 //
 // The loop of one graph launch ends after kWfMaxLoops passes, done or not, so the
 // graph is queued as often as the work could ask for: a path keeps its slot for
@@ -1452,6 +1455,9 @@ static bool render_wavefront_async(hk_scene *s, const hk_render_desc &d, float *
         cudaGetLastError();
         return false;
     }
+    int dev = 0;
+    HK_CUDA(cudaGetDevice(&dev));
+    if (dev != s->device) return false;
     hk_render_desc own = d;
     own.width = own.height = 0;
     hk::WfJob J = hk::make_wf_job(s, own);

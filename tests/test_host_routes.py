@@ -105,3 +105,28 @@ def test_long_and_deep_renders_stay_on_the_wavefront(fake, width, spp, depth, ca
     assert fake.forms() == ["begin"]
     # as many launches of the loop as the work can need if every path reaches its depth
     assert fake.L.fake_passes_left() == 0
+
+
+def _devices(log):
+    return [x.split()[x.split().index("device") + 1] for x in log if x.startswith("loop")]
+
+
+def test_render_on_another_device_than_the_scenes(fake):
+    """The megakernel, which runs where the caller is; the scene's pool stays on the scene's device."""
+    s = _scene(fake, 512, 512)
+    fake.L.fake_device(1)
+    _render(s, 1)
+    assert fake.forms() == ["mega"]
+    fake.L.fake_device(0)
+    _render(s, 1)
+    log = fake.log()
+    assert any(x.startswith("begin") for x in log) and _devices(log) == ["0"]
+
+
+def test_batch_pools_belong_to_the_current_device(fake):
+    s = _scene(fake)
+    film = np.zeros(4, np.float32)
+    for device in (1, 0, 0, 1):
+        fake.L.fake_device(device)
+        s.render_batch([film], 1, 8, stream=0)
+        assert _devices(fake.log()) == [str(device)]
