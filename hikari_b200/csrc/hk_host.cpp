@@ -1023,8 +1023,9 @@ void require_scene_size(const hk_scene *s, const hk_render_desc &d) {
 // The scene's engine of configuration c on the current device.  Pools fitted to the work and pools
 // that a caller sized are kept apart, so that alternating calls of the two kinds
 // do not rebuild them; a fitted one serves every call that needs no more slots.
+// Short of memory, either makes room for the other.
 hk::WfEngine &wf_ensure(hk_scene *s, const hk::WfEngineConfig &c) {
-    std::unique_ptr<hk::WfEngine> &e = c.fit_capacity ? s->wf_fit : s->wf;
+    std::unique_ptr<hk::WfEngine> &e = c.fit_capacity ? s->wf_fit : s->wf, &other = c.fit_capacity ? s->wf : s->wf_fit;
     int dev = 0;
     HK_CUDA(cudaGetDevice(&dev));
     if (e) {
@@ -1041,11 +1042,11 @@ hk::WfEngine &wf_ensure(hk_scene *s, const hk::WfEngineConfig &c) {
     }
     try {
         e.reset(new hk::WfEngine(s->dev, s->sm_count, c));
-    } catch (const HkError &) {
-        if (c.fit_capacity || !s->wf_fit) throw;
-        cudaGetLastError();   // short of memory: the fitted pool makes room
-        if (s->wf_last == s->wf_fit.get()) s->wf_last = nullptr;
-        s->wf_fit.reset();
+    } catch (const HkError &err) {
+        if (!other || err.code != HK_ERR_NOMEM) throw;
+        cudaGetLastError();
+        if (s->wf_last == other.get()) s->wf_last = nullptr;
+        other.reset();
         e.reset(new hk::WfEngine(s->dev, s->sm_count, c));
     }
     s->wf_last = e.get();

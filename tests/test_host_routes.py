@@ -130,3 +130,34 @@ def test_batch_pools_belong_to_the_current_device(fake):
         fake.L.fake_device(device)
         s.render_batch([film], 1, 8, stream=0)
         assert _devices(fake.log()) == [str(device)]
+
+
+def _pool(s, fake, **kw):
+    """Bytes that a batch's pool takes."""
+    film, before = np.zeros(4, np.float32), fake.live()
+    s.render_batch([film], 1, 8, stream=0, **kw)
+    return fake.live() - before
+
+
+# the second pool finds no memory beside the first: the first, idle, makes room
+def test_a_fitted_pool_may_take_the_place_of_a_sized_one(fake):
+    s = _scene(fake, 512, 512)
+    film = np.zeros(4, np.float32)
+    _pool(s, fake, capacity=1 << 20)
+    fake.L.fake_limit(fake.live() + (1 << 20))
+    s.render_batch([film], 1, 8, stream=0)
+    assert [x for x in fake.log() if x.startswith("loop")][-1].endswith("capacity 262144")
+    s.render_batch([film], 1, 8, stream=0, capacity=1 << 20)
+    assert [x for x in fake.log() if x.startswith("loop")][-1].endswith("capacity 1048576")
+
+
+def test_a_film_render_takes_the_place_of_a_sized_pool_once(fake):
+    s = _scene(fake, 512, 512)
+    _pool(s, fake, capacity=1 << 20)
+    fake.L.fake_limit(fake.live() + (1 << 20))
+    fake.log()
+    _render(s, 1)
+    _render(s, 1)
+    log = fake.log()
+    assert [x.split()[0] for x in log if x.startswith(("mega", "begin"))] == ["begin", "begin"]
+    assert log.count("malloc-failed") == 1
