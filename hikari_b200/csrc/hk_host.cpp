@@ -1606,6 +1606,10 @@ int hk_scene_set_image_form(hk_scene *s, int32_t form) {
     return guarded([&] {
         if (!s || form < HK_FORM_AUTO || form > HK_FORM_WAVEFRONT) throw HkError{HK_ERR_INVALID, "bad arguments"};
         s->image_form = form;
+        if (form == HK_FORM_MEGAKERNEL && s->wf_fit) {   // hk_render's pool; one that a caller sized is hk_render_batch's
+            if (s->wf_last == s->wf_fit.get()) s->wf_last = nullptr;
+            s->wf_fit.reset();
+        }
         return HK_OK;
     });
 }

@@ -255,10 +255,16 @@ typedef struct {
  * RGB*w and w, B = ceil(radius - 0.5)); counters_dev (optional, 5 x u64) gets
  * closest-hit rays, shadow rays, dropped (invalid) samples, BVH node visits
  * and triangle tests added.  Asynchronous on `stream`.  Renders of 2^17 paths
- * and more go to the wavefront integrator (its pool, sized to the work, is
- * allocated on first use and kept by the scene), smaller ones, captures of the
- * stream into a graph and calls without memory for the pool to the megakernel;
- * HK_FORM_MEGAKERNEL keeps all of them there.  Both forms draw the same
+ * and more go to the wavefront integrator, smaller ones, captures of the stream
+ * into a graph, calls without memory for the pool, on another device than the
+ * scene's or with a depth above 65535 to the megakernel; HK_FORM_MEGAKERNEL
+ * keeps all of them there.  The wavefront's pool (2^14 to 2^21 slots as the work
+ * asks for, 128 B and 48 B per emitter each and 4 B for each of its queues: 0.9
+ * GB at 2^21 slots and 5 emitters; more than 2^14 slots only up to 13 GB of
+ * shadow records) is made on
+ * first use, which waits for the device, made anew for a larger one, which waits
+ * for the scene's earlier renders, and kept by the scene until it is rebuilt,
+ * destroyed or set to HK_FORM_MEGAKERNEL.  Both forms draw the same
  * per-sample streams. */
 int hk_render(hk_scene *s, const hk_render_desc *desc, float *film_dev, unsigned long long *counters_dev,
               void *stream);
@@ -277,7 +283,9 @@ int hk_render_image(hk_scene *s, const hk_render_desc *desc, float *rgb_host, un
                     void *stream);
 enum { HK_FORM_AUTO = 0, HK_FORM_MEGAKERNEL = 1, HK_FORM_WAVEFRONT = 2 };
 /* The form hk_render_image renders with (HK_FORM_AUTO by default);
- * HK_FORM_MEGAKERNEL holds for hk_render too. */
+ * HK_FORM_MEGAKERNEL holds for hk_render too, and gives the device memory of
+ * the pool that hk_render and hk_render_batch fitted to their work back (it
+ * waits for their renders). */
 int hk_scene_set_image_form(hk_scene *s, int32_t form);
 
 /* ---- wavefront rendering (the batched form) ---- */

@@ -161,3 +161,19 @@ def test_a_film_render_takes_the_place_of_a_sized_pool_once(fake):
     log = fake.log()
     assert [x.split()[0] for x in log if x.startswith(("mega", "begin"))] == ["begin", "begin"]
     assert log.count("malloc-failed") == 1
+
+
+def test_the_megakernel_form_gives_the_film_pool_back(fake):
+    """A pool that a caller sized stays: hk_render_batch goes on using it."""
+    s = _scene(fake, 512, 512)
+    before = fake.live()
+    _render(s, 1)
+    assert fake.live() > before + (1 << 20)
+    s.set_image_form(hk.FORM_MEGAKERNEL)
+    assert fake.live() == before
+    _render(s, 1)
+    assert fake.live() == before
+    s.set_image_form(hk.FORM_AUTO)
+    sized = _pool(s, fake, capacity=1 << 20)
+    s.set_image_form(hk.FORM_MEGAKERNEL)
+    assert fake.live() == before + sized
