@@ -25,9 +25,7 @@ size_t WfEngine::bytes_for(int capacity, int nemitters, uint64_t shade_queues) {
 WfEngine::WfEngine(const DevScene &S, int sm_count, const WfEngineConfig &cfg) : S_(S), cfg_(cfg) {
     if (cfg_.capacity < 1024 || cfg_.capacity > (1 << 26))
         throw HkError{HK_ERR_INVALID, "wavefront capacity must be in [1024, 2^26]"};
-    for (int t : {cfg_.threads_extend, cfg_.threads_shade})
-        if (t % 32 != 0 || t <= 0 || t > 256)
-            throw HkError{HK_ERR_INVALID, "wavefront block sizes must be multiples of 32 up to 256"};
+    if (!valid_threads(cfg_)) throw HkError{HK_ERR_INVALID, "wavefront block sizes must be multiples of 32 up to 256"};
     if (!fits(cfg_.capacity, S.nemitters))
         throw HkError{HK_ERR_INVALID, "wavefront capacity x emitters must be below 2^31"};
     HK_CUDA(cudaGetDevice(&device_));

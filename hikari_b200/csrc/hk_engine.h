@@ -40,6 +40,11 @@ public:
     // Device bytes an engine of this capacity holds for a scene with nemitters emitters and these shade queues.
     // Shadow records are numbered in 32 bits: one for every slot and emitter.
     static bool fits(int capacity, int nemitters) { return (int64_t)capacity * std::max(1, nemitters) < (1ll << 31); }
+    static bool valid_threads(const WfEngineConfig &c) {
+        for (int t : {c.threads_extend, c.threads_shade})
+            if (t % 32 != 0 || t <= 0 || t > 256) return false;
+        return true;
+    }
     static size_t bytes_for(int capacity, int nemitters, uint64_t shade_queues);
     size_t device_bytes() const { return bytes_; }
     const WfEngineConfig &config() const { return cfg_; }

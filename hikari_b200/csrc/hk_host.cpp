@@ -1440,7 +1440,8 @@ static bool work_for_wavefront(const hk_scene *s, const hk_render_desc &d) {
 // loop ends by itself, one for the counters.  False (nothing launched) where
 // the stream is being captured into a graph, which cannot hold a loop, where
 // another device than the scene's is current (the megakernel runs there and
-// reads the scene as a peer), or where there is no memory for the pool.
+// reads the scene as a peer), where the scene's stored configuration is one that
+// a pool refuses, or where there is no memory for the pool.
 //
 // The loop of one graph launch ends after kWfMaxLoops passes, done or not, so the
 // graph is queued as often as the work could ask for: a path keeps its slot for
@@ -1469,12 +1470,11 @@ static bool render_wavefront_async(hk_scene *s, const hk_render_desc &d, float *
     const uint64_t turns = (J.work_count + slots - 1) / slots + 1;   // paths of a slot one after another, and the last of all
     if (turns > (1ull << 40)) return false;                          // 2^54 paths and more
     const uint64_t passes = (turns * (uint64_t)d.depth) / 2 + 2;
-    if (!hk::WfEngine::fits(ec.capacity, s->dev.nemitters)) return false;
+    if (!hk::WfEngine::fits(ec.capacity, s->dev.nemitters) || !hk::WfEngine::valid_threads(ec)) return false;
     hk::WfEngine *E;
     try {
         E = &wf_ensure(s, ec);
-    } catch (const HkError &e) {
-        if (e.code == HK_ERR_INVALID) throw;
+    } catch (const HkError &) {
         cudaGetLastError();
         return false;
     }
@@ -1568,8 +1568,14 @@ int hk_render_image(hk_scene *s, const hk_render_desc *d, float *rgb_host, unsig
         unsigned long long *ctr = (unsigned long long *)s->b_scratch.p + 1;
         unsigned long long *ctr7 = (unsigned long long *)s->b_scratch.p + 8;
         HK_CUDA(cudaMemsetAsync(s->b_film.p, 0, film_bytes, st));
-        // HK_FORM_WAVEFRONT: small images too, through the batch
-        const bool wave = s->image_form == HK_FORM_WAVEFRONT;
+        // HK_FORM_WAVEFRONT: small images too, through the batch.  A stored
+        // configuration that a pool refuses leaves hk_render with the megakernel;
+        // here large images have always been refused then, and the batch does that
+        const hk_wavefront_config c = s->has_wf_cfg ? s->wf_cfg : hk_wavefront_config{};
+        const uint64_t px = (uint64_t)s->width * s->height;
+        const bool refused = px >= 65536 && px * (uint64_t)d->spp >= (1ull << 22) &&
+                             !hk::WfEngine::valid_threads(engine_config(c, 0, s->dev.nemitters));
+        const bool wave = s->image_form == HK_FORM_WAVEFRONT || (s->image_form == HK_FORM_AUTO && refused);
         int rc;
         if (wave) {
             HK_CUDA(cudaMemsetAsync(ctr7, 0, 7 * sizeof(unsigned long long), st));

@@ -177,3 +177,32 @@ def test_the_megakernel_form_gives_the_film_pool_back(fake):
     sized = _pool(s, fake, capacity=1 << 20)
     s.set_image_form(hk.FORM_MEGAKERNEL)
     assert fake.live() == before + sized
+
+
+def _image(s, spp):
+    d = hk.render_desc(spp, 16)
+    out = np.zeros((s.desc.camera.height, s.desc.camera.width, 3), np.float32)
+    hk.check(hk.lib().hk_render_image(s.h, C.byref(d), out.ctypes.data, None, None))
+
+
+def _store(s, **kw):
+    c = hk.WavefrontConfig()
+    for k, v in kw.items():
+        setattr(c, k, v)
+    hk.check(hk.lib().hk_scene_set_wavefront_config(s.h, C.byref(c)))
+
+
+@pytest.mark.parametrize("field", ["threads_extend", "threads_shade"])
+@pytest.mark.parametrize("threads", [100, 288])
+def test_a_stored_configuration_that_the_pool_refuses(fake, field, threads):
+    """hk_render, which does not need it, renders with the megakernel; hk_render_image too, except for the large images
+    (2^22 paths of 256 x 256 pixels) that it has always refused then."""
+    s = _scene(fake, 512, 512)
+    _store(s, **{field: threads})
+    _render(s, 1)
+    _image(s, 15)
+    assert fake.forms() == ["mega", "mega"]
+    with pytest.raises(hk.HikariError):
+        _image(s, 16)
+    with pytest.raises(hk.HikariError):
+        s.render_batch([np.zeros(4, np.float32)], 1, 8, stream=0, **{field: threads})
