@@ -1568,15 +1568,23 @@ int hk_render_image(hk_scene *s, const hk_render_desc *d, float *rgb_host, unsig
         unsigned long long *ctr = (unsigned long long *)s->b_scratch.p + 1;
         unsigned long long *ctr7 = (unsigned long long *)s->b_scratch.p + 8;
         HK_CUDA(cudaMemsetAsync(s->b_film.p, 0, film_bytes, st));
-        // HK_FORM_WAVEFRONT: small images too, through the batch.  A stored
+        // HK_FORM_WAVEFRONT: small images too, through the batch; and the large
+        // ones that hk_render, which returns at once, leaves to the megakernel
+        // though the batch, which waits, renders them with the wavefront: without
+        // a graph, and on another device than the scene's.  A stored
         // configuration that a pool refuses leaves hk_render with the megakernel;
         // here large images have always been refused then, and the batch does that
         const hk_wavefront_config c = s->has_wf_cfg ? s->wf_cfg : hk_wavefront_config{};
         const uint64_t px = (uint64_t)s->width * s->height;
-        const bool refused = px >= 65536 && px * (uint64_t)d->spp >= (1ull << 22) &&
-                             !hk::WfEngine::valid_threads(engine_config(c, 0, s->dev.nemitters));
-        const bool wave = s->image_form == HK_FORM_WAVEFRONT || (s->image_form == HK_FORM_AUTO && refused);
-        int rc;
+        const hk::WfEngineConfig ec = engine_config(c, px * (uint64_t)d->spp, s->dev.nemitters);
+        const bool valid = hk::WfEngine::valid_threads(ec);
+        const bool refused = px >= 65536 && px * (uint64_t)d->spp >= (1ull << 22) && !valid;
+        int dev = 0;
+        HK_CUDA(cudaGetDevice(&dev));
+        const bool waits = work_for_wavefront(s, *d) && (c.no_graph || dev != s->device) && valid &&
+                           hk::WfEngine::fits(ec.capacity, s->dev.nemitters);
+        bool wave = s->image_form == HK_FORM_WAVEFRONT || (s->image_form == HK_FORM_AUTO && (refused || waits));
+        int rc = HK_OK;
         if (wave) {
             HK_CUDA(cudaMemsetAsync(ctr7, 0, 7 * sizeof(unsigned long long), st));
             hk_render_job job;
@@ -1584,7 +1592,9 @@ int hk_render_image(hk_scene *s, const hk_render_desc *d, float *rgb_host, unsig
             job.desc = *d;
             job.desc.width = job.desc.height = 0;
             rc = hk_render_batch(s, &job, 1, s->has_wf_cfg ? &s->wf_cfg : nullptr, ctr7, stream);
-        } else {
+            if (rc == HK_ERR_NOMEM && s->image_form == HK_FORM_AUTO) wave = false;   // as hk_render without memory for the pool
+        }
+        if (!wave) {
             HK_CUDA(cudaMemsetAsync(ctr, 0, 5 * sizeof(unsigned long long), st));
             rc = hk_render(s, d, s->b_film.as<float>(), ctr, stream);
         }

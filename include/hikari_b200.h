@@ -257,12 +257,12 @@ typedef struct {
  * and triangle tests added.  Asynchronous on `stream`.  Renders of 2^17 paths
  * and more go to the wavefront integrator, smaller ones, captures of the stream
  * into a graph, calls without memory for the pool, on another device than the
- * scene's or with a depth above 65535 to the megakernel; HK_FORM_MEGAKERNEL
- * keeps all of them there.  The wavefront's pool (2^14 to 2^21 slots as the work
+ * scene's, with a depth above 65535 or a stored configuration that has no_graph
+ * or that a pool refuses to the megakernel; HK_FORM_MEGAKERNEL keeps all of them
+ * there.  The wavefront's pool (2^14 to 2^21 slots as the work
  * asks for, 128 B and 48 B per emitter each and 4 B for each of its queues: 0.9
  * GB at 2^21 slots and 5 emitters; more than 2^14 slots only up to 13 GB of
- * shadow records) is made on
- * first use, which waits for the device, made anew for a larger one, which waits
+ * shadow records) is made on first use, which waits for the device, made anew for a larger one, which waits
  * for the scene's earlier renders, and kept by the scene until it is rebuilt,
  * destroyed or set to HK_FORM_MEGAKERNEL.  Both forms draw the same
  * per-sample streams. */
@@ -276,7 +276,8 @@ int hk_film_resolve(hk_scene *s, const float *film_dev, float *rgb_dev, void *st
  * rgb_host.  counters (host, 5) optional: as hk_render's (node visits and
  * triangle tests summed over closest-hit and shadow rays).  HK_FORM_WAVEFRONT
  * renders with the wavefront integrator whatever the size (hk_render_batch, one
- * job), otherwise hk_render picks the form.  Both run the same estimator on the
+ * job), otherwise hk_render picks the form, and the batch renders its large
+ * images that hk_render would not (no_graph, another device).  Both run the same estimator on the
  * same per-sample streams: the images agree up to the order of the film's float
  * additions. */
 int hk_render_image(hk_scene *s, const hk_render_desc *desc, float *rgb_host, unsigned long long *counters,

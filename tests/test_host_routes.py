@@ -206,3 +206,33 @@ def test_a_stored_configuration_that_the_pool_refuses(fake, field, threads):
         _image(s, 16)
     with pytest.raises(hk.HikariError):
         s.render_batch([np.zeros(4, np.float32)], 1, 8, stream=0, **{field: threads})
+
+
+def test_a_stored_configuration_without_graphs(fake):
+    """hk_render, which returns at once, has no loop without a graph; hk_render_image waits and launches kernel by kernel."""
+    s = _scene(fake, 512, 512)
+    _store(s, no_graph=1)
+    _render(s, 16)
+    assert fake.forms() == ["mega"]
+    for spp in (1, 16):
+        _image(s, spp)
+        log = fake.log()
+        assert "plain" in log and not any(x.startswith(("mega", "loop")) for x in log)
+    s2 = _scene(fake, 64, 64)   # below 2^17 paths
+    _store(s2, no_graph=1)
+    _image(s2, 1)
+    assert fake.forms() == ["mega"]
+
+
+def test_whole_images_on_another_device(fake):
+    """hk_render_image waits, so it may make a pool there."""
+    s = _scene(fake, 512, 512)
+    fake.L.fake_device(1)
+    _image(s, 1)
+    assert _devices(fake.log()) == ["1"]
+    fake.L.fake_device(0)
+    s = _scene(fake, 512, 512)
+    _store(s, no_graph=1)
+    fake.L.fake_limit(fake.live() + (8 << 20))   # the image's buffers, but no pool
+    _image(s, 1)
+    assert fake.forms() == ["mega"]
