@@ -1464,6 +1464,8 @@ static bool render_wavefront_async(hk_scene *s, const hk_render_desc &d, float *
     own.width = own.height = 0;
     hk::WfJob J = hk::make_wf_job(s, own);
     J.film = film;
+    J.sample_offset = (uint64_t)(int64_t)d.sample_offset;   // signed, as in the megakernel (the batch takes them as unsigned)
+    J.image_index = (uint64_t)(int64_t)d.image_index;
     J.sample_major = c.sample_major ? 1 : 0;
     const hk::WfEngineConfig ec = engine_config(c, J.work_count, s->dev.nemitters);
     const uint64_t slots = std::min<uint64_t>(J.work_count, (uint64_t)ec.capacity);

@@ -64,7 +64,8 @@ struct WfJob {
     unsigned long long *finished;   // work items of this job finished (device counter)
     uint64_t seed;
     uint64_t work_count;            // tiles * spp * 256 work items
-    uint32_t spp, sample_offset, image_index, tiles_x;
+    uint64_t sample_offset, image_index;   // of 64 bits: hk_render's may be negative
+    uint32_t spp, tiles_x;
     uint32_t width, height;
     float cam_aspect;               // width / height (PerspectiveCamera::Activate)
     int32_t depth, rr_start;

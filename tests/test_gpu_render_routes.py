@@ -55,3 +55,16 @@ def test_render_of_more_passes_than_a_launch_of_the_loop_holds():
     a, b = films
     assert np.allclose(a[..., 3], b[..., 3], rtol=1024 * 2.0 ** -24)
     assert abs(b[..., :3].mean() / a[..., :3].mean() - 1) < 1e-4
+
+
+def test_negative_sample_offsets_and_image_indices_in_both_forms():
+    """The same streams, so the same image up to the order of the film's additions (64 samples x 16 taps: 2^-24 each)."""
+    gs = hk.Scene.from_desc(scenes.cornell_box(width=128, height=128))
+    films = []
+    for form in (hk.FORM_MEGAKERNEL, hk.FORM_AUTO):
+        gs.set_image_form(form)
+        film = torch.zeros(gs.film_shape(), device="cuda")
+        gs.render(film, 8, 4, seed=3, sample_offset=-5, image_index=-2)
+        films.append(film.cpu().numpy().astype(np.float64))
+    a, b = films
+    assert np.allclose(a, b, rtol=1024 * 2.0 ** -24, atol=1e-6 * float(a.max()))

@@ -236,3 +236,10 @@ def test_whole_images_on_another_device(fake):
     fake.L.fake_limit(fake.live() + (8 << 20))   # the image's buffers, but no pool
     _image(s, 1)
     assert fake.forms() == ["mega"]
+
+
+def test_negative_sample_offsets_and_image_indices(fake):
+    """hk_render takes both as signed numbers of 64 bits, in either form."""
+    s = _scene(fake, 512, 512)
+    _render(s, 1, sample_offset=-5, image_index=-2)
+    assert [x for x in fake.log() if x.startswith("begin")] == ["begin slots 262144 sample -5 image -2"]
