@@ -228,12 +228,15 @@ void WfEngine::capture_loop() {
     HK_CUDA(cudaGraphInstantiate(&loop_exec_, loop_graph_, 0));
 }
 
+void WfEngine::prepare_loop() {
+    if (loop_exec_) return;
+    if (loop_graph_) cudaGraphDestroy(loop_graph_);   // an earlier attempt failed half way
+    loop_graph_ = nullptr;
+    capture_loop();
+}
+
 void WfEngine::run_to_end() {
-    if (!loop_exec_) {
-        if (loop_graph_) cudaGraphDestroy(loop_graph_);   // an earlier attempt failed half way
-        loop_graph_ = nullptr;
-        capture_loop();
-    }
+    prepare_loop();
     HK_CUDA(cudaGraphLaunch(loop_exec_, stream_));
 }
 

@@ -73,6 +73,8 @@ public:
     // kWfMaxLoops pairs of them: one graph launch whose while node regen
     // steers, so the host neither polls nor overshoots.  Async.
     void run_to_end();
+    // Make run_to_end's graph now (its first use does otherwise).
+    void prepare_loop();
     // Copy the counters and the job table's finished counters to the host mirrors
     // and record done_event(); read them after the event completed.
     void fetch_status();

@@ -1441,7 +1441,7 @@ static bool work_for_wavefront(const hk_scene *s, const hk_render_desc &d) {
 // the stream is being captured into a graph, which cannot hold a loop, where
 // another device than the scene's is current (the megakernel runs there and
 // reads the scene as a peer), where the scene's stored configuration is one that
-// a pool refuses, or where there is no memory for the pool.
+// a pool refuses, or where there is no memory for the pool or the loop's graph.
 //
 // The loop of one graph launch ends after kWfMaxLoops passes, done or not, so the
 // graph is queued as often as the work could ask for: a path keeps its slot for
@@ -1476,6 +1476,7 @@ static bool render_wavefront_async(hk_scene *s, const hk_render_desc &d, float *
     hk::WfEngine *E;
     try {
         E = &wf_ensure(s, ec);
+        E->prepare_loop();
     } catch (const HkError &) {
         cudaGetLastError();
         return false;

@@ -243,3 +243,13 @@ def test_negative_sample_offsets_and_image_indices(fake):
     s = _scene(fake, 512, 512)
     _render(s, 1, sample_offset=-5, image_index=-2)
     assert [x for x in fake.log() if x.startswith("begin")] == ["begin slots 262144 sample -5 image -2"]
+
+
+def test_film_render_without_room_for_the_loops_graph(fake):
+    s = _scene(fake, 512, 512)
+    fake.L.fake_fail_instantiate(1)
+    _render(s, 1)
+    assert fake.forms() == ["mega"]
+    fake.L.fake_fail_instantiate(0)
+    _render(s, 1)
+    assert fake.forms() == ["begin"]
