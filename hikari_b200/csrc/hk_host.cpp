@@ -1475,6 +1475,7 @@ static bool render_wavefront_async(hk_scene *s, const hk_render_desc &d, float *
     if (!hk::WfEngine::fits(ec.capacity, s->dev.nemitters) || !hk::WfEngine::valid_threads(ec)) return false;
     hk::WfEngine *E;
     try {
+        hk::RelaxedCapture relaxed;
         E = &wf_ensure(s, ec);
         E->prepare_loop();
     } catch (const HkError &) {

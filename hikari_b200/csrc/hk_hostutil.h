@@ -49,6 +49,17 @@ int guarded(F &&f) {
     }
 }
 
+// While it lives, the calling thread may allocate, free and wait although
+// another thread, or this one on another stream, captures a stream in the
+// default (global) mode; otherwise such a call fails and breaks that capture.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    RelaxedCapture(const RelaxedCapture &) = delete;
+    RelaxedCapture &operator=(const RelaxedCapture &) = delete;
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 // Owning device allocation (cudaMalloc / cudaFree).
 struct DevBuf {
     void *p = nullptr;

@@ -68,3 +68,25 @@ def test_negative_sample_offsets_and_image_indices_in_both_forms():
         films.append(film.cpu().numpy().astype(np.float64))
     a, b = films
     assert np.allclose(a, b, rtol=1024 * 2.0 ** -24, atol=1e-6 * float(a.max()))
+
+
+def test_first_render_beside_a_capture():
+    """A stream is captured in the default mode while a scene renders for the first time on another stream, which makes
+    its pool: the capture stays whole, and so does the image (64 samples x 16 taps a pixel, 2^-24 each)."""
+    sd = scenes.cornell_box(width=256, height=256)
+    x = torch.zeros(1024, device="cuda")
+    films = [torch.zeros(hk.Scene.from_desc(sd).film_shape(), device="cuda") for _ in range(2)]
+    gs, ref = hk.Scene.from_desc(sd), hk.Scene.from_desc(sd)
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        x.add_(1)
+        gs.render(films[0], 2, 8, seed=3, stream=side)
+    assert _launches(gs) > 0   # the wavefront
+    g.replay()
+    torch.cuda.synchronize()
+    assert float(x.sum()) == 1024
+    ref.render(films[1], 2, 8, seed=3)
+    a, b = (f.cpu().numpy() for f in films)
+    assert np.allclose(a, b, rtol=1024 * 2.0 ** -24, atol=1e-6 * float(b.max()))

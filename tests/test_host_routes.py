@@ -253,3 +253,14 @@ def test_film_render_without_room_for_the_loops_graph(fake):
     fake.L.fake_fail_instantiate(0)
     _render(s, 1)
     assert fake.forms() == ["begin"]
+
+
+def test_pools_are_made_beside_a_capture(fake):
+    """A capture in the default mode forbids other threads, and its own thread on other streams, to allocate; hk_render
+    did not allocate before it had a pool, so its allocations must not break a capture."""
+    s = _scene(fake, 512, 512)
+    fake.L.fake_other_capture(1)
+    _render(s, 1)     # makes the pool and the loop's graph
+    _render(s, 16)    # replaces the pool by a larger one
+    assert fake.forms() == ["begin", "begin"]
+    assert not fake.L.fake_capture_broken()
