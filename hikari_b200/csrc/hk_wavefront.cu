@@ -268,17 +268,18 @@ __global__ void wf_init_kernel(WfState W, int slots, WfJob J) {
 }
 
 // Add the engine's statistics to a caller's 7-slot u64 array, or to a 5-slot one
-// with the traversal totals of both ray kinds (sum).
+// with the traversal totals of both ray kinds (sum).  Other renders may add to
+// the array meanwhile.
 __global__ void wf_counters_add_kernel(const WfCounters *c, unsigned long long *out, bool sum) {
     if (threadIdx.x != 0) return;
-    out[0] += c->rays;
-    out[1] += c->shadow_rays;
-    out[2] += c->dropped;
-    out[3] += c->node_visits + (sum ? c->node_visits_shadow : 0);
-    out[4] += c->tri_tests + (sum ? c->tri_tests_shadow : 0);
+    atomicAdd(out + 0, c->rays);
+    atomicAdd(out + 1, c->shadow_rays);
+    atomicAdd(out + 2, c->dropped);
+    atomicAdd(out + 3, c->node_visits + (sum ? c->node_visits_shadow : 0));
+    atomicAdd(out + 4, c->tri_tests + (sum ? c->tri_tests_shadow : 0));
     if (sum) return;
-    out[5] += c->node_visits_shadow;
-    out[6] += c->tri_tests_shadow;
+    atomicAdd(out + 5, c->node_visits_shadow);
+    atomicAdd(out + 6, c->tri_tests_shadow);
 }
 
 // ------------------------------------------------------------ launchers

@@ -90,3 +90,26 @@ def test_first_render_beside_a_capture():
     ref.render(films[1], 2, 8, seed=3)
     a, b = (f.cpu().numpy() for f in films)
     assert np.allclose(a, b, rtol=1024 * 2.0 ** -24, atol=1e-6 * float(b.max()))
+
+
+def test_counters_shared_by_renders_of_both_forms():
+    """Renders of two scenes on two streams add to one counter array: small ones in the megakernel, whose warps add as
+    they end, and large ones in the wavefront, which adds once per render.  Ray counts of a seed do not vary."""
+    small, large = (hk.Scene.from_desc(scenes.cornell_box(width=128, height=128)), hk.Scene.from_desc(
+        scenes.cornell_box(width=512, height=256)))
+    films = [torch.zeros(s.film_shape(), device="cuda") for s in (small, large)]
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    one = [torch.zeros(5, dtype=torch.int64, device="cuda") for _ in range(2)]
+    both = torch.zeros(5, dtype=torch.int64, device="cuda")
+    for s, f, c in zip((small, large), films, one):
+        s.render(f, 1, 8, seed=3, counters=c)
+    torch.cuda.synchronize()
+    n = (160, 40)
+    for k in range(40):
+        for j in range(4):
+            small.render(films[0], 1, 8, seed=3, counters=both, stream=streams[0])
+        large.render(films[1], 1, 8, seed=3, counters=both, stream=streams[1])
+    torch.cuda.synchronize()
+    assert _launches(large) > 0
+    want = n[0] * one[0].cpu().numpy() + n[1] * one[1].cpu().numpy()
+    assert tuple(both.cpu().numpy()[:3]) == tuple(want[:3])
