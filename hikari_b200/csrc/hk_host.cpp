@@ -1488,6 +1488,11 @@ static bool render_wavefront_async(hk_scene *s, const hk_render_desc &d, float *
         cudaEvent_t e;
         ~EvGuard() { cudaEventDestroy(e); }
     } guard{ev};
+    // the megakernel ran at the priority of the caller's stream
+    int least = 0, greatest = 0, own_prio = 0;
+    HK_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+    HK_CUDA(cudaStreamGetPriority(stream, &own_prio));
+    E->set_priority(own_prio < least);
     HK_CUDA(cudaEventRecord(ev, stream));
     HK_CUDA(cudaStreamWaitEvent(E->stream(), ev, 0));
     E->begin(J, (int)slots);
@@ -1725,6 +1730,7 @@ int hk_render_batch(hk_scene *s, const hk_render_job *jobs, int njobs, const hk_
         }
         const hk::WfEngineConfig ec = engine_config(c, total, s->dev.nemitters);
         hk::WfEngine &E = wf_ensure(s, ec);
+        E.set_priority(false);   // hk_render may have raised it
         cudaStream_t user = (cudaStream_t)stream, st = E.stream();
         // order after the caller's stream (the films may have been cleared there)
         cudaEvent_t ev;

@@ -68,13 +68,13 @@ def fake(fake_lib, monkeypatch):
     f.made = []
     f.log()
     yield f
-    for s in f.made:   # while the fake is the library
-        s.close()
     f.L.fake_limit(C.c_size_t(-1).value)
     f.L.fake_device(0)
     f.L.fake_other_capture(0)
     f.L.fake_user_capturing(0)
     f.L.fake_fail_instantiate(0)
+    for s in f.made:   # while the fake is the library
+        s.close()
 
 
 def _scene(fake, width=64, height=64, lights=1):
@@ -264,3 +264,23 @@ def test_pools_are_made_beside_a_capture(fake):
     _render(s, 16)    # replaces the pool by a larger one
     assert fake.forms() == ["begin", "begin"]
     assert not fake.L.fake_capture_broken()
+
+
+def _priorities(log):
+    return [x.split()[2] for x in log if x.startswith("loop")]
+
+
+def test_film_renders_keep_the_callers_priority(fake):
+    """The pool's streams have the least and the greatest priority; a batch runs at the least, as it always has."""
+    s = _scene(fake, 512, 512)
+    film = np.zeros(4, np.float32)
+    seen = []
+    for priority in (0, -1, -5, 0):
+        stream = fake.L.fake_stream(0, priority)
+        s.render(film, 1, 8, stream=stream)
+        seen += _priorities(fake.log())
+    s.render(film, 1, 8, stream=fake.L.fake_stream(0, -5))
+    fake.log()
+    s.render_batch([film], 1, 8, stream=fake.L.fake_stream(0, -5))
+    seen += _priorities(fake.log())
+    assert seen == ["0", "-5", "-5", "0", "0"]
