@@ -1813,9 +1813,16 @@ int hk_wavefront_autotune(hk_scene *s, const hk_render_desc *probe, hk_wavefront
         hk_render_job job;
         job.film_dev = film.as<float>();
         job.desc = *probe;
-        cudaEvent_t e0, e1;
-        HK_CUDA(cudaEventCreate(&e0));
-        HK_CUDA(cudaEventCreate(&e1));
+        struct Events {
+            cudaEvent_t a = nullptr, b = nullptr;
+            ~Events() {
+                if (a) cudaEventDestroy(a);
+                if (b) cudaEventDestroy(b);
+            }
+        } ev;
+        HK_CUDA(cudaEventCreate(&ev.a));
+        HK_CUDA(cudaEventCreate(&ev.b));
+        const cudaEvent_t e0 = ev.a, e1 = ev.b;
         float best_t = INFINITY;
         hk_wavefront_config bc{};
         const int caps[] = {1 << 20, 1 << 21, 1 << 22};
@@ -1844,7 +1851,14 @@ int hk_wavefront_autotune(hk_scene *s, const hk_render_desc *probe, hk_wavefront
         // coordinate descent: capacity, then block sizes
         hk_wavefront_config c{};
         c.threads_extend = 128; c.threads_shade = 128; c.iterations_per_check = 16;
+        // pools past the bound on shadow records are left out; where all are, the fitted one's size
+        if (!hk::WfEngine::fits(caps[0], s->dev.nemitters)) {
+            c.capacity = engine_config(bc, hk::make_wf_job(s, *probe).work_count, s->dev.nemitters).capacity;
+            best_t = run(c);
+            bc = c;
+        }
         for (int cap : caps) {
+            if (!hk::WfEngine::fits(cap, s->dev.nemitters)) break;
             c.capacity = cap;
             float ms = run(c);
             if (ms < best_t) { best_t = ms; bc = c; }
@@ -1905,8 +1919,6 @@ int hk_wavefront_autotune(hk_scene *s, const hk_render_desc *probe, hk_wavefront
             float ms = run(c);
             if (ms < best_t) { best_t = ms; bc = c; }
         }
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
         *best = bc;
         if (best_ms) *best_ms = best_t;
         s->wf_cfg = bc;   // hk_render_image renders its wavefront calls with it

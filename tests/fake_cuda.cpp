@@ -52,6 +52,10 @@ bool unsafe() {
 void finish(const hk::WfState &W) {
     W.ctr->next_work = W.ctr->total_work;
     W.ctr->active = 0;
+    for (unsigned k = 0; k < W.ctr->seg_count; ++k) {   // the plan's jobs
+        const hk::WfJob &J = W.jobs[W.segs[k].job];
+        *J.finished = J.work_count;
+    }
 }
 }  // namespace
 

@@ -10,7 +10,7 @@ import numpy as np
 import pytest
 
 import hikari_b200 as hk
-from hikari_b200 import build, scenes
+from hikari_b200 import build, scenes, serving
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 SOURCES = [os.path.join(build.CSRC, f) for f in build.SOURCES if f.endswith(".cpp")] + [os.path.join(HERE, "fake_cuda.cpp")]
@@ -284,3 +284,24 @@ def test_film_renders_keep_the_callers_priority(fake):
     s.render_batch([film], 1, 8, stream=fake.L.fake_stream(0, -5))
     seen += _priorities(fake.log())
     assert seen == ["0", "-5", "-5", "0", "0"]
+
+
+def _autotune(s):
+    d, best, ms = hk.render_desc(1, 8), hk.WavefrontConfig(), C.c_float()
+    hk.check(hk.lib().hk_wavefront_autotune(s.h, C.byref(d), C.byref(best), C.byref(ms)))
+    return best.capacity
+
+
+# lights x 2^22 slots: below 2^31, at it (2^21 fits), past it for every candidate (2^20 x 2048 = 2^31): the fitted pool
+@pytest.mark.parametrize("lights,capacities", [(511, [1 << 20, 1 << 21, 1 << 22]), (512, [1 << 20, 1 << 21]), (1024, [1 << 20]),
+                                               (2048, [1 << 16])])
+def test_the_autotuner_tries_the_pools_that_fit(fake, lights, capacities):
+    s = _scene(fake, 512, 512, lights)
+    assert _autotune(s) == capacities[0]   # the fake's clock finds none faster than the first
+    tried = []
+    for x in fake.log():
+        if x.startswith("loop"):
+            c = int(x.split()[-1])
+            if c not in tried:
+                tried.append(c)
+    assert tried == capacities
