@@ -222,7 +222,11 @@ void hk_server::admit(const std::vector<SceneEntry *> &sc) {
         Job *j = queued.front();
         SceneEntry &e = *sc[j->scene];
         const uint64_t need = j->size.film_bytes + j->size.rgb_bytes;
-        const uint64_t pool = e.eng ? 0 : hk::WfEngine::bytes_for(ec.capacity, e.view.dev->nemitters, e.view.dev->shade_queues);
+        // the server's pool size; less for a scene with so many emitters that
+        // the shadow records, one for every slot and emitter, would pass their bound
+        int capacity = ec.capacity;
+        while (capacity > 1024 && !hk::WfEngine::fits(capacity, e.view.dev->nemitters)) capacity = std::max(1024, capacity / 2);
+        const uint64_t pool = e.eng ? 0 : hk::WfEngine::bytes_for(capacity, e.view.dev->nemitters, e.view.dev->shade_queues);
         uint64_t used;
         {
             std::lock_guard<std::mutex> lk(mu);
@@ -230,9 +234,10 @@ void hk_server::admit(const std::vector<SceneEntry *> &sc) {
         }
         if ((int)e.jobs.size() >= cfg.max_jobs || used + need + pool > budget) break;   // arrival order: wait
         if (!e.eng) {
-            // the server's pool size and block sizes; the traversal knobs of
-            // the scene's own configuration where it has one (autotuned)
+            // the server's block sizes; the traversal knobs of the scene's own
+            // configuration where it has one (autotuned)
             hk::WfEngineConfig sec = ec;
+            sec.capacity = capacity;
             sec.serve = true;
             if (*e.view.has_cfg) {
                 const hk_wavefront_config &t = *e.view.cfg;
@@ -559,6 +564,8 @@ int hk_server_add_scene(hk_server *s, hk_scene *scene, int32_t *scene_id) {
         std::unique_ptr<SceneEntry> e(new SceneEntry());
         e->scene = scene;
         e->view = hk::scene_view(scene);
+        if (!hk::WfEngine::fits(1024, e->view.dev->nemitters))
+            throw HkError{HK_ERR_INVALID, "the scene has too many emitters for the least pool of 1024 slots"};
         std::lock_guard<std::mutex> lk(s->mu);
         s->scenes.push_back(std::move(e));
         if (scene_id) *scene_id = (int32_t)s->scenes.size() - 1;

@@ -305,3 +305,17 @@ def test_the_autotuner_tries_the_pools_that_fit(fake, lights, capacities):
             if c not in tried:
                 tried.append(c)
     assert tried == capacities
+
+
+@pytest.mark.parametrize("lights", [4095, 4096, 9000])
+def test_a_served_scene_of_many_lights(fake, lights):
+    """2^19 slots x 4096 lights are 2^31 shadow records: the scene gets a smaller pool, the server goes on."""
+    s = _scene(fake, 64, 64, lights)
+    srv = serving.Server()
+    try:
+        jid, out = srv.submit(srv.add_scene(s), 1, 8, 0)
+        srv.wait(jid, 60)
+    finally:
+        srv.close()
+    slots = {int(x.split()[-1]) for x in fake.log() if x.startswith("pair")}
+    assert slots == {1 << 19 if lights < 4096 else 1 << (18 if lights < 8192 else 17)}
