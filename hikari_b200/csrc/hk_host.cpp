@@ -1504,15 +1504,17 @@ static bool render_wavefront_async(hk_scene *s, const hk_render_desc &d, float *
 }
 // Blocks of a megakernel launch and the lanes of each warp that take paths.  A
 // warp takes as long as the longest of its lanes' walks and BSDFs at every
-// vertex, so few paths are spread over one warp per scheduler before a warp
-// takes more of them; further warps share the schedulers and the instruction
-// cache and cost more than they save (Cornell box, depth 16, paths packed in
-// full warps / one warp per scheduler / four: 256 paths 356 / 226 / 226 us,
-// 16384 paths 417 / 428 / 656 us).
+// vertex, so few paths are spread over one warp per scheduler; further warps
+// share the schedulers and the instruction cache and cost more than they save.
+// Above 16 paths a warp all 32 lanes take part: the fewer SMs then fetch less
+// code (us spread / in full warps: 3072 paths Cornell box 266 / 324, smooth
+// materials 459 / 495; 6912 paths 306 / 314 and 667 / 585; 12288 paths 331 / 324
+// and 811 / 719, a mesh 479 / 567; 16384 paths 349 / 331, 905 / 873 and 625 / 621).
 static int render_grid(const hk_scene *s, int spp, unsigned &lanes) {
     const uint64_t paths = (uint64_t)s->width * s->height * (uint64_t)spp, per_block = hk::kRenderThreads / 32;
     const uint64_t warps = (uint64_t)s->sm_count * 4;
     lanes = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(32, (paths + warps - 1) / warps));
+    if (lanes > 16) lanes = 32;
     const uint64_t blocks = (paths + lanes * per_block - 1) / (lanes * per_block);
     return (int)std::max<uint64_t>(1, std::min<uint64_t>(blocks, (uint64_t)s->sm_count * s->occupancy));
 }

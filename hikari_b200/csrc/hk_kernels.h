@@ -8,11 +8,16 @@ namespace hk {
 
 constexpr int kTile = 16;             // the megakernel numbers paths tile by tile: 16 x 16 pixels
 constexpr int kRenderThreads = 128;
-constexpr int kRenderBlocks = 4;      // resident blocks per SM that the megakernel's register budget allows
+// Resident blocks per SM that the megakernel's register budget allows: two, the
+// 198 registers that it asks for.  With 128 for four blocks it spills 480 B, and
+// more warps per scheduler only take turns in the instruction cache (us at 2 / 3 / 4
+// blocks: Cornell box 346 / 354 / 384 at 2^14 paths, 892 / 903 / 1067 at 2^17;
+// smooth materials 905 / 922 / 981 and 4025 / 4194 / 4583; a mesh 787 / 812 / 874 at 2^16).
+constexpr int kRenderBlocks = 2;
 
 struct RenderLaunch {
     float *film;                          // (H+2B) x (W+2B) x 4 floats, accumulated
-    unsigned long long *work_counter;     // paths dealt; zeroed before launch
+    unsigned long long *work_counter;     // paths dealt past the warps' first chunks; zeroed before launch
     unsigned long long *counters;         // [rays, shadow rays, dropped samples, node visits, triangle tests]
     uint64_t seed;
     int spp;                              // samples per pixel in this launch

@@ -14,16 +14,20 @@ struct PathCounters {
     TravStats trav;
 };
 
-// One path of a lane.
+// One path of a lane.  The BSDF record of a vertex stays here for the next one: where
+// that hits an area light, its MIS weight asks for the previous BSDF's pdf
+// of the sampled direction.  Taken at every vertex instead, the call cost 5 to 10% (Cornell
+// box 423 -> 403 us at 2^14 paths, smooth materials 1076 -> 986).
 struct Path {
     Pcg32 rng;
     Ray ray;          // the next ray to trace
     V3 L, beta;
     float px, py;     // film position
     float w_mats;     // MIS weight of an emitter hit, carried across vertices
-    float prev_pdf;   // the previous vertex's BSDF pdf of the sampled direction
     int depth;
     bool force_mats;  // the previous BSDF sample was EDiscrete
+    int bsdf;         // the last shaded vertex's BSDF, its record and (a bumpMap or normalMap) its frames
+    BRec rec;
 };
 
 // One vertex of PathMISIntegrator::Li (src/integrator/PathMISIntegrator.cpp:16-157):
@@ -36,8 +40,10 @@ struct Path {
 // test on throughput and NEE values.  kTex: the scene has textured materials
 // (texture lookups compiled in); the first hit's lookups filter with the
 // camera ray's differentials, later hits have none (src/core/Intersection.cpp:35).
+// bf: the frames of the last vertex whose BSDF is a bumpMap or normalMap (kTex only).
 template <int kAccel, bool kTex>
-__device__ __forceinline__ bool path_vertex(const DevScene &S, Path &P, int depth_max, int rr_start, PathCounters &pc) {
+__device__ __forceinline__ bool path_vertex(const DevScene &S, Path &P, BumpFrames &bf, int depth_max, int rr_start,
+                                            PathCounters &pc) {
     Hit h;
     pc.rays++;
     if (!trace<kAccel, false>(S, P.ray, h, pc.trav)) {
@@ -59,14 +65,18 @@ __device__ __forceinline__ bool path_vertex(const DevScene &S, Path &P, int dept
                 P.w_mats = 1.0f;
             } else {
                 const float plm = area_pdf(AL, er);
-                if (P.prev_pdf + plm != 0.0f) P.w_mats = P.prev_pdf / (P.prev_pdf + plm);
+                float pbm;
+                if constexpr (kTex) pbm = bsdf_pdf_b(S.bsdfs, P.bsdf, P.rec, bf);
+                else pbm = bsdf_pdf_n(S.bsdfs, P.bsdf, P.rec);
+                if (pbm + plm != 0.0f) P.w_mats = pbm / (pbm + plm);
             }
         }
         P.L = P.L + (P.beta * P.w_mats) * area_eval(AL, er);
     }
     float4 duv = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     float3 geo = make_float3(INFINITY, 0.0f, 0.0f);
-    BumpFrames bf;   // a bumpMap / normalMap vertex's frames (kTex only)
+    P.bsdf = bsdf;
+    BRec &br = P.rec;
     if constexpr (kTex) {
         if (P.depth == 0 && S.ray_diff) {
             V3 rx, ry;
@@ -76,7 +86,6 @@ __device__ __forceinline__ bool path_vertex(const DevScene &S, Path &P, int dept
         if (is_bump(S.bsdfs[bsdf])) bf = perturbed_frames(S, h, it, S.bsdfs[bsdf]);
         if (S.bsdfs[bsdf].geo_tex) geo = tex_geometry(S, h, it);
     }
-    BRec br;
     br.wi = to_local(it.sh, P.ray.d * -1.0f);
     br.eta = 0.0f;
     br.tu = it.u; br.tv = it.v; br.tex = kTex; br.duv = duv; br.geo = geo;
@@ -135,11 +144,7 @@ __device__ __forceinline__ bool path_vertex(const DevScene &S, Path &P, int dept
     }
     ++P.depth;
     if (P.depth >= depth_max) return false;   // the next hit would not be shaded
-    if (S.narea && !P.force_mats) {   // read where the next hit is an area light
-        br.eta = 0.0f;
-        if constexpr (kTex) P.prev_pdf = bsdf_pdf_b(S.bsdfs, bsdf, br, bf);
-        else P.prev_pdf = bsdf_pdf_n(S.bsdfs, bsdf, br);
-    }
+    br.eta = 0.0f;
     P.ray.o = it.p;
     P.ray.d = to_world(it.sh, br.wo);
     P.ray.tmin = kRayEps;
@@ -154,6 +159,15 @@ __device__ __forceinline__ bool path_vertex(const DevScene &S, Path &P, int dept
 // ran its samples one after another, a warp waited at each sample for its
 // longest path (roulette at p = 0.95: the longest of 32 has four times the
 // mean's vertices), and a block for its slowest tile item.
+//
+// Every warp starts with the chunk of its own number, so that the warps of an SM
+// shade neighbouring pixels and share the instruction cache, which bounds this
+// kernel (a warp runs the traversal and the BSDFs of its lanes one after another);
+// claimed in order of arrival, smooth materials took 2510 instead of 2414 us at 2^16 paths.
+// An ended path is splatted when its lane takes the next one, and where none is left all
+// of a warp's together: at each path's own end the filter's taps ran once for every
+// path length in the warp (Cornell box 378 -> 346 us at 2^14 paths, smooth
+// materials 983 -> 905).
 template <int kAccel, bool kTex>
 __global__ void __launch_bounds__(kRenderThreads, kRenderBlocks) render_pathmis_kernel(DevScene S, RenderLaunch P) {
     const unsigned lane = threadIdx.x & 31u;
@@ -161,9 +175,16 @@ __global__ void __launch_bounds__(kRenderThreads, kRenderBlocks) render_pathmis_
     PathCounters pc{0, 0, TravStats()};
     uint32_t dropped = 0;
     Path p;
+    BumpFrames bf;
     // few paths: fewer lanes of each warp take part, so that more warps do
-    bool have = false, exhausted = lane >= P.lanes;
-    uint64_t next = 0, end = 0;   // warp-uniform: undealt paths of the warp's chunk
+    bool have = false, ended = false, exhausted = lane >= P.lanes;
+    // warp-uniform: undealt paths of the warp's chunk; the paths of all warps' first chunks
+    uint64_t next = (blockIdx.x * (uint64_t)(blockDim.x / 32) + threadIdx.x / 32) * P.lanes, end = next + P.lanes;
+    const uint64_t first = gridDim.x * (uint64_t)(blockDim.x / 32) * P.lanes;
+    auto splat = [&] {
+        if (is_valid(p.L)) splat_film(S, P.film, (int)S.width, (int)S.height, p.px, p.py, p.L);
+        else ++dropped;   // ImageBlock::Put (src/core/Block.cpp:97)
+    };
     for (;;) {
         const unsigned want = __ballot_sync(0xffffffffu, !have && !exhausted);
         if (want) {
@@ -173,7 +194,7 @@ __global__ void __launch_bounds__(kRenderThreads, kRenderBlocks) render_pathmis_
             if (k > avail) {   // claim the next chunk for the lanes past the old one
                 unsigned long long base = 0;
                 if ((int)lane == __ffs(want) - 1) base = atomicAdd(P.work_counter, (unsigned long long)P.lanes);
-                base = __shfl_sync(0xffffffffu, base, __ffs(want) - 1);
+                base = __shfl_sync(0xffffffffu, base, __ffs(want) - 1) + first;
                 if (rank >= avail) i = base + (rank - avail);
                 next = base + (k - avail);
                 end = base + P.lanes;
@@ -182,6 +203,8 @@ __global__ void __launch_bounds__(kRenderThreads, kRenderBlocks) render_pathmis_
             }
             if (want >> lane & 1u) {
                 if (i < total) {
+                    if (ended) splat();
+                    ended = false;
                     // path -> sample, row of tiles, tile, pixel (tiles at the right and bottom edges are smaller)
                     const uint64_t s = i / pixels;
                     const uint32_t q = (uint32_t)(i - s * pixels);
@@ -198,7 +221,6 @@ __global__ void __launch_bounds__(kRenderThreads, kRenderBlocks) render_pathmis_
                     p.L = v3(0, 0, 0);
                     p.beta = v3(1, 1, 1);
                     p.w_mats = 1.0f;
-                    p.prev_pdf = 0.0f;
                     p.depth = 0;
                     p.force_mats = false;
                     have = true;
@@ -208,12 +230,12 @@ __global__ void __launch_bounds__(kRenderThreads, kRenderBlocks) render_pathmis_
             }
         }
         if (!__any_sync(0xffffffffu, have)) break;
-        if (have && !(P.depth > 0 && path_vertex<kAccel, kTex>(S, p, P.depth, P.rr_start, pc))) {
+        if (have && !(P.depth > 0 && path_vertex<kAccel, kTex>(S, p, bf, P.depth, P.rr_start, pc))) {
             have = false;
-            if (is_valid(p.L)) splat_film(S, P.film, (int)S.width, (int)S.height, p.px, p.py, p.L);
-            else ++dropped;   // ImageBlock::Put (src/core/Block.cpp:97)
+            ended = true;
         }
     }
+    if (ended) splat();
     // per-warp counter reduction (64-bit: node counts of one thread can pass 2^32)
     unsigned long long r = pc.rays, sh = pc.shadow, dr = dropped, nv = pc.trav.nodes, nt = pc.trav.tris;
     for (int o = 16; o > 0; o >>= 1) {

@@ -113,3 +113,22 @@ def test_counters_shared_by_renders_of_both_forms():
     assert _launches(large) > 0
     want = n[0] * one[0].cpu().numpy() + n[1] * one[1].cpu().numpy()
     assert tuple(both.cpu().numpy()[:3]) == tuple(want[:3])
+
+
+# one path; a lane of every warp and one more path; the last count that is spread and the first in full warps; all resident
+# lanes and more paths than they are, so that lanes take a second one; ragged tiles throughout
+@pytest.mark.parametrize("size,spp", [((1, 1), 1), ((592, 1), 1), ((593, 1), 1), ((128, 74), 1), ((9473, 1), 1), ((37, 29), 9),
+                                      ((592, 64), 1), ((641, 67), 1), ((211, 101), 4)])
+@pytest.mark.parametrize("scene", ["cornell_box", "cornell_smooth", "lights_scene"])
+def test_megakernel_deals_every_path_once(scene, size, spp):
+    """Against the wavefront: the same streams; the samples of 25 pixels, and the up to 64 terms of each, in any order."""
+    kw = dict(textured=True, bitmap=True, bump=True, shading_normals=True) if scene == "lights_scene" else {}
+    gs = hk.Scene.from_desc(getattr(scenes, scene)(width=size[0], height=size[1], **kw))
+    out = []
+    for form in (hk.FORM_MEGAKERNEL, hk.FORM_WAVEFRONT):
+        gs.set_image_form(form)
+        out.append(gs.render_image(spp, 12, seed=5))
+    (a, ca), (b, cb) = out
+    assert tuple(ca[:3]) == tuple(cb[:3])
+    terms = 25 * spp + 64
+    assert np.allclose(a, b, rtol=terms * 2.0 ** -23, atol=terms * 2.0 ** -24 * float(np.abs(a).max()))

@@ -319,3 +319,13 @@ def test_a_served_scene_of_many_lights(fake, lights):
         srv.close()
     slots = {int(x.split()[-1]) for x in fake.log() if x.startswith("pair")}
     assert slots == {1 << 19 if lights < 4096 else 1 << (18 if lights < 8192 else 17)}
+
+
+# 148 x 4 warps: a lane each, 16 each, then full warps; more warps than are resident wait for none: 148 x 2 blocks of 4
+@pytest.mark.parametrize("width,height,spp,lanes,grid", [(1, 1, 1, 1, 1), (592, 1, 1, 1, 148), (593, 1, 1, 2, 75), (592, 16, 1, 16, 148),
+                                                         (9473, 1, 1, 32, 75), (64, 64, 4, 32, 128), (592, 64, 1, 32, 296),
+                                                         (592, 128, 1, 32, 296)])
+def test_few_paths_are_spread_over_one_warp_per_scheduler(fake, width, height, spp, lanes, grid):
+    s = _scene(fake, width, height)
+    _render(s, spp)
+    assert fake.log() == [f"mega grid {grid} lanes {lanes}"]
