@@ -10,6 +10,12 @@ namespace hk {
 namespace {
 // bytes of an allocation's part
 constexpr size_t part(size_t n) { return (n + 255) & ~(size_t)255; }
+// the part of n bytes at p, which moves past it
+char *take(char *&p, size_t n) {
+    char *r = p;
+    p += part(n);
+    return r;
+}
 // queue arrays of one slot id per slot: 2 extend, 2 idle, the scene's shade queues, 1 finished
 int queue_arrays(uint64_t shade_queues) { return 5 + __builtin_popcountll(shade_queues); }
 }  // namespace
@@ -33,14 +39,9 @@ WfEngine::WfEngine(const DevScene &S, int sm_count, const WfEngineConfig &cfg) :
     W_.capacity = cfg_.capacity;
     W_.max_shadow = cfg_.capacity * std::max(1, S.nemitters);
     bytes_ = bytes_for(cfg_.capacity, S.nemitters, S.shade_queues);
-    // one device and one pinned host allocation, carved up (256-byte aligned parts)
+    // one device allocation, carved up (256-byte aligned parts)
     mem_.alloc(bytes_);
     char *at = mem_.as<char>();
-    auto take = [](char *&p, size_t n) {
-        char *r = p;
-        p += part(n);
-        return r;
-    };
     char *rec = take(at, N * kSlotBytes);   // slot records
     int *q = (int *)take(at, N * sizeof(int) * queue_arrays(S.shade_queues));
     float4 *sh = (float4 *)take(at, (size_t)W_.max_shadow * 16 * 3);
@@ -50,16 +51,6 @@ WfEngine::WfEngine(const DevScene &S, int sm_count, const WfEngineConfig &cfg) :
     segs_ = (WfSeg *)take(at, sizeof(WfSeg) * kWfMaxSegs);
     W_.jobs = jobs_;
     W_.segs = segs_;
-    const size_t host_bytes = 2 * part(sizeof(WfCounters)) + part(sizeof(unsigned long long) * kWfMaxJobs) +
-                              part(sizeof(WfJob) * kWfMaxJobs) + part(sizeof(WfSeg) * kWfMaxSegs);
-    host_.alloc(host_bytes);
-    std::memset(host_.p, 0, host_bytes);
-    at = host_.p;
-    h_ctr_ = (WfCounters *)take(at, sizeof(WfCounters));
-    h_head_ = (WfCounters *)take(at, sizeof(WfCounters));
-    h_fin_ = (unsigned long long *)take(at, sizeof(unsigned long long) * kWfMaxJobs);
-    h_jobs_ = (WfJob *)take(at, sizeof(WfJob) * kWfMaxJobs);
-    h_segs_ = (WfSeg *)take(at, sizeof(WfSeg) * kWfMaxSegs);
     W_.ray_o.p = (float4 *)(rec + 0);
     W_.ray_d.p = (float4 *)(rec + 16);
     W_.beta.p = (float4 *)(rec + 32);
@@ -125,7 +116,25 @@ WfEngine::WfEngine(const DevScene &S, int sm_count, const WfEngineConfig &cfg) :
     const int shadow_idle = cfg_.fetch_min_idle_shadow > 0 ? cfg_.fetch_min_idle_shadow : cfg_.fetch_min_idle;
     L_.fetch_min_idle_shadow = shadow_idle > 0 ? std::min(32, shadow_idle) : (w8 ? 8 : 1);
     HK_CUDA(cudaGetLastError());
-    reset();
+    if (cfg_.serve) reset();
+    else HK_CUDA(wf_launch_init(W_, W_.capacity, WfJob{}, stream_));   // begin or reset starts a render
+}
+
+// The host mirrors, in one pinned allocation made when a plan or a status first
+// needs them: it takes 2 ms, twice the rest of an engine, and a render that
+// starts with begin needs neither.
+void WfEngine::pin_host() {
+    if (host_.p) return;
+    const size_t bytes = 2 * part(sizeof(WfCounters)) + part(sizeof(unsigned long long) * kWfMaxJobs) +
+                         part(sizeof(WfJob) * kWfMaxJobs) + part(sizeof(WfSeg) * kWfMaxSegs);
+    host_.alloc(bytes);
+    std::memset(host_.p, 0, bytes);
+    char *at = host_.p;
+    h_ctr_ = (WfCounters *)take(at, sizeof(WfCounters));
+    h_head_ = (WfCounters *)take(at, sizeof(WfCounters));
+    h_fin_ = (unsigned long long *)take(at, sizeof(unsigned long long) * kWfMaxJobs);
+    h_jobs_ = (WfJob *)take(at, sizeof(WfJob) * kWfMaxJobs);
+    h_segs_ = (WfSeg *)take(at, sizeof(WfSeg) * kWfMaxSegs);
 }
 
 WfEngine::~WfEngine() {
@@ -168,6 +177,7 @@ void WfEngine::set_job(int slot, WfJob J) {
     if (slot < 0 || slot >= kWfMaxJobs) throw HkError{HK_ERR_INVALID, "job slot out of range"};
     // Each slot has its own staging entry; a slot is rewritten only after its
     // previous job ended, long after that job's copy ran.
+    pin_host();
     J.finished = finished_ + slot;
     job_count_ = std::max(job_count_, slot + 1);
     h_jobs_[slot] = J;
@@ -177,6 +187,7 @@ void WfEngine::set_job(int slot, WfJob J) {
 
 void WfEngine::set_plan(const std::vector<WfSeg> &segs, uint64_t total) {
     if (segs.size() > (size_t)kWfMaxSegs) throw HkError{HK_ERR_INVALID, "dispatch plan has too many pieces"};
+    pin_host();
     HK_CUDA(cudaEventSynchronize(ev_plan_));   // the staging copies of the previous plan have run
     if (!segs.empty()) {
         std::memcpy(h_segs_, segs.data(), sizeof(WfSeg) * segs.size());
@@ -270,6 +281,7 @@ void WfEngine::run(int iterations, bool use_graph, float *kernel_ms, int32_t *ke
 }
 
 void WfEngine::fetch_status() {
+    pin_host();
     HK_CUDA(cudaMemcpyAsync(h_ctr_, W_.ctr, offsetof(WfCounters, log_n), cudaMemcpyDeviceToHost, stream_));
     HK_CUDA(cudaMemcpyAsync(h_fin_, finished_, sizeof(unsigned long long) * kWfMaxJobs, cudaMemcpyDeviceToHost,
                             stream_));

@@ -92,6 +92,7 @@ public:
 
 private:
     void capture();
+    void pin_host();
     void capture_loop();
     DevScene S_;
     WfEngineConfig cfg_;
@@ -101,7 +102,7 @@ private:
     int device_ = 0;
     int job_count_ = 0;   // highest job slot ever set + 1
     DevBuf mem_;             // slot records, queues, shadow queue, counters, job table, plan
-    PinnedBuf<char> host_;   // the host mirrors below
+    PinnedBuf<char> host_;   // the host mirrors below, on first use
     WfCounters *h_ctr_ = nullptr, *h_head_ = nullptr;
     unsigned long long *h_fin_ = nullptr;
     WfJob *h_jobs_ = nullptr;

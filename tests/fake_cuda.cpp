@@ -31,7 +31,7 @@ struct Fake {
     bool in_capture = false;                      // the library's own
     hk::WfState W{};                              // of the last captured iteration
     uint64_t passes_left = 0;                     // passes that the render begun last needs in the worst case
-    int fail_instantiate = 0;
+    int fail_instantiate = 0, pinned = 0;
     std::string log;
 } g;
 thread_local cudaStreamCaptureMode t_mode = cudaStreamCaptureModeGlobal;
@@ -71,6 +71,7 @@ void fake_other_capture(int on) { g.other_capture = on != 0; g.broken = false; }
 int fake_capture_broken() { return g.broken; }
 void fake_user_capturing(int on) { g.capturing_user = on; }
 void fake_fail_instantiate(int on) { g.fail_instantiate = on; }
+int fake_pinned() { return g.pinned; }
 uint64_t fake_passes_left() { return g.passes_left; }
 void *fake_stream(int device, int priority) { return new Stream{device, priority}; }
 
@@ -110,6 +111,7 @@ cudaError_t cudaFreeAsync(void *p, cudaStream_t) { return cudaFree(p); }
 cudaError_t cudaMallocHost(void **p, size_t n) {
     if (unsafe()) return fail(cudaErrorStreamCaptureUnsupported);
     *p = calloc(1, n);
+    ++g.pinned;
     return cudaSuccess;
 }
 cudaError_t cudaFreeHost(void *p) { free(p); return cudaSuccess; }

@@ -329,3 +329,16 @@ def test_few_paths_are_spread_over_one_warp_per_scheduler(fake, width, height, s
     s = _scene(fake, width, height)
     _render(s, spp)
     assert fake.log() == [f"mega grid {grid} lanes {lanes}"]
+
+
+def test_a_film_render_pins_no_host_memory(fake):
+    """Its job and plan go to the device with a launch: pinned memory, most of what a pool costs to make, is the batch's."""
+    s = _scene(fake, 512, 512)
+    before = fake.L.fake_pinned()
+    _render(s, 1)
+    assert fake.forms() == ["begin"] and fake.L.fake_pinned() == before
+    _pool(s, fake)
+    assert fake.L.fake_pinned() == before + 1
+    _render(s, 1)
+    _pool(s, fake)
+    assert fake.L.fake_pinned() == before + 1
