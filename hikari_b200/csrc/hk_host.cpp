@@ -1074,7 +1074,8 @@ JobSize job_size(const hk_scene *s, const hk_render_desc &d) {
     JobSize z;
     z.width = d.width > 0 ? (uint32_t)d.width : s->width;
     z.height = d.height > 0 ? (uint32_t)d.height : s->height;
-    if (z.width > 16384 || z.height > 16384) throw HkError{HK_ERR_INVALID, "image larger than 16384 x 16384"};
+    if (z.width > kJobMaxSide || z.height > kJobMaxSide)
+        throw HkError{HK_ERR_INVALID, "image larger than " + std::to_string(kJobMaxSide) + " x " + std::to_string(kJobMaxSide)};
     const size_t FW = z.width + 2 * (size_t)s->dev.border, FH = z.height + 2 * (size_t)s->dev.border;
     z.film_bytes = FW * FH * 4 * sizeof(float);
     z.rgb_bytes = (size_t)z.width * z.height * 3 * sizeof(float);
@@ -1435,13 +1436,16 @@ static bool work_for_wavefront(const hk_scene *s, const hk_render_desc &d) {
     if (s->image_form == HK_FORM_MEGAKERNEL || d.depth < 1 || d.depth > 65535) return false;
     return (uint64_t)s->width * s->height * (uint64_t)d.spp >= (1ull << 17);
 }
+// Whether the scene's own image may be a job of the wavefront.
+static bool job_sides_fit(const hk_scene *s) { return s->width <= hk::kJobMaxSide && s->height <= hk::kJobMaxSide; }
 // hk_render through the wavefront, asynchronous on `stream` like the
 // megakernel: one launch that sets the pool, job and plan up, one graph whose
 // loop ends by itself, one for the counters.  False (nothing launched) where
 // the stream is being captured into a graph, which cannot hold a loop, where
 // another device than the scene's is current (the megakernel runs there and
-// reads the scene as a peer), where the scene's stored configuration is one that
-// a pool refuses, or where there is no memory for the pool or the loop's graph.
+// reads the scene as a peer), where the image has more pixels a side than a job
+// may, where the scene's stored configuration is one that a pool refuses, or
+// where there is no memory for the pool or the loop's graph.
 //
 // The loop of one graph launch ends after kWfMaxLoops passes, done or not, so the
 // graph is queued as often as the work could ask for: a path keeps its slot for
@@ -1451,7 +1455,7 @@ static bool work_for_wavefront(const hk_scene *s, const hk_render_desc &d) {
 static bool render_wavefront_async(hk_scene *s, const hk_render_desc &d, float *film, unsigned long long *counters,
                                    cudaStream_t stream) {
     const hk_wavefront_config c = s->has_wf_cfg ? s->wf_cfg : hk_wavefront_config{};
-    if (c.no_graph) return false;
+    if (c.no_graph || !job_sides_fit(s)) return false;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
         cudaGetLastError();
@@ -1583,16 +1587,17 @@ int hk_render_image(hk_scene *s, const hk_render_desc *d, float *rgb_host, unsig
         // ones that hk_render, which returns at once, leaves to the megakernel
         // though the batch, which waits, renders them with the wavefront: without
         // a graph, and on another device than the scene's.  A stored
-        // configuration that a pool refuses leaves hk_render with the megakernel;
-        // here large images have always been refused then, and the batch does that
+        // configuration that a pool refuses and an image of too many pixels a side
+        // leave hk_render with the megakernel; here large images have always been
+        // refused then, and the batch does that
         const hk_wavefront_config c = s->has_wf_cfg ? s->wf_cfg : hk_wavefront_config{};
         const uint64_t px = (uint64_t)s->width * s->height;
         const hk::WfEngineConfig ec = engine_config(c, px * (uint64_t)d->spp, s->dev.nemitters);
         const bool valid = hk::WfEngine::valid_threads(ec);
-        const bool refused = px >= 65536 && px * (uint64_t)d->spp >= (1ull << 22) && !valid;
+        const bool refused = px >= 65536 && px * (uint64_t)d->spp >= (1ull << 22) && (!valid || !job_sides_fit(s));
         int dev = 0;
         HK_CUDA(cudaGetDevice(&dev));
-        const bool waits = work_for_wavefront(s, *d) && (c.no_graph || dev != s->device) && valid &&
+        const bool waits = work_for_wavefront(s, *d) && (c.no_graph || dev != s->device) && valid && job_sides_fit(s) &&
                            hk::WfEngine::fits(ec.capacity, s->dev.nemitters);
         bool wave = s->image_form == HK_FORM_WAVEFRONT || (s->image_form == HK_FORM_AUTO && (refused || waits));
         int rc = HK_OK;

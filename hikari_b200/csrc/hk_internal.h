@@ -21,6 +21,8 @@ struct SceneView {
 // Throws HkError when the scene is null or not built.
 SceneView scene_view(hk_scene *s);
 
+constexpr uint32_t kJobMaxSide = 16384;   // pixels a side of an image that the wavefront renders
+
 // Image size of a render request and the device bytes of its film and RGB image.
 struct JobSize {
     uint32_t width, height;

@@ -238,6 +238,25 @@ def test_whole_images_on_another_device(fake):
     assert fake.forms() == ["mega"]
 
 
+# 2^17 paths and more; 2^22 and more of 65536 pixels and more are refused, as they have always been
+@pytest.mark.parametrize("width,height", [(16385, 8), (8, 16385)])
+@pytest.mark.parametrize("no_graph", [0, 1])
+def test_images_of_more_pixels_a_side_than_a_job_may_have(fake, width, height, no_graph):
+    s = _scene(fake, width, height)
+    if no_graph:
+        _store(s, no_graph=1)
+    _render(s, 1)
+    _image(s, 31)   # below 2^22 paths
+    assert fake.forms() == ["mega", "mega"]
+    with pytest.raises(hk.HikariError):
+        _image(s, 32)
+    _render(s, 32)
+    assert fake.forms() == ["mega"]
+    s = _scene(fake, width - 1 if width > height else width, height - 1 if height > width else height)
+    _render(s, 1)
+    assert fake.forms() == ["begin"]
+
+
 def test_negative_sample_offsets_and_image_indices(fake):
     """hk_render takes both as signed numbers of 64 bits, in either form."""
     s = _scene(fake, 512, 512)
