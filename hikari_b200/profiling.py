@@ -6,7 +6,7 @@ usage: python -m hikari_b200.profiling launches <launches.csv>
        python -m hikari_b200.profiling raw <report.ncu-rep> [regex]
        python -m hikari_b200.profiling render [--workload heterogeneous|textured] [--views V] [--spp S] [--accel bvh2|bvh8] [--out F]
                                               [--threads-extend T] [--threads-shade T] [--fetch-steps K]
-                                              [--fetch-min-idle K] [--shadow-tests M] [--closest-tests M]
+                                              [--fetch-min-idle K]
        python -m hikari_b200.profiling traffic <metrics.csv> <render.json> [skip]
 
 `render` renders the heterogeneous scene once with the wavefront integrator
@@ -159,8 +159,8 @@ def render(argv):
     ap.add_argument("--fetch-steps-shadow", type=int, default=0)
     ap.add_argument("--fetch-min-idle-shadow", type=int, default=0)
     ap.add_argument("--reg-lean", type=int, default=0)
-    ap.add_argument("--shadow-tests", type=int, default=0)
-    ap.add_argument("--closest-tests", type=int, default=0)
+    for name in ("--shadow-tests", "--closest-tests"):   # of earlier kernels: every value runs the one form
+        ap.add_argument(name, type=int, default=0, help=argparse.SUPPRESS)
     ap.add_argument("--sample-major", type=int, default=0)
     ap.add_argument("--config-json", default=None,
                     help="a JSON file with a wavefront configuration (bench.py's config.wavefront); its keys set "
@@ -185,8 +185,7 @@ def render(argv):
                     threads_extend=a.threads_extend, threads_shade=a.threads_shade, fetch_steps=a.fetch_steps,
                     fetch_min_idle=a.fetch_min_idle, iterations_per_check=a.iterations_per_check,
                     fetch_steps_shadow=a.fetch_steps_shadow, fetch_min_idle_shadow=a.fetch_min_idle_shadow,
-                    reg_lean=a.reg_lean, shadow_tests=a.shadow_tests, closest_tests=a.closest_tests,
-                    sample_major=a.sample_major,
+                    reg_lean=a.reg_lean, sample_major=a.sample_major,
                     no_graph=True)   # plain launches: ncu does not list the kernels of a graph's loop
     torch.cuda.synchronize()
     c = [int(x) for x in ctr.cpu().tolist()]
@@ -195,8 +194,7 @@ def render(argv):
            "launch": {"capacity": a.capacity, "threads_extend": a.threads_extend, "threads_shade": a.threads_shade,
                       "fetch_steps": a.fetch_steps, "fetch_min_idle": a.fetch_min_idle,
                       "fetch_steps_shadow": a.fetch_steps_shadow, "fetch_min_idle_shadow": a.fetch_min_idle_shadow,
-                      "reg_lean": a.reg_lean, "shadow_tests": a.shadow_tests, "closest_tests": a.closest_tests,
-                      "sample_major": a.sample_major},
+                      "reg_lean": a.reg_lean, "sample_major": a.sample_major},
            "counters": dict(zip(names, c)),
            # rays of each traversal launch, in launch order (ncu -k <kernel> -s i -c k captures launches i..i+k-1)
            "launch_rays": {"extend": [int(x) for x in gs.wavefront_launch_log(0)],
