@@ -7,14 +7,16 @@
 // the triangles that the visits hit are appended to a 128-entry ring in shared
 // memory as (triangle, owner lane), and a batch of 32 is tested, one triangle
 // per lane, whenever 32 are pending.  The kernels are bound by instruction
-// issue (77% of the slots) and by the ALU pipe (68%: the node test's byte
-// permutes, min / max and compares run there at half rate), not by DRAM (7%),
-// so what counts is warp instructions per ray.  A lane that tests its own
+// issue (76-80% of the slots) with the ALU pipe beside it (60-63%: the node
+// test's byte permutes, min / max and compares run there at half rate), not by
+// DRAM (under 15%), so what counts is warp instructions per ray.  A lane that tests its own
 // triangles keeps the warp for as many rounds as the largest leaf group with
 // the other lanes idle (13 active lanes per instruction); testing each step's
 // triangles at once, shared out over the lanes, fills half of a round (14
 // triangles on average) and pays for numbering triangles and finding owners in
-// every round.  1024^2 x 32 spp, ns per ray, own / shared out at once / ring:
+// every round.  1024^2 x 32 spp, ns per ray when the ring was brought in, before
+// the steps whose figures stand below (now 0.222 and 0.244 ns on the 64-sphere
+// scene, 128 spp), own / shared out at once / ring:
 // 64-sphere scene (1.3M triangles) shadow 0.319 / 0.280 / 0.245, closest hit
 // 0.466 / 0.413 / 0.266; glass sphere (0.33M) shadow 0.485 / 0.391 / 0.324,
 // closest hit 0.549 / 0.473 / 0.307; Cornell box (36 triangles, two visits a

@@ -21,8 +21,9 @@
 // The estimator is the reference's: the next-event MIS weight of an
 // unoccluded emitter is its own pl / (pl + pb) (the reference updates its
 // carried weight exactly when the shadow ray is unoccluded, and uses it right
-// away); the emitter-hit weight is computed from the previous vertex's BSDF
-// record and forced to 1 after an EDiscrete sample; Russian roulette runs
+// away); the emitter-hit weight is computed from the pdf that the previous
+// vertex's BSDF had for the direction it sampled, taken there and kept in the
+// path's record, and forced to 1 after an EDiscrete sample; Russian roulette runs
 // before the continuation ray is traced (the reference traces first and
 // discards the hit of a terminated path, which changes nothing).
 #include "hk_wf_kernels.cuh"

@@ -1,7 +1,7 @@
 // Wavefront pathMIS: device-side structures shared by hk_wavefront.cu and the
 // host driver in hk_host.cpp.
 //
-// A pool of `capacity` path slots lives in HBM as structure-of-arrays.  One
+// A pool of `capacity` path slots lives in HBM, one 128-byte record per slot.  One
 // iteration runs: regen (splat finished paths, claim new work for finished and
 // idle slots, generate camera rays) -> extend (closest hit of every queued ray,
 // classify by material) -> shade<material> (emission, MIS, next-event shadow

@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) wf_shade_kernel(DevScene S, W
         } else {
             // queue -> top-level BSDF type (run-time dispatch for the generic
             // queue) and whether texture lookups are compiled in
-            // kBumpQ: a bumpMap / normalMap over the rough type BT (the
+            // kBumpQ: a bumpMap / normalMap over the type BT (the
             // records move through the perturbed frame, the nested BSDF is
             // evaluated with its type compiled in)
             constexpr bool kBumpQ = kType >= kWfBumpQueue0 && kType != kWfGenericQueue;
@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) wf_shade_kernel(DevScene S, W
             // screen-space partials of a camera ray's first hit (textured
             // materials only: Intersection::ComputeScreenSpacePartial)
             float4 duv = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            BumpFrames bf;   // a bumpMap / normalMap vertex's frames (the generic queue only)
+            BumpFrames bf;   // a bumpMap / normalMap vertex's frames (the bump queues and the generic one)
             if constexpr (BT < 0) {
                 if (is_bump(S.bsdfs[bsdf])) bf = perturbed_frames(S, h, it, S.bsdfs[bsdf]);
             } else if constexpr (kBumpQ) {
