@@ -257,6 +257,7 @@ struct hk_scene {
     double tree_build_s = 0.0;                 // seconds of the last tree build
     bool has_wf_cfg = false;                   // wf_cfg was set (autotuner or caller)
     hk_wavefront_config wf_cfg{};              // wavefront configuration of hk_render_image
+    bool short_paths = false; // most paths leave the scene after a few vertices
     int occupancy = 1;        // resident megakernel CTAs per SM for the traversed tree
     int occupancy_of[2] = {1, 1};
     // wavefront engines, allocated on first use: of the pool size that a caller
@@ -987,6 +988,11 @@ void build_scene(hk_scene *s) {
     HK_CUDA(cudaGetDevice(&dev));
     s->device = dev;
     HK_CUDA(cudaDeviceGetAttribute(&s->sm_count, cudaDevAttrMultiProcessorCount, dev));
+    // under a sky and without transmission; with textures anyhow
+    const bool transmits = std::any_of(bs.begin(), bs.end(), [](const hk::DevBsdf &b) {
+        return b.type == hk::kDielectric || b.type == hk::kRoughDielectric;
+    });
+    s->short_paths = D.env_index >= 0 && (D.textured || !transmits);
     for (int a = 0; a < 2; ++a) s->occupancy_of[a] = std::max(1, hk::render_occupancy(a, D.textured != 0));
     s->occupancy = s->occupancy_of[D.accel];
     HK_CUDA(cudaGetLastError());
@@ -1514,13 +1520,26 @@ static bool render_wavefront_async(hk_scene *s, const hk_render_desc &d, float *
 // code (us spread / in full warps: 3072 paths Cornell box 266 / 324, smooth
 // materials 459 / 495; 6912 paths 306 / 314 and 667 / 585; 12288 paths 331 / 324
 // and 811 / 719, a mesh 479 / 567; 16384 paths 349 / 331, 905 / 873 and 625 / 621).
-static int render_grid(const hk_scene *s, int spp, unsigned &lanes) {
-    const uint64_t paths = (uint64_t)s->width * s->height * (uint64_t)spp, per_block = hk::kRenderThreads / 32;
-    const uint64_t warps = (uint64_t)s->sm_count * 4;
-    lanes = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(32, (paths + warps - 1) / warps));
-    if (lanes > 16) lanes = 32;
-    const uint64_t blocks = (paths + lanes * per_block - 1) / (lanes * per_block);
-    return (int)std::max<uint64_t>(1, std::min<uint64_t>(blocks, (uint64_t)s->sm_count * s->occupancy));
+//
+// Paths in rounds (hk_megakernel.cuh) once they are more than the resident
+// lanes: up to depth 6, and in scenes of short paths at any depth.  Lanes that
+// take paths as they become free / blocks of 128 threads in rounds / of 256, us: depth 2, 2^18 paths, Cornell
+// box 425 / 277 / 273, smooth materials 1945 / 817 / 603, 64 spheres 5972 /
+// 4447 / 4168; depth 6 945 / 1021 / 980, 5406 / 4793 / 4327 and 10190 / 9978 /
+// 9770; depth 8 1082 / 1377 / 1328, 6106 / 6240 / 5760; depth 16 1387 / 2552 /
+// 2486.  Scenes under a sky, depth 16, 2^18 paths: mesh of a conductor 1814 / 1440 / 1410, of
+// plastic 2369 / 1907 / 1857, textures 2639 / 1633 / 1385 (with glass: its code
+// is the largest); not where transmission makes paths longer: mesh of glass 3411 / 4595 / 4671.
+// 256 threads from 2^17 paths on, where they fill the SMs (2^16 paths, textures 857 / 1169 in rounds of 128 / 256).
+static int render_grid(const hk_scene *s, const hk_render_desc &d, hk::RenderLaunch &P) {
+    const uint64_t paths = (uint64_t)s->width * s->height * (uint64_t)d.spp;
+    const uint64_t warps = (uint64_t)s->sm_count * 4, resident = (uint64_t)s->sm_count * s->occupancy * hk::kRenderThreads;
+    P.lanes = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(32, (paths + warps - 1) / warps));
+    if (P.lanes > 16) P.lanes = 32;
+    P.rounds = paths > resident && (d.depth <= 6 || s->short_paths);
+    P.threads = P.rounds && paths >= (1u << 17) ? hk::kRoundThreads : hk::kRenderThreads;
+    const uint64_t per_block = P.lanes * (P.threads / 32);
+    return (int)std::max<uint64_t>(1, std::min<uint64_t>((paths + per_block - 1) / per_block, std::max<uint64_t>(1, resident / P.threads)));
 }
 int hk_render(hk_scene *s, const hk_render_desc *d, float *film, unsigned long long *counters, void *stream) {
     return guarded([&] {
@@ -1543,7 +1562,7 @@ int hk_render(hk_scene *s, const hk_render_desc *d, float *film, unsigned long l
         P.rr_start = d->rr_start;
         P.image_index = d->image_index;
         HK_CUDA(cudaMemsetAsync(s->b_scratch.p, 0, sizeof(unsigned long long), st));
-        const int grid = render_grid(s, P.spp, P.lanes);
+        const int grid = render_grid(s, *d, P);
         if (d->use_camera) {
             hk::DevScene D = s->dev;   // per-call camera pose (passed by value with the launch)
             const float *M = d->camera_to_world;
@@ -1700,7 +1719,7 @@ int hk_render_image_static(hk_scene *s, const hk_render_desc *d, float *rgb_dev,
         P.depth = d->depth;
         P.rr_start = d->rr_start;
         P.image_index = d->image_index;
-        const int grid = render_grid(s, P.spp, P.lanes);
+        const int grid = render_grid(s, *d, P);
         hk::DevScene D = s->dev;
         if (d->use_camera) {
             const float *M = d->camera_to_world;

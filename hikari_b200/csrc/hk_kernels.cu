@@ -180,10 +180,14 @@ static int grid_for(uint64_t n, int threads) {
     return (int)(g < 1 ? 1 : g);
 }
 
+template <int kAccel, bool kTex>
+static cudaError_t launch_render_form(const DevScene &S, const RenderLaunch &P, int grid, cudaStream_t st) {
+    return P.rounds ? launch_render_t<kAccel, kTex, true>(S, P, grid, st) : launch_render_t<kAccel, kTex, false>(S, P, grid, st);
+}
 cudaError_t launch_render(const DevScene &S, const RenderLaunch &P, int grid, cudaStream_t st) {
     if (S.accel == kAccelBvh8)
-        return S.textured ? launch_render_t<kAccelBvh8, true>(S, P, grid, st) : launch_render_t<kAccelBvh8, false>(S, P, grid, st);
-    return S.textured ? launch_render_t<kAccelBvh2, true>(S, P, grid, st) : launch_render_t<kAccelBvh2, false>(S, P, grid, st);
+        return S.textured ? launch_render_form<kAccelBvh8, true>(S, P, grid, st) : launch_render_form<kAccelBvh8, false>(S, P, grid, st);
+    return S.textured ? launch_render_form<kAccelBvh2, true>(S, P, grid, st) : launch_render_form<kAccelBvh2, false>(S, P, grid, st);
 }
 cudaError_t launch_resolve(const float *film, float *rgb, int W, int H, int B, cudaStream_t st) {
     int n = W * H;

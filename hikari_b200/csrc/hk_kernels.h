@@ -14,6 +14,7 @@ constexpr int kRenderThreads = 128;
 // blocks: Cornell box 346 / 354 / 384 at 2^14 paths, 892 / 903 / 1067 at 2^17;
 // smooth materials 905 / 922 / 981 and 4025 / 4194 / 4583; a mesh 787 / 812 / 874 at 2^16).
 constexpr int kRenderBlocks = 2;
+constexpr int kRoundThreads = 256;    // the most threads of a block that deals its paths in rounds
 
 struct RenderLaunch {
     float *film;                          // (H+2B) x (W+2B) x 4 floats, accumulated
@@ -25,6 +26,8 @@ struct RenderLaunch {
     int depth, rr_start;
     int image_index;
     unsigned lanes;                       // lanes of each warp that take paths (1 to 32)
+    unsigned threads;                     // of a block
+    bool rounds;                          // a block's paths start together
 };
 
 // Static scratch of hk_render_image_static: a 256-byte header ([0] work
@@ -55,7 +58,7 @@ int render_occupancy(int accel, bool textured);
 
 // Per-instantiation launchers behind the functions above, each compiled in its
 // own translation unit (megakernel: hk_render_*.cu; BSDF batch: hk_batch_*.cu).
-template <int kAccel, bool kTex>
+template <int kAccel, bool kTex, bool kRounds>
 cudaError_t launch_render_t(const DevScene &S, const RenderLaunch &P, int grid, cudaStream_t st);
 template <int kAccel, bool kTex>
 int render_occupancy_t();

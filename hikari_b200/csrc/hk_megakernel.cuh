@@ -160,6 +160,13 @@ __device__ __forceinline__ bool path_vertex(const DevScene &S, Path &P, BumpFram
 // longest path (roulette at p = 0.95: the longest of 32 has four times the
 // mean's vertices), and a block for its slowest tile item.
 //
+// kRounds: the paths of a block start together.  A warp takes 32 new paths when its last
+// one has ended, after a barrier of its block.  Where all paths are short there is
+// little to wait for, and what a lane gains by going on alone it loses many times over: its warp's lanes are
+// at different vertices, on different materials, and the SM's warps, at
+// different places of a kernel that its instruction cache does not hold, fetch
+// each other's code away.  Which kernel: render_grid (hk_host.cpp).
+//
 // Every warp starts with the chunk of its own number, so that the warps of an SM
 // shade neighbouring pixels and share the instruction cache, which bounds this
 // kernel (a warp runs the traversal and the BSDFs of its lanes one after another);
@@ -168,8 +175,9 @@ __device__ __forceinline__ bool path_vertex(const DevScene &S, Path &P, BumpFram
 // of a warp's together: at each path's own end the filter's taps ran once for every
 // path length in the warp (Cornell box 378 -> 346 us at 2^14 paths, smooth
 // materials 983 -> 905).
-template <int kAccel, bool kTex>
-__global__ void __launch_bounds__(kRenderThreads, kRenderBlocks) render_pathmis_kernel(DevScene S, RenderLaunch P) {
+template <int kAccel, bool kTex, bool kRounds>
+__global__ void __launch_bounds__(kRounds ? kRoundThreads : kRenderThreads, kRounds ? 1 : kRenderBlocks)
+    render_pathmis_kernel(DevScene S, RenderLaunch P) {
     const unsigned lane = threadIdx.x & 31u;
     const uint64_t pixels = (uint64_t)S.width * S.height, total = pixels * (uint64_t)P.spp;
     PathCounters pc{0, 0, TravStats()};
@@ -186,8 +194,12 @@ __global__ void __launch_bounds__(kRenderThreads, kRenderBlocks) render_pathmis_
         else ++dropped;   // ImageBlock::Put (src/core/Block.cpp:97)
     };
     for (;;) {
-        const unsigned want = __ballot_sync(0xffffffffu, !have && !exhausted);
+        unsigned want = __ballot_sync(0xffffffffu, !have && !exhausted);
+        if constexpr (kRounds)
+            if (__any_sync(0xffffffffu, have)) want = 0u;
         if (want) {
+            // warps that find no path leave, and the barrier with them
+            if constexpr (kRounds) __syncthreads();
             const unsigned k = __popc(want), rank = __popc(want & ((1u << lane) - 1u));
             const unsigned avail = (unsigned)(end - next);
             uint64_t i = next + rank;
@@ -254,15 +266,15 @@ __global__ void __launch_bounds__(kRenderThreads, kRenderBlocks) render_pathmis_
     }
 }
 
-template <int kAccel, bool kTex>
+template <int kAccel, bool kTex, bool kRounds>
 cudaError_t launch_render_t(const DevScene &S, const RenderLaunch &P, int grid, cudaStream_t st) {
-    render_pathmis_kernel<kAccel, kTex><<<grid, kRenderThreads, 0, st>>>(S, P);
+    render_pathmis_kernel<kAccel, kTex, kRounds><<<grid, P.threads, 0, st>>>(S, P);
     return cudaGetLastError();
 }
 template <int kAccel, bool kTex>
 int render_occupancy_t() {
     int n = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, render_pathmis_kernel<kAccel, kTex>, kRenderThreads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, render_pathmis_kernel<kAccel, kTex, false>, kRenderThreads, 0);
     return n;
 }
 

@@ -2,6 +2,6 @@
 #include "hk_megakernel.cuh"
 
 namespace hk {
-template cudaError_t launch_render_t<kAccelBvh8, false>(const DevScene &, const RenderLaunch &, int, cudaStream_t);
+template cudaError_t launch_render_t<kAccelBvh8, false, false>(const DevScene &, const RenderLaunch &, int, cudaStream_t);
 template int render_occupancy_t<kAccelBvh8, false>();
 }  // namespace hk

@@ -132,3 +132,35 @@ def test_megakernel_deals_every_path_once(scene, size, spp):
     assert tuple(ca[:3]) == tuple(cb[:3])
     terms = 25 * spp + 64
     assert np.allclose(a, b, rtol=terms * 2.0 ** -23, atol=terms * 2.0 ** -24 * float(np.abs(a).max()))
+
+
+def _room(width, height):
+    return scenes.cornell_box(width=width, height=height)
+
+
+def _sky(width, height):
+    return scenes.mesh_heavy("conductor", width=width, height=height, depth=12, level=3, env_res=(32, 16), seed=2)
+
+
+def _textured_sky(width, height):
+    return scenes.lights_scene(width=width, height=height, textured=True, bitmap=True, bump=True, shading_normals=True)
+
+
+# as many paths as are resident (148 x 256 lanes); two more, in rounds of blocks of 128 threads; 131000, near the last of those;
+# 2^17 and more, of 256 threads; several samples over ragged tiles
+@pytest.mark.parametrize("size,spp", [((592, 64), 1), ((421, 90), 1), ((131, 1000), 1), ((512, 256), 1), ((257, 511), 1), ((37, 29), 123)])
+@pytest.mark.parametrize("scene,depth,accel", [(_room, 6, hk.ACCEL_BVH8), (_room, 2, hk.ACCEL_BVH2), (_sky, 12, hk.ACCEL_BVH8),
+                                               (_sky, 12, hk.ACCEL_BVH2), (_textured_sky, 12, hk.ACCEL_BVH8),
+                                               (_textured_sky, 12, hk.ACCEL_BVH2)])
+def test_rounds_deal_every_path_once(size, spp, scene, depth, accel):
+    """Against the wavefront, as test_megakernel_deals_every_path_once."""
+    gs = hk.Scene.from_desc(scene(*size))
+    gs.set_accel(accel)
+    out = []
+    for form in (hk.FORM_MEGAKERNEL, hk.FORM_WAVEFRONT):
+        gs.set_image_form(form)
+        out.append(gs.render_image(spp, depth, seed=5))
+    (a, ca), (b, cb) = out
+    assert tuple(ca[:3]) == tuple(cb[:3])
+    terms = 25 * spp + 64
+    assert np.allclose(a, b, rtol=terms * 2.0 ** -23, atol=terms * 2.0 ** -24 * float(np.abs(a).max()))

@@ -361,3 +361,21 @@ def test_a_film_render_pins_no_host_memory(fake):
     _render(s, 1)
     _pool(s, fake)
     assert fake.L.fake_pinned() == before + 1
+
+
+def _sky(fake, width, height, material="conductor"):
+    s = hk.Scene.from_desc(scenes.mesh_heavy(material, width=width, height=height, depth=8, level=1, env_res=(8, 4)))
+    fake.made.append(s)
+    fake.log()
+    return s
+
+
+# 148 x 256 lanes are resident: blocks of 128 threads, two an SM; of 256 threads, one an SM, where 2^17 paths start in rounds
+def test_the_blocks_of_the_megakernel(fake):
+    for make, depth, grids in ((_scene, 6, (296, 296, 148)), (_scene, 7, (296, 296, 296)), (_sky, 64, (296, 296, 148)),
+                               (lambda *a: _sky(*a, "dielectric"), 7, (296, 296, 296))):
+        for width, height, grid in ((592, 64, grids[0]), (511, 256, grids[1]), (512, 256, grids[2])):
+            s = make(fake, width, height)
+            s.set_image_form(hk.FORM_MEGAKERNEL)
+            _render(s, 1, depth)
+            assert fake.log() == [f"mega grid {grid} lanes 32"]
