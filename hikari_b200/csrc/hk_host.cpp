@@ -1430,17 +1430,31 @@ static hk::WfEngineConfig engine_config(const hk_wavefront_config &c, uint64_t w
     }
     return ec;
 }
-// Whether a render of the scene's own image goes to the wavefront: from 2^17
-// paths on.  Measured on five scenes (Cornell boxes of diffuse and of smooth
-// materials, a glass sphere, 64 spheres, textures; depth 16), megakernel /
-// wavefront: 2^16 paths 0.8-4.8 / 0.8-2.5 ms, 2^18 paths 1.5-13.8 / 1.2-3.1 ms,
-// 2^20 paths 4-46 / 2.5-4.9 ms; below 2^16 the wavefront's five launches a
-// bounce cost more than the megakernel's divergence, between 2^16 and 2^17 a
-// mesh of one conductor still does better in the megakernel (1.1 / 1.7 ms), and a scene's first
+// Paths from which a render of the scene's own image goes to the wavefront.  The
+// wavefront pays a few launches for every vertex of the longest path, whatever the
+// paths, and sorts them by material; the megakernel pays for each path, and for the materials
+// that differ within a warp.  So the line rises with the depth, most where most
+// paths are short, and is low for many materials.  Megakernel / wavefront, us:
+//   many materials (smooth ones in a Cornell box; 64 spheres)
+//     2^15 paths  depth 2 125 / 258, 1174 / 553    16 1500 / 1235, 3489 / 2496    32 1654 / 2116, 3668 / 3176
+//     2^16 paths  depth 2 214 / 270, 1437 / 594    32 2585 / 2184, 4380 / 3578    64 2609 / 2565, 4327 / 3578
+//   short paths (a mesh of a conductor, of plastic; textures)
+//     2^17 paths  depth 8 884 / 1070, 1048 / 1129, 1173 / 949    16 1073 / 1720, 1325 / 1812, 1169 / 1345
+//     2^18 paths  depth 16 1426-1700 / 2000, 1855-2241 / 2040, 1403-1844 / 1540    32 1496 / 2819, 1962 / 2334, 1593 / 2258
+//     2^19 paths  depth 16 2402 / 2227, 2898 / 2234, 3320 / 1850    32 2516 / 3045, 2943 / 2544, 3352 / 2536
+//   else (Cornell box; a mesh of glass)
+//     2^17 paths  depth 2 162 / 236, 537 / 457    8 661 / 559, 1944 / 1403    16 869 / 924, 2484 / 2280    64 1009 / 1638, 2749 / 3990
+//     2^18 paths  depth 16 1388 / 1118, 3458 / 2680    64 1543 / 1881, 4010 / 4836    3 x 2^17 64 2279 / 2165, 6255 / 5556
+// (the wavefront as a batch of one, which waits: 60 us of it).  A scene's first
 // wavefront render spends 2 ms on its pool and graph.
+static uint64_t wavefront_line(const hk_scene *s, int depth) {
+    if (s->short_paths) return depth <= 8 ? 1u << 17 : depth > 16 ? 3u << 17 : s->dev.textured ? 5u << 15 : 1u << 18;
+    if (__builtin_popcountll(s->dev.shade_queues) > 4) return depth < 4 ? 1u << 17 : depth <= 16 ? 1u << 15 : 1u << 16;   // the misses' queue included
+    return depth <= 16 || depth > 1024 ? 1u << 17 : 5u << 16;   // deeper than 1024: not measured
+}
 static bool work_for_wavefront(const hk_scene *s, const hk_render_desc &d) {
     if (s->image_form == HK_FORM_MEGAKERNEL || d.depth < 1 || d.depth > 65535) return false;
-    return (uint64_t)s->width * s->height * (uint64_t)d.spp >= (1ull << 17);
+    return (uint64_t)s->width * s->height * (uint64_t)d.spp >= wavefront_line(s, d.depth);
 }
 // Whether the scene's own image may be a job of the wavefront.
 static bool job_sides_fit(const hk_scene *s) { return s->width <= hk::kJobMaxSide && s->height <= hk::kJobMaxSide; }

@@ -379,3 +379,30 @@ def test_the_blocks_of_the_megakernel(fake):
             s.set_image_form(hk.FORM_MEGAKERNEL)
             _render(s, 1, depth)
             assert fake.log() == [f"mega grid {grid} lanes 32"]
+
+
+def _smooth(fake, width, height):
+    s = hk.Scene.from_desc(scenes.cornell_smooth(width=width, height=height))
+    fake.made.append(s)
+    fake.log()
+    return s
+
+
+def _textures(fake, width, height):
+    s = hk.Scene.from_desc(scenes.lights_scene(width=width, height=height, textured=True))
+    fake.made.append(s)
+    fake.log()
+    return s
+
+
+# paths x 2^-15: the last that the megakernel renders is a row less
+@pytest.mark.parametrize("make,depth,line", [(_smooth, 3, 4), (_smooth, 4, 1), (_smooth, 16, 1), (_smooth, 17, 2), (_sky, 8, 4),
+                                             (_sky, 9, 8), (_sky, 16, 8), (_sky, 17, 12), (_textures, 8, 4), (_textures, 9, 5),
+                                             (_textures, 16, 5), (_textures, 17, 12), (_scene, 16, 4), (_scene, 17, 10),
+                                             (_scene, 1024, 10), (_scene, 1025, 4)])
+def test_the_line_between_the_forms(fake, make, depth, line):
+    for height, form in ((32 * line - 1, "mega"), (32 * line, "begin")):
+        s = make(fake, 1024, height)
+        _render(s, 1, depth)
+        _image(s, 1) if depth == 16 else None
+        assert set(fake.forms()) == {form}
