@@ -1441,7 +1441,8 @@ static hk::WfEngineConfig engine_config(const hk_wavefront_config &c, uint64_t w
 //   short paths (a mesh of a conductor, of plastic; textures)
 //     2^17 paths  depth 8 884 / 1070, 1048 / 1129, 1173 / 949    16 1073 / 1720, 1325 / 1812, 1169 / 1345
 //     2^18 paths  depth 16 1426-1700 / 2000, 1855-2241 / 2040, 1403-1844 / 1540    32 1496 / 2819, 1962 / 2334, 1593 / 2258
-//     2^19 paths  depth 16 2402 / 2227, 2898 / 2234, 3320 / 1850    32 2516 / 3045, 2943 / 2544, 3352 / 2536
+//     3 x 2^17 paths  depth 32 2438 / 3249, 2941 / 2681, 2275 / 2293    2^19 paths 2516 / 3045, 2943 / 2544, 3352 / 2536
+//     210000 paths of 7 samples a pixel, textures  depth 16 2035 / 1334    64 2073 / 3073
 //   else (Cornell box; a mesh of glass)
 //     2^17 paths  depth 2 162 / 236, 537 / 457    8 661 / 559, 1944 / 1403    16 869 / 924, 2484 / 2280    64 1009 / 1638, 2749 / 3990
 //     2^18 paths  depth 16 1388 / 1118, 3458 / 2680    64 1543 / 1881, 4010 / 4836    3 x 2^17 64 2279 / 2165, 6255 / 5556
@@ -1541,7 +1542,9 @@ static bool render_wavefront_async(hk_scene *s, const hk_render_desc &d, float *
 // box 425 / 277 / 273, smooth materials 1945 / 817 / 603, 64 spheres 5972 /
 // 4447 / 4168; depth 6 945 / 1021 / 980, 5406 / 4793 / 4327 and 10190 / 9978 /
 // 9770; depth 8 1082 / 1377 / 1328, 6106 / 6240 / 5760; depth 16 1387 / 2552 /
-// 2486.  Scenes under a sky, depth 16, 2^18 paths: mesh of a conductor 1814 / 1440 / 1410, of
+// 2486.  Up to twice the resident lanes little is refilled: up to depth 8 (70000 paths
+// 449 / 409, 1978 / 1796, a mesh of glass 1228 / 1208; depth 10 513 / 508, 2179 / 2122, 1416 / 1415;
+// 90000 paths depth 8 493 / 541).  Scenes under a sky, depth 16, 2^18 paths: mesh of a conductor 1814 / 1440 / 1410, of
 // plastic 2369 / 1907 / 1857, textures 2639 / 1633 / 1385 (with glass: its code
 // is the largest); not where transmission makes paths longer: mesh of glass 3411 / 4595 / 4671.
 // 256 threads from 2^17 paths on, where they fill the SMs (2^16 paths, textures 857 / 1169 in rounds of 128 / 256).
@@ -1550,7 +1553,7 @@ static int render_grid(const hk_scene *s, const hk_render_desc &d, hk::RenderLau
     const uint64_t warps = (uint64_t)s->sm_count * 4, resident = (uint64_t)s->sm_count * s->occupancy * hk::kRenderThreads;
     P.lanes = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(32, (paths + warps - 1) / warps));
     if (P.lanes > 16) P.lanes = 32;
-    P.rounds = paths > resident && (d.depth <= 6 || s->short_paths);
+    P.rounds = paths > resident && (d.depth <= (paths <= 2 * resident ? 8 : 6) || s->short_paths);
     P.threads = P.rounds && paths >= (1u << 17) ? hk::kRoundThreads : hk::kRenderThreads;
     const uint64_t per_block = P.lanes * (P.threads / 32);
     return (int)std::max<uint64_t>(1, std::min<uint64_t>((paths + per_block - 1) / per_block, std::max<uint64_t>(1, resident / P.threads)));
