@@ -388,7 +388,7 @@ class Scene:
 
     def set_image_form(self, form: int) -> None:
         """The form render and render_image render with: FORM_AUTO (the wavefront
-        from 2^17 paths on), FORM_MEGAKERNEL, or FORM_WAVEFRONT (render_image
+        from 2^15 to 3 x 2^17 paths on, as the scene and the depth ask for), FORM_MEGAKERNEL, or FORM_WAVEFRONT (render_image
         whatever the size)."""
         check(lib().hk_scene_set_image_form(self.h, form))
 

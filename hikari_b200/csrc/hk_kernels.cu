@@ -198,9 +198,12 @@ template <int kAccel, bool kAnyHit>
 static cudaError_t launch_trace_t(const DevScene &S, uint64_t n, const float *rays, int32_t *tri, float *t, float *u, float *v,
                                   unsigned long long *visits, cudaStream_t st) {
     if constexpr (kAccel == kAccelBvh8) {
-        // 32 rays a warp fill the GPU's 4736 resident warps up to 150 thousand
-        // rays; above, up to 128, so that lanes refill while blocks still
-        // follow one another and even out the warps' times
+        // 32 rays a warp up to 150 thousand rays; above, up to 128, so that lanes
+        // refill while blocks still follow one another and even out the warps'
+        // times.  28 warps an SM are resident (72 registers); dividing by 148 x 28
+        // instead takes 109 instead of 124 us for 200 thousand closest-hit rays of
+        // the 64-sphere scene, 89 / 98 for 450 thousand any-hit ones, but 36.8 / 33.7 for 140
+        // thousand closest-hit rays of a Cornell box and 144 / 141 for 200 thousand of a mesh
         const uint64_t per_warp = std::max<uint64_t>(32, std::min<uint64_t>(128, n / (148 * 32)));
         const uint64_t warps = (n + per_warp - 1) / per_warp, per_block = kTraceThreads / 32;
         const size_t smem = trace8_smem(kAnyHit, kTraceThreads);

@@ -13,6 +13,9 @@ constexpr int kRenderThreads = 128;
 // more warps per scheduler only take turns in the instruction cache (us at 2 / 3 / 4
 // blocks: Cornell box 346 / 354 / 384 at 2^14 paths, 892 / 903 / 1067 at 2^17;
 // smooth materials 905 / 922 / 981 and 4025 / 4194 / 4583; a mesh 787 / 812 / 874 at 2^16).
+// Many paths of the smallest scenes would want four (Cornell box 8.9 / 7.1 ms with two / four
+// at 2^21 paths, smooth materials 52.8 / 52.8, 64 spheres 81.7 / 86.4), but so many come here only from
+// captures and hk_render_image_static: the wavefront renders them otherwise.
 constexpr int kRenderBlocks = 2;
 constexpr int kRoundThreads = 256;    // the most threads of a block that deals its paths in rounds
 

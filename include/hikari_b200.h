@@ -254,10 +254,11 @@ typedef struct {
 /* Accumulate spp samples per pixel into film_dev ((H+2B)*(W+2B)*4 floats of
  * RGB*w and w, B = ceil(radius - 0.5)); counters_dev (optional, 5 x u64) gets
  * closest-hit rays, shadow rays, dropped (invalid) samples, BVH node visits
- * and triangle tests added.  Asynchronous on `stream`.  Renders of 2^17 paths
- * and more go to the wavefront integrator, smaller ones, captures of the stream
- * into a graph, calls without memory for the pool, on another device than the
- * scene's, with a depth above 65535 or a stored configuration that has no_graph
+ * and triangle tests added.  Asynchronous on `stream`.  Renders of many paths
+ * go to the wavefront integrator: from 2^15 (many materials) to 3 x 2^17 paths on (deep renders of open scenes);
+ * smaller ones, captures of the stream into a graph, calls without memory for
+ * the pool, on another device than the scene's, of more than 16384 pixels a
+ * side, with a depth above 65535 or a stored configuration that has no_graph
  * or that a pool refuses to the megakernel; HK_FORM_MEGAKERNEL keeps all of them
  * there.  The wavefront's pool (2^14 to 2^21 slots as the work
  * asks for, 128 B and 48 B per emitter each and 4 B for each of its queues: 0.9
