@@ -1445,13 +1445,14 @@ static hk::WfEngineConfig engine_config(const hk_wavefront_config &c, uint64_t w
 //     210000 paths of 7 samples a pixel, textures  depth 16 2035 / 1334    64 2073 / 3073
 //   else (Cornell box; a mesh of glass)
 //     2^17 paths  depth 2 162 / 236, 537 / 457    8 661 / 559, 1944 / 1403    16 869 / 924, 2484 / 2280    64 1009 / 1638, 2749 / 3990
-//     2^18 paths  depth 16 1388 / 1118, 3458 / 2680    64 1543 / 1881, 4010 / 4836    3 x 2^17 64 2279 / 2165, 6255 / 5556
+//     2^18 paths  depth 2 274 / 321, 870 / 573    16 1388 / 1118, 3458 / 2680    64 1543 / 1881, 4010 / 4836    3 x 2^17 64 2279 / 2165, 6255 / 5556
 // (the wavefront as a batch of one, which waits: 60 us of it).  A scene's first
 // wavefront render spends 2 ms on its pool and graph.
 static uint64_t wavefront_line(const hk_scene *s, int depth) {
     if (s->short_paths) return depth <= 8 ? 1u << 17 : depth > 16 ? 3u << 17 : s->dev.textured ? 5u << 15 : 1u << 18;
     if (__builtin_popcountll(s->dev.shade_queues) > 4) return depth < 4 ? 1u << 17 : depth <= 16 ? 1u << 15 : 1u << 16;   // the misses' queue included
-    return depth <= 16 || depth > 1024 ? 1u << 17 : 5u << 16;   // deeper than 1024: not measured
+    if (depth < 4 && s->info.n_triangles < 4096) return 1u << 18;   // rays that cost next to nothing
+    return depth <= 16 || depth > 1024 ? 1u << 17 : 5u << 16;       // deeper than 1024: not measured
 }
 static bool work_for_wavefront(const hk_scene *s, const hk_render_desc &d) {
     if (s->image_form == HK_FORM_MEGAKERNEL || d.depth < 1 || d.depth > 65535) return false;

@@ -398,7 +398,7 @@ def _textures(fake, width, height):
 # paths x 2^-15: the last that the megakernel renders is a row less
 @pytest.mark.parametrize("make,depth,line", [(_smooth, 3, 4), (_smooth, 4, 1), (_smooth, 16, 1), (_smooth, 17, 2), (_sky, 8, 4),
                                              (_sky, 9, 8), (_sky, 16, 8), (_sky, 17, 12), (_textures, 8, 4), (_textures, 9, 5),
-                                             (_textures, 16, 5), (_textures, 17, 12), (_scene, 16, 4), (_scene, 17, 10),
+                                             (_textures, 16, 5), (_textures, 17, 12), (_scene, 3, 8), (_scene, 4, 4), (_scene, 16, 4), (_scene, 17, 10),
                                              (_scene, 1024, 10), (_scene, 1025, 4)])
 def test_the_line_between_the_forms(fake, make, depth, line):
     for height, form in ((32 * line - 1, "mega"), (32 * line, "begin")):
